@@ -142,93 +142,12 @@ struct Sizes {
 };
 
 
-// ---------------------------------------------------------------------------------------------
-// Launchers of the register-DFT kernels for the sizes they are instantiated for. Each returns
-// false for other sizes; the caller then uses the general shared-memory Stockham kernels.
-// ---------------------------------------------------------------------------------------------
-// Sets a kernel's dynamic shared-memory limit once per device (the attribute is per device context).
-template <typename K>
-void allow_smem(K kernel, std::size_t bytes, unsigned long long& done_mask, const char* what) {
-  int dev = 0;
-  check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
-  if (dev < 64 && (done_mask >> dev & 1ull)) return;
-  check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)), what);
-  if (dev < 64) done_mask |= 1ull << dev;
-}
-
 // The device's largest dynamic shared memory per block (opt-in).
 inline std::size_t smem_optin_bytes() {
   int dev = 0, optin = 0;
   check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
   check_cuda(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "smem attribute");
   return static_cast<std::size_t>(optin);
-}
-
-// Blocks of a persistent kernel: the SMs times the blocks that fit on one (looked up once per kernel).
-template <typename K>
-long long persistent_blocks(K kernel, int threads, std::size_t smem, int& cached) {
-  if (cached <= 0) {
-    int dev = 0, sms = 0, per_sm = 0;
-    check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
-    check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
-    check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem), "occupancy");
-    cached = std::max(1, sms * per_sm);
-  }
-  return cached;
-}
-
-template <typename T, int N1, int N2, int TB>
-bool launch_axis2_tb(const spo::Axis2Args<T>& a, long long outer, cudaStream_t stream) {
-  constexpr int NS = N1 > N2 ? N1 : N2;
-  constexpr int N = N1 * N2;
-  // the tile, then the factors (mixed form: their parts, spo::fmul_t) and the twiddles (mixed form: and their low parts)
-  const std::size_t smem =
-      sizeof(spo::Vec<T>) * (static_cast<std::size_t>(N) * TB + (sizeof(T) == 4 ? spo::kFactorParts + 2 : 2) * N);
-  static unsigned long long configured = 0;
-  allow_smem(spo::axis2_kernel<T, N1, N2, TB>, smem, configured, "axis2 smem");
-  if (a.persistent && a.window == 0) {
-    static unsigned long long configured_p = 0;
-    static int blocks_p = 0;
-    allow_smem(spo::axis2p_kernel<T, N1, N2, TB>, smem, configured_p, "axis2p smem");
-    const long long lane_blocks = (a.inner + TB - 1) / TB;
-    const long long n_tiles = outer * lane_blocks;
-    const long long grid = std::min(n_tiles, persistent_blocks(spo::axis2p_kernel<T, N1, N2, TB>, TB * NS, smem, blocks_p));
-    spo::axis2p_kernel<T, N1, N2, TB><<<static_cast<unsigned>(grid), TB * NS, smem, stream>>>(a, lane_blocks, n_tiles);
-    return true;
-  }
-  if constexpr (N2 == 2 * N1) {
-    if (a.balanced && a.window == 0) {
-      static unsigned long long configured_b = 0;
-      allow_smem(spo::axis2b_kernel<T, N1, N2, TB>, smem, configured_b, "axis2b smem");
-      const dim3 grid(static_cast<unsigned>((a.inner + TB - 1) / TB), static_cast<unsigned>(outer));
-      spo::axis2b_kernel<T, N1, N2, TB><<<grid, TB * N1, smem, stream>>>(a);
-      return true;
-    }
-  }
-  if (a.window > 0) {  // lane windows: groups x ceil(window / TB) blocks
-    spo::Axis2Args<T> w = a;
-    w.blocks_per_group = static_cast<int>((a.window + TB - 1) / TB);
-    const dim3 grid(static_cast<unsigned>(a.groups * w.blocks_per_group), static_cast<unsigned>(outer));
-    spo::axis2_kernel<T, N1, N2, TB><<<grid, TB * NS, smem, stream>>>(w);
-    return true;
-  }
-  const dim3 grid(static_cast<unsigned>((a.inner + TB - 1) / TB), static_cast<unsigned>(outer));
-  spo::axis2_kernel<T, N1, N2, TB><<<grid, TB * NS, smem, stream>>>(a);
-  return true;
-}
-
-// Tile width (batch lanes per block): 32 lanes when a line has at most 8 sub-rows; for more sub-rows
-// 16 lanes by default, or 8 or 32 lanes as the autotuner chose.
-template <typename T, int N1, int N2>
-bool launch_axis2_n(const spo::Axis2Args<T>& a, long long outer, cudaStream_t stream) {
-  constexpr int NS = N1 > N2 ? N1 : N2;
-  if constexpr (NS <= 8) {
-    return launch_axis2_tb<T, N1, N2, 32>(a, outer, stream);
-  } else {
-    if (a.tile == 8) return launch_axis2_tb<T, N1, N2, 8>(a, outer, stream);
-    if (a.tile == 32) return launch_axis2_tb<T, N1, N2, 32>(a, outer, stream);
-    return launch_axis2_tb<T, N1, N2, 16>(a, outer, stream);
-  }
 }
 
 // The prime-factor splits N = N1 x N2 (N1, N2 coprime) with an axis2pfa_kernel instantiation; LT threads per
@@ -254,59 +173,6 @@ std::vector<C> pfa_order(const std::vector<C>& f, int n1, int n2) {
     for (int k2 = 0; k2 < n2; ++k2) out[k1 + n1 * k2] = f[(static_cast<long long>(n2) * u * k1 + static_cast<long long>(n1) * v * k2) % n];
   return out;
 }
-template <typename T, int N1, int N2, int LT>
-bool launch_axis2_pfa_n(const spo::Axis2Args<T>& a, long long outer, cudaStream_t stream) {
-  constexpr int TB = 32, N = N1 * N2;
-  const std::size_t smem = sizeof(spo::Vec<T>) * (static_cast<std::size_t>(N) * TB + (sizeof(T) == 4 ? spo::kFactorParts : 1) * N);
-  static unsigned long long configured = 0;
-  allow_smem(spo::axis2pfa_kernel<T, N1, N2, TB, LT>, smem, configured, "axis2pfa smem");
-  spo::Axis2Args<T> w = a;
-  unsigned blocks_x;
-  if (a.window > 0) {
-    w.blocks_per_group = static_cast<int>((a.window + TB - 1) / TB);
-    blocks_x = static_cast<unsigned>(a.groups * w.blocks_per_group);
-  } else {
-    blocks_x = static_cast<unsigned>((a.inner + TB - 1) / TB);
-  }
-  spo::axis2pfa_kernel<T, N1, N2, TB, LT><<<dim3(blocks_x, static_cast<unsigned>(outer)), TB * LT, smem, stream>>>(w);
-  return true;
-}
-template <typename T>
-bool launch_axis2_pfa(int n, const spo::Axis2Args<T>& a, long long outer, cudaStream_t stream) {
-  switch (n) {
-    case 24: return launch_axis2_pfa_n<T, 3, 8, 4>(a, outer, stream);
-    case 40: return launch_axis2_pfa_n<T, 5, 8, 8>(a, outer, stream);
-    case 48: return launch_axis2_pfa_n<T, 3, 16, 4>(a, outer, stream);
-    case 56: return launch_axis2_pfa_n<T, 7, 8, 8>(a, outer, stream);
-    case 80: return launch_axis2_pfa_n<T, 5, 16, 8>(a, outer, stream);
-    case 112: return launch_axis2_pfa_n<T, 7, 16, 8>(a, outer, stream);
-    default: return false;
-  }
-}
-
-template <typename T>
-bool launch_axis2(int n, const spo::Axis2Args<T>& a, long long outer, cudaStream_t stream) {
-  if (a.factor_pfa && !a.persistent) return launch_axis2_pfa<T>(n, a, outer, stream);
-  switch (n) {
-    // N = N1 N2 with N2 >= N1: the first level, which streams the tile in from HBM, uses every thread.
-    case 24: return launch_axis2_n<T, 4, 6>(a, outer, stream);
-    case 32: return launch_axis2_n<T, 4, 8>(a, outer, stream);
-    case 40: return launch_axis2_n<T, 5, 8>(a, outer, stream);
-    case 48: return launch_axis2_n<T, 6, 8>(a, outer, stream);
-    case 56: return launch_axis2_n<T, 7, 8>(a, outer, stream);
-    case 64: return launch_axis2_n<T, 8, 8>(a, outer, stream);
-    case 80: return launch_axis2_n<T, 8, 10>(a, outer, stream);
-    case 96: return launch_axis2_n<T, 8, 12>(a, outer, stream);
-    case 112: return launch_axis2_n<T, 7, 16>(a, outer, stream);
-    case 128: return launch_axis2_n<T, 8, 16>(a, outer, stream);
-    case 160: return launch_axis2_n<T, 10, 16>(a, outer, stream);
-    case 176: return launch_axis2_n<T, 11, 16>(a, outer, stream);
-    case 192: return launch_axis2_n<T, 12, 16>(a, outer, stream);
-    case 224: return launch_axis2_n<T, 14, 16>(a, outer, stream);
-    case 256: return launch_axis2_n<T, 16, 16>(a, outer, stream);
-    default: return false;
-  }
-}
 // Lengths whose register kernel has more than 8 sub-rows, i.e. a choice of tile widths.
 inline bool axis2_has_tiles(int n) {
   switch (n) {
@@ -326,53 +192,6 @@ inline bool axis2_supported(int n) {
 
 inline bool xy2_supported(int n) { return n == 2 || n == 4 || n == 6 || n == 8 || n == 12 || n == 16; }
 
-template <typename T, int NX, int NY, int TB>
-void launch_xy2_tb(const spo::XyArgs<T>& a, long long n_zr, cudaStream_t stream) {
-  constexpr int NS = NX > NY ? NX : NY;
-  const std::size_t smem =
-      sizeof(spo::Vec<T>) * (static_cast<std::size_t>(NX * NY) * TB + (sizeof(T) == 4 ? spo::kFactorParts : 1) * NX * NY);
-  if (a.persistent) {
-    static unsigned long long configured_p = 0;
-    static int blocks_p = 0;
-    allow_smem(spo::xy2p_kernel<T, NX, NY, TB>, smem, configured_p, "xy2p smem");
-    const long long rot_tiles = (a.n_rot + TB - 1) / TB;
-    const long long n_tiles = n_zr * rot_tiles;
-    const long long grid = std::min(n_tiles, persistent_blocks(spo::xy2p_kernel<T, NX, NY, TB>, TB * NS, smem, blocks_p));
-    spo::xy2p_kernel<T, NX, NY, TB><<<static_cast<unsigned>(grid), TB * NS, smem, stream>>>(a, rot_tiles, n_tiles);
-    return;
-  }
-  static unsigned long long configured = 0;
-  allow_smem(spo::xy2_kernel<T, NX, NY, TB>, smem, configured, "xy2 smem");
-  const dim3 grid(static_cast<unsigned>((a.n_rot + TB - 1) / TB), static_cast<unsigned>(n_zr));
-  spo::xy2_kernel<T, NX, NY, TB><<<grid, TB * NS, smem, stream>>>(a);
-}
-
-template <typename T, int NX, int NY>
-void launch_xy2_n(const spo::XyArgs<T>& a, long long n_zr, cudaStream_t stream) {
-  constexpr int NS = NX > NY ? NX : NY;
-  if constexpr (NS <= 8) {
-    launch_xy2_tb<T, NX, NY, 32>(a, n_zr, stream);
-  } else {
-    if (a.tile == 8) launch_xy2_tb<T, NX, NY, 8>(a, n_zr, stream);
-    else if (a.tile == 32) launch_xy2_tb<T, NX, NY, 32>(a, n_zr, stream);
-    else launch_xy2_tb<T, NX, NY, 16>(a, n_zr, stream);
-  }
-}
-
-template <typename T>
-bool launch_xy2(const spo::XyArgs<T>& a, long long n_zr, cudaStream_t stream) {
-  if (a.nx != a.ny) return false;
-  switch (a.nx) {
-    case 2: launch_xy2_n<T, 2, 2>(a, n_zr, stream); return true;
-    case 4: launch_xy2_n<T, 4, 4>(a, n_zr, stream); return true;
-    case 6: launch_xy2_n<T, 6, 6>(a, n_zr, stream); return true;
-    case 8: launch_xy2_n<T, 8, 8>(a, n_zr, stream); return true;
-    case 12: launch_xy2_n<T, 12, 12>(a, n_zr, stream); return true;
-    case 16: launch_xy2_n<T, 16, 16>(a, n_zr, stream); return true;
-    default: return false;
-  }
-}
-
 // Shared memory of potential2_kernel<T, NPHI, CB>.
 template <typename T>
 std::size_t pot2_smem(int cb, int n_rot, int nt, int nphi, long long n_xy) {
@@ -381,40 +200,6 @@ std::size_t pot2_smem(int cb, int n_rot, int nt, int nphi, long long n_xy) {
          (sizeof(T) == 4 ? 2 : 1) * sizeof(T) * static_cast<std::size_t>(nt) * n_rot;  // matrix (+ low parts)
 }
 
-template <typename T, int NPHI, int CB>
-void launch_pot2_n(const spo::Pot2Args<T>& a, unsigned blocks, std::size_t smem, cudaStream_t stream) {
-  // The shared memory depends on the case's sizes, not only on the instantiation: allow the device's
-  // maximum, so that every case with this instantiation can launch.
-  static unsigned long long configured = 0;
-  allow_smem(spo::potential2_kernel<T, NPHI, CB>, smem_optin_bytes(), configured, "potential2 smem");
-  spo::potential2_kernel<T, NPHI, CB><<<blocks, 128, smem, stream>>>(a);
-}
-
-template <typename T, int NPHI>
-void launch_pot2_phi(const spo::Pot2Args<T>& a, unsigned blocks, std::size_t smem, cudaStream_t stream) {
-  switch (a.cb) {
-    case 32: launch_pot2_n<T, NPHI, 32>(a, blocks, smem, stream); break;
-    case 8: launch_pot2_n<T, NPHI, 8>(a, blocks, smem, stream); break;
-    default: launch_pot2_n<T, NPHI, 4>(a, blocks, smem, stream); break;
-  }
-}
-
-template <typename T>
-void launch_pot2(int nphi, const spo::Pot2Args<T>& a, unsigned blocks, std::size_t smem, cudaStream_t stream) {
-  switch (nphi) {
-    case 6: launch_pot2_phi<T, 6>(a, blocks, smem, stream); break;
-    case 8: launch_pot2_phi<T, 8>(a, blocks, smem, stream); break;
-    case 10: launch_pot2_phi<T, 10>(a, blocks, smem, stream); break;
-    case 12: launch_pot2_phi<T, 12>(a, blocks, smem, stream); break;
-    case 16: launch_pot2_phi<T, 16>(a, blocks, smem, stream); break;
-    case 20: launch_pot2_phi<T, 20>(a, blocks, smem, stream); break;
-    case 24: launch_pot2_phi<T, 24>(a, blocks, smem, stream); break;
-    case 28: launch_pot2_phi<T, 28>(a, blocks, smem, stream); break;
-    case 30: launch_pot2_phi<T, 30>(a, blocks, smem, stream); break;
-    case 32: launch_pot2_phi<T, 32>(a, blocks, smem, stream); break;
-    default: break;
-  }
-}
 // Shared memory of potential3_kernel<T, NPHI, CB>: F (slot-major, jp values per slot) and D share it.
 template <typename T>
 std::size_t pot3_smem(int cb, int jp, int nt, int nphi) {
@@ -422,74 +207,24 @@ std::size_t pot3_smem(int cb, int jp, int nt, int nphi) {
                                         static_cast<std::size_t>(cb) * nt * (nphi + 1));
 }
 
-template <typename T, int NPHI, int CB>
-void launch_pot3_n(const spo::Pot2Args<T>& a, dim3 grid, unsigned threads, std::size_t smem, cudaStream_t stream) {
-  static unsigned long long configured = 0;
-  allow_smem(spo::potential3_kernel<T, NPHI, CB>, smem_optin_bytes(), configured, "potential3 smem");
-  spo::potential3_kernel<T, NPHI, CB><<<grid, threads, smem, stream>>>(a);
-}
-
-template <typename T, int NPHI>
-void launch_pot3_phi(const spo::Pot2Args<T>& a, dim3 grid, unsigned threads, std::size_t smem, cudaStream_t stream) {
-  if (a.cb == 16) launch_pot3_n<T, NPHI, 16>(a, grid, threads, smem, stream);
-  else launch_pot3_n<T, NPHI, 8>(a, grid, threads, smem, stream);
-}
-
-template <typename T>
-void launch_pot3(int nphi, const spo::Pot2Args<T>& a, dim3 grid, unsigned threads, std::size_t smem,
-                 cudaStream_t stream) {
-  switch (nphi) {
-    case 6: launch_pot3_phi<T, 6>(a, grid, threads, smem, stream); break;
-    case 8: launch_pot3_phi<T, 8>(a, grid, threads, smem, stream); break;
-    case 10: launch_pot3_phi<T, 10>(a, grid, threads, smem, stream); break;
-    case 12: launch_pot3_phi<T, 12>(a, grid, threads, smem, stream); break;
-    case 16: launch_pot3_phi<T, 16>(a, grid, threads, smem, stream); break;
-    case 20: launch_pot3_phi<T, 20>(a, grid, threads, smem, stream); break;
-    case 24: launch_pot3_phi<T, 24>(a, grid, threads, smem, stream); break;
-    case 28: launch_pot3_phi<T, 28>(a, grid, threads, smem, stream); break;
-    case 30: launch_pot3_phi<T, 30>(a, grid, threads, smem, stream); break;
-    case 32: launch_pot3_phi<T, 32>(a, grid, threads, smem, stream); break;
-    default: break;
-  }
-}
-
 // The potential4 instantiation for (nphi, ntheta), or null: ntheta 16, 8 and 4 with 8, 16 and 32 columns
 // per chunk, nphi 8, 16 and 32 (and 12 with ntheta 4, a phi grid of the C6v symmetry).
 template <typename T>
 using Pot4Kernel = void (*)(spo::Pot4Args<T>);
-template <typename T>
-Pot4Kernel<T> pot4_kernel_for(int nphi, int nt) {
-  if (nt == 16 && nphi == 32) return spo::potential4_kernel<T, 32, 16, 8>;
-  if (nt == 16 && nphi == 16) return spo::potential4_kernel<T, 16, 16, 8>;
-  if (nt == 8 && nphi == 16) return spo::potential4_kernel<T, 16, 8, 16>;
-  if (nt == 8 && nphi == 32) return spo::potential4_kernel<T, 32, 8, 16>;
-  if (nt == 4 && nphi == 8) return spo::potential4_kernel<T, 8, 4, 32>;
-  if (nt == 4 && nphi == 12) return spo::potential4_kernel<T, 12, 4, 32>;  // C6v grids
-  return nullptr;
-}
 
-// The potential5 instantiation (mixed form only) for (nphi, ntheta), or null.
+// The launchers (defined in spo_launch.cuh, instantiated by spo_launch.cu in one translation unit per family). Those
+// of the register-DFT kernels return false, or launch nothing, for sizes without an instantiation; the caller then
+// uses the general shared-memory Stockham kernels.
 template <typename T>
-using Pot5Kernel = void (*)(spo::Pot4Args<T>, int*);
+bool launch_axis2(int n, const spo::Axis2Args<T>& a, long long outer, cudaStream_t stream);
 template <typename T>
-Pot5Kernel<T> pot5_kernel_for(int nphi, int nt, bool l2e) {
-  if constexpr (sizeof(T) != 4) {
-    return nullptr;
-  } else {
-    if (l2e) {
-      if (nt == 16 && nphi == 32) return spo::potential5_kernel<T, 32, 16, 8, true>;
-      if (nt == 16 && nphi == 28) return spo::potential5_kernel<T, 28, 16, 8, true>;
-      if (nt == 16 && nphi == 24) return spo::potential5_kernel<T, 24, 16, 8, true>;
-    }
-    if (nt == 16 && nphi == 32) return spo::potential5_kernel<T, 32, 16, 8>;
-    if (nt == 16 && nphi == 28) return spo::potential5_kernel<T, 28, 16, 8>;  // JMax 13 (theta 14, padded)
-    if (nt == 16 && nphi == 24) return spo::potential5_kernel<T, 24, 16, 8>;  // JMax 11 (theta 12, padded)
-    if (nt == 8 && nphi == 16) return spo::potential5_kernel<T, 16, 8, 16>;
-    if (nt == 4 && nphi == 8) return spo::potential5_kernel<T, 8, 4, 32>;
-    if (nt == 4 && nphi == 12) return spo::potential5_kernel<T, 12, 4, 32>;
-    return nullptr;
-  }
-}
+bool launch_xy2(const spo::XyArgs<T>& a, long long n_zr, cudaStream_t stream);
+template <typename T>
+void launch_pot2(int nphi, const spo::Pot2Args<T>& a, unsigned blocks, std::size_t smem, cudaStream_t stream);
+template <typename T>
+void launch_pot3(int nphi, const spo::Pot2Args<T>& a, dim3 grid, unsigned threads, std::size_t smem, cudaStream_t stream);
+template <typename T>
+Pot4Kernel<T> pot4_kernel_for(int nphi, int nt);
 
 inline bool pot2_phi_supported(int nphi) {
   switch (nphi) {
@@ -699,8 +434,8 @@ class Step final : public StepBase {
   // and every item's first barrier phase expects extra_bytes more than its copies deliver.
   void set_wait_test(int poll_limit, unsigned extra_bytes) override {
     const int limit = poll_limit > 0 ? poll_limit : spo::pot5::kWaitLimit;
-    pot4_args_.poll_limit = pot6_args_.poll_limit = limit;
-    pot4_args_.extra_tx = pot6_args_.extra_tx = extra_bytes;
+    pot5_args_.poll_limit = pot6_args_.poll_limit = limit;
+    pot5_args_.extra_tx = pot6_args_.extra_tx = extra_bytes;
   }
 
   // A kernel whose bounded wait gave up has set the device flag: report it (and clear it).
@@ -746,9 +481,9 @@ class Step final : public StepBase {
       out += " potential=potential6<nphi=" + std::to_string(s_.nphi) + ",nt=" + std::to_string(s_.nt) +
              ",tcgen05.tf32x3,tile=64,blocks=" + std::to_string(pot6_blocks_) + ">";
     } else if (pot_kind_ == 5) {
-      const int nt_k = (s_.nt == 12 || s_.nt == 14) ? 16 : s_.nt;  // 12 and 14 run on the 16-row tile
-      out += " potential=potential5<nphi=" + std::to_string(s_.nphi) + ",nt=" + std::to_string(nt_k) +
-             ",cb=" + std::to_string(128 / nt_k) + ",blocks=" + std::to_string(pot5_blocks_) + (pot5_l2e_ ? ",l2e" : "") + ">";
+      const int nt_k = 8 * pot5_h_;  // theta in tiles of 8
+      out += " potential=potential5<nphi=" + std::to_string(s_.nphi) + ",nt=" + std::to_string(nt_k) + ",dmma,warps=" +
+             std::to_string(pot5_threads_ / 32) + ",blocks=" + std::to_string(pot5_blocks_) + ">";
       if (nt_k != s_.nt) out += "(theta " + std::to_string(s_.nt) + " padded)";
     }
     else if (pot_kind_ == 4)
@@ -924,7 +659,8 @@ class Step final : public StepBase {
       case SPO_STAGE_ZR: kinetic_zr(half); break;
       case SPO_STAGE_XY: kinetic_xy(half, false); break;
       case SPO_STAGE_POTENTIAL:
-        gas_phase();
+        scale_points("gas_phase", static_cast<long long>(s_.nzp) * s_.nr, s_.n_zr(), gas_step_);
+        if (pot_kind_ == 5) scale_points("scaling", 0, static_cast<long long>(s_.nzp) * s_.nr, before_);
         interaction();
         break;
       default: require(false, "unknown stage");
@@ -1163,6 +899,7 @@ class Step final : public StepBase {
     x.nr = s_.nr;
     x.opt_z = opt_z_;
     x.gas_step = gas_step_;
+    x.before = pot_kind_ == 5 ? before_ : nullptr;
     x.tile = tile_xy_;
     x.persistent = persist_xy_ ? 1 : 0;
     if (n_izr >= 0) {
@@ -1180,13 +917,12 @@ class Step final : public StepBase {
     ++launches_;
   }
 
-  void gas_phase() {
-    const long long first = static_cast<long long>(s_.nzp) * s_.nr;
-    if (first >= s_.n_zr()) return;
+  void scale_points(const char* name, long long first, long long last, const V* table) {
+    if (first >= last) return;
     prof_.begin(stream_);
-    spo::gas_phase_kernel<T><<<1184, 256, 0, stream_>>>(psi_, first, s_.n_zr(), s_.n_rot, static_cast<int>(s_.n_xy()),
-                                                        s_.nr, opt_z_, gas_step_);
-    prof_.end(stream_, "gas_phase", 2.0 * sizeof(V) * (s_.n_zr() - first) * s_.n_xy() * s_.n_rot);
+    spo::scale_points_kernel<T><<<1184, 256, 0, stream_>>>(psi_, first, last, s_.n_rot, static_cast<int>(s_.n_xy()), s_.nr,
+                                                           opt_z_, table);
+    prof_.end(stream_, name, 2.0 * sizeof(V) * (last - first) * s_.n_xy() * s_.n_rot);
     ++launches_;
   }
 
@@ -1202,7 +938,7 @@ class Step final : public StepBase {
       if (pot_kind_ == 6) {
         pot6_kernel_<<<pot6_blocks_, spo::kPot6Threads, pot6_smem_, stream_>>>(pot6_args_, error_flag_);
       } else if (pot_kind_ == 5) {
-        pot5_kernel_<<<pot5_blocks_, 128, pot5_smem_, stream_>>>(pot4_args_, error_flag_);
+        pot5_kernel_<<<pot5_blocks_, pot5_threads_, pot5_smem_, stream_>>>(pot5_args_, error_flag_);
       } else if (pot_kind_ == 4) {
         pot4_kernel_<<<pot4_blocks_, 128, pot4_smem_, stream_>>>(pot4_args_);
       } else {
@@ -1550,6 +1286,7 @@ class Step final : public StepBase {
     host_opt_z_ = opt_z;
     host_opt_r_ = opt_r;
     host_opt_zs_ = opt_zs;
+    host_rot_ = rot;
     const std::vector<cplx> gas = complex_array(d.gas_phase, s.nr, "gas_phase");
     std::vector<cplx> before(rot.size()), gas_step(rot.size());
     for (int ir = 0; ir < s.nr; ++ir)
@@ -1641,6 +1378,12 @@ class Step final : public StepBase {
       }
     }
 
+    identity_maps_ = s.n_rep == nxy;
+    for (long long ixy = 0; ixy < nxy && identity_maps_; ++ixy) {
+      identity_maps_ = rep[ixy] == ixy;
+      for (int p = 0; p < s.nphi && identity_maps_; ++p) identity_maps_ = phi_map[ixy * s.nphi + p] == p;
+    }
+
     // State.
     psi_ = dev<V>(s.n_psi());
     check_cuda(cudaMemsetAsync(psi_, 0, sizeof(V) * s.n_psi(), stream_), "zero psi");
@@ -1650,25 +1393,6 @@ class Step final : public StepBase {
     staging_ = dev<double2>(staging_elems_);
     require(d.chi_initial != nullptr, "chi_initial is null");
     upload(nullptr, d.chi_initial);
-
-    // exp(i A) on the device in FP64, chunk by chunk through the staging buffer.
-    const long long n_e = s.n_expia();
-    require(d.potential != nullptr || n_e == 0, "potential is null");
-    // The mixed form keeps, after the n_e table entries, their n_e modulus corrections (FP16, spo::exp_mul).
-    // (from a 16-byte boundary: the kernels read 8 corrections per load and prefetch rows of them into L2)
-    const long long n_e_even = (n_e + 1) & ~1ll;
-    expia_ = dev<V>(std::max<long long>(n_e_even + (sizeof(T) == 4 ? (n_e + 3) / 4 : 0), 1));
-    __half* exp_mod = sizeof(T) == 4 ? reinterpret_cast<__half*>(expia_ + n_e_even) : nullptr;
-    double* vstage = reinterpret_cast<double*>(staging_);
-    const long long chunk = 2 * staging_elems_;
-    for (long long i = 0; i < n_e; i += chunk) {
-      const long long m = std::min(chunk, n_e - i);
-      check_cuda(cudaMemcpyAsync(vstage, d.potential + i, sizeof(double) * m, cudaMemcpyHostToDevice, stream_),
-                 "upload potential");
-      spo::exp_potential_kernel<T><<<1184, 256, 0, stream_>>>(vstage, expia_ + i, exp_mod ? exp_mod + i : nullptr, m, s.dt);
-      check_cuda(cudaGetLastError(), "exp_potential launch");
-      check_cuda(cudaStreamSynchronize(stream_), "exp_potential");
-    }
 
     // Launch shapes and shared memory.
     int smem_optin = 0, dev_id = 0;
@@ -1722,8 +1446,6 @@ class Step final : public StepBase {
     pot_.rot_half = rot_half_;
     pot_.sp2sc = sp2sc;
     pot_.sc2sp = sc2sp;
-    pot_.expia = expia_;
-    pot_.exp_mod = exp_mod;
     pot_.rep_of = upload_int(rep);
     pot_.phi_map = upload_int(phi_map);
 
@@ -1752,12 +1474,7 @@ class Step final : public StepBase {
       pot2_.p = pot_;
       pot2_.legendre_t = upload_real_lo(leg_t, leg_t64);
       pot2_.cb = pot2_cb_;
-      bool identity = s.n_rep == nxy;
-      for (long long ixy = 0; ixy < nxy && identity; ++ixy) {
-        identity = rep[ixy] == ixy;
-        for (int p = 0; p < s.nphi && identity; ++p) identity = phi_map[ixy * s.nphi + p] == p;
-      }
-      pot2_.identity_maps = identity ? 1 : 0;
+      pot2_.identity_maps = identity_maps_ ? 1 : 0;
     }
     // The chunked potential kernel: one block per (point, chunk of pot3_cb_ columns), one thread per
     // (column, theta) line, F and D in at most the device's opt-in shared memory.
@@ -1793,16 +1510,10 @@ class Step final : public StepBase {
         pot3_args_.jp = jp;
       }
     }
-    // The persistent potential kernels with register-tiled contractions: potential4 (ntheta 4, 8, 16;
-    // nphi 8, 16, 32) and potential5 (mixed form; ntheta 12 and 14 run on its 16-row tile, the matrix
-    // rows of the missing theta zero and their phi lines skipped).
-    const bool pot45_ok = pot2_cb_ > 0 && 2 * s.mj_max + 1 <= s.nphi;
-    const int nt_k = (s.nt == 12 || s.nt == 14) ? 16 : s.nt;
-    pot4_kernel_ = pot45_ok ? pot4_kernel_for<T>(s.nphi, s.nt) : nullptr;
-    pot5_l2e_ = nt_k == 16 && !(std::getenv("SPO_B200_POT5_L2E") && std::string(std::getenv("SPO_B200_POT5_L2E")) == "0");
-    Pot5Kernel<T> pot5_candidate = pot45_ok && s.n_rot % 2 == 0 ? pot5_kernel_for<T>(s.nphi, nt_k, pot5_l2e_) : nullptr;
-    pot5_kernel_ = nullptr;
-    if (pot4_kernel_ || pot5_candidate) {
+    // The persistent potential kernel with register-tiled contractions, potential4 (ntheta 4, 8, 16; nphi 8, 16, 32).
+    const int nt_k = s.nt;
+    pot4_kernel_ = pot2_cb_ > 0 ? pot4_kernel_for<T>(s.nphi, s.nt) : nullptr;
+    if (pot4_kernel_) {
       const int cb = 128 / nt_k;
       // Forward schedule: the slots in (+m, -m) pairs (m = 0 with an empty slot), pairs dealt to the four
       // warps largest first, each to the least loaded warp; half-warp 2w takes the first of each pair
@@ -1871,9 +1582,6 @@ class Step final : public StepBase {
       pot4_args_.chunks = static_cast<int>((nxy + cb - 1) / cb);
       pot4_args_.n_items = static_cast<long long>(s.nzp) * s.nr * pot4_args_.chunks;
       pot4_args_.identity_maps = pot2_.identity_maps;
-      pot4_args_.nt_table = s.nt;
-      pot4_args_.poll_limit = spo::pot5::kWaitLimit;
-      pot4_args_.extra_tx = 0;
       int sms = 0;
       check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev_id), "SM count");
       const long long items = std::max<long long>(pot4_args_.n_items, 1);
@@ -1888,25 +1596,10 @@ class Step final : public StepBase {
       } else {
         pot4_kernel_ = nullptr;
       }
-      // potential5: the same tables, the item data by bulk asynchronous copies (columns of n_rot values:
-      // 16-byte multiples when n_rot is even)
-      pot5_smem_ = spo::pot5_smem<T>(s.n_rot, s.nphi, nt_k, cb, len, pot5_l2e_);
-      if (pot5_candidate && pot5_smem_ <= static_cast<std::size_t>(smem_optin)) {
-        pot5_kernel_ = pot5_candidate;
-        check_cuda(cudaFuncSetAttribute(pot5_kernel_, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin),
-                   "potential5 smem");
-        check_cuda(cudaFuncSetAttribute(pot5_kernel_, cudaFuncAttributePreferredSharedMemoryCarveout, 100),
-                   "potential5 carveout");
-        int per_sm = 0;
-        check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pot5_kernel_, 128, pot5_smem_),
-                   "potential5 occupancy");
-        pot5_blocks_per_sm_ = std::max(per_sm, 1);
-        pot5_sms_ = sms;
-        pot5_blocks_ = static_cast<int>(std::min<long long>(static_cast<long long>(pot5_blocks_per_sm_) * sms, items));
-        error_flag_ = dev<int>(1);
-        check_cuda(cudaMemset(error_flag_, 0, sizeof(int)), "error flag");
-      }
     }
+    // potential5 (mixed form): the contractions on the FP64 tensor cores, any ntheta up to 16.
+    pot5_kernel_ = nullptr;
+    if constexpr (std::is_same_v<T, float>) build_pot5(pot5_args_, first, size, slot, offset, legendre64, phi_map, smem_optin, dev_id);
     // potential6 (mixed form): both theta contractions as split-precision TF32 tcgen05 GEMMs over 64-column
     // tiles, for the square heteronuclear basis JMax = MJMax = 15 with ntheta 16 and nphi 32 (configuration
     // 2's angular grid); one block of 256 threads per SM holding all 512 tensor-memory columns.
@@ -2003,8 +1696,141 @@ class Step final : public StepBase {
           }
       pot_source_ = "fixed";
     }
+    build_exp_table(d);
     check_cuda(cudaStreamSynchronize(stream_), "set-up");
     autotune();
+  }
+
+  // potential5's matrix fragments (spo_pot5.cuh), rotation factors and launch shape.
+  template <typename A>
+  void build_pot5(A& a, const std::vector<int>& first, const std::vector<int>& size, const std::vector<int>& slot,
+                  const std::vector<int>& offset, const std::vector<double>& legendre, const std::vector<int>& phi_map,
+                  int smem_optin, int dev_id) {
+    const Sizes& s = s_;
+    const long long n_cols = static_cast<long long>(s.nzp) * s.nr * s.n_xy();
+    if (s.nt > 16 || s.nphi > 255 || s.n_rot > 8192 || n_cols > (1ll << 30) || static_cast<long long>(s.nr) * s.n_rot > (1ll << 30)) return;
+    const int h_n = s.nt > 8 ? 2 : 1;
+    auto kernel = spo::pot5::kernel_for(s.nphi, h_n);
+    if (!kernel) return;
+    // Fragments of 32 values: forward [theta half][J quad], lane l the entry (theta 8 half + l / 4, J 4 quad + l % 4);
+    // transposed [J octet][theta half][i], lane l the entry (theta 8 half + 2 (l % 4) + i, J 8 octet + l / 8 + 4 (l / 4 % 2)).
+    // Blocks of equal matrices (m and -m) share theirs.
+    std::vector<double> fwd, back;
+    std::vector<int4> slots(s.nphi, make_int4(0, 0, 0, 0));
+    for (int b = 0; b < s.n_blocks; ++b) {
+      const double* m = legendre.data() + offset[b];
+      const int nj = size[b];
+      const int nk = (std::max(nj, size[s.n_blocks - 1 - b]) + 3) / 4;  // as many steps as the block of -m
+      int4 e = make_int4(first[b], nj + 65536 * nk, -1, -1);
+      for (int o = 0; o < b && e.z < 0; ++o)
+        if (slots[slot[o]].y == e.y && std::equal(m, m + static_cast<std::size_t>(s.nt) * nj, legendre.data() + offset[o])) {
+          e.z = slots[slot[o]].z;
+          e.w = slots[slot[o]].w;
+        }
+      if (e.z < 0) {
+        auto at = [&](int theta, int j) { return theta < s.nt && j < nj ? m[static_cast<std::size_t>(theta) * nj + j] : 0.0; };
+        e.z = static_cast<int>(fwd.size() / 32);
+        for (int h = 0; h < h_n; ++h)
+          for (int q = 0; q < nk; ++q)
+            for (int l = 0; l < 32; ++l) fwd.push_back(at(8 * h + l / 4, 4 * q + l % 4));
+        e.w = static_cast<int>(back.size() / 32);
+        for (int q = 0; 8 * q < nj; ++q)
+          for (int h = 0; h < h_n; ++h)
+            for (int i = 0; i < 2; ++i)
+              for (int l = 0; l < 32; ++l) back.push_back(at(8 * h + 2 * (l % 4) + i, 8 * q + l / 8 + 4 * (l / 4 % 2)));
+      }
+      slots[slot[b]] = e;
+    }
+    const int n_fwd = static_cast<int>(fwd.size() / 32), n_back = static_cast<int>(back.size() / 32);
+    fwd.insert(fwd.end(), back.begin(), back.end());
+    int teams = spo::pot5::threads_of(s.nphi) / (32 * h_n);
+    while (teams > 0 && spo::pot5::smem_bytes(s.n_rot, s.nphi, h_n, n_fwd + n_back, teams) > static_cast<std::size_t>(smem_optin)) --teams;
+    if (teams == 0) return;
+    a.p = pot_;
+    a.frags = upload_f64(fwd);
+    a.n_fwd = n_fwd;
+    a.n_back = n_back;
+    int4* ds = dev<int4>(slots.size());
+    check_cuda(cudaMemcpy(ds, slots.data(), sizeof(int4) * slots.size(), cudaMemcpyHostToDevice), "potential5 slots");
+    a.slots = ds;
+    a.rot = upload_c128(host_rot_);
+    a.phi_map = nullptr;
+    if (!identity_maps_) {
+      std::vector<std::uint8_t> map(phi_map.begin(), phi_map.end());
+      std::uint8_t* dm = dev<std::uint8_t>(map.size());
+      check_cuda(cudaMemcpy(dm, map.data(), map.size(), cudaMemcpyHostToDevice), "potential5 maps");
+      a.phi_map = dm;
+    }
+    a.pairs = (s.nt + 1) / 2;
+    a.n_cols = static_cast<int>(n_cols);
+    a.n_items = (a.n_cols + spo::pot5::kCols - 1) / spo::pot5::kCols;
+    a.bulk = s.n_rot % 2 == 0 ? 1 : 0;
+    a.poll_limit = spo::pot5::kWaitLimit;
+    a.extra_tx = 0;
+    int sms = 0;
+    check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev_id), "SM count");
+    pot5_kernel_ = kernel;
+    pot5_h_ = h_n;
+    // one block per SM; few items: fewer teams per block, so that every SM has some
+    while (teams > 1 && a.n_items <= static_cast<long long>(sms) * (teams - 1)) --teams;
+    pot5_threads_ = teams * 32 * h_n;
+    pot5_smem_ = spo::pot5::smem_bytes(s.n_rot, s.nphi, h_n, n_fwd + n_back, teams);
+    check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin), "potential5 smem");
+    pot5_blocks_ = static_cast<int>(std::max<long long>(1, std::min<long long>(sms, (a.n_items + teams - 1) / teams)));
+    if (!error_flag_) {
+      error_flag_ = dev<int>(1);
+      check_cuda(cudaMemset(error_flag_, 0, sizeof(int)), "error flag");
+    }
+  }
+
+  // exp(i A) on the device in FP64, chunk by chunk through the staging buffer, in the order of the handle's potential
+  // kernel: potential5's, or (point, representative, theta, phi) for the others.
+  void build_exp_table(const spo_desc& d) {
+    const Sizes& s = s_;
+    const long long n_e = s.n_expia(), n_tp = static_cast<long long>(s.nt) * s.nphi;
+    require(d.potential != nullptr || n_e == 0, "potential is null");
+    double* vstage = reinterpret_cast<double*>(staging_);
+    if (pot_kind_ == 5) {
+      const long long reps = static_cast<long long>(s.nzp) * s.nr * s.n_rep;
+      const long long per_rep = static_cast<long long>(s.nphi) * pot5_args_.pairs;
+      float4* table = dev<float4>(std::max<long long>(reps * per_rep, 1));
+      __half2* mods = dev<__half2>(std::max<long long>(reps * per_rep, 1));
+      pot5_args_.table = table;
+      pot5_args_.mods = mods;
+      const long long chunk = 2 * staging_elems_ / n_tp;
+      for (long long i = 0; i < reps; i += chunk) {
+        const long long m = std::min(chunk, reps - i);
+        check_cuda(cudaMemcpyAsync(vstage, d.potential + i * n_tp, sizeof(double) * m * n_tp, cudaMemcpyHostToDevice, stream_),
+                   "upload potential");
+        spo::exp_pairs_kernel<<<1184, 256, 0, stream_>>>(vstage, table + i * per_rep, mods + i * per_rep, m, s.nt, s.nphi,
+                                                        pot5_args_.pairs, spo::pot5::group_of(s.nphi), s.dt);
+        check_cuda(cudaGetLastError(), "exp_potential launch");
+        check_cuda(cudaStreamSynchronize(stream_), "exp_potential");
+      }
+      return;
+    }
+    // The mixed form keeps, after the n_e table entries, their n_e modulus corrections (FP16, spo::exp_mul)
+    // (from a 16-byte boundary: the kernels read 8 corrections per load and prefetch rows of them into L2)
+    const long long n_e_even = (n_e + 1) & ~1ll;
+    expia_ = dev<V>(std::max<long long>(n_e_even + (sizeof(T) == 4 ? (n_e + 3) / 4 : 0), 1));
+    __half* exp_mod = sizeof(T) == 4 ? reinterpret_cast<__half*>(expia_ + n_e_even) : nullptr;
+    const long long chunk = 2 * staging_elems_;
+    for (long long i = 0; i < n_e; i += chunk) {
+      const long long m = std::min(chunk, n_e - i);
+      check_cuda(cudaMemcpyAsync(vstage, d.potential + i, sizeof(double) * m, cudaMemcpyHostToDevice, stream_),
+                 "upload potential");
+      spo::exp_potential_kernel<T><<<1184, 256, 0, stream_>>>(vstage, expia_ + i, exp_mod ? exp_mod + i : nullptr, m, s.dt);
+      check_cuda(cudaGetLastError(), "exp_potential launch");
+      check_cuda(cudaStreamSynchronize(stream_), "exp_potential");
+    }
+    for (auto* p : {&pot_, &pot2_.p, &pot3_args_.p, &pot4_args_.p}) {
+      p->expia = expia_;
+      p->exp_mod = exp_mod;
+    }
+    if constexpr (std::is_same_v<T, float>) {
+      pot6_args_.p.expia = expia_;
+      pot6_args_.p.exp_mod = exp_mod;
+    }
   }
 
   // Host FP64 complex -> device T, through the staging buffer.
@@ -2069,10 +1895,12 @@ class Step final : public StepBase {
   spo::Pot4Args<T> pot4_args_{};
   int pot4_blocks_ = 0;
   std::size_t pot4_smem_ = 0;
-  Pot5Kernel<T> pot5_kernel_ = nullptr;
-  int pot5_blocks_ = 0, pot5_blocks_per_sm_ = 1, pot5_sms_ = 0;
+  spo::pot5::Kernel pot5_kernel_ = nullptr;  // mixed form
+  spo::Pot5Args pot5_args_{};
+  int pot5_blocks_ = 0, pot5_threads_ = 0, pot5_h_ = 1;
   std::size_t pot5_smem_ = 0;
-  bool pot5_l2e_ = false;  // potential5's L2E form (exp(i A) rows through L2, three blocks per SM)
+  std::vector<cplx> host_rot_;   // rot(dt/2), (ir, irot)
+  bool identity_maps_ = true;    // no symmetry: representative = (x, y) point and phi maps = identity
   int* error_flag_ = nullptr;  // set by a kernel whose bounded wait gave up
   // the norm budget (norm_budget_setup / norm_budget_add) and the FP64 absorber factors it is built from
   std::vector<double> host_opt_z_, host_opt_r_, host_opt_zs_;

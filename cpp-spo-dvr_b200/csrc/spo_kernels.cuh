@@ -417,11 +417,20 @@ struct XyArgs {
   int nr;
   const T* opt_z;          // nz
   const Vec<T>* gas_step;  // (ir, irot): opt_r rot gas rot
+  const Vec<T>* before;    // (ir, irot): opt_r rot(dt/2), applied with opt_z to the points below izr_gas_first when
+                           // `apply_gas` is set (a potential kernel that takes psi scaled follows); or null
   int tile;                // launch choice of the register-DFT xy kernel: rotational states per block
                            // (8, 16 or 32; 0: the default) for grids of more than 8 points per axis
   long long izr_offset;    // register-DFT xy kernel: block y serves point izr = izr_offset + y
   int persistent;          // launch choice: the persistent form of the register-DFT xy kernel (xy2p_kernel)
 };
+
+// The factor table (ir, irot) that follows T_xy at a point: the gas-phase step, or the scaling of the interaction
+// region's potential step, or none (null).
+template <typename T>
+__device__ __forceinline__ const Vec<T>* xy_post(const XyArgs<T>& a, long long izr) {
+  return !a.apply_gas ? nullptr : izr >= a.izr_gas_first ? a.gas_step : a.before;
+}
 
 template <typename T>
 __global__ void __launch_bounds__(256) xy_pass_kernel(XyArgs<T> a) {
@@ -459,16 +468,16 @@ __global__ void __launch_bounds__(256) xy_pass_kernel(XyArgs<T> a) {
   cur = smem_fft(cur, oth, twx, a.px, +1, a.ny * tb, a.ny * tb, 0, a.ny * tb);
   oth = cur == buf0 ? buf1 : buf0;
   cur = smem_fft(cur, oth, twy, a.py, +1, a.nx * tb, tb, a.ny * tb, tb);
-  const bool gas = a.apply_gas && izr >= a.izr_gas_first;
+  const Vec<T>* const post = xy_post(a, izr);
   const int ir = static_cast<int>(izr % a.nr);
-  const T oz = gas ? a.opt_z[izr / a.nr] : T(1);
+  const T oz = post ? a.opt_z[izr / a.nr] : T(1);
   for (int e = threadIdx.x; e < nxy * tb; e += blockDim.x) {
     const int ixy = e / tb, b = e % tb;
     if (r0 + b < a.n_rot) {
       V v = cur[e];
       if (a.shift_b) v = fmul_t(v, a.shift_b, nxy, ixy);
-      if (gas) {
-        v = fmul_t(v, a.gas_step, static_cast<long long>(a.nr) * a.n_rot, ir * a.n_rot + r0 + b);
+      if (post) {
+        v = fmul_t(v, post, static_cast<long long>(a.nr) * a.n_rot, ir * a.n_rot + r0 + b);
         v = cscale(v, oz);
       }
       a.psi[(col0 + ixy) * a.n_rot + r0 + b] = v;
@@ -624,41 +633,46 @@ __global__ void __launch_bounds__(256) potential_kernel(PotArgs<T> a) {
 // Utilities
 // ---------------------------------------------------------------------------------------------
 
-// Potential step of the gas-phase region alone (izr >= izr_first): optical_z * gas_step(ir, irot)
-// (src/propagation/potential_operator.cpp:104-112). The propagation fuses this into the xy pass;
-// this kernel serves the stage-by-stage entry point.
+// The factors opt_z * table(ir, irot) of the potential step at the points izr_first <= izr < izr_last: the whole
+// step in the gas-phase region (src/propagation/potential_operator.cpp:104-112), or the scaling before a potential
+// kernel that takes psi scaled. The propagation fuses this into the xy pass; this kernel serves the stage-by-stage
+// entry point.
 template <typename T>
-__global__ void gas_phase_kernel(Vec<T>* __restrict__ psi, long long izr_first, long long n_zr, int n_rot, int n_xy,
-                                 int nr, const T* __restrict__ opt_z, const Vec<T>* __restrict__ gas_step) {
+__global__ void scale_points_kernel(Vec<T>* __restrict__ psi, long long izr_first, long long izr_last, int n_rot, int n_xy,
+                                    int nr, const T* __restrict__ opt_z, const Vec<T>* __restrict__ table) {
   const long long per_izr = static_cast<long long>(n_xy) * n_rot;
-  const long long n = (n_zr - izr_first) * per_izr;
+  const long long n = (izr_last - izr_first) * per_izr;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     const long long izr = izr_first + i / per_izr;
     const int irot = static_cast<int>(i % n_rot);
     const int ir = static_cast<int>(izr % nr);
     const long long g = izr_first * per_izr + i;
-    psi[g] = cscale(fmul_t(psi[g], gas_step, static_cast<long long>(nr) * n_rot, ir * n_rot + irot), opt_z[izr / nr]);
+    psi[g] = cscale(fmul_t(psi[g], table, static_cast<long long>(nr) * n_rot, ir * n_rot + irot), opt_z[izr / nr]);
   }
 }
 
 // exp(i A), A = -V dt, formed in FP64 (src/propagation/potential_operator.cpp:55-65 with
-// src/potential/potential_grid.cpp:164-167), then rounded to T.
+// src/potential/potential_grid.cpp:164-167), then rounded to T. Mixed form: g = exp(i A) - 1 and the modulus
+// correction of 1 + g (see exp_mul).
+__device__ __forceinline__ void exp_entry(double v, double dt, float2& g, __half& m) {
+  const double a = -v * dt;
+  const float gx = static_cast<float>(-2.0 * sin(0.5 * a) * sin(0.5 * a));  // cos A - 1 without cancellation
+  const float gy = static_cast<float>(sin(a));
+  g = make_float2(gx, gy);
+  const double rx = 1.0 + static_cast<double>(gx), ry = gy;
+  m = __double2half((1.0 / sqrt(rx * rx + ry * ry) - 1.0) * 16777216.0);
+}
 template <typename T>
 __global__ void exp_potential_kernel(const double* __restrict__ v, Vec<T>* __restrict__ out, __half* __restrict__ mod,
                                      long long n, double dt) {
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const double a = -v[i] * dt;
-    double s, c;
-    sincos(a, &s, &c);
-    if constexpr (sizeof(T) == 4) {  // g = exp(i A) - 1 and the modulus correction of 1 + g (see exp_mul)
-      const double cm1 = -2.0 * sin(0.5 * a) * sin(0.5 * a);  // cos A - 1 without cancellation
-      const float gx = static_cast<float>(cm1), gy = static_cast<float>(s);
-      out[i] = cmake<Vec<T>>(gx, gy);
-      const double rx = 1.0 + static_cast<double>(gx), ry = gy;
-      mod[i] = __double2half((1.0 / sqrt(rx * rx + ry * ry) - 1.0) * 16777216.0);
+    if constexpr (sizeof(T) == 4) {
+      exp_entry(v[i], dt, out[i], mod[i]);
     } else {
+      double s, c;
+      sincos(-v[i] * dt, &s, &c);
       out[i] = cmake<Vec<T>>(static_cast<T>(c), static_cast<T>(s));
     }
   }

@@ -1,0 +1,314 @@
+// The kinetic passes of the scattering wave (src/propagation/kinetic_operators.cpp:77-172) as one kernel: a two-level
+// transform of N = N1 N2 points along an axis, times the kinetic factor, and back, for tiles of adjacent lanes. Three
+// maps between the points and the two levels:
+//   kTwiddle  n = n2 + N2 n1, k = k1 + N1 k2, twiddles w_N^(n2 k1) between the levels (T_Z, T_r)
+//   kPrime    n = (N2 n1 + N1 n2) mod N for coprime N1, N2: no twiddles, the factors permuted (axis2pfa_kernel)
+//   kXy       n = n1 + N1 n2: the two levels are y (N1) and x (N2) of the (x, y) grid, no twiddles (T_xy), with the
+//             momentum shift before and after and, as the last factor, the gas-phase step or the scaling of the
+//             interaction region's potential step.
+//
+// The mixed form takes two adjacent lanes per thread as packed FP32 pairs (spo_pair.cuh): 16-byte accesses and half
+// the instructions. Issue bound it before (65 to 75 % of the slots at 4 TB/s: every constant is exact to ~2^-48, which
+// costs two to three times the instructions of plain FP32 products); one lane per thread took 1.64, 1.59 and 1.84 ms
+// on configuration 3 (Z 128, r 48, 16 x 16). A grid of resident blocks loops over the tiles, so that the tables are
+// staged in shared memory once per block, not once per tile. kinetic factors s e^{i phi} are applied as p (x + x g)
+// with p the power of two in s, folded into g and exact, and a product with the rest s / p only where it is not 1.
+//
+// N1, N2 > 0: compile-time sizes. N1 = N2 = 0: any two sizes up to 16 that rdft has (a switch per level), for the
+// lengths without an instantiation and for rectangular (x, y) grids, in both forms; the shared-memory Stockham kernels
+// they ran on before are 3 to 10 times slower (T_Z of 90 points, r 36, x = y = 10: 1.12 ms).
+#pragma once
+
+#include "spo_pair.cuh"
+
+namespace spo {
+
+enum KinMap : int { kTwiddle = 0, kPrime = 1, kXy = 2 };
+
+template <typename T>
+struct KinArgs {
+  Vec<T>* data;
+  int n1, n2;
+  long long stride, outer_stride;  // between a line's points, between the line sets of consecutive outer indices
+  // lanes: groups of `window` adjacent lanes, group_stride apart, the first at lane_offset
+  long long group_stride, lane_offset, window;
+  unsigned groups, blocks_per_group, n_tiles;
+  int log_lines;          // lines per tile = 1 << log_lines (mixed form: pairs of lanes)
+  int aligned;            // mixed form: every pair of lanes starts on a 16-byte boundary
+  const double2* table;   // N factors (see KinTable), then N twiddles (kTwiddle), as stored in shared memory
+  T scale;                // p
+  int unit;               // s = p: no remaining scale
+  XyArgs<T> xy;           // kXy: shift, gas-phase and scaling tables
+};
+
+// Table entries: mixed form: N pairs (p g.x, p g.x, p g.y, p g.y) and (their low parts), N scales (s/p, s/p, low, low),
+// then for kTwiddle N twiddles (w.x, w.x, w.y, w.y) and (their low parts); FP64 form: N factors, then N twiddles.
+template <typename T> struct KinLine;
+template <> struct KinLine<float> {
+  using type = C2;
+  static constexpr int lanes = 2;
+  static constexpr int factor_words = 3, twiddle_words = 2;  // 16-byte words per entry
+};
+template <> struct KinLine<double> {
+  using type = double2;
+  static constexpr int lanes = 1;
+  static constexpr int factor_words = 1, twiddle_words = 1;
+};
+
+#ifdef __CUDACC__
+
+
+// factor k on x
+__device__ __forceinline__ C2 kin_factor(C2 x, const C2* f, int n, int k, F2 p, bool unit) {
+  const C2 m = cmul2(x, f[2 * k], f[2 * k + 1]);
+  C2 z = c2(fma2(x.x, p, m.x), fma2(x.y, p, m.y));
+  if (!unit) {
+    const C2 s = f[2 * n + k];  // (s/p twice, its low part twice)
+    z = c2(fma2(z.x, s.x, z.x * s.y), fma2(z.y, s.x, z.y * s.y));
+  }
+  return z;
+}
+__device__ __forceinline__ double2 kin_factor(double2 x, const double2* f, int, int k, double, bool) { return cmul(f[k], x); }
+// twiddle j on x, conjugated for S > 0
+template <bool ODD, int S>
+__device__ __forceinline__ C2 kin_twiddle(C2 x, const C2* tw, int j) {
+  C2 w = tw[2 * j], l = tw[2 * j + 1];
+  if constexpr (S > 0) {
+    w.y = -w.y;
+    l.y = -l.y;
+  }
+  if constexpr (ODD) return cmul_comp(x, w, l);
+  else return cmul2(x, w, l);
+}
+template <bool ODD, int S>
+__device__ __forceinline__ double2 kin_twiddle(double2 x, const double2* tw, int j) {
+  return S > 0 ? cmul(x, cconj(tw[j])) : cmul(x, tw[j]);
+}
+__device__ __forceinline__ F2 kin_scale(float p) { return f2(p); }
+__device__ __forceinline__ double kin_scale(double p) { return p; }
+
+// The lane(s) of a line: `ok` counts those that exist.
+__device__ __forceinline__ C2 kin_load(const float2* p, int ok, bool aligned) {
+  float2 a = make_float2(0.0f, 0.0f), b = a;
+  if (aligned && ok == 2) {
+    const float4 v = *reinterpret_cast<const float4*>(p);
+    a = make_float2(v.x, v.y);
+    b = make_float2(v.z, v.w);
+  } else {
+    if (ok > 0) a = p[0];
+    if (ok > 1) b = p[1];
+  }
+  return c2(a, b);
+}
+__device__ __forceinline__ void kin_store(float2* p, C2 v, int ok, bool aligned) {
+  float2 a, b;
+  c2_split(v, a, b);
+  if (aligned && ok == 2) {
+    *reinterpret_cast<float4*>(p) = make_float4(a.x, a.y, b.x, b.y);
+  } else {
+    if (ok > 0) p[0] = a;
+    if (ok > 1) p[1] = b;
+  }
+}
+__device__ __forceinline__ double2 kin_load(const double2* p, int ok, bool) { return ok ? *p : make_double2(0.0, 0.0); }
+__device__ __forceinline__ void kin_store(double2* p, double2 v, int ok, bool) {
+  if (ok) *p = v;
+}
+
+// The factor of the potential step that follows T_xy at a point, for the lane(s) of a line.
+struct KinPostPair {
+  C2 g, gl, s;
+  F2 oz;
+  bool unit;
+};
+struct KinPostF64 {
+  double2 g;
+  double oz;
+};
+__device__ __forceinline__ KinPostPair kin_post(const float2* t, long long n, long long k, int ok, float oz) {
+  const long long j = ok > 1 ? k + 1 : k;
+  const float2 s = t[2 * n + k];  // the scale depends on the r point only
+  return KinPostPair{c2(t[k], t[j]), c2(t[n + k], t[n + j]), c2(f2(s.x), f2(s.y)), f2(oz), s.x == 1.0f && s.y == 0.0f && oz == 1.0f};
+}
+__device__ __forceinline__ C2 kin_apply(C2 x, const KinPostPair& w) {
+  C2 z = cadd(x, cmul2(x, w.g, w.gl));
+  if (!w.unit) {
+    z = c2(fma2(z.x, w.s.x, z.x * w.s.y), fma2(z.y, w.s.x, z.y * w.s.y));
+    z = c2(z.x * w.oz, z.y * w.oz);
+  }
+  return z;
+}
+__device__ __forceinline__ KinPostF64 kin_post(const double2* t, long long, long long k, int ok, double oz) {
+  return KinPostF64{ok ? t[k] : make_double2(0.0, 0.0), oz};
+}
+__device__ __forceinline__ double2 kin_apply(double2 x, const KinPostF64& w) { return cscale(cmul(w.g, x), w.oz); }
+// x times entry k of a factor table in global memory (the momentum shift), the same for every lane
+__device__ __forceinline__ C2 kin_shift(C2 x, const float2* t, int n, int k) {
+  return fmul_parts(x, __ldg(t + k), __ldg(t + n + k), __ldg(t + 2 * n + k));
+}
+__device__ __forceinline__ double2 kin_shift(double2 x, const double2* t, int, int k) { return cmul(t[k], x); }
+
+// A thread's share of a tile.
+template <typename T>
+struct KinTile {
+  using L = typename KinLine<T>::type;
+  Vec<T>* base;   // the line's first point
+  long long stride;
+  int ok;         // existing lanes of the line
+  bool aligned;
+  int b, s, nt, log_lines;  // line of the tile, thread of the line, threads per line
+  L* Y;           // [n2][k1][line]
+};
+
+template <int MAP>
+__device__ __forceinline__ int kin_point(int n1, int n2, int N1, int N2) {
+  if constexpr (MAP == kTwiddle) return n2 + N2 * n1;
+  else if constexpr (MAP == kXy) return n1 + N1 * n2;
+  else {
+    const int n = N2 * n1 + N1 * n2;
+    return n >= N1 * N2 ? n - N1 * N2 : n;
+  }
+}
+
+// Level 1: DFT over n1 for the thread's n2.
+template <typename T, int MAP, int N1, bool ODD>
+__device__ __forceinline__ void kin_forward(const KinTile<T>& t, const KinArgs<T>& a, int N2, const typename KinLine<T>::type* tw) {
+  using L = typename KinLine<T>::type;
+#pragma unroll 1
+  for (int n2 = t.s; n2 < N2; n2 += t.nt) {
+    L x[N1];
+    static_for<0, N1>([&](auto n1) {
+      x[n1] = kin_load(t.base + kin_point<MAP>(SPO_CV(n1), n2, N1, N2) * t.stride, t.ok, t.aligned);
+      if constexpr (MAP == kXy)
+        if (a.xy.shift_f) x[n1] = kin_shift(x[n1], a.xy.shift_f, N1 * N2, kin_point<MAP>(SPO_CV(n1), n2, N1, N2));
+    });
+    rdft<N1, -1>(x);
+    static_for<0, N1>([&](auto k1) {
+      if constexpr (MAP == kTwiddle && SPO_CV(k1) > 0) x[k1] = kin_twiddle<ODD, -1>(x[k1], tw, n2 * SPO_CV(k1));
+      t.Y[((n2 * N1 + SPO_CV(k1)) << t.log_lines) + t.b] = x[k1];
+    });
+  }
+}
+// Level 2: DFT over n2 for the thread's k1, the factor, and back.
+template <typename T, int MAP, int N2, bool ODD>
+__device__ __forceinline__ void kin_middle(const KinTile<T>& t, const KinArgs<T>& a, int N1, const typename KinLine<T>::type* f,
+                                           const typename KinLine<T>::type* tw) {
+  using L = typename KinLine<T>::type;
+  const auto p = kin_scale(a.scale);
+  const bool unit = a.unit != 0;
+#pragma unroll 1
+  for (int k1 = t.s; k1 < N1; k1 += t.nt) {
+    L y[N2];
+    L* const row = t.Y + (k1 << t.log_lines) + t.b;
+    static_for<0, N2>([&](auto n2) { y[n2] = row[(SPO_CV(n2) * N1) << t.log_lines]; });
+    rdft<N2, -1>(y);
+    static_for<0, N2>([&](auto k2) { y[k2] = kin_factor(y[k2], f, N1 * N2, k1 + N1 * SPO_CV(k2), p, unit); });
+    rdft<N2, +1>(y);
+    static_for<0, N2>([&](auto n2) {
+      if constexpr (MAP == kTwiddle && SPO_CV(n2) > 0) y[n2] = kin_twiddle<ODD, +1>(y[n2], tw, SPO_CV(n2) * k1);
+      row[(SPO_CV(n2) * N1) << t.log_lines] = y[n2];
+    });
+  }
+}
+template <typename T, int MAP, int N1, typename P>
+__device__ __forceinline__ void kin_back(const KinTile<T>& t, const KinArgs<T>& a, int N2, bool post, const P& w) {
+  using L = typename KinLine<T>::type;
+  if (t.ok == 0) return;
+#pragma unroll 1
+  for (int n2 = t.s; n2 < N2; n2 += t.nt) {
+    L x[N1];
+    static_for<0, N1>([&](auto k1) { x[k1] = t.Y[((n2 * N1 + SPO_CV(k1)) << t.log_lines) + t.b]; });
+    rdft<N1, +1>(x);
+    static_for<0, N1>([&](auto n1) {
+      const int n = kin_point<MAP>(SPO_CV(n1), n2, N1, N2);
+      if constexpr (MAP == kXy) {
+        if (a.xy.shift_b) x[n1] = kin_shift(x[n1], a.xy.shift_b, N1 * N2, n);
+        if (post) x[n1] = kin_apply(x[n1], w);
+      }
+      kin_store(t.base + n * t.stride, x[n1], t.ok, t.aligned);
+    });
+  }
+}
+
+// f(size) for a runtime size among those of rdft up to 16.
+template <typename F>
+__device__ __forceinline__ void kin_switch(int n, F&& f) {
+  switch (n) {
+    case 1: f(std::integral_constant<int, 1>{}); break;
+    case 2: f(std::integral_constant<int, 2>{}); break;
+    case 3: f(std::integral_constant<int, 3>{}); break;
+    case 4: f(std::integral_constant<int, 4>{}); break;
+    case 5: f(std::integral_constant<int, 5>{}); break;
+    case 6: f(std::integral_constant<int, 6>{}); break;
+    case 7: f(std::integral_constant<int, 7>{}); break;
+    case 8: f(std::integral_constant<int, 8>{}); break;
+    case 9: f(std::integral_constant<int, 9>{}); break;
+    case 10: f(std::integral_constant<int, 10>{}); break;
+    case 11: f(std::integral_constant<int, 11>{}); break;
+    case 12: f(std::integral_constant<int, 12>{}); break;
+    case 14: f(std::integral_constant<int, 14>{}); break;
+    case 15: f(std::integral_constant<int, 15>{}); break;
+    default: f(std::integral_constant<int, 16>{}); break;
+  }
+}
+
+// Registers: the lines of the larger level (4 per point and pair of lanes) and its temporaries.
+constexpr int kin_max_threads(int n) { return n > 16 ? 128 : 256; }
+constexpr int kin_min_blocks(int n) { return n > 16 ? 3 : n > 8 || n == 0 ? 2 : 3; }
+
+template <typename T, int MAP, int N1C, int N2C>
+__global__ void __launch_bounds__(kin_max_threads(N1C > N2C ? N1C : N2C), kin_min_blocks(N1C > N2C ? N1C : N2C))
+    kin_kernel(const __grid_constant__ KinArgs<T> a) {
+  using L = typename KinLine<T>::type;
+  constexpr bool ANY = N1C == 0;
+  const int N1 = ANY ? a.n1 : N1C, N2 = ANY ? a.n2 : N2C, N = N1 * N2;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  L* const f = reinterpret_cast<L*>(smem_raw);
+  L* const tw = f + KinLine<T>::factor_words * N;
+  KinTile<T> t;
+  t.Y = tw + (MAP == kTwiddle ? KinLine<T>::twiddle_words * N : 0);
+  {
+    const int words = static_cast<int>(t.Y - f);
+    const L* src = reinterpret_cast<const L*>(a.table);
+    for (int k = threadIdx.x; k < words; k += blockDim.x) f[k] = src[k];
+  }
+  t.log_lines = a.log_lines;
+  t.b = threadIdx.x & ((1 << a.log_lines) - 1);
+  t.s = threadIdx.x >> a.log_lines;
+  t.nt = blockDim.x >> a.log_lines;
+  t.stride = a.stride;
+  t.aligned = a.aligned != 0;
+  // twiddle products of lengths with an odd factor are nearly correctly rounded (cmul_comp)
+  constexpr bool ODD = ANY || ((N1C * N2C) & (N1C * N2C - 1)) != 0;
+  __syncthreads();
+  for (unsigned tile = blockIdx.x; tile < a.n_tiles; tile += gridDim.x) {
+    const unsigned rest = tile / a.blocks_per_group, blk = tile - rest * a.blocks_per_group;
+    const unsigned outer = rest / a.groups, grp = rest - outer * a.groups;
+    const long long lane = (static_cast<long long>(blk) << a.log_lines) * KinLine<T>::lanes + t.b * KinLine<T>::lanes;
+    t.ok = lane >= a.window ? 0 : static_cast<int>(min(static_cast<long long>(KinLine<T>::lanes), a.window - lane));
+    t.base = a.data + outer * a.outer_stride + grp * a.group_stride + a.lane_offset + lane;
+    if constexpr (ANY) kin_switch(N1, [&](auto n) { kin_forward<T, MAP, SPO_CV(n), ODD>(t, a, N2, tw); });
+    else kin_forward<T, MAP, N1C, ODD>(t, a, N2C, tw);
+    __syncthreads();
+    if constexpr (ANY) kin_switch(N2, [&](auto n) { kin_middle<T, MAP, SPO_CV(n), ODD>(t, a, N1, f, tw); });
+    else kin_middle<T, MAP, N2C, ODD>(t, a, N1C, f, tw);
+    __syncthreads();
+    if constexpr (MAP == kXy) {
+      const long long izr = a.xy.izr_offset + outer;
+      const Vec<T>* const table = xy_post(a.xy, izr);
+      decltype(kin_post(table, 0ll, 0ll, 0, T(0))) w{};
+      if (table && t.ok)
+        w = kin_post(table, static_cast<long long>(a.xy.nr) * a.xy.n_rot, (izr % a.xy.nr) * a.xy.n_rot + lane, t.ok, a.xy.opt_z[izr / a.xy.nr]);
+      if constexpr (ANY) kin_switch(N1, [&](auto n) { kin_back<T, MAP, SPO_CV(n)>(t, a, N2, table != nullptr, w); });
+      else kin_back<T, MAP, N1C>(t, a, N2C, table != nullptr, w);
+    } else {
+      if constexpr (ANY) kin_switch(N1, [&](auto n) { kin_back<T, MAP, SPO_CV(n)>(t, a, N2, false, 0); });
+      else kin_back<T, MAP, N1C>(t, a, N2C, false, 0);
+    }
+    __syncthreads();  // Y is read before the next tile's first level writes it
+  }
+}
+
+#endif  // __CUDACC__
+
+}  // namespace spo

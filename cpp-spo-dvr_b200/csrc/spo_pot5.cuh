@@ -1,31 +1,42 @@
-// Potential step of the interaction region, mixed form, with the item data moved by bulk asynchronous
-// copies (src/propagation/potential_operator.cpp:84-135, angular_transform.cpp:54-114).
+// Potential step of the interaction region, mixed form (src/propagation/potential_operator.cpp:84-135,
+// angular_transform.cpp:54-114): both theta contractions on the FP64 tensor cores (mma.m8n8k4.f64), the phi
+// transforms in registers between them.
 //
-// potential4_kernel loads each item's wave packet and exp(i A) rows with ordinary per-thread loads when
-// it needs them; with 12 warps per SM that keeps too few bytes in flight (1.8 TB/s on configuration 3).
-// This kernel issues them one item ahead with cp.async.bulk (global -> shared, completion counted in
-// bytes on an mbarrier), so the copies of item k + 1 run while item k computes:
-//   - psi: the CB columns of the item (n_rot contiguous values each) into the F buffer, column c at
-//     F + c (n_rot + 2) (the 16-byte pad puts the columns on different banks); issued for item k + 1
-//     as soon as item k's forward sums have read F;
-//   - exp(i A): each thread's phi line (NPHI contiguous values of its column's representative) into its
-//     own row of E (rows of NPHI + 2 values: 16-byte loads of 8 consecutive rows on distinct banks);
-//     issued for item k + 1 when item k's phi phase is done.
-//   - the item's rows of the scaling tables (opt_r rot(dt/2) and rot(dt/2) at its r point) with the
-//     columns; its opt_z value, incoming specular amplitude and sp2sc coefficients into registers when
-//     the copies are issued, so that no global load sits on the path between two barriers.
-// Per item: wait for F; scale it in place (absorbers, rot(dt/2), the specular wave into the initial
-// channel); forward theta sums (potential4's tiles, F read column-major); wait for E; phi DFT, exp(i A),
-// inverse DFT; transposed theta sums, rot(dt/2), store. The matrix rows are staged in shared memory as
-// in potential4 (about 105 KB per block on configuration 3: two blocks per SM). The projection onto the
-// specular grid is projection_finalize_kernel's.
+// A team of H warps (H = 1 for ntheta <= 8, 2 for ntheta <= 16) owns 8 (x, y) columns at a time, warp h the
+// theta 8h .. 8h + 7 of every one of them:
+//   - forward: X_m[c, theta] = sum_J F[c, J] M_m[theta, J] for every mJ block m, columns as the rows of the
+//     product. Lane (c = lane / 4, t = lane % 4) then holds theta 8h + 2t and 8h + 2t + 1 of column c for
+//     every phi slot, real and imaginary parts (two products share each matrix fragment): two complete phi lines
+//     per lane, so the phi transforms, exp(i A) and the inverse transforms need no exchange at all;
+//   - back: out[c, J] = sum_theta X[c, theta] M_m[theta, J]. The accumulator layout of the forward product is the
+//     A operand layout of this one when the summed theta are taken in the order 8h + 2 (lane % 4) + i, i = 0, 1:
+//     the values go from registers into the tensor core. With H = 2 each warp takes every other phi slot and gets
+//     the other warp's eight theta of it through shared memory (FP32).
+// Products and sums are FP64 (the matrix exactly as given), rounded once to FP32 per contraction: the FP32 state
+// of the mixed form is kept, its contractions lose nothing.
 //
-// Every wait on an mbarrier is bounded. A block whose wait gives up sets *error_flag, waits (bounded)
-// for the copies it has in flight and returns as a whole; the host reads the flag after the step.
+// What bounds it: on configuration 3 (2.6e8 values of psi per launch) the tensor core needs 84 multiply-adds per
+// value with its padding (1.2 ms), the FP32 pipe about 100 operations per value for the phi transforms and
+// exp(i A) (0.8 ms), HBM 9.5 GB (1.5 ms). The FP32 form of the contractions (a 12-bit high part and the rest of
+// each matrix entry, two FMAs per term, operands through shared memory) spent 128 FMA-pipe operations and as many
+// bytes of shared memory per value and took 5.62 ms.
+//
+// Data movement: the 8 columns of a team's next item (n_rot contiguous values each) are copied into its F buffer
+// by cp.async.bulk as soon as F is free (H = 2: after the exchange, which uses the same memory) (completion counted in bytes on the team's
+// mbarrier; odd n_rot, whose columns are not 16-byte multiples, by plain loads). The exp(i A) entries are stored
+// in the order in which the lanes read them: per (Z, r) point and representative [phi][pair of theta] as
+// (re, re', im, im') with the modulus corrections of G phi together, so the four lanes of a column read 64
+// contiguous bytes; the next item's are requested into L2 one item ahead.
+//
+// psi comes scaled by the absorbers and rot(dt/2): the xy pass before this kernel multiplies every value anyway.
+//
+// Every wait on an mbarrier is bounded. A team whose wait gives up sets *error_flag, waits (bounded) for the
+// copies it has in flight and leaves; the host reads the flag after the step.
 #pragma once
 
 #include <cstdint>
 
+#include "spo_pair.cuh"
 #include "spo_pot4.cuh"
 
 namespace spo {
@@ -96,433 +107,379 @@ __device__ __forceinline__ void bulk_copy(void* dst, const void* src, uint32_t b
       : "memory");
 }
 
-}  // namespace pot5
-
-// Shared memory of potential5_kernel: 2 barriers (padded to 32 bytes), F (CB columns of n_rot + 2
-// values), E (NT CB rows of NPHI + 2 values), X (NPHI padded slot blocks), the scaling rows with their
-// low parts (one opt_r rot(dt/2) row, two rot(dt/2) rows, CB incoming amplitudes), the matrix rows (n_rot rows of NT + 4),
-// irot -> slot (n_rot ints), the slot sizes and first rows (2 NPHI ints), the schedule (8 sched_len ints).
-// The L2E form keeps neither E nor the scaling rows in shared memory.
-template <typename T>
-constexpr std::size_t pot5_smem(int n_rot, int nphi, int nt, int cb, int sched_len, bool l2e = false) {
-  return 32 + sizeof(Vec<T>) * (static_cast<std::size_t>(cb) * (n_rot + 2) +
-                                (l2e ? 0 : static_cast<std::size_t>(nt) * cb * (nphi + 2)) +
-                                static_cast<std::size_t>(nphi) * pot4_slot_stride<T>(nt, cb) +
-                                (l2e ? 0 : 6) * static_cast<std::size_t>(n_rot) + cb) +
-         sizeof(T) * static_cast<std::size_t>(n_rot) * (nt + 4) +
-         sizeof(int) * (static_cast<std::size_t>(n_rot) + 2 * nphi + 8 * sched_len);
+// Vote of a team (64 threads on named barrier `id`, or one warp): true when any thread's `fail` is set; also a
+// barrier of the team.
+template <int H>
+__device__ __forceinline__ bool team_any(int id, bool fail) {
+  if constexpr (H == 1) {
+    __syncwarp();
+    return __any_sync(0xffffffffu, fail);
+  } else {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 q, %1, 0;\n\t"
+        "barrier.cta.red.or.pred p, %2, 64, q;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(r)
+        : "r"(fail ? 1u : 0u), "r"(id)
+        : "memory");
+    return r != 0;
+  }
+}
+template <int H>
+__device__ __forceinline__ void team_sync(int id) {
+  if constexpr (H == 1) __syncwarp();
+  else asm volatile("barrier.cta.sync %0, 64;" ::"r"(id) : "memory");
 }
 
-// The theta contractions use the matrix as a 12-bit high part (staged in shared memory) plus the FP32
-// rounding of the rest (read through L1), each term as fma(hi, x, fma(lo, x, acc)): hi + lo is the FP64
-// matrix to ~2^-36, and the lo products (~2^-13 of a term) stay well above the rounding unit of the sum, so
-// the sums round without bias. With the matrix rounded to FP32 alone (even with each rotational state's
-// sum of squares kept), the forward and transposed contractions of a physical wave packet (few rotational
-// states with turning relative phases, smooth in theta, the potential varying with theta) changed its norm
-// by up to ~1e-8 per step, the same sign every step: 5e-5 in P_reaction over 20000 steps of configuration 3.
-// With hi + lo as an FP32 value and its small remainder, the remainders lie below half an ulp of the
-// running sum and are rounded away.
-//
-// L2E: the exp(i A) rows are not staged in shared memory; each item's block of them is prefetched into
-// L2 one item ahead (cp.async.bulk.prefetch.L2) and every thread reads its row from there at the start of
-// its phi phase; the opt_r rot(dt/2) values of a thread's rotational states come one item ahead into
-// registers, and its rot(dt/2) values (with their low parts) are read through L1 at the start of the back
-// sums. That leaves ~72 KB of shared memory per block: three blocks (12 warps) per SM instead of two.
-template <typename T, int NPHI, int NT, int CB, bool L2E = false>
-__global__ void __launch_bounds__(NT * CB, L2E ? 3 : 2) potential5_kernel(Pot4Args<T> g, int* __restrict__ error_flag) {
-  using V = Vec<T>;
-  static_assert(sizeof(T) == 4, "the mixed form");
-  static_assert(NT * CB == 128 && NT % 4 == 0 && CB % 2 == 0, "tile shape");
-  constexpr int NTH = NT * CB;
-  constexpr int LDL = NT + 4;
-  constexpr int QUADS = NT / 4;
-  constexpr int PAIRS = CB / 2;
-  static_assert(QUADS * PAIRS == 16, "a slot tile is one half-warp");
-  constexpr int SS = pot4_slot_stride<T>(NT, CB);
-  constexpr int ERS = NPHI + 2;  // E row stride (values)
-  const PotArgs<T>& a = g.p;
-  const int n_rot = a.n_rot;
-  const int FCS = n_rot + 2;     // F column stride (values); n_rot is even
+// D += A B, 8 x 8 x 4 in FP64: lane l holds A[l / 4][l % 4], B[l % 4][l / 4], D[l / 4][2 (l % 4) + {0, 1}].
+__device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(d0), "+d"(d1)
+      : "d"(a), "d"(b));
+}
+
+// Loads of values that are read once, past L1 (whose 28 KB beside the shared memory hold the rotation factors).
+__device__ __forceinline__ float4 ld_stream4(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint2 ld_stream2(const void* p) {
+  uint2 v;
+  asm volatile("ld.global.nc.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+  return v;
+}
+
+// phi whose modulus corrections are stored together (16 or 8 bytes per pair of theta).
+constexpr int group_of(int nphi) { return nphi % 4 == 0 ? 4 : 2; }
+constexpr int kCols = 8;       // columns per item
+// F column stride (values): n_rot and at least 4 zeros behind it, 4 or 12 mod 16 so that the 4 x 8 values of a
+// fragment fall on distinct banks.
+constexpr int f_stride(int n_rot) {
+  int s = (n_rot + 4 + 3) / 4 * 4;
+  while (s % 16 != 4 && s % 16 != 12) s += 4;
+  return s;
+}
+// Threads per block: the phi lines of a lane take 4 nphi registers.
+constexpr int threads_of(int nphi) { return nphi > 16 ? 384 : nphi > 8 ? 512 : 640; }
+// Bytes of a team's buffer: the columns of its item, then (H = 2) the values that its warps exchange.
+constexpr std::size_t team_bytes(int n_rot, int nphi, int h) {
+  const std::size_t f = sizeof(float2) * kCols * static_cast<std::size_t>(f_stride(n_rot));
+  const std::size_t x = h == 2 ? static_cast<std::size_t>(nphi) * 32 * sizeof(float4) : 0;
+  return f > x ? f : x;
+}
+
+}  // namespace pot5
+
+struct Pot5Args {
+  PotArgs<float> p;
+  const float4* table;   // exp(i A) - 1: [(Z, r) point][representative][phi][pair of theta] (re, re', im, im')
+  const __half2* mods;   // modulus corrections: [point][representative][phi / G][pair of theta][phi % G]
+  const double* frags;   // matrix fragments of 32 values: the forward ones, then the transposed ones
+  int n_fwd, n_back;     // their numbers
+  const int4* slots;     // per phi slot: first irot, J count + 65536 forward steps, first forward and transposed fragment
+  const double2* rot;    // (ir, irot): rot(dt/2)
+  const uint8_t* phi_map;  // n_xy * nphi, or null (no symmetry)
+  int pairs;             // pairs of theta in the table
+  int n_cols, n_items;   // columns of the interaction region, items of kCols columns
+  int bulk;              // columns are 16-byte multiples: bulk copies
+  int poll_limit;        // polls before a wait on an mbarrier gives up
+  unsigned extra_tx;     // bytes announced beyond those copied (0; a failure-detection test sets it so that a
+                         // barrier phase cannot complete and the wait gives up)
+};
+
+template <int NPHI, int H>
+__global__ void __launch_bounds__(pot5::threads_of(NPHI), 1) potential5_kernel(Pot5Args g, int* __restrict__ error_flag) {
+  using namespace pot5;
+  constexpr int G = group_of(NPHI);
+  const PotArgs<float>& a = g.p;
+  const int n_rot = a.n_rot, n_xy = a.n_xy, nr = a.nr;
+  const int fcs = f_stride(n_rot);
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw);  // 0: F, 1: E
-  V* const F = reinterpret_cast<V*>(smem_raw + 32);  // [c][irot], columns of FCS values
-  V* E = F + CB * FCS;                     // [line][phi], line = thread (not with L2E)
-  V* X = E + (L2E ? 0 : NTH * ERS);        // [p][theta][c], slot blocks of SS values
-  // The scaling rows hold each value and its low part (see cmul2): rows of n_rot values, then n_rot low parts.
-  V* Bf = X + NPHI * SS;                   // [irot]: opt_r rot(dt/2) at the item's r point (not with L2E)
-  V* R = Bf + (L2E ? 0 : 2 * n_rot);       // [item parity][irot]: rot(dt/2) at the item's r point (not with L2E)
-  V* SP = R + (L2E ? 0 : 4 * n_rot);       // [c]: sp2sc(c) * chi, the item's incoming amplitudes
-  T* L = reinterpret_cast<T*>(SP + CB);    // [irot][position of theta], rows of LDL
-  int* irot_slot = reinterpret_cast<int*>(L + n_rot * LDL);
-  int* s_nj = irot_slot + n_rot;           // [slot]: J count
-  int* s_first = s_nj + NPHI;              // [slot]: first irot
-  int* sched = s_first + NPHI;
-  const int tid = threadIdx.x;
-  if (tid == 0) {
-    for (int k = 0; k < 2; ++k) pot5::mbar_init(bars + k, NTH);
-    pot5::mbar_init_fence();
-  }
-  for (int k = tid; k < n_rot * LDL; k += NTH) L[k] = g.leg_rows12[k];
-  for (int k = tid; k < n_rot; k += NTH) irot_slot[k] = g.irot_slot[k];
-  for (int k = tid; k < NPHI; k += NTH) {
-    s_nj[k] = g.slot_nj[k];
-    s_first[k] = g.slot_nj[k] > 0 ? g.slot_first[k] : 0;
-  }
-  for (int k = tid; k < 8 * g.sched_len; k += NTH) sched[k] = g.fwd_sched[k];
+  double* const mats = reinterpret_cast<double*>(smem_raw);
+  int4* const slots = reinterpret_cast<int4*>(mats + 32 * (g.n_fwd + g.n_back));
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, teams = blockDim.x / (32 * H);
+  const int team = warp / H, h = warp % H, bar_id = 1 + team;
+  uint64_t* const bars = reinterpret_cast<uint64_t*>(slots + NPHI);
+  uint64_t* const bar = bars + team;
+  unsigned char* const own = reinterpret_cast<unsigned char*>(bars + ((teams + 1) & ~1)) + team * team_bytes(n_rot, NPHI, H);
+  float2* const F = reinterpret_cast<float2*>(own);               // [c][irot], columns of fcs values
+  float4* const EX = reinterpret_cast<float4*>(own);              // [reading warp][slot pair][lane], after F is consumed
+  if (lane == 0 && h == 0) mbar_init(bar, 1);
+  mbar_init_fence();
+  for (int k = threadIdx.x; k < 32 * (g.n_fwd + g.n_back); k += blockDim.x) mats[k] = g.frags[k];
+  for (int k = threadIdx.x; k < NPHI; k += blockDim.x) slots[k] = g.slots[k];
+  for (int k = h * 32 + lane; k < kCols * fcs; k += 32 * H) F[k] = make_float2(0.0f, 0.0f);
   __syncthreads();
+  const double* const mf = mats + lane;
+  const double* const mb = mats + 32 * g.n_fwd + lane;
 
-  const int fc = tid % PAIRS;
-  const int fq = (tid / PAIRS) % QUADS;
-  const int fg = tid / 16;
-  const int line_c = tid % CB;
-  const int line_t = tid / CB;
-  const int nt_table = g.nt_table;
+  const int c = lane >> 2, t = lane & 3;
   const int i0 = a.initial_channel;
-  const uint32_t col_bytes = static_cast<uint32_t>(n_rot * sizeof(V));
-  constexpr uint32_t row_bytes = NPHI * sizeof(V);
-  // The item's opt_z value, incoming amplitude chi(point) and (threads c < CB) sp2sc(column c), loaded
-  // when the item's copies are issued and used in its scaling phase.
-  T oz = 0;
-  V chi_in = cmake<V>(0, 0), sp_in = cmake<V>(0, 0), sp_lo = cmake<V>(0, 0);
-  V bq[2] = {cmake<V>(0, 0), cmake<V>(0, 0)};  // L2E: opt_r rot(dt/2) of irot tid and tid + NTH
-  V bql[2] = {cmake<V>(0, 0), cmake<V>(0, 0)};  // and their low parts
-  V sb = cmake<V>(1, 0);  // the item's opt_r (and its low part): the scale of its opt_r rot(dt/2) row (fmul_t)
-  const V one = cmake<V>(1, 0);
-  const long long n_scale = static_cast<long long>(a.nr) * n_rot;  // entries of the scaling tables
+  const uint32_t col_bytes = static_cast<uint32_t>(n_rot * sizeof(float2));
+  const int step = gridDim.x * teams;
 
-  auto item_columns = [&](long long item, int& izr, int& c0, int& ncol) {
-    izr = static_cast<int>(item / g.chunks);
-    c0 = static_cast<int>(item - static_cast<long long>(izr) * g.chunks) * CB;
-    ncol = min(CB, a.n_xy - c0);
-  };
-  // Every thread arrives on each barrier once per phase; the threads that copy announce their bytes.
-  // Threads c < ncol copy column c; in the staged form thread CB the opt_r rot(dt/2) row, thread CB + 1 the
-  // rot(dt/2) row (into R[parity]), CB + 2 its low parts, CB + 3 those of the opt_r rot(dt/2) row.
-  auto issue_psi = [&](long long item, int parity_r) {
-    int izr, c0, ncol;
-    item_columns(item, izr, c0, ncol);
-    const int ir = izr % a.nr;
-    if (tid < ncol) {
-      pot5::fence_proxy_async();
-      pot5::mbar_arrive_tx(bars, col_bytes + (tid == 0 ? g.extra_tx : 0u));
-      pot5::bulk_copy(F + tid * FCS, a.psi + (static_cast<long long>(izr) * a.n_xy + c0 + tid) * n_rot, col_bytes,
-                      bars);
-    } else if (!L2E && tid >= CB && tid <= CB + 3) {
-      pot5::fence_proxy_async();
-      pot5::mbar_arrive_tx(bars, col_bytes);
-      const long long row = static_cast<long long>(ir) * n_rot;
-      if (tid == CB)
-        pot5::bulk_copy(Bf, a.before + row, col_bytes, bars);
-      else if (tid == CB + 3)
-        pot5::bulk_copy(Bf + n_rot, a.before + n_scale + row, col_bytes, bars);
-      else if (tid == CB + 1)
-        pot5::bulk_copy(R + parity_r * 2 * n_rot, a.rot_half + row, col_bytes, bars);
-      else
-        pot5::bulk_copy(R + parity_r * 2 * n_rot + n_rot, a.rot_half + n_scale + row, col_bytes, bars);
-    } else {
-      pot5::mbar_arrive(bars);
-    }
-    if constexpr (L2E) {
-#pragma unroll
-      for (int u = 0; u < 2; ++u)
-        if (tid + u * NTH < n_rot) {
-          bq[u] = a.before[static_cast<long long>(ir) * n_rot + tid + u * NTH];
-          bql[u] = a.before[n_scale + static_cast<long long>(ir) * n_rot + tid + u * NTH];
-        }
-    }
-    oz = a.opt_z[izr / a.nr];
-    sb = a.before[2 * n_scale + static_cast<long long>(ir) * n_rot];
-    chi_in = a.chi[izr];
-    if (tid < ncol) {
-      sp_in = a.sp2sc[c0 + tid];
-      sp_lo = a.sp2sc[a.n_xy + c0 + tid];
-    }
-  };
-  auto issue_exp = [&](long long item) {
-    int izr, c0, ncol;
-    item_columns(item, izr, c0, ncol);
-    if constexpr (L2E) {  // column tid's rows (nt_table NPHI contiguous values) into L2
-      if (tid < ncol) {
-        const int ixy = c0 + tid;
-        const int rep = g.identity_maps ? ixy : __ldg(a.rep_of + ixy);
-        const long long e0 = (static_cast<long long>(izr) * a.n_rep + rep) * nt_table * NPHI;
-        pot5::prefetch_l2(a.expia + e0, static_cast<uint32_t>(nt_table * row_bytes));
-        // and the rows' modulus corrections (see exp_mul): 2 bytes per entry
-        if ((nt_table * NPHI) % 8 == 0) pot5::prefetch_l2(a.exp_mod + e0, static_cast<uint32_t>(nt_table * NPHI * 2));
+  // The columns of an item into F: one warp's lanes issue a bulk copy each (H = 2: warp 0), or every lane loads.
+  auto issue = [&](int item) {
+    const int col0 = item * kCols;
+    const int ncol = min(kCols, g.n_cols - col0);
+    if (g.bulk) {
+      if (h == 0) {
+        fence_proxy_async();
+        if (lane == 0) mbar_arrive_tx(bar, col_bytes * ncol + g.extra_tx);
+        __syncwarp();
+        if (lane < ncol) bulk_copy(F + lane * fcs, a.psi + static_cast<long long>(col0 + lane) * n_rot, col_bytes, bar);
       }
-      return;
-    }
-    if (line_c < ncol && line_t < nt_table) {
-      const int ixy = c0 + line_c;
-      const int rep = g.identity_maps ? ixy : __ldg(a.rep_of + ixy);
-      pot5::fence_proxy_async();
-      pot5::mbar_arrive_tx(bars + 1, row_bytes);
-      pot5::bulk_copy(E + tid * ERS, a.expia + ((static_cast<long long>(izr) * a.n_rep + rep) * nt_table + line_t) * NPHI,
-                      row_bytes, bars + 1);
     } else {
-      pot5::mbar_arrive(bars + 1);
+      for (int k = h * 32 + lane; k < ncol * n_rot; k += 32 * H) {
+        const int cc = k / n_rot;
+        F[cc * fcs + k - cc * n_rot] = a.psi[static_cast<long long>(col0) * n_rot + k];
+      }
     }
   };
-  // A bounded wait by every thread; true (for the whole block) when one of them gave up.
-  auto wait_failed = [&](uint64_t* bar, uint32_t parity) {
-    const bool ok = pot5::mbar_wait(bar, parity, g.poll_limit);
-    return __syncthreads_or(!ok) != 0;
-  };
-  // Phase parities (bit 0: F, bit 1: E) and copies issued but not yet waited for (same bits).
-  uint32_t parity = 0, pending = 0;
-  auto give_up = [&]() {
-    if (tid == 0) atomicExch(error_flag, 1);
-    // bounded waits for this block's copies in flight, so that none lands after the block has left
-    for (int k = 0; k < 2; ++k)
-      if (pending >> k & 1u) pot5::mbar_wait(bars + k, parity >> k & 1u, g.poll_limit);
+  // The columns, exp(i A) rows and corrections of an item into L2 (column c by one lane).
+  auto prefetch = [&](int item) {
+    const int col = item * kCols + lane;
+    if (h == 0 && lane < kCols && col < g.n_cols) {
+      const int izr = col / n_xy, ixy = col - izr * n_xy;
+      const long long e = (static_cast<long long>(izr) * a.n_rep + (g.phi_map ? __ldg(a.rep_of + ixy) : ixy)) * NPHI * g.pairs;
+      prefetch_l2(g.table + e, static_cast<uint32_t>(NPHI * g.pairs * sizeof(float4)));
+      const uint32_t mod_bytes = static_cast<uint32_t>(NPHI * g.pairs * sizeof(__half2));
+      if (mod_bytes % 16 == 0) prefetch_l2(g.mods + e, mod_bytes);
+      if (H == 2 && g.bulk) prefetch_l2(a.psi + static_cast<long long>(col) * n_rot, col_bytes);
+    }
   };
 
-  long long item = blockIdx.x;
-  int rp = 0;  // parity of the item count: the R row the current item reads
+  int item = blockIdx.x * teams + team;
+  uint32_t parity = 0;
   if (item < g.n_items) {
-    issue_psi(item, rp);
-    issue_exp(item);
-    pending = L2E ? 1u : 3u;
+    issue(item);
+    prefetch(item);
   }
-  for (; item < g.n_items; item += gridDim.x, rp ^= 1) {
-    int izr, c0, ncol;
-    item_columns(item, izr, c0, ncol);
-    const long long col_base = static_cast<long long>(izr) * a.n_xy + c0;
-    const int ir_item = izr % a.nr;
-    // rot(dt/2) at the item's r point, then its n_rot low parts
-    const V* rh_row = L2E ? a.rot_half + static_cast<long long>(ir_item) * n_rot : R + rp * 2 * n_rot;
-    const long long rh_lo = L2E ? n_scale : n_rot;
-    if (tid < CB) SP[tid] = cmul2(chi_in, sp_in, sp_lo);  // the previous item's scaling phase has read SP
-
-    // ---- wait for the columns and rows, scale the columns in place (absorbers, rot(dt/2), the
-    // specular wave into the initial channel)
-    if (wait_failed(bars, parity & 1u)) {
-      give_up();
+  for (; item < g.n_items; item += step) {
+    const bool ok = !g.bulk || mbar_wait(bar, parity, g.poll_limit);
+    if (team_any<H>(bar_id, !ok)) {
+      if (lane == 0 && h == 0) {
+        atomicExch(error_flag, 1);
+        mbar_wait(bar, parity, g.poll_limit);  // bounded: no copy lands after the team has left
+      }
       return;
     }
     parity ^= 1u;
-    pending &= ~1u;
-    // Two rotational states per pass, all their loads before the first store (the compiler cannot tell
-    // that the runtime-strided stores to F miss the later loads, and would otherwise serialise them).
-    {
-      const V rot_i0 = rh_row[i0], rot_i0_lo = rh_row[rh_lo + i0];
-      const V sbi = sb;
-      for (int ia = tid; ia < n_rot; ia += 2 * NTH) {
-        const int ib = ia + NTH;
-        const bool has_b = ib < n_rot;
-        const int irs[2] = {ia, has_b ? ib : ia};
-        V b[2], bl[2], v[2][CB];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          if constexpr (L2E) {
-            b[u] = ia == tid ? bq[u] : a.before[static_cast<long long>(ir_item) * n_rot + irs[u]];
-            bl[u] = ia == tid ? bql[u] : a.before[n_scale + static_cast<long long>(ir_item) * n_rot + irs[u]];
-          } else {
-            b[u] = Bf[irs[u]];
-            bl[u] = Bf[n_rot + irs[u]];
-          }
-#pragma unroll
-          for (int c = 0; c < CB; ++c) v[u][c] = F[c * FCS + irs[u]];
-        }
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          if (u == 1 && !has_b) break;
-          const bool at_i0 = irs[u] == i0;
-#pragma unroll
-          for (int c = 0; c < CB; ++c) {
-            V w = cmake<V>(0, 0);
-            if (c < ncol) {
-              w = cscale(fmul_parts(v[u][c], b[u], bl[u], sbi), oz);
-              if (at_i0) w = cadd(w, fmul_parts(SP[c], rot_i0, rot_i0_lo, one));  // the specular wave into the initial channel
-            }
-            F[c * FCS + irs[u]] = w;
-          }
-        }
-      }
-    }
-    __syncthreads();
-    const long long next = item + gridDim.x;
 
-    // ---- forward theta contraction
-    for (int s = 0; s < g.sched_len; ++s) {
-      const int slot = sched[fg * g.sched_len + s];
-      if (slot < 0) continue;
-      const int nj = s_nj[slot];
-      const int first = s_first[slot];
-      T acc[4][4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int r = 0; r < 4; ++r) acc[q][r] = 0;
-      const V* f0p = F + (2 * fc) * FCS + first;
-      const V* f1p = f0p + FCS;
-      const T* lp = L + first * LDL + 4 * fq;                 // the entries' 12-bit high parts
-      const T* lq = g.leg_rows_lo + first * LDL + 4 * fq;     // and the rest (through L1)
-      for (int j = 0; j < nj; ++j) {
-        T l[4], m[4];
-        ld4(lp + j * LDL, l);
-        ld4(lq + j * LDL, m);
-        const V f0 = f0p[j];
-        const V f1 = f1p[j];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          acc[q][0] = fmaf(l[q], f0.x, fmaf(m[q], f0.x, acc[q][0]));
-          acc[q][1] = fmaf(l[q], f0.y, fmaf(m[q], f0.y, acc[q][1]));
-          acc[q][2] = fmaf(l[q], f1.x, fmaf(m[q], f1.x, acc[q][2]));
-          acc[q][3] = fmaf(l[q], f1.y, fmaf(m[q], f1.y, acc[q][3]));
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        st2c(X + slot * SS + (fq + QUADS * q) * CB + 2 * fc, cmake<V>(acc[q][0], acc[q][1]),
-             cmake<V>(acc[q][2], acc[q][3]));
+    // ---- the item's columns: the specular wave into the initial channel (the absorbers and rot(dt/2) are in psi)
+    const int col = item * kCols + c;
+    const bool col_ok = col < g.n_cols;
+    const int izr = min(col, g.n_cols - 1) / n_xy, ixy = min(col, g.n_cols - 1) - izr * n_xy;
+    const int ir = izr % nr;
+    if (!col_ok) {
+      for (int j = h * 4 + t; j < n_rot; j += 4 * H) F[c * fcs + j] = make_float2(0.0f, 0.0f);
+    } else if (h == 0 && t == 0) {
+      const float2 chi = a.chi[izr], s = a.sp2sc[ixy], sl = a.sp2sc[n_xy + ixy];
+      const double2 r0 = g.rot[ir * n_rot + i0];
+      const double sx = static_cast<double>(s.x) + sl.x, sy = static_cast<double>(s.y) + sl.y;
+      const double ux = sx * chi.x - sy * chi.y, uy = sx * chi.y + sy * chi.x;
+      float2* const v = F + c * fcs + i0;
+      *v = make_float2(static_cast<float>(v->x + (ux * r0.x - uy * r0.y)), static_cast<float>(v->y + (ux * r0.y + uy * r0.x)));
     }
-    __syncthreads();
-    // the next item's columns (every thread has finished reading F)
-    if (next < g.n_items) {
-      issue_psi(next, rp ^ 1);
-      pending |= 1u;
-    }
+    team_sync<H>(bar_id);
 
-    // ---- phi transform, exp(i A), inverse phi transform
-    if constexpr (L2E) {
-      if (line_c < ncol && line_t < nt_table) {  // padding lines (theta >= nt_table) hold zeros
-        const int ixy = c0 + line_c;
-        const int rep = g.identity_maps ? ixy : __ldg(a.rep_of + ixy);
-        const long long e0 = ((static_cast<long long>(izr) * a.n_rep + rep) * nt_table + line_t) * NPHI;
-        const V* eg = a.expia + e0;
-        V* xl = X + line_t * CB + line_c;
-        V x[NPHI];
-        if (g.identity_maps) {
-          V e[NPHI];  // this line's row from L2, requested before the transform
-          static_for<0, NPHI / 2>([&](auto h) {
-            constexpr int P = 2 * SPO_CV(h);
-            const float4 q = __ldg(reinterpret_cast<const float4*>(eg + P));
-            e[P] = cmake<V>(q.x, q.y);
-            e[P + 1] = cmake<V>(q.z, q.w);
-          });
-          if constexpr (sizeof(T) == 4 && NPHI % 8 == 0) {  // the row's corrections, 16 bytes per load
-            uint32_t mw[NPHI / 2];
-            static_for<0, NPHI / 8>([&](auto h) {
-              const uint4 q = __ldg(reinterpret_cast<const uint4*>(a.exp_mod + e0) + SPO_CV(h));
-              mw[4 * SPO_CV(h)] = q.x;
-              mw[4 * SPO_CV(h) + 1] = q.y;
-              mw[4 * SPO_CV(h) + 2] = q.z;
-              mw[4 * SPO_CV(h) + 3] = q.w;
-            });
-            static_for<0, NPHI>([&](auto p) { x[SPO_CV(p)] = xl[SPO_CV(p) * SS]; });
-            rdft<NPHI, +1>(x);
-            static_for<0, NPHI / 2>([&](auto h) {
-              constexpr int P = 2 * SPO_CV(h);
-              x[P] = exp_mul_m(x[P], e[P], mod_lo(mw[SPO_CV(h)]));
-              x[P + 1] = exp_mul_m(x[P + 1], e[P + 1], mod_hi(mw[SPO_CV(h)]));
-            });
-          } else {
-            static_for<0, NPHI>([&](auto p) { x[SPO_CV(p)] = xl[SPO_CV(p) * SS]; });
-            rdft<NPHI, +1>(x);
-            static_for<0, NPHI>([&](auto p) { x[SPO_CV(p)] = exp_mul(x[SPO_CV(p)], e[SPO_CV(p)], a.exp_mod, e0 + SPO_CV(p)); });
-          }
-        } else {
-          const int* map = a.phi_map + ixy * NPHI;
-          static_for<0, NPHI>([&](auto p) { x[SPO_CV(p)] = xl[SPO_CV(p) * SS]; });
-          rdft<NPHI, +1>(x);
-          static_for<0, NPHI>([&](auto p) {
-            const int pm = __ldg(map + SPO_CV(p));
-            x[SPO_CV(p)] = exp_mul(x[SPO_CV(p)], eg[pm], a.exp_mod, e0 + pm);
-          });
-        }
-        rdft<NPHI, -1>(x);
-        static_for<0, NPHI>([&](auto p) { xl[SPO_CV(p) * SS] = x[SPO_CV(p)]; });
-      }
-    } else {
-    if (wait_failed(bars + 1, parity >> 1 & 1u)) {
-      give_up();
-      return;
-    }
-    parity ^= 2u;
-    pending &= ~2u;
-    if (line_c < ncol && line_t < nt_table) {  // padding lines (theta >= nt_table) hold zeros
-      const int ixy = c0 + line_c;
-      V* xl = X + line_t * CB + line_c;
-      const V* el = E + tid * ERS;
-      const int rep = g.identity_maps ? ixy : __ldg(a.rep_of + ixy);
-      const long long e0 = ((static_cast<long long>(izr) * a.n_rep + rep) * nt_table + line_t) * NPHI;
-      V x[NPHI];
-      static_for<0, NPHI>([&](auto p) { x[SPO_CV(p)] = xl[SPO_CV(p) * SS]; });
-      rdft<NPHI, +1>(x);
-      if (g.identity_maps) {
-        static_for<0, NPHI / 2>([&](auto h) {
-          constexpr int P = 2 * SPO_CV(h);
-          V ea, eb;
-          ld2c(el + P, ea, eb);
-          x[P] = exp_mul(x[P], ea, a.exp_mod, e0 + P);
-          x[P + 1] = exp_mul(x[P + 1], eb, a.exp_mod, e0 + P + 1);
-        });
-      } else {
-        const int* map = a.phi_map + ixy * NPHI;
-        static_for<0, NPHI>([&](auto p) {
-          const int pm = __ldg(map + SPO_CV(p));
-          x[SPO_CV(p)] = exp_mul(x[SPO_CV(p)], el[pm], a.exp_mod, e0 + pm);
-        });
-      }
-      rdft<NPHI, -1>(x);
-      static_for<0, NPHI>([&](auto p) { xl[SPO_CV(p) * SS] = x[SPO_CV(p)]; });
-    }
-    }
-    __syncthreads();
-    // the next item's exp(i A) rows (every thread has read its row of this item)
-    if (next < g.n_items) {
-      issue_exp(next);
-      if (!L2E) pending |= 2u;
-    }
-
-    // ---- transposed theta contraction, rot(dt/2), store: two rotational states per pass (irot and
-    // irot + NTH), their sums interleaved as independent chains
-    for (int ia = tid; ia < n_rot; ia += 2 * NTH) {
-      const int ib = ia + NTH;
-      const bool has_b = ib < n_rot;
-      const int ibb = has_b ? ib : ia;
-      const V rh[2] = {rh_row[ia], rh_row[ibb]}, rhl[2] = {rh_row[rh_lo + ia], rh_row[rh_lo + ibb]};
-      T acc[2][CB][2];
-#pragma unroll
-      for (int u = 0; u < 2; ++u)
-#pragma unroll
-        for (int c = 0; c < CB; ++c) acc[u][c][0] = acc[u][c][1] = 0;
-      const V* ys[2] = {X + irot_slot[ia] * SS, X + irot_slot[ibb] * SS};
-      const T* lrow[2] = {L + ia * LDL, L + ibb * LDL};                          // 12-bit high parts
-      const T* lrest[2] = {g.leg_rows_lo + ia * LDL, g.leg_rows_lo + ibb * LDL};  // the rest, through L1
+    // ---- forward contraction, two slots at a time (p and nphi - p, usually of equal J count)
+    C2 x[NPHI];  // the lane's two phi lines: theta 8 h + 2 t and 8 h + 2 t + 1
+    const float2* const fl = F + c * fcs + t;
+    static_for<0, NPHI / 2>([&](auto q) {
+      constexpr int PA = SPO_CV(q) == 0 ? 0 : SPO_CV(q);
+      constexpr int PB = SPO_CV(q) == 0 ? NPHI / 2 : NPHI - SPO_CV(q);
+      const int4 sa = slots[PA], sb = slots[PB];
+      const int nk = sa.y >> 16;  // the same for both (the shorter block's fragments end in zeros)
+      double ar0 = 0, ar1 = 0, ai0 = 0, ai1 = 0, br0 = 0, br1 = 0, bi0 = 0, bi1 = 0;
+      const float2 *fa = fl + sa.x, *fb = fl + sb.x;
+      const double *ma = mf + 32 * (sa.z + h * nk), *mc = mf + 32 * (sb.z + h * nk);
 #pragma unroll 1
-      for (int kq = 0; kq < QUADS; ++kq) {
-        T l[2][4], m[2][4];
-        ld4(lrow[0] + 4 * kq, l[0]);
-        ld4(lrow[1] + 4 * kq, l[1]);
-        ld4(lrest[0] + 4 * kq, m[0]);
-        ld4(lrest[1] + 4 * kq, m[1]);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-#pragma unroll
-          for (int c = 0; c < CB; c += 2) {
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-              V y0, y1;
-              ld2c(ys[u] + (kq + QUADS * q) * CB + c, y0, y1);
-              acc[u][c][0] = fmaf(l[u][q], y0.x, fmaf(m[u][q], y0.x, acc[u][c][0]));
-              acc[u][c][1] = fmaf(l[u][q], y0.y, fmaf(m[u][q], y0.y, acc[u][c][1]));
-              acc[u][c + 1][0] = fmaf(l[u][q], y1.x, fmaf(m[u][q], y1.x, acc[u][c + 1][0]));
-              acc[u][c + 1][1] = fmaf(l[u][q], y1.y, fmaf(m[u][q], y1.y, acc[u][c + 1][1]));
-            }
-          }
+      for (int k = 0; k < nk; ++k) {
+        const float2 u = fa[4 * k];
+        const double m = ma[32 * k];
+        dmma(ar0, ar1, u.x, m);
+        dmma(ai0, ai1, u.y, m);
+        if constexpr (SPO_CV(q) != 0) {
+          const float2 v = fb[4 * k];
+          const double n = mc[32 * k];
+          dmma(br0, br1, v.x, n);
+          dmma(bi0, bi1, v.y, n);
         }
       }
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int irot = u == 0 ? ia : ib;
-        if (u == 1 && !has_b) break;
-#pragma unroll
-        for (int c = 0; c < CB; ++c)
-          if (c < ncol) a.psi[(col_base + c) * n_rot + irot] = fmul_parts(cmake<V>(acc[u][c][0], acc[u][c][1]), rh[u], rhl[u], one);
-      }
+      x[PA] = c2(f2(static_cast<float>(ar0), static_cast<float>(ar1)), f2(static_cast<float>(ai0), static_cast<float>(ai1)));
+      x[PB] = c2(f2(static_cast<float>(br0), static_cast<float>(br1)), f2(static_cast<float>(bi0), static_cast<float>(bi1)));
+    });
+    team_sync<H>(bar_id);
+    const int next = item + step;
+    if (next < g.n_items) {
+      if (H == 1) issue(next);  // every lane of the team has read F
+      prefetch(next);
     }
+
+    // ---- phi transform, exp(i A), inverse phi transform of the lane's two lines
+    rdft<NPHI, +1>(x);
+    {
+      const int tp = min(4 * h + t, g.pairs - 1);  // theta beyond the grid: zero lines
+      const long long e = (static_cast<long long>(izr) * a.n_rep + (g.phi_map ? __ldg(a.rep_of + ixy) : ixy)) * NPHI * g.pairs;
+      const float4* et = g.table + e + tp;
+      const __half2* em = g.mods + e + tp * G;
+      // Two phi per batch, the next batch's loads in flight while one is applied. The empty asm statements tie a batch's
+      // address to values of the batch before the last, so that the compiler does not collect all loads in front (and
+      // spill the lines to make room for them).
+      constexpr int NB = NPHI / 2;
+      float4 w[2][2];
+      uint32_t m2[2][2];
+      auto load = [&](auto b) {
+        constexpr int P = 2 * SPO_CV(b), U = SPO_CV(b) % 2;
+        if (g.phi_map == nullptr) {
+          const uint2 m = ld_stream2(em + (P / G) * G * g.pairs + P % G);
+          m2[U][0] = m.x;
+          m2[U][1] = m.y;
+          w[U][0] = ld_stream4(et + P * g.pairs);
+          w[U][1] = ld_stream4(et + (P + 1) * g.pairs);
+        } else {
+          const uint8_t* map = g.phi_map + ixy * NPHI;
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const int pm = __ldg(map + P + i);
+            m2[U][i] = __ldg(reinterpret_cast<const uint32_t*>(em + (pm / G) * G * g.pairs + pm % G));
+            w[U][i] = ld_stream4(et + pm * g.pairs);
+          }
+        }
+      };
+      auto apply = [&](auto p, float4 e4, uint32_t m2) {  // exp_mul_m on both lines
+        const F2 m = f2(mod_lo(m2), mod_hi(m2)) * f2(5.9604644775390625e-8f);  // 2^-24
+        const C2 e = c2(f2(e4.x, e4.y), f2(e4.z, e4.w));
+        x[p] = cadd(x[p], cmul2(x[p], e, c2(m * (f2(1.0f) + e.x), m * e.y)));
+      };
+      asm volatile("" : "+l"(et), "+l"(em), "+l"(x[NPHI - 1].x.v));
+      load(std::integral_constant<int, 0>{});
+      static_for<0, NB>([&](auto b) {
+        constexpr int B = SPO_CV(b), U = B % 2;
+        if constexpr (B + 1 < NB) load(std::integral_constant<int, B + 1>{});
+        apply(std::integral_constant<int, 2 * B>{}, w[U][0], m2[U][0]);
+        apply(std::integral_constant<int, 2 * B + 1>{}, w[U][1], m2[U][1]);
+        asm volatile("" : "+l"(et), "+l"(em), "+l"(x[2 * B + 1].y.v));
+      });
+    }
+    rdft<NPHI, -1>(x);
+
+    // ---- transposed contraction, rot(dt/2), store
+    float2* const out = a.psi + static_cast<long long>(col) * n_rot;
+    const double2* const rot = g.rot + ir * n_rot;
+    auto finish = [&](int irot, double2 w, double re, double im) {
+      out[irot] = make_float2(static_cast<float>(re * w.x - im * w.y), static_cast<float>(re * w.y + im * w.x));
+    };
+    // One slot: the warp's own theta in v[0..3], the other warp's in v[4..7].
+    auto back = [&](int p, const double (&v)[4 * H]) {
+      const int4 s = slots[p];
+      const int nj = s.y & 0xffff;
+#pragma unroll 1
+      for (int jt = 0; 8 * jt < nj; ++jt) {
+        const double* const m0 = mb + 32 * (s.w + (jt * H + h) * 2);
+        const double* const m1 = mb + 32 * (s.w + (jt * H + H - 1 - h) * 2);
+        const int j = 8 * jt + t;
+        const double2 wa = __ldg(rot + s.x + min(j, nj - 1)), wb = __ldg(rot + s.x + min(j + 4, nj - 1));
+        double r0 = 0, r1 = 0, q0 = 0, q1 = 0;
+#pragma unroll
+        for (int i = 0; i < 2 * H; ++i) {
+          const double w = (i < 2 ? m0 : m1)[32 * (i % 2)];
+          dmma(r0, r1, v[2 * i], w);
+          dmma(q0, q1, v[2 * i + 1], w);
+        }
+        if (col_ok) {
+          if (j < nj) finish(s.x + j, wa, r0, q0);
+          if (j + 4 < nj) finish(s.x + j + 4, wb, r1, q1);
+        }
+      }
+    };
+    if constexpr (H == 1) {
+      static_for<0, NPHI>([&](auto p) {
+        float2 u, w;
+        c2_split(x[p], u, w);
+        const double v[4] = {u.x, u.y, w.x, w.y};
+        back(SPO_CV(p), v);
+      });
+    } else {
+      // Warp h takes the slots 2 q + h: it keeps its own theta of them and gets the other warp's through F.
+      float4* const to = EX + (h ^ 1) * (NPHI / 2) * 32 + lane;
+      const float4* const from = EX + h * (NPHI / 2) * 32 + lane;
+      float4 mine[NPHI / 2];
+      static_for<0, NPHI / 2>([&](auto q) {
+        float2 e0, e1, o0, o1;
+        c2_split(x[2 * SPO_CV(q)], e0, e1);
+        c2_split(x[2 * SPO_CV(q) + 1], o0, o1);
+        const float4 xe = make_float4(e0.x, e0.y, e1.x, e1.y), xo = make_float4(o0.x, o0.y, o1.x, o1.y);
+        to[SPO_CV(q) * 32] = h == 0 ? xo : xe;
+        mine[SPO_CV(q)] = h == 0 ? xe : xo;
+      });
+      team_sync<H>(bar_id);
+      static_for<0, NPHI / 2>([&](auto q) {
+        const float4 z = mine[SPO_CV(q)], y = from[SPO_CV(q) * 32];
+        const double v[8] = {z.x, z.y, z.z, z.w, y.x, y.y, y.z, y.w};
+        back(2 * SPO_CV(q) + h, v);
+      });
+      team_sync<H>(bar_id);
+      // the zeros behind the columns again, then the next item's columns
+      if (h == 0) F[c * fcs + n_rot + t] = make_float2(0.0f, 0.0f);
+      if (next < g.n_items) issue(next);
+    }
+    if (!g.bulk) team_sync<H>(bar_id);
+  }
+}
+
+namespace pot5 {
+
+// The instantiation for (nphi, H), or null (spo_pot5.cu, one translation unit per part).
+using Kernel = void (*)(Pot5Args, int*);
+template <int PART>
+Kernel kernel_of_part(int nphi, int h);
+template <> Kernel kernel_of_part<0>(int nphi, int h);
+template <> Kernel kernel_of_part<1>(int nphi, int h);
+template <> Kernel kernel_of_part<2>(int nphi, int h);
+template <> Kernel kernel_of_part<3>(int nphi, int h);
+template <> Kernel kernel_of_part<4>(int nphi, int h);
+template <> Kernel kernel_of_part<5>(int nphi, int h);
+inline Kernel kernel_for(int nphi, int h) {
+  Kernel k = nullptr;
+  for (Kernel (*part)(int, int) : {kernel_of_part<0>, kernel_of_part<1>, kernel_of_part<2>, kernel_of_part<3>,
+                                   kernel_of_part<4>, kernel_of_part<5>})
+    if (!k) k = part(nphi, h);
+  return k;
+}
+// Dynamic shared memory of a block of `teams` teams: matrix fragments, slots, barriers, per team F and exchange.
+inline std::size_t smem_bytes(int n_rot, int nphi, int h, int frags, int teams) {
+  return 256u * static_cast<std::size_t>(frags) + sizeof(int4) * static_cast<std::size_t>(nphi) +
+         8u * static_cast<std::size_t>((teams + 1) & ~1) + teams * team_bytes(n_rot, nphi, h);
+}
+
+}  // namespace pot5
+
+// exp(i A) - 1 and the modulus corrections (exp_potential_kernel) in the order of potential5, from n_reps blocks of
+// ntheta x nphi values of V, phi fastest.
+static __global__ void exp_pairs_kernel(const double* __restrict__ v, float4* __restrict__ table, __half2* __restrict__ mods,
+                                        long long n_reps, int n_theta, int n_phi, int pairs, int group, double dt) {
+  const long long n = n_reps * n_phi * pairs;
+  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
+       i += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const int tp = static_cast<int>(i % pairs);
+    const long long q = i / pairs;
+    const int p = static_cast<int>(q % n_phi);
+    const long long rep = q / n_phi;
+    float2 g[2];
+    __half m[2];
+    for (int k = 0; k < 2; ++k) {
+      const int th = 2 * tp + k;
+      g[k] = make_float2(0.0f, 0.0f);
+      m[k] = __float2half(0.0f);
+      if (th < n_theta) exp_entry(v[(rep * n_theta + th) * n_phi + p], dt, g[k], m[k]);
+    }
+    table[i] = make_float4(g[0].x, g[1].x, g[0].y, g[1].y);
+    mods[rep * n_phi * pairs + (p / group) * group * pairs + tp * group + p % group] = __halves2half2(m[0], m[1]);
   }
 }
 
