@@ -23,6 +23,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <limits>
+#include <map>
 #include <memory>
 #include <mutex>
 #include <stdexcept>
@@ -36,6 +37,7 @@
 #include "spo_pot5.cuh"
 #include "spo_pot6.cuh"
 #include "spo_persist.cuh"
+#include "spo_kin.cuh"
 
 namespace spo_host {
 
@@ -225,6 +227,37 @@ template <typename T>
 void launch_pot3(int nphi, const spo::Pot2Args<T>& a, dim3 grid, unsigned threads, std::size_t smem, cudaStream_t stream);
 template <typename T>
 Pot4Kernel<T> pot4_kernel_for(int nphi, int nt);
+
+// A launch of kin_kernel (spo_kin.cuh): the instantiation for (map, n1, n2), or the one for any sizes, with its block.
+template <typename T>
+struct KinLaunch {
+  void (*kernel)(spo::KinArgs<T>) = nullptr;
+  int threads = 0, log_lines = 0;
+  long long blocks = 0;  // resident blocks of the device
+  std::size_t smem = 0;
+};
+template <typename T>
+KinLaunch<T> kin_configure(int map, int n1, int n2, int lanes_per_tile, long long window);
+
+// The levels of kin_kernel for an axis of n points, false if it has none: two coprime sizes up to 16 (no twiddles), else
+// any two.
+inline bool kin_split(int n, bool prime, int& map, int& n1, int& n2) {
+  auto size_ok = [](int k) { return k >= 2 && k <= 16 && k != 13; };
+  for (const bool coprime : {true, false}) {
+    if (coprime && !prime) continue;
+    for (int b = 16; b >= 2; --b) {  // the most balanced split: the smallest larger factor
+      const int larger = 18 - b;
+      if (n % larger != 0 || !size_ok(larger) || !size_ok(n / larger) || n / larger > larger) continue;
+      int x = larger, y = n / larger;
+      while (y) std::swap(x %= y, y);
+      if (coprime && x != 1) continue;
+      map = coprime ? spo::kPrime : spo::kTwiddle, n1 = n / larger, n2 = larger;
+      return true;
+    }
+  }
+  return false;
+}
+inline bool kin_xy_size(int n) { return n >= 1 && n <= 16 && n != 13; }
 
 inline bool pot2_phi_supported(int nphi) {
   switch (nphi) {
@@ -418,6 +451,16 @@ template <typename T>
 class Step final : public StepBase {
   using V = spo::Vec<T>;
 
+  // kin_kernel on one axis: its levels (map < 0: not used), tables and scales of the full and the half step, launch
+  // shapes by (lanes per tile, lanes).
+  struct KinAxis {
+    int map = -1, n1 = 0, n2 = 0;
+    double2* table[2] = {nullptr, nullptr};
+    T scale[2] = {T(1), T(1)};
+    int unit[2] = {1, 1};
+    std::map<std::pair<int, long long>, KinLaunch<T>> launches;
+  };
+
  public:
   Step(const spo_desc& d, const Sizes& s, cudaStream_t stream) : s_(s), stream_(stream), own_stream_(stream) {
     build(d);
@@ -463,7 +506,9 @@ class Step final : public StepBase {
 
   std::string describe() const override {
     auto lanes = [](int tile, bool has_tiles) { return "tb" + std::to_string(!has_tiles ? 32 : tile ? tile : 16); };
-    auto axis_name = [&](int n, int tile, bool persistent) {
+    auto axis_name = [&](int n, int tile, bool persistent, const KinAxis& kin) {
+      if (kin.map >= 0 && !axis2_supported(n))
+        return "kin<" + std::to_string(n) + "=" + std::to_string(kin.n1) + "x" + std::to_string(kin.n2) + ">";
       if (!(use_v2_ && axis2_supported(n))) return std::string("axis_pass(general)");
       int n1 = 0, n2 = 0;
       if (use_pfa_ && !persistent && pfa_split(n, n1, n2))
@@ -472,8 +517,8 @@ class Step final : public StepBase {
       return form + std::string("<") + std::to_string(n) + "," + lanes(tile, axis2_has_tiles(n)) + ">";
     };
     std::string out = std::string(sizeof(T) == 8 ? "fp64" : "mixed");
-    out += " z=" + axis_name(s_.nz, tile_z_, persist_z_);
-    out += " r=" + axis_name(s_.nr, tile_r_, persist_r_);
+    out += " z=" + axis_name(s_.nz, tile_z_, persist_z_, kin_z_);
+    out += " r=" + axis_name(s_.nr, tile_r_, persist_r_, kin_r_);
     const bool xy2 = use_v2_ && s_.nx == s_.ny && xy2_supported(s_.nx);
     out += std::string(" xy=") + (xy2 ? std::string(persist_xy_ ? "xy2p<" : "xy2<") + std::to_string(s_.nx) + "," + lanes(tile_xy_, s_.nx > 8) + ">"
                                       : std::string("xy_pass(general)"));
@@ -786,11 +831,15 @@ class Step final : public StepBase {
     const long long plane = static_cast<long long>(s_.nr) * s_.n_xy() * s_.n_rot;
     for (int iz0 = 0; iz0 < s_.nz; iz0 += rxy_planes_) {
       const int g = std::min(rxy_planes_, s_.nz - iz0);
-      spo::Axis2Args<T> r{psi_ + plane * iz0, s_.n_xy() * s_.n_rot, half ? rk_half_ : rk_full_, tw_r_, tile_r_};
-      r.factor_pfa = pfa_of(r.factor);
-      r.persistent = persist_r_ ? 1 : 0;
       prof_.begin(stream_);
-      launch_axis2<T>(plan_r_.n, r, g, stream_);
+      if (kin_r_.map >= 0) {
+        kin_axis(kin_r_, half, tile_r_, psi_ + plane * iz0, s_.n_xy() * s_.n_rot, g, 1, 0, 0, s_.n_xy() * s_.n_rot);
+      } else {
+        spo::Axis2Args<T> r{psi_ + plane * iz0, s_.n_xy() * s_.n_rot, half ? rk_half_ : rk_full_, tw_r_, tile_r_};
+        r.factor_pfa = pfa_of(r.factor);
+        r.persistent = persist_r_ ? 1 : 0;
+        launch_axis2<T>(plan_r_.n, r, g, stream_);
+      }
       prof_.end(stream_, "kinetic_r", 2.0 * sizeof(V) * plane * g);
       ++launches_;
       kinetic_xy(half, with_gas, static_cast<long long>(iz0) * s_.nr, static_cast<long long>(g) * s_.nr);
@@ -833,7 +882,8 @@ class Step final : public StepBase {
       z.line_stride = static_cast<long long>(s_.nr) * lanes;
       z.outer_stride = 0;
       prof_.begin(stream_);
-      launch_axis2<T>(plan_z_.n, z, 1, stream_);
+      if (kin_z_.map >= 0) kin_axis(kin_z_, half, tile_z_, psi_, static_cast<long long>(s_.nr) * lanes, 1, s_.nr, lanes, l0, w);
+      else launch_axis2<T>(plan_z_.n, z, 1, stream_);
       prof_.end(stream_, "kinetic_z", bw);
       ++launches_;
       spo::Axis2Args<T> r{psi_, 0, rf, tw_r_, tile_r_};
@@ -845,7 +895,8 @@ class Step final : public StepBase {
       r.line_stride = lanes;
       r.outer_stride = static_cast<long long>(s_.nr) * lanes;  // block y = iz
       prof_.begin(stream_);
-      launch_axis2<T>(plan_r_.n, r, s_.nz, stream_);
+      if (kin_r_.map >= 0) kin_axis(kin_r_, half, tile_r_, psi_, lanes, s_.nz, 1, 0, l0, w);
+      else launch_axis2<T>(plan_r_.n, r, s_.nz, stream_);
       prof_.end(stream_, "kinetic_r", bw);
       ++launches_;
     }
@@ -862,8 +913,49 @@ class Step final : public StepBase {
     if (factor == rk_half_) return rk_half_pfa_;
     return nullptr;
   }
+  // kin_kernel along an axis of `data`: points `stride` apart, `outer` consecutive line sets, lanes as KinArgs has them.
+  void kin_axis(KinAxis& ax, bool half, int tile, V* data, long long stride, long long outer, long long groups,
+                long long group_stride, long long lane_offset, long long window) {
+    spo::KinArgs<T> a{};
+    a.data = data;
+    a.stride = stride;
+    a.outer_stride = stride * ax.n1 * ax.n2;
+    a.group_stride = group_stride;
+    a.lane_offset = lane_offset;
+    a.window = window;
+    a.groups = static_cast<unsigned>(groups);
+    kin_launch(ax, half, tile, a, outer);
+  }
+  void kin_launch(KinAxis& ax, bool half, int tile, spo::KinArgs<T>& a, long long outer) {
+    const int lanes = tile > 0 ? tile : ax.n1 * ax.n2 >= 80 ? 16 : 32;
+    auto it = ax.launches.find({lanes, a.window});
+    if (it == ax.launches.end())
+      it = ax.launches.emplace(std::make_pair(lanes, a.window), kin_configure<T>(ax.map, ax.n1, ax.n2, lanes, a.window)).first;
+    const KinLaunch<T>& l = it->second;
+    const long long per_tile = static_cast<long long>(spo::KinLine<T>::lanes) << l.log_lines;
+    const long long blocks_per_group = (a.window + per_tile - 1) / per_tile, n_tiles = blocks_per_group * a.groups * outer;
+    require(n_tiles < (1ll << 32), "kinetic pass: too many tiles");
+    a.n1 = ax.n1;
+    a.n2 = ax.n2;
+    a.blocks_per_group = static_cast<unsigned>(blocks_per_group);
+    a.n_tiles = static_cast<unsigned>(n_tiles);
+    a.log_lines = l.log_lines;
+    a.aligned = (a.stride | a.outer_stride | a.group_stride | a.lane_offset | (a.data - psi_)) % 2 == 0 ? 1 : 0;
+    a.table = ax.table[half];
+    a.scale = ax.scale[half];
+    a.unit = ax.unit[half];
+    l.kernel<<<static_cast<unsigned>(std::min(n_tiles, l.blocks)), l.threads, l.smem, stream_>>>(a);
+  }
   void axis_psi(const char* name, double bytes, long long outer, const spo::FftPlan& plan, const V* tw,
                 long long inner, const V* factor, int tile, bool persistent = false, bool balanced = false) {
+    KinAxis& kin = factor == zk_full_ || factor == zk_half_ ? kin_z_ : kin_r_;
+    if (kin.map >= 0) {
+      prof_.begin(stream_);
+      kin_axis(kin, factor == zk_half_ || factor == rk_half_, tile, psi_, inner, outer, 1, 0, 0, inner);
+      prof_.end(stream_, name, bytes);
+      ++launches_;
+      return;
+    }
     if (use_v2_ && axis2_supported(plan.n)) {
       spo::Axis2Args<T> a{psi_, inner, factor, tw, tile};
       a.factor_pfa = pfa_of(factor);
@@ -902,6 +994,22 @@ class Step final : public StepBase {
     x.before = pot_kind_ == 5 ? before_ : nullptr;
     x.tile = tile_xy_;
     x.persistent = persist_xy_ ? 1 : 0;
+    if (kin_xy_.map >= 0) {
+      const long long n = n_izr >= 0 ? n_izr : s_.n_zr();
+      spo::KinArgs<T> a{};
+      a.data = psi_ + izr_first * s_.n_xy() * s_.n_rot;
+      a.stride = s_.n_rot;
+      a.outer_stride = s_.n_xy() * s_.n_rot;
+      a.window = s_.n_rot;
+      a.groups = 1;
+      x.izr_offset = izr_first;
+      a.xy = x;
+      prof_.begin(stream_);
+      kin_launch(kin_xy_, half, tile_xy_ > 0 ? tile_xy_ : s_.nx > 8 || s_.ny > 8 ? 16 : 32, a, n);
+      prof_.end(stream_, "kinetic_xy", 2.0 * sizeof(V) * n * s_.n_xy() * s_.n_rot);
+      ++launches_;
+      return;
+    }
     if (n_izr >= 0) {
       x.izr_offset = izr_first;
       prof_.begin(stream_);
@@ -1195,6 +1303,47 @@ class Step final : public StepBase {
       return upload_complex(f);
     }
   }
+  // kin_kernel's table for an axis (KinArgs::table): the factors in the order of its levels (s e^{i phi} as p (1 + g) r with
+  // p the power of two below the first factor's s and r = s / p), then the twiddles.
+  void kin_table(KinAxis& ax, int half, const std::vector<cplx>& natural) {
+    const int n = ax.n1 * ax.n2;
+    const std::vector<cplx> f = ax.map == spo::kPrime ? pfa_order(natural, ax.n1, ax.n2) : natural;
+    const std::vector<cplx> tw = ax.map == spo::kTwiddle ? twiddles(n) : std::vector<cplx>();
+    ax.scale[half] = T(1);
+    ax.unit[half] = 1;
+    if constexpr (sizeof(T) == 8) {
+      std::vector<cplx> t = f;
+      t.insert(t.end(), tw.begin(), tw.end());
+      ax.table[half] = upload_c128(t);
+    } else {
+      const double s0 = std::abs(f[0]);
+      double p = 1.0;
+      if (std::isfinite(s0) && s0 > 1e-30 && s0 < 1e30) p = std::exp2(std::floor(std::log2(s0) + 1e-9));
+      std::vector<float> h(static_cast<std::size_t>(12 * n));
+      auto put = [&](std::size_t word, double x, double y) {
+        h[4 * word] = h[4 * word + 1] = static_cast<float>(x);
+        h[4 * word + 2] = h[4 * word + 3] = static_cast<float>(y);
+      };
+      for (int k = 0; k < n; ++k) {
+        const double s = std::abs(f[k]), r = s / p;
+        const cplx g = s > 0.0 ? cplx(p * (f[k].real() / s - 1.0), p * (f[k].imag() / s)) : cplx(-p, 0.0);
+        put(2 * k, g.real(), g.imag());
+        put(2 * k + 1, g.real() - static_cast<float>(g.real()), g.imag() - static_cast<float>(g.imag()));
+        put(2 * static_cast<std::size_t>(n) + k, r, r - static_cast<float>(r));
+        if (!(std::fabs(r - 1.0) < 1e-14)) ax.unit[half] = 0;  // rounding of |s e^{i phi}| in FP64
+      }
+      ax.scale[half] = static_cast<float>(p);
+      h.resize(12 * static_cast<std::size_t>(n) + 8 * tw.size());
+      for (std::size_t k = 0; k < tw.size(); ++k) {
+        put(3 * static_cast<std::size_t>(n) + 2 * k, tw[k].real(), tw[k].imag());
+        put(3 * static_cast<std::size_t>(n) + 2 * k + 1, tw[k].real() - static_cast<float>(tw[k].real()),
+            tw[k].imag() - static_cast<float>(tw[k].imag()));
+      }
+      double2* d = dev<double2>(h.size() / 4);
+      check_cuda(cudaMemcpy(d, h.data(), sizeof(float) * h.size(), cudaMemcpyHostToDevice), "upload table");
+      ax.table[half] = d;
+    }
+  }
   T* upload_real_lo(const std::vector<double>& v, const std::vector<double>& exact) {
     if constexpr (sizeof(T) == 4) {
       std::vector<double> both(2 * v.size());
@@ -1272,6 +1421,25 @@ class Step final : public StepBase {
     const double xy_scale = (sx * sy) * ((1.0 / (s.nx * sx)) * (1.0 / (s.ny * sy)));
     xyk_full_ = upload_factor(scaled(complex_array(d.xy_kinetic_full, nxy, "xy_kinetic_full"), xy_scale));
     xyk_half_ = upload_factor(scaled(complex_array(d.xy_kinetic_half, nxy, "xy_kinetic_half"), xy_scale));
+    // kin_kernel: the kinetic passes of sizes the other register kernels do not have.
+    use_v2_ = !(std::getenv("SPO_B200_KERNELS") && std::string(std::getenv("SPO_B200_KERNELS")) == "v1");
+    use_pfa_ = !(std::getenv("SPO_B200_PFA") && std::string(std::getenv("SPO_B200_PFA")) == "0");
+    if (use_v2_) {
+      auto axis = [&](KinAxis& ax, int n, const double* full, const double* half) {
+        if (axis2_supported(n) || !kin_split(n, use_pfa_, ax.map, ax.n1, ax.n2)) return;
+        kin_table(ax, 0, scaled(complex_array(full, n, "kinetic factors"), 1.0 / n));
+        kin_table(ax, 1, scaled(complex_array(half, n, "kinetic factors"), 1.0 / n));
+      };
+      axis(kin_z_, s.nz, d.z_kinetic_full, d.z_kinetic_half);
+      axis(kin_r_, s.nr, d.r_kinetic_full, d.r_kinetic_half);
+      if (kin_xy_size(s.nx) && kin_xy_size(s.ny) && (s.nx != s.ny || !xy2_supported(s.nx))) {
+        kin_xy_.map = spo::kXy;
+        kin_xy_.n1 = s.ny;
+        kin_xy_.n2 = s.nx;
+        kin_table(kin_xy_, 0, scaled(complex_array(d.xy_kinetic_full, nxy, "xy_kinetic_full"), xy_scale));
+        kin_table(kin_xy_, 1, scaled(complex_array(d.xy_kinetic_half, nxy, "xy_kinetic_half"), xy_scale));
+      }
+    }
     const double sz = d.fft_scale_z, sr = d.fft_scale_r;
     const double spec_scale = (sz * sr) * ((1.0 / (s.nzs * sz)) * (1.0 / (s.nr * sr)));
     spec_full_ = upload_factor(scaled(complex_array(d.specular_kinetic_full, s.n_chi(), "specular_kinetic_full"), spec_scale));
@@ -1673,8 +1841,6 @@ class Step final : public StepBase {
     if (use_v2_ && pot4_kernel_) pot_kind_ = 4;
     if (use_v2_ && pot5_kernel_) pot_kind_ = 5;
     pot_source_ = "default";
-    use_pfa_ = true;
-    if (const char* env = std::getenv("SPO_B200_PFA")) use_pfa_ = std::string(env) != "0";
     if (const char* env = std::getenv("SPO_B200_KERNELS")) {
       const std::string k(env);
       require(k == "v1" || k == "v2" || k == "v3" || k == "v4" || k == "v5" || k == "v6",
@@ -1860,6 +2026,8 @@ class Step final : public StepBase {
       }
     }
   }
+
+  KinAxis kin_z_, kin_r_, kin_xy_;
 
   Sizes s_;
   cudaStream_t stream_;

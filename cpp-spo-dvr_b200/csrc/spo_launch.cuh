@@ -263,4 +263,43 @@ Pot4Kernel<T> pot4_kernel_for(int nphi, int nt) {
   return nullptr;
 }
 
+template <typename T>
+using KinKernel = void (*)(spo::KinArgs<T>);
+template <typename T>
+KinKernel<T> kin_kernel_for(int map) {
+  return map == spo::kTwiddle ? spo::kin_kernel<T, spo::kTwiddle, 0, 0>
+         : map == spo::kPrime ? spo::kin_kernel<T, spo::kPrime, 0, 0>
+                              : spo::kin_kernel<T, spo::kXy, 0, 0>;
+}
+
+// Threads per line: the number that wastes the fewest thread slots over the two levels (N2 lines of N1 points, then N1 of
+// N2) in whole warps.
+template <typename T>
+KinLaunch<T> kin_configure(int map, int n1, int n2, int lanes_per_tile, long long window) {
+  KinLaunch<T> l;
+  l.kernel = kin_kernel_for<T>(map);
+  while ((spo::KinLine<T>::lanes << (l.log_lines + 1)) <= lanes_per_tile) ++l.log_lines;
+  while (l.log_lines > 0 && (static_cast<long long>(spo::KinLine<T>::lanes) << (l.log_lines - 1)) >= window) --l.log_lines;
+  const int lines = 1 << l.log_lines, limit = spo::kin_max_threads(std::max(n1, n2));
+  long long best = 0;
+  for (int nt = 1; nt <= std::max(n1, n2) && nt * lines <= limit; ++nt) {
+    const int threads = (nt * lines + 31) / 32 * 32;
+    const long long cost = static_cast<long long>((n2 + nt - 1) / nt * n1 + (n1 + nt - 1) / nt * n2) * threads;
+    if (best == 0 || cost < best || (cost == best && nt * lines <= 128)) {
+      best = cost;
+      l.threads = nt * lines;
+    }
+  }
+  const std::size_t n = static_cast<std::size_t>(n1) * n2;
+  l.smem = 16 * (n * (spo::KinLine<T>::factor_words + (map == spo::kTwiddle ? spo::KinLine<T>::twiddle_words : 0)) + n * lines);
+  check_cuda(cudaFuncSetAttribute(l.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_optin_bytes())),
+             "kin smem");
+  int dev = 0, sms = 0, per_sm = 0;
+  check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
+  check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
+  check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, l.kernel, l.threads, l.smem), "occupancy");
+  l.blocks = static_cast<long long>(sms) * std::max(per_sm, 1);
+  return l;
+}
+
 }  // namespace spo_host
