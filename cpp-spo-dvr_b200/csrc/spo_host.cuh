@@ -34,6 +34,7 @@
 #include "spo_kernels.cuh"
 #include "spo_regfft.cuh"
 #include "spo_pot4.cuh"
+#include "spo_pot4d.cuh"
 #include "spo_pot5.cuh"
 #include "spo_pot6.cuh"
 #include "spo_persist.cuh"
@@ -531,6 +532,9 @@ class Step final : public StepBase {
              std::to_string(pot5_threads_ / 32) + ",blocks=" + std::to_string(pot5_blocks_) + ">";
       if (nt_k != s_.nt) out += "(theta " + std::to_string(s_.nt) + " padded)";
     }
+    else if (pot_kind_ == 4 && pot4d_kernel_)
+      out += " potential=potential4<nphi=" + std::to_string(s_.nphi) + ",nt=" + std::to_string(s_.nt) + ",dmma,warps=" +
+             std::to_string(pot4d_threads_ / 32) + ",blocks=" + std::to_string(pot4_blocks_) + ">";
     else if (pot_kind_ == 4)
       out += " potential=potential4<nphi=" + std::to_string(s_.nphi) + ",nt=" + std::to_string(s_.nt) +
              ",cb=" + std::to_string(128 / s_.nt) + ",blocks=" + std::to_string(pot4_blocks_) + ">";
@@ -705,7 +709,7 @@ class Step final : public StepBase {
       case SPO_STAGE_XY: kinetic_xy(half, false); break;
       case SPO_STAGE_POTENTIAL:
         scale_points("gas_phase", static_cast<long long>(s_.nzp) * s_.nr, s_.n_zr(), gas_step_);
-        if (pot_kind_ == 5) scale_points("scaling", 0, static_cast<long long>(s_.nzp) * s_.nr, before_);
+        if (prescaled_) scale_points("scaling", 0, static_cast<long long>(s_.nzp) * s_.nr, before_);
         interaction();
         break;
       default: require(false, "unknown stage");
@@ -991,7 +995,7 @@ class Step final : public StepBase {
     x.nr = s_.nr;
     x.opt_z = opt_z_;
     x.gas_step = gas_step_;
-    x.before = pot_kind_ == 5 ? before_ : nullptr;
+    x.before = prescaled_ ? before_ : nullptr;
     x.tile = tile_xy_;
     x.persistent = persist_xy_ ? 1 : 0;
     if (kin_xy_.map >= 0) {
@@ -1048,7 +1052,8 @@ class Step final : public StepBase {
       } else if (pot_kind_ == 5) {
         pot5_kernel_<<<pot5_blocks_, pot5_threads_, pot5_smem_, stream_>>>(pot5_args_, error_flag_);
       } else if (pot_kind_ == 4) {
-        pot4_kernel_<<<pot4_blocks_, 128, pot4_smem_, stream_>>>(pot4_args_);
+        if (pot4d_kernel_) pot4d_kernel_<<<pot4_blocks_, pot4d_threads_, pot4_smem_, stream_>>>(pot4d_args_);
+        else pot4_kernel_<<<pot4_blocks_, 128, pot4_smem_, stream_>>>(pot4_args_);
       } else {
         const dim3 grid(static_cast<unsigned>(pot3_chunks_), points);
         launch_pot3<T>(s_.nphi, pot3_args_, grid, static_cast<unsigned>(pot3_cb_ * s_.nt), pot3_smem_, stream_);
@@ -1768,6 +1773,8 @@ class Step final : public StepBase {
     // potential5 (mixed form): the contractions on the FP64 tensor cores, any ntheta up to 16.
     pot5_kernel_ = nullptr;
     if constexpr (std::is_same_v<T, float>) build_pot5(pot5_args_, first, size, slot, offset, legendre64, phi_map, smem_optin, dev_id);
+    // potential4 of the FP64 form: the same for FP64 columns.
+    if constexpr (std::is_same_v<T, double>) build_pot4d(pot4d_args_, first, size, slot, offset, legendre64, phi_map, smem_optin, dev_id);
     // potential6 (mixed form): both theta contractions as split-precision TF32 tcgen05 GEMMs over 64-column
     // tiles, for the square heteronuclear basis JMax = MJMax = 15 with ntheta 16 and nphi 32 (configuration
     // 2's angular grid); one block of 256 threads per SM holding all 512 tensor-memory columns.
@@ -1827,7 +1834,7 @@ class Step final : public StepBase {
         }
       }
     }
-    if (pot3_cb_ > 0 || pot4_kernel_ || pot5_kernel_ || pot6_kernel_) {
+    if (pot3_cb_ > 0 || pot4_kernel_ || pot4d_kernel_ || pot5_kernel_ || pot6_kernel_) {
       require(sizeof(V) * (nxy + 1) <= static_cast<std::size_t>(smem_optin), "nx*ny too large for the projection kernel");
       check_cuda(cudaFuncSetAttribute(spo::projection_finalize_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       smem_optin), "projection smem");
@@ -1838,7 +1845,7 @@ class Step final : public StepBase {
     pot_kind_ = 1;
     if (use_v2_ && pot2_cb_ > 0) pot_kind_ = 2;
     if (use_v2_ && pot3_cb_ > 0) pot_kind_ = 3;
-    if (use_v2_ && pot4_kernel_) pot_kind_ = 4;
+    if (use_v2_ && (pot4_kernel_ || pot4d_kernel_)) pot_kind_ = 4;
     if (use_v2_ && pot5_kernel_) pot_kind_ = 5;
     pot_source_ = "default";
     if (const char* env = std::getenv("SPO_B200_KERNELS")) {
@@ -1848,10 +1855,10 @@ class Step final : public StepBase {
       use_v2_ = k != "v1";
       const int want = k[1] - '0';
       const bool have = want == 1 || (want == 2 && pot2_cb_ > 0) || (want == 3 && pot3_cb_ > 0) ||
-                        (want == 4 && pot4_kernel_ != nullptr) || (want == 5 && pot5_kernel_ != nullptr) ||
+                        (want == 4 && (pot4_kernel_ != nullptr || pot4d_kernel_ != nullptr)) || (want == 5 && pot5_kernel_ != nullptr) ||
                         (want == 6 && pot6_kernel_ != nullptr);
       // an unavailable kernel falls back to the best available one below it
-      const bool avail[7] = {false, true, pot2_cb_ > 0, pot3_cb_ > 0, pot4_kernel_ != nullptr, pot5_kernel_ != nullptr,
+      const bool avail[7] = {false, true, pot2_cb_ > 0, pot3_cb_ > 0, pot4_kernel_ != nullptr || pot4d_kernel_ != nullptr, pot5_kernel_ != nullptr,
                              pot6_kernel_ != nullptr};
       pot_kind_ = have ? want : 1;
       if (!have)
@@ -1862,9 +1869,114 @@ class Step final : public StepBase {
           }
       pot_source_ = "fixed";
     }
+    prescaled_ = pot_kind_ == 5 || (pot_kind_ == 4 && pot4d_kernel_);
     build_exp_table(d);
     check_cuda(cudaStreamSynchronize(stream_), "set-up");
     autotune();
+  }
+
+  // The fragments of 32 matrix entries that the DMMA potential kernels multiply with, the forward ones, then the transposed
+  // ones, and per phi slot (first irot, J count [+ 65536 forward steps in the interleaved order], first fragments). Blocks of
+  // equal matrices (m and -m) share theirs. Lane l holds
+  //   forward, J quad q, theta half h: theta 8 h + a(l / 4), J 4 q + l % 4;
+  //   transposed, J octet q, half h, i = 0, 1: theta 8 h + b(l % 4, i), J 8 q + (l / 4) / 2 + 4 (l / 4 % 2);
+  // potential5 (registers between the products): a(n) = n, b(k, i) = 2 k + i, forward order [h][q];
+  // potential4_dmma (shared memory between them): a(n) = n / 2 + 4 (n % 2), b(k, i) = k + 4 i, forward order [q][h].
+  std::vector<double> dmma_fragments(const std::vector<int>& first, const std::vector<int>& size, const std::vector<int>& slot,
+                                     const std::vector<int>& offset, const std::vector<double>& legendre, int h_n, bool fp64,
+                                     std::vector<int4>& slots, int& n_fwd, int& n_back) const {
+    const Sizes& s = s_;
+    std::vector<double> fwd, back;
+    slots.assign(s.nphi, make_int4(0, 0, 0, 0));
+    for (int b = 0; b < s.n_blocks; ++b) {
+      const double* m = legendre.data() + offset[b];
+      const int nj = size[b];
+      const int nk = ((fp64 ? nj : std::max(nj, size[s.n_blocks - 1 - b])) + 3) / 4;  // potential5: as many steps as the block of -m
+      int4 e = make_int4(first[b], fp64 ? nj : nj + 65536 * nk, -1, -1);
+      for (int o = 0; o < b && e.z < 0; ++o)
+        if (slots[slot[o]].y == e.y && std::equal(m, m + static_cast<std::size_t>(s.nt) * nj, legendre.data() + offset[o])) {
+          e.z = slots[slot[o]].z;
+          e.w = slots[slot[o]].w;
+        }
+      if (e.z < 0) {
+        auto at = [&](int theta, int j) { return theta < s.nt && j < nj ? m[static_cast<std::size_t>(theta) * nj + j] : 0.0; };
+        e.z = static_cast<int>(fwd.size() / 32);
+        for (int x = 0; x < nk * h_n; ++x) {
+          const int h = fp64 ? x % h_n : x / nk, q = fp64 ? x / h_n : x % nk;
+          for (int l = 0; l < 32; ++l) fwd.push_back(at(8 * h + (fp64 ? l / 8 + 4 * (l / 4 % 2) : l / 4), 4 * q + l % 4));
+        }
+        e.w = static_cast<int>(back.size() / 32);
+        for (int q = 0; 8 * q < nj; ++q)
+          for (int h = 0; h < h_n; ++h)
+            for (int i = 0; i < 2; ++i)
+              for (int l = 0; l < 32; ++l)
+                back.push_back(at(8 * h + (fp64 ? l % 4 + 4 * i : 2 * (l % 4) + i), 8 * q + l / 8 + 4 * (l / 4 % 2)));
+      }
+      slots[slot[b]] = e;
+    }
+    n_fwd = static_cast<int>(fwd.size() / 32);
+    n_back = static_cast<int>(back.size() / 32);
+    fwd.insert(fwd.end(), back.begin(), back.end());
+    return fwd;
+  }
+
+  // potential4 of the FP64 form (spo_pot4d.cuh): fragments, task lists, rotation factors and launch shape.
+  template <typename A>
+  void build_pot4d(A& a, const std::vector<int>& first, const std::vector<int>& size, const std::vector<int>& slot,
+                   const std::vector<int>& offset, const std::vector<double>& legendre, const std::vector<int>& phi_map,
+                   int smem_optin, int dev_id) {
+    const Sizes& s = s_;
+    const long long n_cols = static_cast<long long>(s.nzp) * s.nr * s.n_xy();
+    if (s.nt > 16 || s.nphi > 255 || n_cols > (1ll << 30) || static_cast<long long>(s.nr) * s.n_rot > (1ll << 30)) return;
+    const int h_n = s.nt > 8 ? 2 : 1, cols = 16 / h_n;
+    auto kernel = spo::pot4d::kernel_for(s.nphi, h_n);
+    if (!kernel) return;
+    int n_fwd = 0, n_back = 0;
+    std::vector<int4> slots;
+    const std::vector<double> frags = dmma_fragments(first, size, slot, offset, legendre, h_n, true, slots, n_fwd, n_back);
+    std::vector<int> order(s.nphi);
+    for (int p = 0; p < s.nphi; ++p) order[p] = p;
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return slots[x].y > slots[y].y; });
+    std::vector<int2> tiles;
+    for (int p = 0; p < s.nphi; ++p)
+      for (int q = 0; 8 * q < slots[p].y; ++q) tiles.push_back(make_int2(p, q));
+    int teams = spo::pot4d::threads_of(s.nphi) / spo::pot4d::kTeam;
+    auto need = [&](int n) { return spo::pot4d::smem_bytes(s.nphi, n_fwd + n_back, static_cast<int>(tiles.size()), n); };
+    while (teams > 0 && need(teams) > static_cast<std::size_t>(smem_optin)) --teams;
+    if (teams == 0) return;
+    a.p = pot_;
+    a.frags = upload_f64(frags);
+    a.n_fwd = n_fwd;
+    a.n_back = n_back;
+    int4* ds = dev<int4>(slots.size());
+    check_cuda(cudaMemcpy(ds, slots.data(), sizeof(int4) * slots.size(), cudaMemcpyHostToDevice), "potential4 slots");
+    a.slots = ds;
+    a.fwd_tasks = upload_int(order);
+    int2* dt = dev<int2>(tiles.size());
+    check_cuda(cudaMemcpy(dt, tiles.data(), sizeof(int2) * tiles.size(), cudaMemcpyHostToDevice), "potential4 tasks");
+    a.back_tasks = dt;
+    a.n_back_tasks = static_cast<int>(tiles.size());
+    a.rot = upload_c128(host_rot_);
+    a.phi_map = upload_phi_map(phi_map);
+    a.n_cols = static_cast<int>(n_cols);
+    a.n_items = (a.n_cols + cols - 1) / cols;
+    int sms = 0;
+    check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev_id), "SM count");
+    while (teams > 1 && a.n_items <= static_cast<long long>(sms) * (teams - 1)) --teams;
+    pot4d_kernel_ = kernel;
+    pot4d_threads_ = teams * spo::pot4d::kTeam;
+    pot4_smem_ = need(teams);
+    check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin), "potential4 smem");
+    pot4_blocks_ = static_cast<int>(std::max<long long>(1, std::min<long long>(sms, (a.n_items + teams - 1) / teams)));
+  }
+
+  // The phi maps as bytes, or null without symmetry.
+  std::uint8_t* upload_phi_map(const std::vector<int>& phi_map) {
+    if (identity_maps_) return nullptr;
+    const std::vector<std::uint8_t> map(phi_map.begin(), phi_map.end());
+    std::uint8_t* dm = dev<std::uint8_t>(map.size());
+    check_cuda(cudaMemcpy(dm, map.data(), map.size(), cudaMemcpyHostToDevice), "phi maps");
+    return dm;
   }
 
   // potential5's matrix fragments (spo_pot5.cuh), rotation factors and launch shape.
@@ -1878,55 +1990,21 @@ class Step final : public StepBase {
     const int h_n = s.nt > 8 ? 2 : 1;
     auto kernel = spo::pot5::kernel_for(s.nphi, h_n);
     if (!kernel) return;
-    // Fragments of 32 values: forward [theta half][J quad], lane l the entry (theta 8 half + l / 4, J 4 quad + l % 4);
-    // transposed [J octet][theta half][i], lane l the entry (theta 8 half + 2 (l % 4) + i, J 8 octet + l / 8 + 4 (l / 4 % 2)).
-    // Blocks of equal matrices (m and -m) share theirs.
-    std::vector<double> fwd, back;
-    std::vector<int4> slots(s.nphi, make_int4(0, 0, 0, 0));
-    for (int b = 0; b < s.n_blocks; ++b) {
-      const double* m = legendre.data() + offset[b];
-      const int nj = size[b];
-      const int nk = (std::max(nj, size[s.n_blocks - 1 - b]) + 3) / 4;  // as many steps as the block of -m
-      int4 e = make_int4(first[b], nj + 65536 * nk, -1, -1);
-      for (int o = 0; o < b && e.z < 0; ++o)
-        if (slots[slot[o]].y == e.y && std::equal(m, m + static_cast<std::size_t>(s.nt) * nj, legendre.data() + offset[o])) {
-          e.z = slots[slot[o]].z;
-          e.w = slots[slot[o]].w;
-        }
-      if (e.z < 0) {
-        auto at = [&](int theta, int j) { return theta < s.nt && j < nj ? m[static_cast<std::size_t>(theta) * nj + j] : 0.0; };
-        e.z = static_cast<int>(fwd.size() / 32);
-        for (int h = 0; h < h_n; ++h)
-          for (int q = 0; q < nk; ++q)
-            for (int l = 0; l < 32; ++l) fwd.push_back(at(8 * h + l / 4, 4 * q + l % 4));
-        e.w = static_cast<int>(back.size() / 32);
-        for (int q = 0; 8 * q < nj; ++q)
-          for (int h = 0; h < h_n; ++h)
-            for (int i = 0; i < 2; ++i)
-              for (int l = 0; l < 32; ++l) back.push_back(at(8 * h + 2 * (l % 4) + i, 8 * q + l / 8 + 4 * (l / 4 % 2)));
-      }
-      slots[slot[b]] = e;
-    }
-    const int n_fwd = static_cast<int>(fwd.size() / 32), n_back = static_cast<int>(back.size() / 32);
-    fwd.insert(fwd.end(), back.begin(), back.end());
+    int n_fwd = 0, n_back = 0;
+    std::vector<int4> slots;
+    const std::vector<double> frags = dmma_fragments(first, size, slot, offset, legendre, h_n, false, slots, n_fwd, n_back);
     int teams = spo::pot5::threads_of(s.nphi) / (32 * h_n);
     while (teams > 0 && spo::pot5::smem_bytes(s.n_rot, s.nphi, h_n, n_fwd + n_back, teams) > static_cast<std::size_t>(smem_optin)) --teams;
     if (teams == 0) return;
     a.p = pot_;
-    a.frags = upload_f64(fwd);
+    a.frags = upload_f64(frags);
     a.n_fwd = n_fwd;
     a.n_back = n_back;
     int4* ds = dev<int4>(slots.size());
     check_cuda(cudaMemcpy(ds, slots.data(), sizeof(int4) * slots.size(), cudaMemcpyHostToDevice), "potential5 slots");
     a.slots = ds;
     a.rot = upload_c128(host_rot_);
-    a.phi_map = nullptr;
-    if (!identity_maps_) {
-      std::vector<std::uint8_t> map(phi_map.begin(), phi_map.end());
-      std::uint8_t* dm = dev<std::uint8_t>(map.size());
-      check_cuda(cudaMemcpy(dm, map.data(), map.size(), cudaMemcpyHostToDevice), "potential5 maps");
-      a.phi_map = dm;
-    }
+    a.phi_map = upload_phi_map(phi_map);
     a.pairs = (s.nt + 1) / 2;
     a.n_cols = static_cast<int>(n_cols);
     a.n_items = (a.n_cols + spo::pot5::kCols - 1) / spo::pot5::kCols;
@@ -1974,6 +2052,23 @@ class Step final : public StepBase {
         check_cuda(cudaStreamSynchronize(stream_), "exp_potential");
       }
       return;
+    }
+    if constexpr (std::is_same_v<T, double>) {
+      if (prescaled_) {
+        const long long reps = static_cast<long long>(s.nzp) * s.nr * s.n_rep;
+        double2* table = dev<double2>(std::max<long long>(n_e, 1));
+        pot4d_args_.table = table;
+        const long long chunk = 2 * staging_elems_ / n_tp;
+        for (long long i = 0; i < reps; i += chunk) {
+          const long long m = std::min(chunk, reps - i);
+          check_cuda(cudaMemcpyAsync(vstage, d.potential + i * n_tp, sizeof(double) * m * n_tp, cudaMemcpyHostToDevice, stream_),
+                     "upload potential");
+          spo::exp_rows_kernel<<<1184, 256, 0, stream_>>>(vstage, table + i * n_tp, m, s.nt, s.nphi, s.dt);
+          check_cuda(cudaGetLastError(), "exp_potential launch");
+          check_cuda(cudaStreamSynchronize(stream_), "exp_potential");
+        }
+        return;
+      }
     }
     // The mixed form keeps, after the n_e table entries, their n_e modulus corrections (FP16, spo::exp_mul)
     // (from a 16-byte boundary: the kernels read 8 corrections per load and prefetch rows of them into L2)
@@ -2063,6 +2158,10 @@ class Step final : public StepBase {
   spo::Pot4Args<T> pot4_args_{};
   int pot4_blocks_ = 0;
   std::size_t pot4_smem_ = 0;
+  spo::pot4d::Kernel pot4d_kernel_ = nullptr;  // potential4 of the FP64 form
+  spo::Pot4dArgs pot4d_args_{};
+  int pot4d_threads_ = 0;
+  bool prescaled_ = false;       // the potential kernel takes psi scaled by the absorbers and rot(dt/2) (the xy pass)
   spo::pot5::Kernel pot5_kernel_ = nullptr;  // mixed form
   spo::Pot5Args pot5_args_{};
   int pot5_blocks_ = 0, pot5_threads_ = 0, pot5_h_ = 1;
