@@ -467,8 +467,22 @@ class Step final : public StepBase {
     build(d);
   }
 
+  ~Step() override {
+    if (graph_) cudaGraphExecDestroy(graph_);
+    if (side_) cudaStreamDestroy(side_);
+    for (cudaEvent_t e : fork_)
+      if (e) cudaEventDestroy(e);
+    if (host_flag_) cudaFreeHost(host_flag_);
+  }
+
   void propagate_analysis_step() override {
-    enqueue_analysis_step();
+    if (graph_ && !prof_.on()) {
+      launches_ = graph_launches_;
+      check_cuda(cudaGraphLaunch(graph_, stream_), "propagate_analysis_step launch");
+    } else {
+      enqueue_analysis_step();
+      read_device_error();
+    }
     check_cuda(cudaStreamSynchronize(stream_), "propagate_analysis_step");
     prof_.resolve();
     check_device_error();
@@ -480,17 +494,58 @@ class Step final : public StepBase {
     const int limit = poll_limit > 0 ? poll_limit : spo::pot5::kWaitLimit;
     pot5_args_.poll_limit = pot6_args_.poll_limit = limit;
     pot5_args_.extra_tx = pot6_args_.extra_tx = extra_bytes;
+    capture_graph();  // the graph holds the kernels' arguments
   }
 
-  // A kernel whose bounded wait gave up has set the device flag: report it (and clear it).
+  // A kernel whose bounded wait gave up has set the device flag, which each step copies to host_flag_ at its end: report
+  // it (and clear it).
+  void read_device_error() {
+    if (error_flag_)
+      check_cuda(cudaMemcpyAsync(host_flag_, error_flag_, sizeof(int), cudaMemcpyDeviceToHost, stream_), "error flag");
+  }
   void check_device_error() {
-    if (!error_flag_) return;
-    int flag = 0;
-    check_cuda(cudaMemcpy(&flag, error_flag_, sizeof(int), cudaMemcpyDeviceToHost), "error flag");
-    if (flag) {
-      check_cuda(cudaMemset(error_flag_, 0, sizeof(int)), "error flag");
-      throw SpoError(SPO_ERR_TIMEOUT, std::string(pot_kind_ == 6 ? "potential6" : "potential5") +
-                                          ": a bounded wait for an asynchronous copy or tensor-core work gave up");
+    if (!error_flag_ || *host_flag_ == 0) return;
+    *host_flag_ = 0;
+    check_cuda(cudaMemset(error_flag_, 0, sizeof(int)), "error flag");
+    throw SpoError(SPO_ERR_TIMEOUT, std::string(pot_kind_ == 6 ? "potential6" : "potential5") +
+                                        ": a bounded wait for an asynchronous copy or tensor-core work gave up");
+  }
+
+  // One analysis step as a CUDA graph (about 8 (n + 1) small kernels: on the smallest grids the gaps between separate
+  // launches and the wait for the copy of the error flag cost as much as the kernels). Captured on a stream of its own
+  // when the handle is built, so it can be launched into any stream.
+  void capture_graph() {
+    if (graph_) {
+      check_cuda(cudaStreamSynchronize(stream_), "graph");
+      cudaGraphExecDestroy(graph_);
+      graph_ = nullptr;
+    }
+    const cudaStream_t current = stream_;
+    cudaStream_t capture = nullptr;
+    check_cuda(cudaStreamCreateWithFlags(&capture, cudaStreamNonBlocking), "cudaStreamCreate");
+    cudaGraph_t graph = nullptr;
+    cudaError_t e = cudaStreamBeginCapture(capture, cudaStreamCaptureModeThreadLocal);
+    if (e == cudaSuccess) {
+      stream_ = capture;
+      const bool was_on = prof_.on();
+      std::string failed;
+      try {
+        require(!was_on, "profiling");
+        enqueue_analysis_step();
+        read_device_error();
+      } catch (const std::exception& x) {
+        failed = x.what();
+      }
+      stream_ = current;
+      e = cudaStreamEndCapture(capture, &graph);
+      if (e == cudaSuccess && failed.empty()) e = cudaGraphInstantiate(&graph_, graph, 0);
+      if (graph) cudaGraphDestroy(graph);
+      graph_launches_ = launches_;
+    }
+    cudaStreamDestroy(capture);
+    if (e != cudaSuccess) {  // the step then launches its kernels one by one
+      (void)cudaGetLastError();
+      graph_ = nullptr;
     }
   }
 
@@ -814,14 +869,28 @@ class Step final : public StepBase {
 
  private:
   // ------------------------------------------------------------------ one sub-step
+  // The specular grid's step needs nothing of the scattering wave's kinetic step, so its three short passes (20 to 50 us
+  // each, a few blocks) run beside it on a second stream; profiling runs them one after another.
   void sub_step(bool half, bool kinetic_only) {
-    specular(half, kinetic_only);
+    const bool fork = side_ && !prof_.on();
+    if (fork) {
+      const cudaStream_t main = stream_;
+      check_cuda(cudaEventRecord(fork_[0], main), "cudaEventRecord");
+      check_cuda(cudaStreamWaitEvent(side_, fork_[0], 0), "cudaStreamWaitEvent");
+      stream_ = side_;
+      specular(half, kinetic_only);
+      stream_ = main;
+      check_cuda(cudaEventRecord(fork_[1], side_), "cudaEventRecord");
+    } else {
+      specular(half, kinetic_only);
+    }
     if (rxy_planes_ > 0) {
       kinetic_rxy_slabs(half, !kinetic_only);
     } else {
       kinetic_zr(half);
       kinetic_xy(half, !kinetic_only);  // the gas-phase potential step rides along
     }
+    if (fork) check_cuda(cudaStreamWaitEvent(stream_, fork_[1], 0), "cudaStreamWaitEvent");
     if (!kinetic_only) interaction();
   }
 
@@ -1061,8 +1130,8 @@ class Step final : public StepBase {
       prof_.end(stream_, "potential", bytes);
       ++launches_;
       prof_.begin(stream_);
-      spo::projection_finalize_kernel<T><<<points, 128, sizeof(V) * (s_.n_xy() + 1), stream_>>>(
-          psi_, chi_, s_.n_rot, static_cast<int>(s_.n_xy()), s_.i0, pot_.sc2sp, pot_.sp2sc);
+      spo::projection_finalize_kernel<T><<<(points + spo::kProjectWarps - 1) / spo::kProjectWarps, 32 * spo::kProjectWarps, 0, stream_>>>(
+          psi_, chi_, static_cast<int>(points), s_.n_rot, static_cast<int>(s_.n_xy()), s_.i0, pot_.sc2sp, pot_.sp2sc);
       prof_.end(stream_, "projection", 2.0 * sizeof(V) * points * s_.n_xy());
       ++launches_;
       return;
@@ -1829,15 +1898,9 @@ class Step final : public StepBase {
         check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev_id), "SM count");
         pot6_blocks_ = static_cast<int>(std::min<long long>(sms, std::max<long long>(pot6_args_.n_items, 1)));
         if (!error_flag_) {
-          error_flag_ = dev<int>(1);
-          check_cuda(cudaMemset(error_flag_, 0, sizeof(int)), "error flag");
+          make_error_flag();
         }
       }
-    }
-    if (pot3_cb_ > 0 || pot4_kernel_ || pot4d_kernel_ || pot5_kernel_ || pot6_kernel_) {
-      require(sizeof(V) * (nxy + 1) <= static_cast<std::size_t>(smem_optin), "nx*ny too large for the projection kernel");
-      check_cuda(cudaFuncSetAttribute(spo::projection_finalize_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      smem_optin), "projection smem");
     }
     // The potential kernel is not chosen by timing: the kernels agree only to rounding (the compiler may
     // contract the products of a complex multiply into FMAs differently in each), and a timing choice
@@ -1873,6 +1936,9 @@ class Step final : public StepBase {
     build_exp_table(d);
     check_cuda(cudaStreamSynchronize(stream_), "set-up");
     autotune();
+    check_cuda(cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking), "cudaStreamCreate");
+    for (cudaEvent_t& e : fork_) check_cuda(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
+    capture_graph();
   }
 
   // The fragments of 32 matrix entries that the DMMA potential kernels multiply with, the forward ones, then the transposed
@@ -1970,6 +2036,13 @@ class Step final : public StepBase {
     pot4_blocks_ = static_cast<int>(std::max<long long>(1, std::min<long long>(sms, (a.n_items + teams - 1) / teams)));
   }
 
+  void make_error_flag() {
+    error_flag_ = dev<int>(1);
+    check_cuda(cudaMemset(error_flag_, 0, sizeof(int)), "error flag");
+    check_cuda(cudaMallocHost(&host_flag_, sizeof(int)), "error flag");
+    *host_flag_ = 0;
+  }
+
   // The phi maps as bytes, or null without symmetry.
   std::uint8_t* upload_phi_map(const std::vector<int>& phi_map) {
     if (identity_maps_) return nullptr;
@@ -2022,8 +2095,7 @@ class Step final : public StepBase {
     check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin), "potential5 smem");
     pot5_blocks_ = static_cast<int>(std::max<long long>(1, std::min<long long>(sms, (a.n_items + teams - 1) / teams)));
     if (!error_flag_) {
-      error_flag_ = dev<int>(1);
-      check_cuda(cudaMemset(error_flag_, 0, sizeof(int)), "error flag");
+      make_error_flag();
     }
   }
 
@@ -2127,6 +2199,11 @@ class Step final : public StepBase {
   Sizes s_;
   cudaStream_t stream_;
   cudaStream_t own_stream_;
+  cudaGraphExec_t graph_ = nullptr;  // one analysis step
+  int graph_launches_ = 0;
+  cudaStream_t side_ = nullptr;      // the specular grid's passes
+  cudaEvent_t fork_[2] = {nullptr, nullptr};
+  int* host_flag_ = nullptr;         // pinned copy of the error flag
   DeviceArena arena_;
   Profiler prof_;
   int launches_ = 0;

@@ -654,41 +654,41 @@ __global__ void __launch_bounds__(CB * 16) potential3_kernel(Pot2Args<T> args) {
 }
 
 // The projection of each interaction-region point onto the specular grid
-// (src/propagation/potential_operator.cpp:129-135): chi(ir, iz) = sum over the (x, y) columns, in column
-// order, of scattering_to_specular times the initial channel, then specular_to_scattering times it
-// subtracted from the initial channel of every column. One block per point; the initial channel of the
-// point's columns is gathered into shared memory (n_xy values) and summed by one thread.
+// (src/propagation/potential_operator.cpp:129-135): chi(ir, iz) = sum over the (x, y) columns of
+// scattering_to_specular times the initial channel, then specular_to_scattering times it subtracted from the
+// initial channel of every column. One warp per point (a block has kProjectWarps): every lane sums the columns
+// lane, lane + 32, ... in FP64, then a fixed tree over the lanes, so the sum is repeatable and does not depend on
+// the potential kernel's chunking. The pass reads one value per column from as many 32-byte sectors (configuration
+// 3: 1.03e6 of them, twice); a serial sum by one thread per point made it 95 us of latency.
+constexpr int kProjectWarps = 4;
 template <typename T>
-__global__ void projection_finalize_kernel(Vec<T>* __restrict__ psi, Vec<T>* __restrict__ chi, int n_rot, int n_xy,
-                                           int i0, const Vec<T>* __restrict__ sc2sp, const Vec<T>* __restrict__ sp2sc) {
+__global__ void __launch_bounds__(32 * kProjectWarps)
+    projection_finalize_kernel(Vec<T>* __restrict__ psi, Vec<T>* __restrict__ chi, int n_points, int n_rot, int n_xy, int i0,
+                               const Vec<T>* __restrict__ sc2sp, const Vec<T>* __restrict__ sp2sc) {
   using V = Vec<T>;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  V* col = reinterpret_cast<V*>(smem_raw);  // n_xy
-  V& proj = col[n_xy];                      // dynamic shared memory: (n_xy + 1) values
-  const long long base = static_cast<long long>(blockIdx.x) * n_xy;  // blockIdx.x = ir + nr iz
-  for (int ixy = threadIdx.x; ixy < n_xy; ixy += blockDim.x) col[ixy] = psi[(base + ixy) * n_rot + i0];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    if constexpr (sizeof(T) == 4) {  // mixed form: the sum in FP64, the coefficients with their low parts
-      double px = 0.0, py = 0.0;
-      for (int ixy = 0; ixy < n_xy; ++ixy) {
-        const V w = sc2sp[ixy], wl = sc2sp[n_xy + ixy], v = col[ixy];
-        const double wx = static_cast<double>(w.x) + wl.x, wy = static_cast<double>(w.y) + wl.y;
-        px += wx * v.x - wy * v.y;
-        py += wx * v.y + wy * v.x;
-      }
-      proj = cmake<V>(static_cast<T>(px), static_cast<T>(py));
-    } else {
-      V p = cmake<V>(0, 0);
-      for (int ixy = 0; ixy < n_xy; ++ixy) p = cadd(p, cmul(sc2sp[ixy], col[ixy]));
-      proj = p;
-    }
-    chi[blockIdx.x] = proj;
+  const int point = blockIdx.x * kProjectWarps + threadIdx.x / 32, lane = threadIdx.x % 32;  // point = ir + nr iz
+  if (point >= n_points) return;
+  V* const col = psi + static_cast<long long>(point) * n_xy * n_rot + i0;
+  double px = 0.0, py = 0.0;
+#pragma unroll 4
+  for (int ixy = lane; ixy < n_xy; ixy += 32) {
+    const V w = sc2sp[ixy], wl = lo_part(sc2sp, n_xy, ixy), v = col[static_cast<long long>(ixy) * n_rot];
+    const double wx = static_cast<double>(w.x) + wl.x, wy = static_cast<double>(w.y) + wl.y;
+    px += wx * v.x - wy * v.y;
+    py += wx * v.y + wy * v.x;
   }
-  __syncthreads();
-  const V p = proj;
-  for (int ixy = threadIdx.x; ixy < n_xy; ixy += blockDim.x)
-    psi[(base + ixy) * n_rot + i0] = csub(col[ixy], cmul_t(p, sp2sc, n_xy, ixy));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    px += __shfl_xor_sync(0xffffffffu, px, o);
+    py += __shfl_xor_sync(0xffffffffu, py, o);
+  }
+  const V p = cmake<V>(static_cast<T>(px), static_cast<T>(py));
+  if (lane == 0) chi[point] = p;
+#pragma unroll 4
+  for (int ixy = lane; ixy < n_xy; ixy += 32) {
+    V* const v = col + static_cast<long long>(ixy) * n_rot;
+    *v = csub(*v, cmul_t(p, sp2sc, n_xy, ixy));
+  }
 }
 
 }  // namespace spo
