@@ -39,6 +39,7 @@
 #include "spo_pot6.cuh"
 #include "spo_persist.cuh"
 #include "spo_kin.cuh"
+#include "spo_hostcopy.cuh"
 
 namespace spo_host {
 
@@ -2166,8 +2167,15 @@ class Step final : public StepBase {
     }
   }
 
-  // Host FP64 complex -> device T, through the staging buffer.
+  // Host FP64 complex -> device T, by several threads or through the staging buffer.
   void copy_in(const double* src, V* dst, long long n) {
+    if (HostCopier<T>::wanted(src, n)) {
+      int device = 0;
+      check_cuda(cudaGetDevice(&device), "cudaGetDevice");
+      check_cuda(cudaStreamSynchronize(stream_), "upload");
+      check_cuda(copier_.to_device(src, dst, n, device), "upload");
+      return;
+    }
     for (long long i = 0; i < n; i += staging_elems_) {
       const long long m = std::min(staging_elems_, n - i);
       if constexpr (std::is_same_v<T, double>) {
@@ -2181,6 +2189,13 @@ class Step final : public StepBase {
     }
   }
   void copy_out(const V* src, double* dst, long long n) {
+    if (HostCopier<T>::wanted(dst, n)) {
+      int device = 0;
+      check_cuda(cudaGetDevice(&device), "cudaGetDevice");
+      check_cuda(cudaStreamSynchronize(stream_), "download");
+      check_cuda(copier_.to_host(src, dst, n, device), "download");
+      return;
+    }
     for (long long i = 0; i < n; i += staging_elems_) {
       const long long m = std::min(staging_elems_, n - i);
       if constexpr (std::is_same_v<T, double>) {
@@ -2205,6 +2220,7 @@ class Step final : public StepBase {
   cudaEvent_t fork_[2] = {nullptr, nullptr};
   int* host_flag_ = nullptr;         // pinned copy of the error flag
   DeviceArena arena_;
+  HostCopier<T> copier_;
   Profiler prof_;
   int launches_ = 0;
   spo::FftPlan plan_z_{}, plan_r_{}, plan_x_{}, plan_y_{}, plan_zs_{}, plan_phi_{};

@@ -14,6 +14,8 @@
 //     and writes FP32, BF16, or bias + SiLU (pre-activation FP32, activation BF16);
 //   - split K: blockIdx.y takes a share of the K chunks and writes its own FP32 partial, summed in a
 //     fixed order afterwards (weight gradients, where K is the batch).
+// Prediction on many points is one kernel (mlp_predict_kernel): a block keeps the activations of 128 points in shared
+// memory through all layers.
 // Everything else (output layer, loss, SiLU derivative, transposes, Adam) is plain SIMT, with fixed-
 // order reductions so that a training run is repeatable.
 #include <cuda_bf16.h>
@@ -29,6 +31,7 @@
 #include <vector>
 
 #include "../../include/spo_b200.h"
+#include "spo_hostcopy.cuh"
 #include "../../include/spo_mlp.h"
 
 namespace {
@@ -102,6 +105,19 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t a_desc, uint6
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}" ::"r"(tmem_d),
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0), "r"(0), "r"(0), "r"(0)
       : "memory");
+}
+// Arrives on the barrier, announcing `bytes` of asynchronous copies, and one such copy (global -> shared).
+__device__ __forceinline__ void mbar_arrive_tx(uint64_t* bar, uint32_t bytes) {
+  asm volatile(
+      "{\n\t.reg .b64 state;\n\t"
+      "mbarrier.arrive.expect_tx.shared::cta.b64 state, [%0], %1;\n\t}" ::"r"(smem_addr(bar)),
+      "r"(bytes)
+      : "memory");
+}
+__device__ __forceinline__ void bulk_copy(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_addr(dst)),
+               "l"(src), "r"(bytes), "r"(smem_addr(bar))
+               : "memory");
 }
 // Arrives on the barrier when this thread's earlier tcgen05.mma have completed.
 __device__ __forceinline__ void commit(uint64_t* bar) {
@@ -286,6 +302,174 @@ __global__ void __launch_bounds__(128) gemm_tn_kernel(GemmArgs g) {
   tc::fence_before_sync();
   __syncthreads();
   if (warp == 0) tc::tmem_dealloc(tmem, 256);
+}
+
+// ------------------------------------------------------------------------------------------------
+// Prediction
+// ------------------------------------------------------------------------------------------------
+// y[i] = network(x[i]): a block of 128 threads takes tiles of 128 points through all layers. The activations stay in
+// shared memory as the A operand (BF16, canonical layout), the accumulator in tensor memory, and the weights come in
+// chunks of 32 inputs (packed in the B operand's layout by pack_weights_kernel) by bulk copies into three slots, two
+// chunks ahead of the products; two blocks per SM, so that one's SiLU overlaps the other's products. The separate
+// kernels (input rounding, one GEMM per layer with its pre-activations in FP32, output layer) moved 1.5 KB per point
+// and layer through memory. Bound: the SiLU (two special-function operations per unit: 0.5 ms for 1e6 points of
+// 4 x 256), then the weights from L2 (3.2 GB).
+struct PredictArgs {
+  const float* x;       // n x n_in
+  long long n;
+  int n_in, width, depth;
+  const bf16* weights;  // chunk after chunk, layer after layer
+  const float* bias;    // depth x width
+  const float* wo;
+  const float* bo;
+  float* y;
+  int* error_flag;
+};
+constexpr int kPredictSlots = 3, kPredictChunk = 32;
+constexpr std::size_t predict_smem(int width) {
+  const std::size_t k = width > 64 ? width : 64;
+  return 128 * k * 2 + kPredictSlots * static_cast<std::size_t>(width) * kPredictChunk * 2 + 64 + 64;
+}
+
+__global__ void __launch_bounds__(128) mlp_predict_kernel(PredictArgs g) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  const int width = g.width, n8 = width / 8;
+  unsigned char* const A = smem;
+  unsigned char* const W = smem + 128 * (width > 64 ? width : 64) * 2;
+  const uint32_t chunk_bytes = static_cast<uint32_t>(width * kPredictChunk * 2);
+  uint64_t* const full = reinterpret_cast<uint64_t*>(W + kPredictSlots * chunk_bytes);  // per slot: the chunk has arrived
+  uint64_t* const empty = full + kPredictSlots;                                         // per slot: its products are done
+  uint64_t* const done = empty + kPredictSlots;                                         // a layer's products are done
+  uint32_t* const tslot = reinterpret_cast<uint32_t*>(done + 1);
+  const int tid = threadIdx.x, warp = tid >> 5;
+  if (warp == 0) tc::tmem_alloc(tslot, static_cast<uint32_t>(width));
+  if (tid == 0)
+    for (int k = 0; k < 2 * kPredictSlots + 1; ++k) tc::mbar_init(full + k, 1);
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = *tslot;
+  const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(width >> 3) << 17) |
+                         (static_cast<uint32_t>(kBM >> 4) << 24);
+  const long long tiles = (g.n + kBM - 1) / kBM;
+  const int per_tile = 64 / kPredictChunk + (g.depth - 1) * (width / kPredictChunk);  // chunks
+  const long long my_tiles = tiles > blockIdx.x ? (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+  const long long chunks = my_tiles * per_tile;
+  // Thread 0: chunks requested and multiplied so far; chunk k is the k % per_tile-th of the weights, in slot k % 3.
+  long long requested = 0, used = 0;
+  uint32_t done_parity = 0;
+  bool failed = false;
+  auto request = [&] {  // every slot whose products are done, in order; false when a wait gave up
+    while (requested < chunks && requested < used + kPredictSlots) {
+      const int slot = static_cast<int>(requested % kPredictSlots);
+      if (requested >= kPredictSlots &&
+          !tc::mbar_wait(empty + slot, static_cast<uint32_t>(requested / kPredictSlots - 1) & 1u))
+        return false;
+      tc::mbar_arrive_tx(full + slot, chunk_bytes);
+      tc::bulk_copy(W + slot * chunk_bytes, reinterpret_cast<const unsigned char*>(g.weights) + (requested % per_tile) * chunk_bytes,
+                    chunk_bytes, full + slot);
+      ++requested;
+    }
+    return true;
+  };
+  if (tid == 0) request();
+  for (long long tile = blockIdx.x; tile < tiles && !failed; tile += gridDim.x) {
+    const long long row = tile * kBM + tid;
+    {  // the point's features, rounded to BF16, zero-padded to 64
+      const float* const x = g.x + row * g.n_in;
+      for (int c = 0; c < 8; ++c) {
+        __align__(16) bf16 v[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = __float2bfloat16_rn(row < g.n && 8 * c + e < g.n_in ? x[8 * c + e] : 0.0f);
+        *reinterpret_cast<uint4*>(A + (c * (kBM / 8) + (tid >> 3)) * 128 + (tid & 7) * 16) = *reinterpret_cast<const uint4*>(v);
+      }
+    }
+    float out = 0.0f;
+    for (int l = 0; l < g.depth; ++l) {
+      tc::fence_proxy_async();  // the activations, visible to the tensor core
+      tc::fence_before_sync();
+      __syncthreads();
+      if (tid == 0) {
+        tc::fence_after_sync();
+        const int nc = (l == 0 ? 64 : width) / kPredictChunk;
+        const uint32_t a0 = tc::smem_addr(A);
+        bool ok = true;
+        for (int c = 0; c < nc && ok; ++c) {
+          const int slot = static_cast<int>(used % kPredictSlots);
+          ok = tc::mbar_wait(full + slot, static_cast<uint32_t>(used / kPredictSlots) & 1u);
+          if (!ok) break;
+          const uint32_t b0 = tc::smem_addr(W + slot * chunk_bytes);
+#pragma unroll
+          for (int s = 0; s < kPredictChunk / 16; ++s) {
+            const uint64_t ad = tc::smem_desc(a0 + (c * (kPredictChunk / 8) + 2 * s) * (kBM / 8) * 128, (kBM / 8) * 128, 128);
+            const uint64_t bd = tc::smem_desc(b0 + 2 * s * n8 * 128, static_cast<uint32_t>(n8 * 128), 128);
+            tc::mma_bf16(tmem, ad, bd, idesc, (c > 0 || s > 0) ? 1u : 0u);
+          }
+          tc::commit(empty + slot);
+          ++used;
+          if (c == nc - 1) tc::commit(done);
+          // the chunk after the next two, into the slot of the chunk before this one
+          if (c + 1 < nc || l + 1 < g.depth || tile + gridDim.x < tiles) {
+            const long long keep = used;
+            used = keep - 1;  // this chunk's slot is not waited for yet
+            ok = request();
+            used = keep;
+          }
+        }
+        if (!ok) atomicExch(g.error_flag, 1);
+      }
+      const bool ok = tc::mbar_wait(done, done_parity);
+      if (__syncthreads_or(!ok)) {
+        failed = true;
+        break;
+      }
+      done_parity ^= 1u;
+      tc::fence_after_sync();
+      // bias, SiLU, BF16: the next layer's A operand, or the output layer's sum
+      const float* const bias = g.bias + l * width;
+      for (int j = 0; j < width / 16; ++j) {
+        uint32_t r[16];
+        tc::tmem_ld16(tmem + (static_cast<uint32_t>(warp * 32) << 16) + static_cast<uint32_t>(j * 16), r);
+        __align__(16) bf16 v[16];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) v[e] = __float2bfloat16_rn(silu(__uint_as_float(r[e]) + __ldg(bias + j * 16 + e)));
+        if (l + 1 < g.depth) {
+#pragma unroll
+          for (int c = 0; c < 2; ++c)
+            *reinterpret_cast<uint4*>(A + ((2 * j + c) * (kBM / 8) + (tid >> 3)) * 128 + (tid & 7) * 16) =
+                reinterpret_cast<const uint4*>(v)[c];
+        } else {
+#pragma unroll
+          for (int e = 0; e < 16; ++e) out += __bfloat162float(v[e]) * __ldg(g.wo + j * 16 + e);
+        }
+      }
+    }
+    if (!failed && row < g.n) g.y[row] = out + g.bo[0];
+  }
+  if (failed) {
+    if (tid == 0) {
+      atomicExch(g.error_flag, 1);
+      // bounded waits for this block's copies and products in flight, so that none lands after the block has left
+      for (long long k = used; k < requested; ++k)
+        tc::mbar_wait(full + k % kPredictSlots, static_cast<uint32_t>(k / kPredictSlots) & 1u);
+      for (long long k = used > kPredictSlots ? used - kPredictSlots : 0; k < used; ++k)
+        tc::mbar_wait(empty + k % kPredictSlots, static_cast<uint32_t>(k / kPredictSlots) & 1u);
+    }
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  if (warp == 0) tc::tmem_dealloc(tmem, static_cast<uint32_t>(width));
+}
+
+// W (out x in, FP32) -> BF16 chunks of 32 inputs in the B operand's layout: core matrices of 8 outputs x 8 inputs, outputs
+// adjacent (n8 = out / 8 of them), inputs n8 apart.
+__global__ void pack_weights_kernel(const float* __restrict__ w, int out, int in, bf16* __restrict__ packed) {
+  const int total = out * in, n8 = out / 8;
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+    const int n = t / in, k = t - n * in;
+    packed[(k / kPredictChunk) * out * kPredictChunk + (((k % kPredictChunk) / 8) * n8 + n / 8) * 64 + (n % 8) * 8 + k % 8] =
+        __float2bfloat16_rn(w[t]);
+  }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -491,6 +675,13 @@ struct spo_mlp {
   DevBuf<bf16> g16, dz16, dzt, at;
   DevBuf<long long> idx;
   long long step = 0;
+  // prediction: features and outputs of a chunk of points (grown to the largest call's, at most kPredictRows points),
+  // packed weights and the biases of all layers
+  static constexpr long long kPredictRows = 1 << 20;
+  DevBuf<float> px, py, pbias;
+  DevBuf<bf16> packed;
+  int sms = 0;
+  spo_host::RawCopier copier;
 
   ~spo_mlp() {
     if (stream) cudaStreamDestroy(stream);
@@ -806,18 +997,45 @@ int spo_mlp_set_parameters(spo_mlp* m, const float* in) {
 int spo_mlp_predict(spo_mlp* m, const float* x, long long n, float* y) {
   return guarded_mlp(m, [&] {
     need(x && y && n > 0, "spo_mlp_predict: bad arguments");
-    constexpr long long chunk = 1 << 16;
-    m->ensure_capacity(std::min(n, chunk));
-    DevBuf<float> xd;
-    xd.alloc(static_cast<std::size_t>(std::min(n, chunk) * m->n_in));
-    for (long long i0 = 0; i0 < n; i0 += chunk) {
-      const long long rows = std::min(chunk, n - i0);
-      ck(cudaMemcpyAsync(xd.p, x + i0 * m->n_in, sizeof(float) * rows * m->n_in, cudaMemcpyHostToDevice, m->stream),
-         "upload");
-      m->load_rows(xd.p, nullptr, nullptr, rows);
-      m->forward(rows);
-      ck(cudaMemcpyAsync(y + i0, m->out.p, sizeof(float) * rows, cudaMemcpyDeviceToHost, m->stream), "download");
-      ck(cudaStreamSynchronize(m->stream), "predict");
+    const long long most = std::min(n, spo_mlp::kPredictRows);
+    if (m->px.n < static_cast<std::size_t>(most * m->n_in)) m->px.alloc(static_cast<std::size_t>(most * m->n_in));
+    if (m->py.n < static_cast<std::size_t>(most)) m->py.alloc(static_cast<std::size_t>(most));
+    if (!m->packed.p) {
+      std::size_t total = 0;
+      for (const auto& l : m->layers) total += static_cast<std::size_t>(l->in) * l->out;
+      m->packed.alloc(total);
+      m->pbias.alloc(static_cast<std::size_t>(m->depth) * m->width);
+      ck(cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, m->device), "SM count");
+      ck(cudaFuncSetAttribute(mlp_predict_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              static_cast<int>(predict_smem(256))), "predict smem");
+    }
+    std::size_t off = 0;
+    for (int l = 0; l < m->depth; ++l) {
+      const Layer& L = *m->layers[l];
+      pack_weights_kernel<<<grid_for(static_cast<long long>(L.in) * L.out), 256, 0, m->stream>>>(L.w.p, L.out, L.in, m->packed.p + off);
+      off += static_cast<std::size_t>(L.in) * L.out;
+      ck(cudaMemcpyAsync(m->pbias.p + static_cast<std::size_t>(l) * m->width, L.b.p, sizeof(float) * m->width,
+                         cudaMemcpyDeviceToDevice, m->stream), "biases");
+    }
+    ck(cudaGetLastError(), "pack weights");
+    for (long long i0 = 0; i0 < n; i0 += most) {
+      const long long rows = std::min(most, n - i0);
+      const std::size_t in_bytes = sizeof(float) * static_cast<std::size_t>(rows * m->n_in), out_bytes = sizeof(float) * rows;
+      if (spo_host::RawCopier::wanted(x, in_bytes))
+        ck(m->copier.to_device(x + i0 * m->n_in, m->px.p, in_bytes, m->device), "upload");
+      else
+        ck(cudaMemcpyAsync(m->px.p, x + i0 * m->n_in, in_bytes, cudaMemcpyHostToDevice, m->stream), "upload");
+      PredictArgs g{m->px.p, rows, m->n_in, m->width, m->depth, m->packed.p, m->pbias.p, m->wo.p, m->bo.p, m->py.p, m->error_flag.p};
+      const long long tiles = (rows + kBM - 1) / kBM;
+      mlp_predict_kernel<<<static_cast<unsigned>(std::min<long long>(tiles, 2ll * m->sms)), 128, predict_smem(m->width), m->stream>>>(g);
+      ck(cudaGetLastError(), "predict launch");
+      if (spo_host::RawCopier::wanted(y, out_bytes)) {
+        ck(cudaStreamSynchronize(m->stream), "predict");
+        ck(m->copier.to_host(m->py.p, y + i0, out_bytes, m->device), "download");
+      } else {
+        ck(cudaMemcpyAsync(y + i0, m->py.p, out_bytes, cudaMemcpyDeviceToHost, m->stream), "download");
+        ck(cudaStreamSynchronize(m->stream), "predict");
+      }
     }
     m->check_flag();
   });
