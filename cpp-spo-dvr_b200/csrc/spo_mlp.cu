@@ -2,22 +2,24 @@
 // B200 tensor cores through tcgen05.mma, FP32 accumulators in tensor memory.
 //
 // One GEMM kernel serves the forward pass and both backward products: C[M x N] = A[M x K] B[N x K]^T
-// with A and B BF16, K-major (row-major with K contiguous), K a multiple of 64, N <= 256:
-//   - a block of 128 threads owns 128 rows of C; warp 0 allocates 256 tensor-memory columns;
-//   - per K chunk of 64, the threads stage A (128 x 64) and B (N x 64) in shared memory in the
+// with A and B BF16, K-major (row-major with K contiguous), K and N multiples of 64:
+//   - a block of 128 threads owns 128 rows and 64 columns of C (tiles of 256 columns left the forward product of a
+//     batch of 4096 on 32 blocks: 48 us, 4096 x 256 x 256); warp 0 allocates 64 tensor-memory columns;
+//   - per K chunk of 64, the threads stage A (128 x 64) and B (64 x 64) in shared memory in the
 //     canonical K-major layout without swizzle (8-row x 16-byte core matrices: K chunks LBO bytes
 //     apart, 8-row groups SBO = 128 bytes apart), make the writes visible to the tensor core
 //     (fence.proxy.async), and one thread issues four tcgen05.mma (M 128, N, K 16) and a
 //     tcgen05.commit on the stage's mbarrier; two stages alternate, so chunk k + 1 is staged while
 //     the tensor core multiplies chunk k (a stage is rewritten after its previous commit, bounded wait);
 //   - epilogue: each warp reads its 32 accumulator lanes (tcgen05.ld 32x32b, 16 columns at a time)
-//     and writes FP32, BF16, or bias + SiLU (pre-activation FP32, activation BF16);
+//     and writes FP32, BF16, or bias + SiLU (pre-activation FP32, activation BF16, row-major and transposed);
 //   - split K: blockIdx.y takes a share of the K chunks and writes its own FP32 partial, summed in a
 //     fixed order afterwards (weight gradients, where K is the batch).
 // Prediction on many points is one kernel (mlp_predict_kernel): a block keeps the activations of 128 points in shared
 // memory through all layers.
-// Everything else (output layer, loss, SiLU derivative, transposes, Adam) is plain SIMT, with fixed-
-// order reductions so that a training run is repeatable.
+// Everything else (output layer, loss, SiLU derivative, Adam) is plain SIMT, with fixed-order reductions so that a
+// training run is repeatable. A training step of 4 layers is 23 launches and no wait for the host (losses are summed on
+// the device and read once per epoch); as 60 launches with two waits it took 0.9 ms, 0.5 of them the products.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -151,15 +153,16 @@ struct GemmArgs {
   const float* bias;
   bf16* out16;  // kEpiBf16: the product; kEpiBiasSilu: the activation
   long long ld16;
+  bf16* out16t;  // kEpiBiasSilu: the activation transposed (column c at c * ldt), or null
+  long long ldt;
   int* error_flag;
 };
 
-constexpr int kBM = 128, kBK = 64, kBNMax = 256;
-constexpr std::size_t kStageBytes = static_cast<std::size_t>(kBM + kBNMax) * kBK * 2;  // one A and one B chunk
-constexpr std::size_t kGemmSmem = 2 * kStageBytes + 64;                                  // two stages, barriers
-// At most two blocks per SM: the number whose 256 tensor-memory columns fit the SM's 512 together.
-constexpr std::size_t kGemmLaunchSmem = kGemmSmem;
-static_assert(3 * kGemmLaunchSmem > 228 * 1024, "two blocks per SM at most");
+constexpr int kBM = 128, kBK = 64, kBN = 64;
+constexpr std::size_t kStageBytes = static_cast<std::size_t>(kBM + kBN) * kBK * 2;  // one A and one B chunk
+// Two stages, barriers: at most four blocks per SM, whose 64 tensor-memory columns each fit the SM's 512 together.
+constexpr std::size_t kGemmLaunchSmem = 2 * kStageBytes + 64;
+static_assert(5 * kGemmLaunchSmem > 228 * 1024, "four blocks per SM at most");
 
 __device__ __forceinline__ float silu(float z) { return z / (1.0f + __expf(-z)); }
 
@@ -170,7 +173,7 @@ __global__ void __launch_bounds__(128) gemm_tn_kernel(GemmArgs g) {
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem + 2 * kStageBytes);  // one per stage
   uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 2);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (warp == 0) tc::tmem_alloc(tslot, 256);
+  if (warp == 0) tc::tmem_alloc(tslot, kBN);
   if (tid == 0) {
     tc::mbar_init(bar, 1);
     tc::mbar_init(bar + 1, 1);
@@ -179,19 +182,19 @@ __global__ void __launch_bounds__(128) gemm_tn_kernel(GemmArgs g) {
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = *tslot;
-  const int m0 = blockIdx.x * kBM;
-  const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(g.n >> 3) << 17) |
+  const int m0 = blockIdx.x * kBM, n0 = blockIdx.z * kBN;
+  const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kBN >> 3) << 17) |
                          (static_cast<uint32_t>(kBM >> 4) << 24);
   const int nk = g.k / kBK;
   const int kc_first = static_cast<int>(static_cast<long long>(nk) * blockIdx.y / gridDim.y);
   const int kc_last = static_cast<int>(static_cast<long long>(nk) * (blockIdx.y + 1) / gridDim.y);
-  // A: core (r8, kc) at (kc * 16 + r8) * 128; B: core (r8, kc) at (kc * 32 + r8) * 128
+  // A: core (r8, kc) at (kc * 16 + r8) * 128; B: core (r8, kc) at (kc * 8 + r8) * 128
   // All of a thread's 16-byte loads of a chunk are issued before the first is stored.
   auto stage = [&](int st, int kc) {
     unsigned char* As = smem + st * kStageBytes;
     unsigned char* Bs = As + kBM * kBK * 2;
     const int k0 = kc * kBK;
-    constexpr int NA = kBM * 8 / 128, NB = kBNMax * 8 / 128;
+    constexpr int NA = kBM * 8 / 128, NB = kBN * 8 / 128;
     uint4 va[NA], vb[NB];
 #pragma unroll
     for (int i = 0; i < NA; ++i) {
@@ -202,7 +205,7 @@ __global__ void __launch_bounds__(128) gemm_tn_kernel(GemmArgs g) {
 #pragma unroll
     for (int i = 0; i < NB; ++i) {
       const int p = tid + 128 * i, r = p >> 3, c = p & 7;
-      if (p < g.n * 8) vb[i] = *reinterpret_cast<const uint4*>(g.b + static_cast<long long>(r) * g.ldb + k0 + 8 * c);
+      vb[i] = *reinterpret_cast<const uint4*>(g.b + static_cast<long long>(n0 + r) * g.ldb + k0 + 8 * c);
     }
 #pragma unroll
     for (int i = 0; i < NA; ++i) {
@@ -212,7 +215,7 @@ __global__ void __launch_bounds__(128) gemm_tn_kernel(GemmArgs g) {
 #pragma unroll
     for (int i = 0; i < NB; ++i) {
       const int p = tid + 128 * i, r = p >> 3, c = p & 7;
-      if (p < g.n * 8) *reinterpret_cast<uint4*>(Bs + (c * (kBNMax / 8) + (r >> 3)) * 128 + (r & 7) * 16) = vb[i];
+      *reinterpret_cast<uint4*>(Bs + (c * (kBN / 8) + (r >> 3)) * 128 + (r & 7) * 16) = vb[i];
     }
     tc::fence_proxy_async();  // the generic writes, visible to the tensor core
   };
@@ -231,7 +234,7 @@ __global__ void __launch_bounds__(128) gemm_tn_kernel(GemmArgs g) {
 #pragma unroll
       for (int s = 0; s < kBK / 16; ++s) {
         const uint64_t ad = tc::smem_desc(a0 + 2 * s * (kBM / 8) * 128, (kBM / 8) * 128, 128);
-        const uint64_t bd = tc::smem_desc(b0 + 2 * s * (kBNMax / 8) * 128, (kBNMax / 8) * 128, 128);
+        const uint64_t bd = tc::smem_desc(b0 + 2 * s * (kBN / 8) * 128, (kBN / 8) * 128, 128);
         tc::mma_bf16(tmem, ad, bd, idesc, (kc > kc_first || s > 0) ? 1u : 0u);
       }
       tc::commit(bar + st);
@@ -272,36 +275,48 @@ __global__ void __launch_bounds__(128) gemm_tn_kernel(GemmArgs g) {
       if (pending >> k & 1u) tc::mbar_wait(bar + k, parity >> k & 1u);
   } else if (kc_last > kc_first) {
     const int row = m0 + warp * 32 + lane;
-    for (int j = 0; j < g.n / 16; ++j) {
+    for (int j = 0; j < kBN / 16; ++j) {
+      const int col = n0 + j * 16;
       uint32_t r[16];
       tc::tmem_ld16(tmem + (static_cast<uint32_t>(warp * 32) << 16) + static_cast<uint32_t>(j * 16), r);
       if (row < g.m) {
         if (g.epi == kEpiF32) {
-          float* dst = g.c + blockIdx.y * g.c_split_stride + static_cast<long long>(row) * g.ldc + j * 16;
+          float* dst = g.c + blockIdx.y * g.c_split_stride + static_cast<long long>(row) * g.ldc + col;
 #pragma unroll
           for (int e = 0; e < 16; e += 4)
             *reinterpret_cast<float4*>(dst + e) = make_float4(__uint_as_float(r[e]), __uint_as_float(r[e + 1]),
                                                               __uint_as_float(r[e + 2]), __uint_as_float(r[e + 3]));
         } else if (g.epi == kEpiBf16) {
-          bf16* dst = g.out16 + static_cast<long long>(row) * g.ld16 + j * 16;
+          bf16* dst = g.out16 + static_cast<long long>(row) * g.ld16 + col;
+          __align__(16) bf16 v[16];
 #pragma unroll
-          for (int e = 0; e < 16; ++e) dst[e] = __float2bfloat16_rn(__uint_as_float(r[e]));
+          for (int e = 0; e < 16; ++e) v[e] = __float2bfloat16_rn(__uint_as_float(r[e]));
+          reinterpret_cast<uint4*>(dst)[0] = reinterpret_cast<const uint4*>(v)[0];
+          reinterpret_cast<uint4*>(dst)[1] = reinterpret_cast<const uint4*>(v)[1];
         } else {
-          float* zd = g.c + static_cast<long long>(row) * g.ldc + j * 16;
-          bf16* ad = g.out16 + static_cast<long long>(row) * g.ld16 + j * 16;
+          float* zd = g.c + static_cast<long long>(row) * g.ldc + col;
+          bf16* ad = g.out16 + static_cast<long long>(row) * g.ld16 + col;
+          __align__(16) float z[16];
+          __align__(16) bf16 v[16];
 #pragma unroll
           for (int e = 0; e < 16; ++e) {
-            const float z = __uint_as_float(r[e]) + g.bias[j * 16 + e];
-            zd[e] = z;
-            ad[e] = __float2bfloat16_rn(silu(z));
+            z[e] = __uint_as_float(r[e]) + __ldg(g.bias + col + e);
+            v[e] = __float2bfloat16_rn(silu(z[e]));
           }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) reinterpret_cast<float4*>(zd)[e] = reinterpret_cast<const float4*>(z)[e];
+          reinterpret_cast<uint4*>(ad)[0] = reinterpret_cast<const uint4*>(v)[0];
+          reinterpret_cast<uint4*>(ad)[1] = reinterpret_cast<const uint4*>(v)[1];
+          if (g.out16t)
+#pragma unroll
+            for (int e = 0; e < 16; ++e) g.out16t[(col + e) * g.ldt + row] = v[e];
         }
       }
     }
   }
   tc::fence_before_sync();
   __syncthreads();
-  if (warp == 0) tc::tmem_dealloc(tmem, 256);
+  if (warp == 0) tc::tmem_dealloc(tmem, kBN);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -475,142 +490,163 @@ __global__ void pack_weights_kernel(const float* __restrict__ w, int out, int in
 // ------------------------------------------------------------------------------------------------
 // SIMT kernels
 // ------------------------------------------------------------------------------------------------
-// x (n x n_in, FP32) rows idx[i] (or i) -> BF16 rows of width w (zero-padded).
-__global__ void gather_inputs_kernel(const float* __restrict__ x, int n_in, const long long* __restrict__ idx,
-                                     long long rows, int w, bf16* __restrict__ out) {
-  const long long total = rows * w;
-  for (long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; t < total;
-       t += static_cast<long long>(gridDim.x) * blockDim.x) {
+// The batch: rows idx[i] (or i) of x (n x n_in, FP32) as BF16 rows of width w (zero-padded) and transposed, and of y.
+__global__ void gather_kernel(const float* __restrict__ x, const float* __restrict__ y, int n_in, const long long* __restrict__ idx,
+                              long long rows, int w, bf16* __restrict__ out, bf16* __restrict__ out_t, float* __restrict__ yb) {
+  const long long total = rows * w, step = static_cast<long long>(gridDim.x) * blockDim.x;
+  const long long first = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+  for (long long t = first; t < total; t += step) {
     const long long i = t / w;
     const int c = static_cast<int>(t - i * w);
-    const long long src = idx ? idx[i] : i;
-    out[t] = __float2bfloat16_rn(c < n_in ? x[src * n_in + c] : 0.0f);
+    out[t] = __float2bfloat16_rn(c < n_in ? x[(idx ? idx[i] : i) * n_in + c] : 0.0f);
   }
-}
-__global__ void gather_targets_kernel(const float* __restrict__ y, const long long* __restrict__ idx, long long rows,
-                                      float* __restrict__ out) {
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < rows;
-       i += static_cast<long long>(gridDim.x) * blockDim.x)
-    out[i] = y[idx ? idx[i] : i];
-}
-
-// out[i] = sum_k a[i][k] w[k] + b, one warp per row, fixed order (lane-strided sums, then a fixed tree).
-__global__ void output_layer_kernel(const bf16* __restrict__ a, int w, const float* __restrict__ wo,
-                                    const float* __restrict__ bo, long long rows, float* __restrict__ out) {
-  const long long row = blockIdx.x * static_cast<long long>(blockDim.x / 32) + threadIdx.x / 32;
-  const int lane = threadIdx.x & 31;
-  if (row >= rows) return;
-  float s = 0.0f;
-  for (int k = lane; k < w; k += 32) s += __bfloat162float(a[row * w + k]) * wo[k];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) out[row] = s + bo[0];
+  for (long long t = first; t < total; t += step) {
+    const int c = static_cast<int>(t / rows);
+    const long long i = t - c * rows;
+    out_t[t] = __float2bfloat16_rn(c < n_in ? x[(idx ? idx[i] : i) * n_in + c] : 0.0f);
+  }
+  for (long long i = first; i < rows; i += step) yb[i] = y[idx ? idx[i] : i];
 }
 
-// d[i] = 2 (out[i] - y[i]) / rows; the squared errors summed per block in a fixed order.
-__global__ void loss_kernel(const float* __restrict__ out, const float* __restrict__ y, long long rows,
-                            float* __restrict__ d, double* __restrict__ block_sums) {
-  __shared__ double part[256];
-  double s = 0.0;
-  for (long long i = blockIdx.x * 256ll + threadIdx.x; i < rows; i += 256ll * gridDim.x) {
-    const float e = out[i] - y[i];
-    d[i] = 2.0f * e / static_cast<float>(rows);
-    s += static_cast<double>(e) * e;
-  }
-  part[threadIdx.x] = s;
-  __syncthreads();
-  for (int w = 128; w > 0; w >>= 1) {
-    if (threadIdx.x < w) part[threadIdx.x] += part[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) block_sums[blockIdx.x] = part[0];
-}
-
-// Column sums over rows, one block per column, fixed order: sum_i v(i, col).
-// mode 0: gw_out[col] = sum_i d[i] a[i][col]; mode 1: gb[col] = sum_i dzf[i][col] (FP32 matrix).
-__global__ void column_sums_kernel(int mode, const float* __restrict__ d, const bf16* __restrict__ a,
-                                   const float* __restrict__ m32, int w, long long rows, float* __restrict__ out) {
-  __shared__ float part[256];
-  const int col = blockIdx.x;
-  float s = 0.0f;
-  for (long long i = threadIdx.x; i < rows; i += 256) {
-    s += mode == 0 ? d[i] * __bfloat162float(a[i * w + col]) : m32[i * w + col];
-  }
-  part[threadIdx.x] = s;
-  __syncthreads();
-  for (int k = 128; k > 0; k >>= 1) {
-    if (threadIdx.x < k) part[threadIdx.x] += part[threadIdx.x + k];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[col] = part[0];
-}
-
-// Gradient into the last hidden activation: g[i][k] = d[i] w_out[k] (FP32).
-__global__ void output_backward_kernel(const float* __restrict__ d, const float* __restrict__ wo, int w,
-                                       long long rows, float* __restrict__ g) {
-  const long long total = rows * w;
-  for (long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; t < total;
-       t += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const long long i = t / w;
-    g[t] = d[i] * wo[t - i * w];
-  }
-}
-
-// dz = g * SiLU'(z), kept in FP32 (bias gradient) and BF16 (the products), both row-major.
-__global__ void silu_backward_kernel(const float* __restrict__ g, const bf16* __restrict__ g16, const float* __restrict__ z,
-                                     long long total, float* __restrict__ dz, bf16* __restrict__ dz16) {
-  for (long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; t < total;
-       t += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const float zz = z[t];
-    const float s = 1.0f / (1.0f + __expf(-zz));
-    const float gv = g ? g[t] : __bfloat162float(g16[t]);
-    const float v = gv * s * (1.0f + zz * (1.0f - s));
-    dz[t] = v;
-    dz16[t] = __float2bfloat16_rn(v);
-  }
-}
-
-// out[c][r] = in[r][c] for an R x C BF16 matrix (32 x 32 tiles through shared memory).
-__global__ void transpose_kernel(const bf16* __restrict__ in, long long rows, int cols, bf16* __restrict__ out) {
-  __shared__ bf16 tile[32][33];
-  const long long r0 = static_cast<long long>(blockIdx.y) * 32;
-  const int c0 = blockIdx.x * 32;
-  for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-    const long long r = r0 + k;
-    const int c = c0 + threadIdx.x;
-    tile[k][threadIdx.x] = (r < rows && c < cols) ? in[r * cols + c] : __float2bfloat16_rn(0.0f);
-  }
-  __syncthreads();
-  for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-    const int c = c0 + k;
-    const long long r = r0 + threadIdx.x;
-    if (c < cols && r < rows) out[static_cast<long long>(c) * rows + r] = tile[threadIdx.x][k];
-  }
-}
-
-// out[i] = sum over the split partials in order.
-__global__ void sum_partials_kernel(const float* __restrict__ parts, int n_parts, long long stride, long long n,
-                                    float* __restrict__ out) {
-  for (long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; t < n;
-       t += static_cast<long long>(gridDim.x) * blockDim.x) {
+// The output layer, the error and the loss of a batch: out = sum_k a[i][k] w[k] + b, d[i] = 2 (out - y[i]) / rows, and per
+// block of 64 rows the sum of its squared errors. One warp per row at a time, fixed order (lane-strided sums, then a fixed
+// tree).
+__global__ void __launch_bounds__(256) output_loss_kernel(const bf16* __restrict__ a, int w, const float* __restrict__ wo,
+                                                          const float* __restrict__ bo, const float* __restrict__ y,
+                                                          long long rows, float* __restrict__ d, double* __restrict__ block_sums) {
+  __shared__ double part[8];
+  const int warp = threadIdx.x / 32, lane = threadIdx.x & 31;
+  double sq = 0.0;
+#pragma unroll 2
+  for (int r = 0; r < 8; ++r) {
+    const long long row = blockIdx.x * 64ll + warp * 8 + r;
+    if (row >= rows) break;
     float s = 0.0f;
-    for (int p = 0; p < n_parts; ++p) s += parts[p * stride + t];
-    out[t] = s;
+    for (int k = lane; k < w; k += 32) s += __bfloat162float(a[row * w + k]) * wo[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    const float e = s + bo[0] - y[row];
+    if (lane == 0) d[row] = 2.0f * e / static_cast<float>(rows);
+    sq += static_cast<double>(e) * e;
+  }
+  if (lane == 0) part[warp] = sq;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int k = 0; k < 8; ++k) t += part[k];
+    block_sums[blockIdx.x] = t;
   }
 }
 
-// Adam on FP32 parameters.
-__global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
-                            float* __restrict__ v, long long n, float lr, float b1, float b2, float c1, float c2,
-                            float eps) {
-  for (long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; t < n;
+// dz = g SiLU'(z) for a tile of 64 rows x 64 columns: BF16 row-major and transposed (the operands of the products) and the
+// tile's column sums of dz (bias gradient). g is the BF16 gradient of the layer above, or for the last hidden layer (top)
+// d[i] w_out[k]; there also the column sums of d[i] a[i][k] (output weights) and, in column tile 0, of d (output bias).
+__global__ void __launch_bounds__(256) silu_backward_kernel(const bf16* __restrict__ g16, const float* __restrict__ d,
+                                                            const float* __restrict__ wo, const bf16* __restrict__ a,
+                                                            const float* __restrict__ z, long long rows, int w, bf16* __restrict__ dz16,
+                                                            bf16* __restrict__ dzt, float* __restrict__ db, float* __restrict__ dwo,
+                                                            float* __restrict__ dbo) {
+  __shared__ bf16 tile[64][66];
+  __shared__ float part[2][4][64];
+  const int c = threadIdx.x % 64, q = threadIdx.x / 64;
+  const int col = blockIdx.x * 64 + c;
+  const long long r0 = blockIdx.y * 64ll;
+  float sum = 0.0f, sum_wo = 0.0f;
+#pragma unroll 4
+  for (int k = 0; k < 16; ++k) {
+    const long long i = r0 + q * 16 + k;
+    const float zz = z[i * w + col];
+    const float s = 1.0f / (1.0f + __expf(-zz));
+    const float gv = g16 ? __bfloat162float(g16[i * w + col]) : d[i] * wo[col];
+    const float v = gv * s * (1.0f + zz * (1.0f - s));
+    const bf16 h = __float2bfloat16_rn(v);
+    dz16[i * w + col] = h;
+    tile[q * 16 + k][c] = h;
+    sum += v;
+    if (!g16) sum_wo += d[i] * __bfloat162float(a[i * w + col]);
+  }
+  part[0][q][c] = sum;
+  part[1][q][c] = sum_wo;
+  __syncthreads();
+  if (q == 0) {
+    db[blockIdx.y * static_cast<long long>(w) + col] = part[0][0][c] + part[0][1][c] + part[0][2][c] + part[0][3][c];
+    if (!g16) dwo[blockIdx.y * static_cast<long long>(w) + col] = part[1][0][c] + part[1][1][c] + part[1][2][c] + part[1][3][c];
+  }
+  if (!g16 && blockIdx.x == 0 && threadIdx.x == 0) {
+    float t = 0.0f;
+    for (int k = 0; k < 64; ++k) t += d[r0 + k];
+    dbo[blockIdx.y] = t;
+  }
+  for (int k = q; k < 64; k += 4) dzt[(blockIdx.x * 64ll + k) * rows + r0 + c] = tile[c][k];
+}
+
+// Sums of partials in order: weights (n_parts of nw), then biases (n_rows_parts of w); for the last hidden layer also the
+// output layer's gradients and the loss (the block sums of output_loss_kernel over `rows`).
+__global__ void sum_partials_kernel(const float* __restrict__ parts, int n_parts, long long nw, float* __restrict__ gw,
+                                    const float* __restrict__ db, int n_row_parts, int w, float* __restrict__ gb,
+                                    const float* __restrict__ dwo, float* __restrict__ gwo, const float* __restrict__ dbo,
+                                    float* __restrict__ gbo, const double* __restrict__ loss_parts, int n_loss, long long rows,
+                                    double* __restrict__ loss) {
+  const long long total = nw + w + (dwo ? w + 2 : 0);
+  for (long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; t < total;
        t += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const float gt = g[t];
-    const float mt = b1 * m[t] + (1.0f - b1) * gt;
-    const float vt = b2 * v[t] + (1.0f - b2) * gt * gt;
-    m[t] = mt;
-    v[t] = vt;
-    p[t] -= lr * (mt / c1) / (sqrtf(vt / c2) + eps);
+    if (t < nw) {
+      float s = 0.0f;
+#pragma unroll 8
+      for (int p = 0; p < n_parts; ++p) s += parts[p * nw + t];
+      gw[t] = s;
+    } else if (t < nw + 2 * w) {
+      const bool hidden = t < nw + w;
+      const int k = static_cast<int>(t - nw) - (hidden ? 0 : w);
+      const float* const src = hidden ? db : dwo;
+      float s = 0.0f;
+#pragma unroll 8
+      for (int p = 0; p < n_row_parts; ++p) s += src[static_cast<long long>(p) * w + k];
+      (hidden ? gb : gwo)[k] = s;
+    } else if (t == nw + 2 * w) {
+      float s = 0.0f;
+#pragma unroll 8
+      for (int p = 0; p < n_row_parts; ++p) s += dbo[p];
+      gbo[0] = s;
+    } else {
+      double s = 0.0;
+#pragma unroll 8
+      for (int p = 0; p < n_loss; ++p) s += loss_parts[p];
+      loss[0] = s / static_cast<double>(rows);
+    }
+  }
+}
+
+// Adam on FP32 parameters, all tensors in one launch (blockIdx.y), with the BF16 copies of the weight matrices (rows x
+// cols): row-major and transposed.
+struct AdamTensor {
+  float *p, *m, *v;
+  const float* g;
+  long long n;
+  int cols;  // 0: no BF16 copies
+  bf16 *wb, *wt;
+};
+constexpr int kAdamTensors = 18;  // 8 layers of W and b, the output layer's
+struct AdamArgs {
+  AdamTensor t[kAdamTensors];
+};
+__global__ void adam_kernel(const __grid_constant__ AdamArgs args, float lr, float b1, float b2, float c1, float c2, float eps) {
+  const AdamTensor& a = args.t[blockIdx.y];
+  for (long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; t < a.n;
+       t += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const float gt = a.g[t];
+    const float mt = b1 * a.m[t] + (1.0f - b1) * gt;
+    const float vt = b2 * a.v[t] + (1.0f - b2) * gt * gt;
+    a.m[t] = mt;
+    a.v[t] = vt;
+    const float p = a.p[t] - lr * (mt / c1) / (sqrtf(vt / c2) + eps);
+    a.p[t] = p;
+    if (a.cols > 0) {
+      const int r = static_cast<int>(t / a.cols), c = static_cast<int>(t - static_cast<long long>(r) * a.cols);
+      const bf16 h = __float2bfloat16_rn(p);
+      a.wb[t] = h;
+      a.wt[c * (a.n / a.cols) + r] = h;
+    }
   }
 }
 
@@ -627,6 +663,8 @@ __global__ void weights_to_bf16_kernel(const float* __restrict__ w, int rows, in
   }
 }
 
+constexpr int kSplits = 32;  // K splits of the weight gradients
+
 unsigned grid_for(long long n, int threads = 256) {
   return static_cast<unsigned>(std::min<long long>(std::max<long long>((n + threads - 1) / threads, 1), 148 * 16));
 }
@@ -639,14 +677,16 @@ struct DevBuf {
   U* p = nullptr;
   std::size_t n = 0;
   void alloc(std::size_t count) {
+    free();
+    ck(cudaMalloc(&p, sizeof(U) * std::max<std::size_t>(count, 1)), "cudaMalloc");
+    n = count;
+  }
+  void free() {
     if (p) cudaFree(p);
     p = nullptr;
-    n = count;
-    ck(cudaMalloc(&p, sizeof(U) * std::max<std::size_t>(count, 1)), "cudaMalloc");
+    n = 0;
   }
-  ~DevBuf() {
-    if (p) cudaFree(p);
-  }
+  ~DevBuf() { free(); }
 };
 
 struct Layer {
@@ -667,17 +707,31 @@ struct spo_mlp {
   DevBuf<int> error_flag;
   // per-batch work space (capacity rows)
   long long cap = 0;
-  DevBuf<bf16> x16;                        // rows x in_pad
-  std::vector<std::unique_ptr<DevBuf<float>>> z;   // per layer: rows x width (pre-activation)
-  std::vector<std::unique_ptr<DevBuf<bf16>>> act;  // per layer: rows x width (activation)
-  DevBuf<float> out, yb, d, g32, dz32, partials;
-  DevBuf<double> loss_parts;
-  DevBuf<bf16> g16, dz16, dzt, at;
-  DevBuf<long long> idx;
+  DevBuf<bf16> x16, x16t;                  // rows x in_pad, and transposed
+  std::vector<std::unique_ptr<DevBuf<float>>> z;           // per layer: rows x width (pre-activation)
+  std::vector<std::unique_ptr<DevBuf<bf16>>> act, act_t;   // per layer: rows x width (activation), and transposed
+  DevBuf<float> yb, d, db, dwo, dbo, partials;             // db, dwo, dbo: column sums per 64 rows
+  DevBuf<double> loss_parts, loss;                         // per 64 rows; per step of an epoch
+  DevBuf<bf16> g16, dz16, dzt;
   long long step = 0;
   // prediction: features and outputs of a chunk of points (grown to the largest call's, at most kPredictRows points),
   // packed weights and the biases of all layers
   static constexpr long long kPredictRows = 1 << 20;
+  // and the points of a training set, kept for the next call up to kKeepBytes
+  static constexpr std::size_t kKeepBytes = 64ull << 20;
+  DevBuf<float> tx, ty;
+  DevBuf<long long> tperm;
+  void training_set(long long n, bool order) {
+    if (tx.n < static_cast<std::size_t>(n * n_in)) tx.alloc(static_cast<std::size_t>(n * n_in));
+    if (ty.n < static_cast<std::size_t>(n)) ty.alloc(static_cast<std::size_t>(n));
+    if (order && tperm.n < static_cast<std::size_t>(n)) tperm.alloc(static_cast<std::size_t>(n));
+  }
+  void release_training_set() {
+    if (sizeof(float) * (tx.n + ty.n) + sizeof(long long) * tperm.n <= kKeepBytes) return;
+    tx.free();
+    ty.free();
+    tperm.free();
+  }
   DevBuf<float> px, py, pbias;
   DevBuf<bf16> packed;
   int sms = 0;
@@ -697,25 +751,28 @@ struct spo_mlp {
     if (rows <= cap) return;
     cap = ((rows + 127) / 128) * 128;
     x16.alloc(cap * in_pad);
+    x16t.alloc(cap * in_pad);
     z.clear();
     act.clear();
+    act_t.clear();
     for (int l = 0; l < depth; ++l) {
       z.push_back(std::make_unique<DevBuf<float>>());
       z.back()->alloc(cap * width);
-      act.push_back(std::make_unique<DevBuf<bf16>>());
-      act.back()->alloc(cap * width);
+      for (auto* v : {&act, &act_t}) {
+        v->push_back(std::make_unique<DevBuf<bf16>>());
+        v->back()->alloc(cap * width);
+      }
     }
-    out.alloc(cap);
     yb.alloc(cap);
     d.alloc(cap);
-    g32.alloc(cap * width);
-    dz32.alloc(cap * width);
+    db.alloc(cap / 64 * width);
+    dwo.alloc(cap / 64 * width);
+    dbo.alloc(cap / 64);
     g16.alloc(cap * width);
     dz16.alloc(cap * width);
     dzt.alloc(cap * width);
-    at.alloc(cap * std::max(width, in_pad));
-    idx.alloc(cap);
-    loss_parts.alloc(256);
+    loss_parts.alloc(cap / 64);
+    if (!loss.p) loss.alloc(1);
   }
 
   void refresh_bf16() {
@@ -726,70 +783,53 @@ struct spo_mlp {
   }
 
   void gemm(const bf16* a, long long lda, const bf16* b, long long ldb, int m, int n, int k, int epi, float* c,
-            long long ldc, const float* bias, bf16* out16, long long ld16, int splits = 1, long long split_stride = 0) {
-    need(k % kBK == 0 && n % 16 == 0 && n >= 16 && n <= kBNMax && lda % 8 == 0 && ldb % 8 == 0, "gemm shape");
-    GemmArgs g{a, lda, b, ldb, m, n, k, epi, c, ldc, split_stride, bias, out16, ld16, error_flag.p};
-    const dim3 grid(static_cast<unsigned>((m + kBM - 1) / kBM), static_cast<unsigned>(splits));
+            long long ldc, const float* bias, bf16* out16, long long ld16, int splits = 1, long long split_stride = 0,
+            bf16* out16t = nullptr, long long ldt = 0) {
+    need(k % kBK == 0 && n % kBN == 0 && n > 0 && lda % 8 == 0 && ldb % 8 == 0, "gemm shape");
+    GemmArgs g{a, lda, b, ldb, m, n, k, epi, c, ldc, split_stride, bias, out16, ld16, out16t, ldt, error_flag.p};
+    const dim3 grid(static_cast<unsigned>((m + kBM - 1) / kBM), static_cast<unsigned>(splits), static_cast<unsigned>(n / kBN));
     gemm_tn_kernel<<<grid, 128, kGemmLaunchSmem, stream>>>(g);
     ck(cudaGetLastError(), "gemm launch");
   }
 
-  // Forward pass of `rows` rows already in x16; output in out.
+  // Forward pass of `rows` rows already in x16 / yb; the output layer's errors in d, the squared ones in loss_parts.
   void forward(long long rows) {
     const bf16* a = x16.p;
     int k = in_pad;
     for (int l = 0; l < depth; ++l) {
       Layer& L = *layers[l];
-      gemm(a, k, L.wb.p, L.in, static_cast<int>(rows), width, k, kEpiBiasSilu, z[l]->p, width, L.b.p, act[l]->p, width);
+      gemm(a, k, L.wb.p, L.in, static_cast<int>(rows), width, k, kEpiBiasSilu, z[l]->p, width, L.b.p, act[l]->p, width, 1, 0,
+           l + 1 < depth ? act_t[l]->p : nullptr, rows);
       a = act[l]->p;
       k = width;
     }
-    output_layer_kernel<<<static_cast<unsigned>((rows + 7) / 8), 256, 0, stream>>>(act[depth - 1]->p, width, wo.p, bo.p,
-                                                                                  rows, out.p);
+    output_loss_kernel<<<static_cast<unsigned>((rows + 63) / 64), 256, 0, stream>>>(act[depth - 1]->p, width, wo.p, bo.p, yb.p, rows,
+                                                                                 d.p, loss_parts.p);
     ck(cudaGetLastError(), "output layer");
   }
 
-  // Loss and all gradients for `rows` rows in x16 / yb. Returns the loss.
-  double backward(long long rows) {
-    const unsigned lb = static_cast<unsigned>(std::min<long long>((rows + 255) / 256, 256));
-    loss_kernel<<<lb, 256, 0, stream>>>(out.p, yb.p, rows, d.p, loss_parts.p);
-    column_sums_kernel<<<width, 256, 0, stream>>>(0, d.p, act[depth - 1]->p, nullptr, width, rows, gwo.p);
-    column_sums_kernel<<<1, 256, 0, stream>>>(1, nullptr, nullptr, d.p, 1, rows, gbo.p);
-    output_backward_kernel<<<grid_for(rows * width), 256, 0, stream>>>(d.p, wo.p, width, rows, g32.p);
-    ck(cudaGetLastError(), "output backward");
-    const int splits = static_cast<int>(std::min<long long>(64, rows / kBK));
+  // All gradients for `rows` rows (a multiple of 64) after forward(); the mean squared error into loss[slot].
+  void backward(long long rows, long long slot) {
+    // split K so that the weight gradients (few tiles of C) fill the GPU; every split has its chunks of kBK rows
+    const int splits = static_cast<int>(std::min<long long>(kSplits, rows / kBK));
+    const int row_parts = static_cast<int>(rows / 64);
     for (int l = depth - 1; l >= 0; --l) {
       Layer& L = *layers[l];
-      const bool first_grad = l == depth - 1;
-      silu_backward_kernel<<<grid_for(rows * width), 256, 0, stream>>>(first_grad ? g32.p : nullptr, g16.p, z[l]->p,
-                                                                      rows * width, dz32.p, dz16.p);
-      column_sums_kernel<<<width, 256, 0, stream>>>(1, nullptr, nullptr, dz32.p, width, rows, L.gb.p);
+      const bool top = l == depth - 1;
+      silu_backward_kernel<<<dim3(static_cast<unsigned>(width / 64), static_cast<unsigned>(row_parts)), 256, 0, stream>>>(
+          top ? nullptr : g16.p, d.p, wo.p, act[l]->p, z[l]->p, rows, width, dz16.p, dzt.p, db.p, dwo.p, dbo.p);
+      ck(cudaGetLastError(), "silu backward");
       // gW = dz^T a_in : A = dz^T (width x rows), B = a_in^T (in x rows), K = rows
-      const bf16* a_in = l == 0 ? x16.p : act[l - 1]->p;
-      const dim3 tb(32, 8);
-      transpose_kernel<<<dim3((width + 31) / 32, static_cast<unsigned>((rows + 31) / 32)), tb, 0, stream>>>(
-          dz16.p, rows, width, dzt.p);
-      transpose_kernel<<<dim3((L.in + 31) / 32, static_cast<unsigned>((rows + 31) / 32)), tb, 0, stream>>>(
-          a_in, rows, L.in, at.p);
-      ck(cudaGetLastError(), "transposes");
       const long long wsz = static_cast<long long>(L.out) * L.in;
-      gemm(dzt.p, rows, at.p, rows, L.out, L.in, static_cast<int>(rows), kEpiF32, partials.p, L.in, nullptr, nullptr, 0,
-           splits, wsz);
-      sum_partials_kernel<<<grid_for(wsz), 256, 0, stream>>>(partials.p, splits, wsz, wsz, L.gw.p);
+      gemm(dzt.p, rows, l == 0 ? x16t.p : act_t[l - 1]->p, rows, L.out, L.in, static_cast<int>(rows), kEpiF32, partials.p, L.in,
+           nullptr, nullptr, 0, splits, wsz);
+      sum_partials_kernel<<<grid_for(wsz + 2 * width + 2), 256, 0, stream>>>(
+          partials.p, splits, wsz, L.gw.p, db.p, row_parts, width, L.gb.p, top ? dwo.p : nullptr, gwo.p, dbo.p, gbo.p, loss_parts.p,
+          static_cast<int>((rows + 63) / 64), rows, loss.p + slot);
       ck(cudaGetLastError(), "sum partials");
-      if (l > 0) {
-        // d a_in = dz W : A = dz (rows x width), B = W^T (in x width)
-        gemm(dz16.p, width, L.wt.p, L.out, static_cast<int>(rows), L.in, width, kEpiBf16, nullptr, 0, nullptr, g16.p,
-             L.in);
-      }
+      if (l > 0)  // d a_in = dz W : A = dz (rows x width), B = W^T (in x width)
+        gemm(dz16.p, width, L.wt.p, L.out, static_cast<int>(rows), L.in, width, kEpiBf16, nullptr, 0, nullptr, g16.p, L.in);
     }
-    std::vector<double> parts(lb);
-    ck(cudaMemcpyAsync(parts.data(), loss_parts.p, sizeof(double) * lb, cudaMemcpyDeviceToHost, stream), "loss");
-    ck(cudaStreamSynchronize(stream), "backward");
-    check_flag();
-    double s = 0.0;
-    for (double p : parts) s += p;
-    return s / static_cast<double>(rows);
   }
 
   void check_flag() {
@@ -802,8 +842,7 @@ struct spo_mlp {
   }
 
   void load_rows(const float* x_dev, const float* y_dev, const long long* idx_dev, long long rows) {
-    gather_inputs_kernel<<<grid_for(rows * in_pad), 256, 0, stream>>>(x_dev, n_in, idx_dev, rows, in_pad, x16.p);
-    if (y_dev) gather_targets_kernel<<<grid_for(rows), 256, 0, stream>>>(y_dev, idx_dev, rows, yb.p);
+    gather_kernel<<<grid_for(rows * in_pad), 256, 0, stream>>>(x_dev, y_dev, n_in, idx_dev, rows, in_pad, x16.p, x16t.p, yb.p);
     ck(cudaGetLastError(), "gather");
   }
 
@@ -811,15 +850,16 @@ struct spo_mlp {
     ++step;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     const float c1 = 1.0f - std::pow(b1, static_cast<float>(step)), c2 = 1.0f - std::pow(b2, static_cast<float>(step));
+    AdamArgs args{};
+    int n = 0;
     for (auto& l : layers) {
-      const long long nw = static_cast<long long>(l->in) * l->out;
-      adam_kernel<<<grid_for(nw), 256, 0, stream>>>(l->w.p, l->gw.p, l->mw.p, l->vw.p, nw, lr, b1, b2, c1, c2, eps);
-      adam_kernel<<<grid_for(l->out), 256, 0, stream>>>(l->b.p, l->gb.p, l->mb.p, l->vb.p, l->out, lr, b1, b2, c1, c2, eps);
+      args.t[n++] = {l->w.p, l->mw.p, l->vw.p, l->gw.p, static_cast<long long>(l->in) * l->out, l->in, l->wb.p, l->wt.p};
+      args.t[n++] = {l->b.p, l->mb.p, l->vb.p, l->gb.p, l->out, 0, nullptr, nullptr};
     }
-    adam_kernel<<<grid_for(width), 256, 0, stream>>>(wo.p, gwo.p, mwo.p, vwo.p, width, lr, b1, b2, c1, c2, eps);
-    adam_kernel<<<1, 256, 0, stream>>>(bo.p, gbo.p, mbo.p, vbo.p, 1, lr, b1, b2, c1, c2, eps);
+    args.t[n++] = {wo.p, mwo.p, vwo.p, gwo.p, width, 0, nullptr, nullptr};
+    args.t[n++] = {bo.p, mbo.p, vbo.p, gbo.p, 1, 0, nullptr, nullptr};
+    adam_kernel<<<dim3(64, static_cast<unsigned>(n)), 256, 0, stream>>>(args, lr, b1, b2, c1, c2, eps);
     ck(cudaGetLastError(), "adam");
-    refresh_bf16();
   }
 
   // Parameter transfer in the documented order.
@@ -937,7 +977,7 @@ int spo_mlp_create(int n_in, int width, int depth, unsigned long long seed, int 
     zeros(m->vbo, 1);
     m->error_flag.alloc(1);
     ck(cudaMemset(m->error_flag.p, 0, sizeof(int)), "error flag");
-    m->partials.alloc(static_cast<std::size_t>(64) * width * std::max(width, m->in_pad));
+    m->partials.alloc(static_cast<std::size_t>(kSplits) * width * std::max(width, m->in_pad));
     m->refresh_bf16();
     ck(cudaStreamSynchronize(m->stream), "create");
   } catch (const MlpError& e) {
@@ -1046,14 +1086,16 @@ int spo_mlp_gradients(spo_mlp* m, const float* x, const float* y, long long n, d
     need(x && y && grad && n >= kBK && n <= 65536 && n % kBK == 0,
          "spo_mlp_gradients: n must be a multiple of 64, at most 65536");
     m->ensure_capacity(n);
-    DevBuf<float> xd, yd;
-    xd.alloc(static_cast<std::size_t>(n * m->n_in));
-    yd.alloc(static_cast<std::size_t>(n));
-    ck(cudaMemcpy(xd.p, x, sizeof(float) * n * m->n_in, cudaMemcpyHostToDevice), "upload");
-    ck(cudaMemcpy(yd.p, y, sizeof(float) * n, cudaMemcpyHostToDevice), "upload");
-    m->load_rows(xd.p, yd.p, nullptr, n);
+    m->training_set(n, false);
+    ck(cudaMemcpyAsync(m->tx.p, x, sizeof(float) * n * m->n_in, cudaMemcpyHostToDevice, m->stream), "upload");
+    ck(cudaMemcpyAsync(m->ty.p, y, sizeof(float) * n, cudaMemcpyHostToDevice, m->stream), "upload");
+    m->load_rows(m->tx.p, m->ty.p, nullptr, n);
     m->forward(n);
-    const double l = m->backward(n);
+    m->backward(n, 0);
+    double l = 0.0;
+    ck(cudaMemcpyAsync(&l, m->loss.p, sizeof(double), cudaMemcpyDeviceToHost, m->stream), "loss");
+    ck(cudaStreamSynchronize(m->stream), "gradients");
+    m->check_flag();
     if (loss) *loss = l;
     long long off = 0;
     m->for_each_param([&](DevBuf<float>&, DevBuf<float>& g, long long cnt) {
@@ -1069,36 +1111,39 @@ int spo_mlp_train(spo_mlp* m, const float* x, const float* y, long long n, int e
     need(x && y && n >= batch && epochs > 0 && batch >= 128 && batch % 128 == 0 && batch <= 65536 && lr > 0.0f,
          "spo_mlp_train: bad arguments");
     m->ensure_capacity(batch);
-    DevBuf<float> xd, yd;
-    DevBuf<long long> perm;
-    xd.alloc(static_cast<std::size_t>(n * m->n_in));
-    yd.alloc(static_cast<std::size_t>(n));
-    perm.alloc(static_cast<std::size_t>(n));
-    ck(cudaMemcpy(xd.p, x, sizeof(float) * n * m->n_in, cudaMemcpyHostToDevice), "upload");
-    ck(cudaMemcpy(yd.p, y, sizeof(float) * n, cudaMemcpyHostToDevice), "upload");
+    m->training_set(n, true);
+    ck(cudaMemcpyAsync(m->tx.p, x, sizeof(float) * n * m->n_in, cudaMemcpyHostToDevice, m->stream), "upload");
+    ck(cudaMemcpyAsync(m->ty.p, y, sizeof(float) * n, cudaMemcpyHostToDevice, m->stream), "upload");
     SplitMix rng{seed};
     std::vector<long long> order(static_cast<std::size_t>(n));
     const long long steps_per_epoch = n / batch;
     const long long total_steps = steps_per_epoch * epochs;
+    if (m->loss.n < static_cast<std::size_t>(steps_per_epoch)) m->loss.alloc(static_cast<std::size_t>(steps_per_epoch));
+    std::vector<double> losses(static_cast<std::size_t>(steps_per_epoch));
     long long t = 0;
     double epoch_loss = 0.0;
     for (int e = 0; e < epochs; ++e) {
       for (long long i = 0; i < n; ++i) order[i] = i;
       for (long long i = n - 1; i > 0; --i) std::swap(order[i], order[rng.next() % static_cast<uint64_t>(i + 1)]);
-      ck(cudaMemcpy(perm.p, order.data(), sizeof(long long) * n, cudaMemcpyHostToDevice), "order");
-      epoch_loss = 0.0;
+      ck(cudaMemcpyAsync(m->tperm.p, order.data(), sizeof(long long) * n, cudaMemcpyHostToDevice, m->stream), "order");
       for (long long s = 0; s < steps_per_epoch; ++s, ++t) {
         const double frac = static_cast<double>(t) / static_cast<double>(std::max<long long>(total_steps - 1, 1));
         const float rate = static_cast<float>(lr * (0.05 + 0.95 * 0.5 * (1.0 + std::cos(3.14159265358979 * frac))));
-        m->load_rows(xd.p, yd.p, perm.p + s * batch, batch);
+        m->load_rows(m->tx.p, m->ty.p, m->tperm.p + s * batch, batch);
         m->forward(batch);
-        epoch_loss += m->backward(batch);
+        m->backward(batch, s);
         m->adam(rate);
       }
+      ck(cudaMemcpyAsync(losses.data(), m->loss.p, sizeof(double) * steps_per_epoch, cudaMemcpyDeviceToHost, m->stream), "losses");
+      ck(cudaStreamSynchronize(m->stream), "epoch");  // and before the next epoch's order is uploaded
+      m->check_flag();
+      epoch_loss = 0.0;
+      for (const double v : losses) epoch_loss += v;
       epoch_loss /= static_cast<double>(steps_per_epoch);
     }
     ck(cudaStreamSynchronize(m->stream), "train");
     m->check_flag();
+    m->release_training_set();
     if (last_epoch_loss) *last_epoch_loss = epoch_loss;
   });
 }
