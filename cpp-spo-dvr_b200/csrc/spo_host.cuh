@@ -693,7 +693,7 @@ class Step final : public StepBase {
     budget_spec_.z_absorber = up_i(za1);
     budget_spec_.r_absorber = up_i(ra1);
     budget_spec_.previous = dev<double>(e1.size());
-    budget_out_ = dev<double>(2 * spo::kBudgetMaxAbsorbers + 2);
+    budget_out_ = dev<double>(spo::kBudgetSums * (1 + spo::kSumBlocks));
     budget_abs_ = n_abs;
     budget_vol_scat_ = d.volume_scattering;
     budget_vol_spec_ = d.volume_specular;
@@ -710,9 +710,10 @@ class Step final : public StepBase {
     require(budget_abs_ > 0, "spo_norm_budget_add: spo_norm_budget_setup was not called");
     spo::block_density_kernel<T><<<static_cast<unsigned>(s_.n_zr()), 256, 0, stream_>>>(
         psi_, s_.n_xy() * s_.n_rot, densities_);
-    spo::norm_budget_kernel<T><<<1, 256, 0, stream_>>>(densities_, budget_vol_scat_, chi_, budget_vol_spec_,
-                                                      budget_scat_, budget_spec_, budget_abs_,
-                                                      budget_has_previous_ ? 1 : 0, budget_out_);
+    double* const partial = budget_out_ + spo::kBudgetSums;
+    spo::norm_budget_kernel<T><<<spo::kSumBlocks, 256, 0, stream_>>>(densities_, budget_vol_scat_, chi_, budget_vol_spec_,
+                                                                    budget_scat_, budget_spec_, budget_has_previous_ ? 1 : 0, partial);
+    spo::norm_budget_finish_kernel<<<1, 32, 0, stream_>>>(partial, spo::kSumBlocks, budget_abs_, budget_out_);
     check_cuda(cudaGetLastError(), "norm budget launch");
     const bool window = budget_has_previous_;
     if (window)
@@ -727,18 +728,19 @@ class Step final : public StepBase {
                 int surface_index, double* out) override {
     require(z && zs && r && out, "averages: null pointer");
     require(iz_analysis >= -1 && iz_analysis < s_.nzs && surface_index < s_.nzs, "averages: index out of range");
-    // The grids and the four results pass through the staging buffer (>= 8M doubles).
+    // The grids, the four results and the partial sums pass through the staging buffer (>= 8M doubles).
     double* g = reinterpret_cast<double*>(staging_);
     const long long ng = static_cast<long long>(s_.nz) + s_.nzs + s_.nr;
-    require(ng + 4 <= 2 * staging_elems_, "averages: grids larger than the staging buffer");
+    require(ng + 4 + 7 * spo::kSumBlocks <= 2 * staging_elems_, "averages: grids larger than the staging buffer");
     check_cuda(cudaMemcpyAsync(g, z, sizeof(double) * s_.nz, cudaMemcpyHostToDevice, stream_), "averages grids");
     check_cuda(cudaMemcpyAsync(g + s_.nz, zs, sizeof(double) * s_.nzs, cudaMemcpyHostToDevice, stream_), "averages grids");
     check_cuda(cudaMemcpyAsync(g + s_.nz + s_.nzs, r, sizeof(double) * s_.nr, cudaMemcpyHostToDevice, stream_),
                "averages grids");
     spo::block_density_kernel<T><<<static_cast<unsigned>(s_.n_zr()), 256, 0, stream_>>>(
         psi_, s_.n_xy() * s_.n_rot, densities_);
-    spo::averages_kernel<T><<<1, 256, 0, stream_>>>(densities_, chi_, g, s_.nz, s_.nr, s_.nzs, iz_analysis,
-                                                    surface_index, vol_scat, vol_spec, g + ng);
+    spo::averages_kernel<T><<<spo::kSumBlocks, 256, 0, stream_>>>(densities_, chi_, g, s_.nz, s_.nr, s_.nzs, iz_analysis,
+                                                                 surface_index, g + ng + 4);
+    spo::averages_finish_kernel<<<1, 32, 0, stream_>>>(g + ng + 4, spo::kSumBlocks, vol_scat, vol_spec, g + ng);
     check_cuda(cudaGetLastError(), "averages launch");
     check_cuda(cudaMemcpyAsync(out, g + ng, sizeof(double) * 4, cudaMemcpyDeviceToHost, stream_), "averages copy");
     check_cuda(cudaStreamSynchronize(stream_), "averages");

@@ -685,8 +685,8 @@ __global__ void exp_potential_kernel(const double* __restrict__ v, Vec<T>* __res
 //   loss = rho_start (1 - F) + (rho_end - F rho_start) (gamma / (1 - F) - 1),
 //   error = gamma^2 / 6 |rho_end - rho_start + loss|,
 // shared between the cell's Z absorber (z_share) and its r absorber (the rest), and the norms at the window's
-// start and end. One block, a fixed assignment of cells to threads and a fixed tree: the sums are repeatable
-// (not in the reference's serial order; they agree to rounding). The current cells replace the previous ones.
+// start and end. A fixed assignment of cells to threads and a fixed tree: the sums are repeatable (not in the reference's
+// serial order; they agree to rounding). The current cells replace the previous ones.
 constexpr int kBudgetMaxAbsorbers = 6;
 struct BudgetGrid {
   const double* exponent;  // per cell: 2 n V_opt dt of the window (0: the cell does not absorb)
@@ -696,19 +696,41 @@ struct BudgetGrid {
   double* previous;        // the cells of the previous call
   long long cells;
 };
+// kSumBlocks blocks leave their partial sums, one block adds them in order: a single block took 0.1 ms of latency for
+// 3e4 cells.
+constexpr int kSumBlocks = 64;
+// The block's sums of NV values per thread (fixed tree) into out[k * gridDim.x + blockIdx.x].
+template <int NV>
+__device__ __forceinline__ void block_sums(const double (&acc)[NV], double* __restrict__ out) {
+  __shared__ double part[NV][8];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    double v = acc[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (threadIdx.x % 32 == 0) part[k][threadIdx.x / 32] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x < NV) {
+    double v = 0.0;
+    for (int w = 0; w < 8; ++w) v += part[threadIdx.x][w];
+    out[threadIdx.x * gridDim.x + blockIdx.x] = v;
+  }
+}
+constexpr int kBudgetSums = 2 * kBudgetMaxAbsorbers + 2;  // loss, error per absorber; norm at start, at end
 template <typename T>
 __global__ void __launch_bounds__(256) norm_budget_kernel(const double* __restrict__ densities, double vol_scat,
                                                           const Vec<T>* __restrict__ chi, double vol_spec,
-                                                          BudgetGrid scat, BudgetGrid spec, int n_absorbers,
-                                                          int has_previous, double* __restrict__ out) {
-  constexpr int NV = 2 * kBudgetMaxAbsorbers + 2;  // loss, error per absorber; norm at start, at end
-  __shared__ double part[NV][256];
+                                                          BudgetGrid scat, BudgetGrid spec, int has_previous,
+                                                          double* __restrict__ partial) {
+  constexpr int NV = kBudgetSums;
   double acc[NV];
 #pragma unroll
   for (int k = 0; k < NV; ++k) acc[k] = 0.0;
   for (int grid = 0; grid < 2; ++grid) {
     const BudgetGrid& g = grid == 0 ? scat : spec;
-    for (long long k = threadIdx.x; k < g.cells; k += blockDim.x) {
+    for (long long k = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; k < g.cells;
+         k += static_cast<long long>(gridDim.x) * blockDim.x) {
       double rho_end;
       if (grid == 0) {
         rho_end = densities[k] * vol_scat;
@@ -744,40 +766,56 @@ __global__ void __launch_bounds__(256) norm_budget_kernel(const double* __restri
       g.previous[k] = rho_end;
     }
   }
-#pragma unroll
-  for (int k = 0; k < NV; ++k) part[k][threadIdx.x] = acc[k];
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w)
-#pragma unroll
-      for (int k = 0; k < NV; ++k) part[k][threadIdx.x] += part[k][threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    for (int a = 0; a < n_absorbers; ++a) {
-      out[a] = part[a][0];
-      out[n_absorbers + a] = part[kBudgetMaxAbsorbers + a][0];
-    }
-    out[2 * n_absorbers] = part[NV - 2][0];
-    out[2 * n_absorbers + 1] = part[NV - 1][0];
-  }
+  block_sums(acc, partial);
+}
+// out = losses, errors (n_absorbers each), norm at start, at end, from the blocks' partial sums.
+static __global__ void norm_budget_finish_kernel(const double* __restrict__ partial, int blocks, int n_absorbers,
+                                                 double* __restrict__ out) {
+  const int k = threadIdx.x;
+  if (k >= kBudgetSums) return;
+  double v = 0.0;
+  for (int b = 0; b < blocks; ++b) v += partial[k * blocks + b];
+  const int a = k % kBudgetMaxAbsorbers;
+  if (k >= 2 * kBudgetMaxAbsorbers) out[2 * n_absorbers + k - 2 * kBudgetMaxAbsorbers] = v;
+  else if (a < n_absorbers) out[(k / kBudgetMaxAbsorbers) * n_absorbers + a] = v;
 }
 
-// sum |psi|^2 over one (Z, r) block (n_block values) in FP64, fixed order: strided per thread, then
-// a fixed tree (src/propagation/averages.cpp:20-29).
+// sum |psi|^2 over one (Z, r) block (n_block values) in FP64, fixed order: strided per thread into four sums (16-byte
+// loads where the blocks are aligned), then a fixed tree (src/propagation/averages.cpp:20-29). Bound by the one read of psi.
 template <typename T>
-__global__ void block_density_kernel(const Vec<T>* __restrict__ psi, long long n_block, double* __restrict__ out) {
+__global__ void __launch_bounds__(256) block_density_kernel(const Vec<T>* __restrict__ psi, long long n_block,
+                                                            double* __restrict__ out) {
   __shared__ double part[256];
-  const long long base = static_cast<long long>(blockIdx.x) * n_block;
-  double s = 0.0;
-  for (long long i = threadIdx.x; i < n_block; i += blockDim.x) {
-    const Vec<T> v = psi[base + i];
-    const double re = v.x, im = v.y;
-    s += re * re + im * im;
+  const Vec<T>* const p = psi + static_cast<long long>(blockIdx.x) * n_block;
+  double s[4] = {0.0, 0.0, 0.0, 0.0};
+  auto add = [](double& t, T re, T im) {
+    const double x = re, y = im;
+    t = fma(x, x, fma(y, y, t));
+  };
+  long long done = 0;  // values taken by the 16-byte loads
+  if (sizeof(T) == 8 || (n_block % 2 == 0 && reinterpret_cast<uintptr_t>(psi) % 16 == 0)) {
+    using W = std::conditional_t<sizeof(T) == 4, float4, double2>;
+    constexpr int per = sizeof(W) / sizeof(Vec<T>);
+    const W* const w = reinterpret_cast<const W*>(p);
+    const long long n = n_block / per, whole = n / 1024 * 1024;
+    auto take = [&](double& t, const W& v) {
+      add(t, v.x, v.y);
+      if constexpr (per == 2) add(t, v.z, v.w);
+    };
+    for (long long i = threadIdx.x; i < whole; i += 1024) {
+      const W v0 = w[i], v1 = w[i + 256], v2 = w[i + 512], v3 = w[i + 768];
+      take(s[0], v0);
+      take(s[1], v1);
+      take(s[2], v2);
+      take(s[3], v3);
+    }
+    for (long long i = whole + threadIdx.x; i < n; i += 256) take(s[0], w[i]);
+    done = n * per;
   }
-  part[threadIdx.x] = s;
+  for (long long i = done + threadIdx.x; i < n_block; i += 256) add(s[0], p[i].x, p[i].y);
+  part[threadIdx.x] = (s[0] + s[1]) + (s[2] + s[3]);
   __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
+  for (int w = 128; w > 0; w >>= 1) {
     if (threadIdx.x < w) part[threadIdx.x] += part[threadIdx.x + w];
     __syncthreads();
   }
@@ -899,31 +937,28 @@ __global__ void convert_kernel(const Vec<TI>* __restrict__ in, Vec<TO>* __restri
   }
 }
 
-// Norm and position averages of the scattering plus specular wave in one block of 256 threads, FP64
-// (src/propagation/averages.cpp:37-80). grids = [z (nz) | z_specular (nzs) | r (nr)]; densities are
-// the block densities (izr = ir + nr iz). Seven sums, each strided per thread and then added in a
-// fixed tree: the scattering norm, Z and r moments, the same three on the specular grid, and the
-// specular norm between the analysis line (exclusive) and the analysis surface (inclusive).
+// Norm and position averages of the scattering plus specular wave, FP64 (src/propagation/averages.cpp:37-80). grids =
+// [z (nz) | z_specular (nzs) | r (nr)]; densities are the block densities (izr = ir + nr iz). Seven sums (the scattering
+// norm, Z and r moments, the same three on the specular grid, and the specular norm between the analysis line
+// (exclusive) and the analysis surface (inclusive)) as block sums, which one block adds in order:
 // out = {norm, <Z>, <r>, rest norm}.
 template <typename T>
 __global__ void __launch_bounds__(256) averages_kernel(const double* __restrict__ densities, const Vec<T>* __restrict__ chi,
                                                        const double* __restrict__ grids, int nz, int nr, int nzs,
-                                                       int iz_analysis, int surface_index, double vol_scat,
-                                                       double vol_spec, double* __restrict__ out) {
-  __shared__ double part[7][256];
+                                                       int iz_analysis, int surface_index, double* __restrict__ partial) {
   const double* zg = grids;
   const double* zsg = grids + nz;
   const double* rg = grids + nz + nzs;
   double acc[7] = {0, 0, 0, 0, 0, 0, 0};
-  const int n_scat = nz * nr;
-  for (int izr = threadIdx.x; izr < n_scat; izr += blockDim.x) {
+  const int n_scat = nz * nr, first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+  for (int izr = first; izr < n_scat; izr += step) {
     const double d = densities[izr];
     acc[0] += d;
     acc[1] += zg[izr / nr] * d;
     acc[2] += rg[izr % nr] * d;
   }
   const int n_spec = nzs * nr;
-  for (int k = threadIdx.x; k < n_spec; k += blockDim.x) {
+  for (int k = first; k < n_spec; k += step) {
     const int iz = k / nr;
     const int ir = k - iz * nr;
     const Vec<T> c = chi[k];
@@ -934,22 +969,23 @@ __global__ void __launch_bounds__(256) averages_kernel(const double* __restrict_
     acc[5] += rg[ir] * d;
     if (iz > iz_analysis && iz <= surface_index) acc[6] += d;
   }
-#pragma unroll
-  for (int q = 0; q < 7; ++q) part[q][threadIdx.x] = acc[q];
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) {
-#pragma unroll
-      for (int q = 0; q < 7; ++q) part[q][threadIdx.x] += part[q][threadIdx.x + w];
-    }
-    __syncthreads();
+  block_sums(acc, partial);
+}
+static __global__ void averages_finish_kernel(const double* __restrict__ partial, int blocks, double vol_scat, double vol_spec,
+                                              double* __restrict__ out) {
+  __shared__ double part[7];
+  if (threadIdx.x < 7) {
+    double v = 0.0;
+    for (int b = 0; b < blocks; ++b) v += partial[threadIdx.x * blocks + b];
+    part[threadIdx.x] = v;
   }
+  __syncthreads();
   if (threadIdx.x == 0) {
-    const double norm = part[0][0] * vol_scat + part[3][0] * vol_spec;
+    const double norm = part[0] * vol_scat + part[3] * vol_spec;
     out[0] = norm;
-    out[1] = (part[1][0] * vol_scat + part[4][0] * vol_spec) / norm;
-    out[2] = (part[2][0] * vol_scat + part[5][0] * vol_spec) / norm;
-    out[3] = part[6][0] * vol_spec;
+    out[1] = (part[1] * vol_scat + part[4] * vol_spec) / norm;
+    out[2] = (part[2] * vol_scat + part[5] * vol_spec) / norm;
+    out[3] = part[6] * vol_spec;
   }
 }
 
