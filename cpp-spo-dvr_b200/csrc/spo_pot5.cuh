@@ -152,6 +152,16 @@ __device__ __forceinline__ uint2 ld_stream2(const void* p) {
   return v;
 }
 
+// This thread's own asynchronous copies (global -> shared, past L1), in groups.
+__device__ __forceinline__ void copy16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void copy_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
+}
+
 // phi whose modulus corrections are stored together (16 or 8 bytes per pair of theta).
 constexpr int group_of(int nphi) { return nphi % 4 == 0 ? 4 : 2; }
 constexpr int kCols = 8;       // columns per item
@@ -164,11 +174,24 @@ constexpr int f_stride(int n_rot) {
 }
 // Threads per block: the phi lines of a lane take 4 nphi registers.
 constexpr int threads_of(int nphi) { return nphi > 16 ? 384 : nphi > 8 ? 512 : 640; }
-// Bytes of a team's buffer: the columns of its item, then (H = 2) the values that its warps exchange.
-constexpr std::size_t team_bytes(int n_rot, int nphi, int h) {
-  const std::size_t f = sizeof(float2) * kCols * static_cast<std::size_t>(f_stride(n_rot));
+// With two warps per team and 28 or 32 phi, the lines (112 or 128 registers) leave no registers for exp(i A) entries in
+// flight: each lane copies its entries into the team's buffer instead, kBatches batches of 4 phi (and their corrections)
+// ahead, and the row of rot(dt/2) comes with the columns. Configuration 3: 4.31 ms against 4.92 with loads two batches of
+// two phi ahead in registers and rot(dt/2) through L1; phi 24 with symmetry maps 1.35 against 1.25 ms, phi 18 0.547
+// against 0.525, one warp per team 0.78 against 0.55: there the loads in registers stay.
+constexpr bool ring_of(int nphi, int h) { return h == 2 && nphi >= 28 && nphi % 4 == 0; }
+constexpr int kBatches = 3, kBatchBytes = 5 * 512;
+// Bytes of a team's buffer, used in turn for the columns of its item, (ring) its warps' exp(i A) entries and (H = 2) the
+// values that the warps exchange; with (ring) the row of rot(dt/2).
+constexpr std::size_t buffer_bytes(int n_rot, int nphi, int h) {
+  std::size_t f = sizeof(float2) * kCols * static_cast<std::size_t>(f_stride(n_rot));
   const std::size_t x = h == 2 ? static_cast<std::size_t>(nphi) * 32 * sizeof(float4) : 0;
-  return f > x ? f : x;
+  const std::size_t r = ring_of(nphi, h) ? 2 * kBatches * kBatchBytes : 0;
+  f = f > x ? f : x;
+  return f > r ? f : r;
+}
+constexpr std::size_t team_bytes(int n_rot, int nphi, int h) {
+  return buffer_bytes(n_rot, nphi, h) + (ring_of(nphi, h) ? sizeof(double2) * static_cast<std::size_t>(n_rot) : 0);
 }
 
 }  // namespace pot5
@@ -194,6 +217,7 @@ template <int NPHI, int H>
 __global__ void __launch_bounds__(pot5::threads_of(NPHI), 1) potential5_kernel(Pot5Args g, int* __restrict__ error_flag) {
   using namespace pot5;
   constexpr int G = group_of(NPHI);
+  constexpr bool RING = ring_of(NPHI, H);
   const PotArgs<float>& a = g.p;
   const int n_rot = a.n_rot, n_xy = a.n_xy, nr = a.nr;
   const int fcs = f_stride(n_rot);
@@ -207,6 +231,7 @@ __global__ void __launch_bounds__(pot5::threads_of(NPHI), 1) potential5_kernel(P
   unsigned char* const own = reinterpret_cast<unsigned char*>(bars + ((teams + 1) & ~1)) + team * team_bytes(n_rot, NPHI, H);
   float2* const F = reinterpret_cast<float2*>(own);               // [c][irot], columns of fcs values
   float4* const EX = reinterpret_cast<float4*>(own);              // [reading warp][slot pair][lane], after F is consumed
+  double2* const rot_row = reinterpret_cast<double2*>(own + buffer_bytes(n_rot, NPHI, H));  // RING: rot(dt/2) at the item's r point
   if (lane == 0 && h == 0) mbar_init(bar, 1);
   mbar_init_fence();
   for (int k = threadIdx.x; k < 32 * (g.n_fwd + g.n_back); k += blockDim.x) mats[k] = g.frags[k];
@@ -228,8 +253,11 @@ __global__ void __launch_bounds__(pot5::threads_of(NPHI), 1) potential5_kernel(P
     if (g.bulk) {
       if (h == 0) {
         fence_proxy_async();
-        if (lane == 0) mbar_arrive_tx(bar, col_bytes * ncol + g.extra_tx);
+        const int izr = col0 / n_xy;
+        const bool row = RING && (col0 + ncol - 1) / n_xy == izr;  // one r point
+        if (lane == 0) mbar_arrive_tx(bar, col_bytes * ncol + (row ? 2 * col_bytes : 0u) + g.extra_tx);
         __syncwarp();
+        if (row && lane == kCols) bulk_copy(rot_row, g.rot + (izr % nr) * n_rot, 2 * col_bytes, bar);
         if (lane < ncol) bulk_copy(F + lane * fcs, a.psi + static_cast<long long>(col0 + lane) * n_rot, col_bytes, bar);
       }
     } else {
@@ -316,17 +344,55 @@ __global__ void __launch_bounds__(pot5::threads_of(NPHI), 1) potential5_kernel(P
     team_sync<H>(bar_id);
     const int next = item + step;
     if (next < g.n_items) {
-      if (H == 1) issue(next);  // every lane of the team has read F
+      if (H == 1 && g.bulk) issue(next);  // every lane of the team has read F
       prefetch(next);
     }
 
     // ---- phi transform, exp(i A), inverse phi transform of the lane's two lines
-    rdft<NPHI, +1>(x);
-    {
-      const int tp = min(4 * h + t, g.pairs - 1);  // theta beyond the grid: zero lines
-      const long long e = (static_cast<long long>(izr) * a.n_rep + (g.phi_map ? __ldg(a.rep_of + ixy) : ixy)) * NPHI * g.pairs;
-      const float4* et = g.table + e + tp;
-      const __half2* em = g.mods + e + tp * G;
+    const int tp = min(4 * h + t, g.pairs - 1);  // theta beyond the grid: zero lines
+    const long long e0 = (static_cast<long long>(izr) * a.n_rep + (g.phi_map ? __ldg(a.rep_of + ixy) : ixy)) * NPHI * g.pairs;
+    const float4* et = g.table + e0 + tp;
+    const __half2* em = g.mods + e0 + tp * G;
+    auto apply = [&](auto p, float4 e4, uint32_t m2) {  // exp_mul_m on both lines
+      const F2 m = f2(mod_lo(m2), mod_hi(m2)) * f2(5.9604644775390625e-8f);  // 2^-24
+      const C2 e = c2(f2(e4.x, e4.y), f2(e4.z, e4.w));
+      x[p] = cadd(x[p], cmul2(x[p], e, c2(m * (f2(1.0f) + e.x), m * e.y)));
+    };
+    if constexpr (RING) {
+      constexpr int NB = NPHI / G;
+      unsigned char* const ring = own + h * kBatches * kBatchBytes + lane * 16;
+      auto request = [&](auto b) {
+        constexpr int B = SPO_CV(b);
+        unsigned char* const to = ring + (B % kBatches) * kBatchBytes;
+        if (g.phi_map == nullptr) {
+          static_for<0, G>([&](auto i) { copy16(to + SPO_CV(i) * 512, et + (B * G + SPO_CV(i)) * g.pairs); });
+          copy16(to + G * 512, em + B * G * g.pairs);
+        } else {
+          const uint8_t* const map = g.phi_map + ixy * NPHI + B * G;
+          uint32_t* const m = reinterpret_cast<uint32_t*>(to + G * 512);
+          static_for<0, G>([&](auto i) {
+            const int pm = __ldg(map + SPO_CV(i));
+            copy16(to + SPO_CV(i) * 512, et + pm * g.pairs);
+            m[SPO_CV(i)] = __ldg(reinterpret_cast<const uint32_t*>(em + (pm / G) * G * g.pairs + pm % G));
+          });
+        }
+        copy_commit();
+      };
+      static_for<0, kBatches>([&](auto b) { request(b); });
+      rdft<NPHI, +1>(x);
+      static_for<0, NB>([&](auto b) {
+        constexpr int B = SPO_CV(b);
+        copy_wait<(NB - 1 - B < kBatches - 1 ? NB - 1 - B : kBatches - 1)>();
+        const unsigned char* const from = ring + (B % kBatches) * kBatchBytes;
+        const uint4 m = *reinterpret_cast<const uint4*>(from + G * 512);
+        const uint32_t m2[4] = {m.x, m.y, m.z, m.w};
+        static_for<0, G>([&](auto i) {
+          apply(std::integral_constant<int, B * G + SPO_CV(i)>{}, *reinterpret_cast<const float4*>(from + SPO_CV(i) * 512), m2[SPO_CV(i)]);
+        });
+        if constexpr (B + kBatches < NB) request(std::integral_constant<int, B + kBatches>{});
+      });
+    } else {
+      rdft<NPHI, +1>(x);
       // Two phi per batch, the next batch's loads in flight while one is applied. The empty asm statements tie a batch's
       // address to values of the batch before the last, so that the compiler does not collect all loads in front (and
       // spill the lines to make room for them).
@@ -351,11 +417,6 @@ __global__ void __launch_bounds__(pot5::threads_of(NPHI), 1) potential5_kernel(P
           }
         }
       };
-      auto apply = [&](auto p, float4 e4, uint32_t m2) {  // exp_mul_m on both lines
-        const F2 m = f2(mod_lo(m2), mod_hi(m2)) * f2(5.9604644775390625e-8f);  // 2^-24
-        const C2 e = c2(f2(e4.x, e4.y), f2(e4.z, e4.w));
-        x[p] = cadd(x[p], cmul2(x[p], e, c2(m * (f2(1.0f) + e.x), m * e.y)));
-      };
       asm volatile("" : "+l"(et), "+l"(em), "+l"(x[NPHI - 1].x.v));
       load(std::integral_constant<int, 0>{});
       static_for<0, NB>([&](auto b) {
@@ -370,7 +431,13 @@ __global__ void __launch_bounds__(pot5::threads_of(NPHI), 1) potential5_kernel(P
 
     // ---- transposed contraction, rot(dt/2), store
     float2* const out = a.psi + static_cast<long long>(col) * n_rot;
-    const double2* const rot = g.rot + ir * n_rot;
+    // (RING: the row in shared memory, if the item lies at one point, as in issue())
+    const bool row = RING && g.bulk && (item * kCols) / n_xy == min(item * kCols + kCols - 1, g.n_cols - 1) / n_xy;
+    const double2* const rot = row ? rot_row : g.rot + ir * n_rot;
+    auto rot_at = [&](int irot) {
+      if constexpr (RING) return rot[irot];
+      else return __ldg(rot + irot);
+    };
     auto finish = [&](int irot, double2 w, double re, double im) {
       out[irot] = make_float2(static_cast<float>(re * w.x - im * w.y), static_cast<float>(re * w.y + im * w.x));
     };
@@ -383,7 +450,7 @@ __global__ void __launch_bounds__(pot5::threads_of(NPHI), 1) potential5_kernel(P
         const double* const m0 = mb + 32 * (s.w + (jt * H + h) * 2);
         const double* const m1 = mb + 32 * (s.w + (jt * H + H - 1 - h) * 2);
         const int j = 8 * jt + t;
-        const double2 wa = __ldg(rot + s.x + min(j, nj - 1)), wb = __ldg(rot + s.x + min(j + 4, nj - 1));
+        const double2 wa = rot_at(s.x + min(j, nj - 1)), wb = rot_at(s.x + min(j + 4, nj - 1));
         double r0 = 0, r1 = 0, q0 = 0, q1 = 0;
 #pragma unroll
         for (int i = 0; i < 2 * H; ++i) {
@@ -409,6 +476,7 @@ __global__ void __launch_bounds__(pot5::threads_of(NPHI), 1) potential5_kernel(P
       float4* const to = EX + (h ^ 1) * (NPHI / 2) * 32 + lane;
       const float4* const from = EX + h * (NPHI / 2) * 32 + lane;
       float4 mine[NPHI / 2];
+      if (RING) team_sync<H>(bar_id);  // both warps have read their exp(i A) entries
       static_for<0, NPHI / 2>([&](auto q) {
         float2 e0, e1, o0, o1;
         c2_split(x[2 * SPO_CV(q)], e0, e1);
@@ -426,6 +494,10 @@ __global__ void __launch_bounds__(pot5::threads_of(NPHI), 1) potential5_kernel(P
       team_sync<H>(bar_id);
       // the zeros behind the columns again, then the next item's columns
       if (h == 0) F[c * fcs + n_rot + t] = make_float2(0.0f, 0.0f);
+      if (next < g.n_items) issue(next);
+    }
+    if (H == 1 && !g.bulk) {
+      __syncwarp();
       if (next < g.n_items) issue(next);
     }
     if (!g.bulk) team_sync<H>(bar_id);
