@@ -239,16 +239,41 @@ struct KinLaunch {
   std::size_t smem = 0;
 };
 template <typename T>
-KinLaunch<T> kin_configure(int map, int n1, int n2, int lanes_per_tile, long long window);
+KinLaunch<T> kin_configure(int map, int n1, int n2, bool unit, int lanes_per_tile, long long window);
 
-// The levels of kin_kernel for an axis of n points, false if it has none: two coprime sizes up to 16 (no twiddles), else
-// any two.
-inline bool kin_split(int n, bool prime, int& map, int& n1, int& n2) {
+// The lengths and square grids whose mixed form runs kin_kernel on pairs of lanes although another register kernel has
+// them: where pairs measured faster (ms per launch of 0.2 to 0.8 GB, pairs against one lane per thread):
+//   Z, r: 48 0.242/0.259, 96 0.485/0.560, 128 1.56/1.64 (configuration 3), 160 0.256/0.296, 176 0.170/0.226, 192
+//     0.288/0.300, 224 0.182/0.223, 256 0.162/0.188;
+//   x = y: 2 0.034/0.036, 4 0.074/0.098, 8 0.173/0.227, 16 2.07/2.13 (configuration 3).
+// Not 24, 32 and 64 (short lines: the other kernels keep more warps in flight and run at 4.1 to 4.9 TB/s; 0.056/0.050,
+// 0.189/0.190, 0.232/0.224), 40, 56, 80 and 112 (radices 5 and 7 sum in FP64, line by line; 0.173/0.130, 0.090/0.066,
+// 0.120/0.114, 0.134/0.125), 6 and 12 (0.199/0.188, 0.463/0.445).
+inline bool kin_paired(int n, int& map, int& n1, int& n2) {
+  switch (n) {
+    case 48: map = spo::kPrime, n1 = 3, n2 = 16; return true;
+    case 96: map = spo::kPrime, n1 = 3, n2 = 32; return true;
+    case 128: map = spo::kTwiddle, n1 = 8, n2 = 16; return true;
+    case 160: map = spo::kPrime, n1 = 5, n2 = 32; return true;
+    case 176: map = spo::kPrime, n1 = 11, n2 = 16; return true;
+    case 192: map = spo::kTwiddle, n1 = 12, n2 = 16; return true;
+    case 224: map = spo::kPrime, n1 = 7, n2 = 32; return true;
+    case 256: map = spo::kTwiddle, n1 = 16, n2 = 16; return true;
+    default: return false;
+  }
+}
+inline bool kin_paired_xy(int n) { return n == 2 || n == 4 || n == 8 || n == 16; }
+
+// The levels of kin_kernel for an axis of n points, false if another kernel takes it: the mixed form's pairs above, or for
+// lengths no register kernel has two coprime sizes up to 16 (no twiddles), else any two, the most balanced split first.
+inline bool kin_split(int n, bool mixed, bool prime, int& map, int& n1, int& n2) {
+  if (mixed && kin_paired(n, map, n1, n2) && (prime || map != spo::kPrime)) return true;
+  map = -1;
+  if (axis2_supported(n)) return false;
   auto size_ok = [](int k) { return k >= 2 && k <= 16 && k != 13; };
   for (const bool coprime : {true, false}) {
     if (coprime && !prime) continue;
-    for (int b = 16; b >= 2; --b) {  // the most balanced split: the smallest larger factor
-      const int larger = 18 - b;
+    for (int larger = 2; larger <= 16; ++larger) {
       if (n % larger != 0 || !size_ok(larger) || !size_ok(n / larger) || n / larger > larger) continue;
       int x = larger, y = n / larger;
       while (y) std::swap(x %= y, y);
@@ -1006,7 +1031,7 @@ class Step final : public StepBase {
     const int lanes = tile > 0 ? tile : ax.n1 * ax.n2 >= 80 ? 16 : 32;
     auto it = ax.launches.find({lanes, a.window});
     if (it == ax.launches.end())
-      it = ax.launches.emplace(std::make_pair(lanes, a.window), kin_configure<T>(ax.map, ax.n1, ax.n2, lanes, a.window)).first;
+      it = ax.launches.emplace(std::make_pair(lanes, a.window), kin_configure<T>(ax.map, ax.n1, ax.n2, ax.unit[0] && ax.unit[1], lanes, a.window)).first;
     const KinLaunch<T>& l = it->second;
     const long long per_tile = static_cast<long long>(spo::KinLine<T>::lanes) << l.log_lines;
     const long long blocks_per_group = (a.window + per_tile - 1) / per_tile, n_tiles = blocks_per_group * a.groups * outer;
@@ -1016,10 +1041,10 @@ class Step final : public StepBase {
     a.blocks_per_group = static_cast<unsigned>(blocks_per_group);
     a.n_tiles = static_cast<unsigned>(n_tiles);
     a.log_lines = l.log_lines;
-    a.aligned = (a.stride | a.outer_stride | a.group_stride | a.lane_offset | (a.data - psi_)) % 2 == 0 ? 1 : 0;
+    a.aligned = sizeof(T) == 8 || (a.stride | a.outer_stride | a.group_stride | a.lane_offset | (a.data - psi_)) % 2 == 0 ? 1 : 0;
     a.table = ax.table[half];
     a.scale = ax.scale[half];
-    a.unit = ax.unit[half];
+    a.unit = ax.unit[0] && ax.unit[1] ? 1 : 0;
     l.kernel<<<static_cast<unsigned>(std::min(n_tiles, l.blocks)), l.threads, l.smem, stream_>>>(a);
   }
   void axis_psi(const char* name, double bytes, long long outer, const spo::FftPlan& plan, const V* tw,
@@ -1396,7 +1421,7 @@ class Step final : public StepBase {
       const double s0 = std::abs(f[0]);
       double p = 1.0;
       if (std::isfinite(s0) && s0 > 1e-30 && s0 < 1e30) p = std::exp2(std::floor(std::log2(s0) + 1e-9));
-      std::vector<float> h(static_cast<std::size_t>(12 * n));
+      std::vector<float> h(12 * static_cast<std::size_t>(n) + 8 * tw.size());
       auto put = [&](std::size_t word, double x, double y) {
         h[4 * word] = h[4 * word + 1] = static_cast<float>(x);
         h[4 * word + 2] = h[4 * word + 3] = static_cast<float>(y);
@@ -1406,14 +1431,13 @@ class Step final : public StepBase {
         const cplx g = s > 0.0 ? cplx(p * (f[k].real() / s - 1.0), p * (f[k].imag() / s)) : cplx(-p, 0.0);
         put(2 * k, g.real(), g.imag());
         put(2 * k + 1, g.real() - static_cast<float>(g.real()), g.imag() - static_cast<float>(g.imag()));
-        put(2 * static_cast<std::size_t>(n) + k, r, r - static_cast<float>(r));
+        put(2 * n + 2 * tw.size() + k, r, r - static_cast<float>(r));
         if (!(std::fabs(r - 1.0) < 1e-14)) ax.unit[half] = 0;  // rounding of |s e^{i phi}| in FP64
       }
       ax.scale[half] = static_cast<float>(p);
-      h.resize(12 * static_cast<std::size_t>(n) + 8 * tw.size());
       for (std::size_t k = 0; k < tw.size(); ++k) {
-        put(3 * static_cast<std::size_t>(n) + 2 * k, tw[k].real(), tw[k].imag());
-        put(3 * static_cast<std::size_t>(n) + 2 * k + 1, tw[k].real() - static_cast<float>(tw[k].real()),
+        put(2 * n + 2 * k, tw[k].real(), tw[k].imag());
+        put(2 * n + 2 * k + 1, tw[k].real() - static_cast<float>(tw[k].real()),
             tw[k].imag() - static_cast<float>(tw[k].imag()));
       }
       double2* d = dev<double2>(h.size() / 4);
@@ -1498,18 +1522,19 @@ class Step final : public StepBase {
     const double xy_scale = (sx * sy) * ((1.0 / (s.nx * sx)) * (1.0 / (s.ny * sy)));
     xyk_full_ = upload_factor(scaled(complex_array(d.xy_kinetic_full, nxy, "xy_kinetic_full"), xy_scale));
     xyk_half_ = upload_factor(scaled(complex_array(d.xy_kinetic_half, nxy, "xy_kinetic_half"), xy_scale));
-    // kin_kernel: the kinetic passes of sizes the other register kernels do not have.
+    // kin_kernel: where the mixed form's pairs are faster, and both forms' sizes that no other register kernel has.
     use_v2_ = !(std::getenv("SPO_B200_KERNELS") && std::string(std::getenv("SPO_B200_KERNELS")) == "v1");
     use_pfa_ = !(std::getenv("SPO_B200_PFA") && std::string(std::getenv("SPO_B200_PFA")) == "0");
     if (use_v2_) {
+      constexpr bool mixed = sizeof(T) == 4;
       auto axis = [&](KinAxis& ax, int n, const double* full, const double* half) {
-        if (axis2_supported(n) || !kin_split(n, use_pfa_, ax.map, ax.n1, ax.n2)) return;
+        if (!kin_split(n, mixed, use_pfa_, ax.map, ax.n1, ax.n2)) return;
         kin_table(ax, 0, scaled(complex_array(full, n, "kinetic factors"), 1.0 / n));
         kin_table(ax, 1, scaled(complex_array(half, n, "kinetic factors"), 1.0 / n));
       };
       axis(kin_z_, s.nz, d.z_kinetic_full, d.z_kinetic_half);
       axis(kin_r_, s.nr, d.r_kinetic_full, d.r_kinetic_half);
-      if (kin_xy_size(s.nx) && kin_xy_size(s.ny) && (s.nx != s.ny || !xy2_supported(s.nx))) {
+      if (kin_xy_size(s.nx) && kin_xy_size(s.ny) && (s.nx != s.ny || !xy2_supported(s.nx) || (mixed && kin_paired_xy(s.nx)))) {
         kin_xy_.map = spo::kXy;
         kin_xy_.n1 = s.ny;
         kin_xy_.n2 = s.nx;

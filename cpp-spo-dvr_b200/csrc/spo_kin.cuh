@@ -8,7 +8,8 @@
 //             interaction region's potential step.
 //
 // The mixed form takes two adjacent lanes per thread as packed FP32 pairs (spo_pair.cuh): 16-byte accesses and half
-// the instructions. Issue bound it before (65 to 75 % of the slots at 4 TB/s: every constant is exact to ~2^-48, which
+// the instructions; the next tile's points are copied to shared memory (cp.async, each thread its own) while a tile is
+// transformed. Issue bound it before (65 to 75 % of the slots at 4 TB/s: every constant is exact to ~2^-48, which
 // costs two to three times the instructions of plain FP32 products); one lane per thread took 1.64, 1.59 and 1.84 ms
 // on configuration 3 (Z 128, r 48, 16 x 16). A grid of resident blocks loops over the tiles, so that the tables are
 // staged in shared memory once per block, not once per tile. kinetic factors s e^{i phi} are applied as p (x + x g)
@@ -19,7 +20,7 @@
 // they ran on before are 3 to 10 times slower (T_Z of 90 points, r 36, x = y = 10: 1.12 ms).
 #pragma once
 
-#include "spo_pair.cuh"
+#include "spo_pot5.cuh"
 
 namespace spo {
 
@@ -41,34 +42,40 @@ struct KinArgs {
   XyArgs<T> xy;           // kXy: shift, gas-phase and scaling tables
 };
 
-// Table entries: mixed form: N pairs (p g.x, p g.x, p g.y, p g.y) and (their low parts), N scales (s/p, s/p, low, low),
-// then for kTwiddle N twiddles (w.x, w.x, w.y, w.y) and (their low parts); FP64 form: N factors, then N twiddles.
+// Table entries: mixed form: N pairs (p g.x, p g.x, p g.y, p g.y) and (their low parts), for kTwiddle N twiddles
+// (w.x, w.x, w.y, w.y) and (their low parts), and where some s is not p N scales (s/p, s/p, low, low); FP64 form: N
+// factors, then N twiddles.
 template <typename T> struct KinLine;
 template <> struct KinLine<float> {
   using type = C2;
   static constexpr int lanes = 2;
-  static constexpr int factor_words = 3, twiddle_words = 2;  // 16-byte words per entry
+  static constexpr int factor_words = 2, twiddle_words = 2, scale_words = 1;  // 16-byte words per entry
 };
 template <> struct KinLine<double> {
   using type = double2;
   static constexpr int lanes = 1;
-  static constexpr int factor_words = 1, twiddle_words = 1;
+  static constexpr int factor_words = 1, twiddle_words = 1, scale_words = 0;
 };
+// 16-byte words of a table in shared memory.
+template <typename T>
+constexpr int kin_words(int map, int n, bool unit) {
+  return n * (KinLine<T>::factor_words + (map == kTwiddle ? KinLine<T>::twiddle_words : 0) + (unit ? 0 : KinLine<T>::scale_words));
+}
 
 #ifdef __CUDACC__
 
 
 // factor k on x
-__device__ __forceinline__ C2 kin_factor(C2 x, const C2* f, int n, int k, F2 p, bool unit) {
+__device__ __forceinline__ C2 kin_factor(C2 x, const C2* f, const C2* scale, int k, F2 p, bool unit) {
   const C2 m = cmul2(x, f[2 * k], f[2 * k + 1]);
   C2 z = c2(fma2(x.x, p, m.x), fma2(x.y, p, m.y));
   if (!unit) {
-    const C2 s = f[2 * n + k];  // (s/p twice, its low part twice)
+    const C2 s = scale[k];  // (s/p twice, its low part twice)
     z = c2(fma2(z.x, s.x, z.x * s.y), fma2(z.y, s.x, z.y * s.y));
   }
   return z;
 }
-__device__ __forceinline__ double2 kin_factor(double2 x, const double2* f, int, int k, double, bool) { return cmul(f[k], x); }
+__device__ __forceinline__ double2 kin_factor(double2 x, const double2* f, const double2*, int k, double, bool) { return cmul(f[k], x); }
 // twiddle j on x, conjugated for S > 0
 template <bool ODD, int S>
 __device__ __forceinline__ C2 kin_twiddle(C2 x, const C2* tw, int j) {
@@ -111,6 +118,18 @@ __device__ __forceinline__ void kin_store(float2* p, C2 v, int ok, bool aligned)
   }
 }
 __device__ __forceinline__ double2 kin_load(const double2* p, int ok, bool) { return ok ? *p : make_double2(0.0, 0.0); }
+// A point of a thread's line(s) as it lies in memory (mixed form: re, im, re', im') in a word of shared memory, and back.
+__device__ __forceinline__ C2 kin_unpack(const float4* w) {
+  const float4 v = *w;
+  return c2(make_float2(v.x, v.y), make_float2(v.z, v.w));
+}
+__device__ __forceinline__ float4 kin_pack(C2 v) {
+  float2 a, b;
+  c2_split(v, a, b);
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ double2 kin_unpack(const double2* w) { return *w; }
+__device__ __forceinline__ double2 kin_pack(double2 v) { return v; }
 __device__ __forceinline__ void kin_store(double2* p, double2 v, int ok, bool) {
   if (ok) *p = v;
 }
@@ -152,12 +171,13 @@ __device__ __forceinline__ double2 kin_shift(double2 x, const double2* t, int, i
 template <typename T>
 struct KinTile {
   using L = typename KinLine<T>::type;
+  using W = std::conditional_t<sizeof(T) == 4, float4, double2>;
   Vec<T>* base;   // the line's first point
   long long stride;
   int ok;         // existing lanes of the line
   bool aligned;
   int b, s, nt, log_lines;  // line of the tile, thread of the line, threads per line
-  L* Y;           // [n2][k1][line]
+  L* Y;           // the tile: [n2][n1][line] as loaded, then [n2][k1][line]
 };
 
 template <int MAP>
@@ -170,6 +190,21 @@ __device__ __forceinline__ int kin_point(int n1, int n2, int N1, int N2) {
   }
 }
 
+// The thread's points of a tile into its own words of `buffer` (asynchronous copies; the ragged edge by plain loads).
+template <typename T, int MAP>
+__device__ __forceinline__ void kin_request(const KinTile<T>& t, typename KinTile<T>::L* buffer, const Vec<T>* base, int ok, int N1, int N2) {
+  for (int n2 = t.s; n2 < N2; n2 += t.nt) {
+    auto* const to = reinterpret_cast<typename KinTile<T>::W*>(buffer) + ((n2 * N1) << t.log_lines) + t.b;
+    if (ok == KinLine<T>::lanes && t.aligned) {
+#pragma unroll 4
+      for (int n1 = 0; n1 < N1; ++n1) pot5::copy16(to + (n1 << t.log_lines), base + kin_point<MAP>(n1, n2, N1, N2) * t.stride);
+    } else {
+      for (int n1 = 0; n1 < N1; ++n1)
+        to[n1 << t.log_lines] = kin_pack(kin_load(base + kin_point<MAP>(n1, n2, N1, N2) * t.stride, ok, t.aligned));
+    }
+  }
+  pot5::copy_commit();
+}
 // Level 1: DFT over n1 for the thread's n2.
 template <typename T, int MAP, int N1, bool ODD>
 __device__ __forceinline__ void kin_forward(const KinTile<T>& t, const KinArgs<T>& a, int N2, const typename KinLine<T>::type* tw) {
@@ -178,7 +213,7 @@ __device__ __forceinline__ void kin_forward(const KinTile<T>& t, const KinArgs<T
   for (int n2 = t.s; n2 < N2; n2 += t.nt) {
     L x[N1];
     static_for<0, N1>([&](auto n1) {
-      x[n1] = kin_load(t.base + kin_point<MAP>(SPO_CV(n1), n2, N1, N2) * t.stride, t.ok, t.aligned);
+      x[n1] = kin_unpack(reinterpret_cast<const typename KinTile<T>::W*>(t.Y) + ((n2 * N1 + SPO_CV(n1)) << t.log_lines) + t.b);
       if constexpr (MAP == kXy)
         if (a.xy.shift_f) x[n1] = kin_shift(x[n1], a.xy.shift_f, N1 * N2, kin_point<MAP>(SPO_CV(n1), n2, N1, N2));
     });
@@ -196,13 +231,14 @@ __device__ __forceinline__ void kin_middle(const KinTile<T>& t, const KinArgs<T>
   using L = typename KinLine<T>::type;
   const auto p = kin_scale(a.scale);
   const bool unit = a.unit != 0;
+  const L* const scale = f + (KinLine<T>::factor_words + (MAP == kTwiddle ? KinLine<T>::twiddle_words : 0)) * N1 * N2;
 #pragma unroll 1
   for (int k1 = t.s; k1 < N1; k1 += t.nt) {
     L y[N2];
     L* const row = t.Y + (k1 << t.log_lines) + t.b;
     static_for<0, N2>([&](auto n2) { y[n2] = row[(SPO_CV(n2) * N1) << t.log_lines]; });
     rdft<N2, -1>(y);
-    static_for<0, N2>([&](auto k2) { y[k2] = kin_factor(y[k2], f, N1 * N2, k1 + N1 * SPO_CV(k2), p, unit); });
+    static_for<0, N2>([&](auto k2) { y[k2] = kin_factor(y[k2], f, scale, k1 + N1 * SPO_CV(k2), p, unit); });
     rdft<N2, +1>(y);
     static_for<0, N2>([&](auto n2) {
       if constexpr (MAP == kTwiddle && SPO_CV(n2) > 0) y[n2] = kin_twiddle<ODD, +1>(y[n2], tw, SPO_CV(n2) * k1);
@@ -266,9 +302,9 @@ __global__ void __launch_bounds__(kin_max_threads(N1C > N2C ? N1C : N2C), kin_mi
   L* const f = reinterpret_cast<L*>(smem_raw);
   L* const tw = f + KinLine<T>::factor_words * N;
   KinTile<T> t;
-  t.Y = tw + (MAP == kTwiddle ? KinLine<T>::twiddle_words * N : 0);
+  const int words = kin_words<T>(MAP, N, a.unit != 0);
+  L* const tiles = f + words;  // two tiles
   {
-    const int words = static_cast<int>(t.Y - f);
     const L* src = reinterpret_cast<const L*>(a.table);
     for (int k = threadIdx.x; k < words; k += blockDim.x) f[k] = src[k];
   }
@@ -280,13 +316,38 @@ __global__ void __launch_bounds__(kin_max_threads(N1C > N2C ? N1C : N2C), kin_mi
   t.aligned = a.aligned != 0;
   // twiddle products of lengths with an odd factor are nearly correctly rounded (cmul_comp)
   constexpr bool ODD = ANY || ((N1C * N2C) & (N1C * N2C - 1)) != 0;
-  __syncthreads();
-  for (unsigned tile = blockIdx.x; tile < a.n_tiles; tile += gridDim.x) {
+  auto locate = [&](unsigned tile, Vec<T>*& base, int& ok, unsigned& outer, long long& lane) {
     const unsigned rest = tile / a.blocks_per_group, blk = tile - rest * a.blocks_per_group;
-    const unsigned outer = rest / a.groups, grp = rest - outer * a.groups;
-    const long long lane = (static_cast<long long>(blk) << a.log_lines) * KinLine<T>::lanes + t.b * KinLine<T>::lanes;
-    t.ok = lane >= a.window ? 0 : static_cast<int>(min(static_cast<long long>(KinLine<T>::lanes), a.window - lane));
-    t.base = a.data + outer * a.outer_stride + grp * a.group_stride + a.lane_offset + lane;
+    outer = rest / a.groups;
+    const unsigned grp = rest - outer * a.groups;
+    lane = (static_cast<long long>(blk) << a.log_lines) * KinLine<T>::lanes + t.b * KinLine<T>::lanes;
+    ok = lane >= a.window ? 0 : static_cast<int>(min(static_cast<long long>(KinLine<T>::lanes), a.window - lane));
+    base = a.data + outer * a.outer_stride + grp * a.group_stride + a.lane_offset + lane;
+  };
+  unsigned tile = blockIdx.x, outer = 0;
+  long long lane = 0;
+  if (tile < a.n_tiles) {
+    locate(tile, t.base, t.ok, outer, lane);
+    kin_request<T, MAP>(t, tiles, t.base, t.ok, N1, N2);
+  }
+  __syncthreads();
+  // Levels 1 and 3 touch the thread's own words of a tile only, so that the next tile but one may overwrite them without
+  // a barrier; level 2 lies between two.
+  int side = 0;
+  for (; tile < a.n_tiles; tile += gridDim.x, side ^= 1) {
+    // the next tile's points, on their way during this one
+    Vec<T>* next_base = nullptr;
+    int next_ok = 0;
+    unsigned next_outer = 0;
+    long long next_lane = 0;
+    if (tile + gridDim.x < a.n_tiles) {
+      locate(tile + gridDim.x, next_base, next_ok, next_outer, next_lane);
+      kin_request<T, MAP>(t, tiles + (side ^ 1) * (N << t.log_lines), next_base, next_ok, N1, N2);
+    } else {
+      pot5::copy_commit();
+    }
+    t.Y = tiles + side * (N << t.log_lines);
+    pot5::copy_wait<1>();  // this tile's points
     if constexpr (ANY) kin_switch(N1, [&](auto n) { kin_forward<T, MAP, SPO_CV(n), ODD>(t, a, N2, tw); });
     else kin_forward<T, MAP, N1C, ODD>(t, a, N2C, tw);
     __syncthreads();
@@ -305,7 +366,10 @@ __global__ void __launch_bounds__(kin_max_threads(N1C > N2C ? N1C : N2C), kin_mi
       if constexpr (ANY) kin_switch(N1, [&](auto n) { kin_back<T, MAP, SPO_CV(n)>(t, a, N2, false, 0); });
       else kin_back<T, MAP, N1C>(t, a, N2C, false, 0);
     }
-    __syncthreads();  // Y is read before the next tile's first level writes it
+    t.base = next_base;
+    t.ok = next_ok;
+    outer = next_outer;
+    lane = next_lane;
   }
 }
 

@@ -14,7 +14,7 @@ template void launch_pot2<T>(int, const spo::Pot2Args<T>&, unsigned, std::size_t
 #elif SPO_LAUNCH_PART == 3
 template void launch_pot3<T>(int, const spo::Pot2Args<T>&, dim3, unsigned, std::size_t, cudaStream_t);
 #elif SPO_LAUNCH_PART == 5
-template KinLaunch<T> kin_configure<T>(int, int, int, int, long long);
+template KinLaunch<T> kin_configure<T>(int, int, int, bool, int, long long);
 #else
 template Pot4Kernel<T> pot4_kernel_for<T>(int, int);
 #endif

@@ -266,32 +266,52 @@ Pot4Kernel<T> pot4_kernel_for(int nphi, int nt) {
 template <typename T>
 using KinKernel = void (*)(spo::KinArgs<T>);
 template <typename T>
-KinKernel<T> kin_kernel_for(int map) {
+KinKernel<T> kin_kernel_for(int map, int n1, int n2) {
+  if constexpr (sizeof(T) == 4) {  // kin_paired, kin_paired_xy
+    if (map == spo::kTwiddle) {
+      if (n1 == 8 && n2 == 16) return spo::kin_kernel<T, spo::kTwiddle, 8, 16>;
+      if (n1 == 12 && n2 == 16) return spo::kin_kernel<T, spo::kTwiddle, 12, 16>;
+      if (n1 == 16 && n2 == 16) return spo::kin_kernel<T, spo::kTwiddle, 16, 16>;
+    } else if (map == spo::kPrime) {
+      if (n1 == 3 && n2 == 16) return spo::kin_kernel<T, spo::kPrime, 3, 16>;
+      if (n1 == 11 && n2 == 16) return spo::kin_kernel<T, spo::kPrime, 11, 16>;
+      if (n1 == 3 && n2 == 32) return spo::kin_kernel<T, spo::kPrime, 3, 32>;
+      if (n1 == 5 && n2 == 32) return spo::kin_kernel<T, spo::kPrime, 5, 32>;
+      if (n1 == 7 && n2 == 32) return spo::kin_kernel<T, spo::kPrime, 7, 32>;
+    } else if (n1 == n2) {
+      if (n1 == 2) return spo::kin_kernel<T, spo::kXy, 2, 2>;
+      if (n1 == 4) return spo::kin_kernel<T, spo::kXy, 4, 4>;
+      if (n1 == 8) return spo::kin_kernel<T, spo::kXy, 8, 8>;
+      if (n1 == 16) return spo::kin_kernel<T, spo::kXy, 16, 16>;
+    }
+  }
   return map == spo::kTwiddle ? spo::kin_kernel<T, spo::kTwiddle, 0, 0>
          : map == spo::kPrime ? spo::kin_kernel<T, spo::kPrime, 0, 0>
                               : spo::kin_kernel<T, spo::kXy, 0, 0>;
 }
 
 // Threads per line: the number that wastes the fewest thread slots over the two levels (N2 lines of N1 points, then N1 of
-// N2) in whole warps.
+// N2) in whole warps, among those that keep about 14 warps per SM beside the tiles' shared memory.
 template <typename T>
-KinLaunch<T> kin_configure(int map, int n1, int n2, int lanes_per_tile, long long window) {
+KinLaunch<T> kin_configure(int map, int n1, int n2, bool unit, int lanes_per_tile, long long window) {
   KinLaunch<T> l;
-  l.kernel = kin_kernel_for<T>(map);
+  l.kernel = kin_kernel_for<T>(map, n1, n2);
   while ((spo::KinLine<T>::lanes << (l.log_lines + 1)) <= lanes_per_tile) ++l.log_lines;
   while (l.log_lines > 0 && (static_cast<long long>(spo::KinLine<T>::lanes) << (l.log_lines - 1)) >= window) --l.log_lines;
   const int lines = 1 << l.log_lines, limit = spo::kin_max_threads(std::max(n1, n2));
-  long long best = 0;
+  const std::size_t n = static_cast<std::size_t>(n1) * n2;
+  l.smem = 16 * (spo::kin_words<T>(map, n1 * n2, unit) + 2 * n * lines);
+  const double fit = std::floor((228 << 10) / static_cast<double>(l.smem + 1024));
+  double best = 0.0;
   for (int nt = 1; nt <= std::max(n1, n2) && nt * lines <= limit; ++nt) {
     const int threads = (nt * lines + 31) / 32 * 32;
-    const long long cost = static_cast<long long>((n2 + nt - 1) / nt * n1 + (n1 + nt - 1) / nt * n2) * threads;
-    if (best == 0 || cost < best || (cost == best && nt * lines <= 128)) {
+    const double warps = std::max(1.0, fit) * threads / 32;
+    const double cost = static_cast<double>((n2 + nt - 1) / nt * n1 + (n1 + nt - 1) / nt * n2) * threads * std::max(1.0, 14.0 / warps);
+    if (best == 0.0 || cost < 0.999 * best) {
       best = cost;
       l.threads = nt * lines;
     }
   }
-  const std::size_t n = static_cast<std::size_t>(n1) * n2;
-  l.smem = 16 * (n * (spo::KinLine<T>::factor_words + (map == spo::kTwiddle ? spo::KinLine<T>::twiddle_words : 0)) + n * lines);
   check_cuda(cudaFuncSetAttribute(l.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_optin_bytes())),
              "kin smem");
   int dev = 0, sms = 0, per_sm = 0;
