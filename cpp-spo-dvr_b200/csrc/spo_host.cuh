@@ -2035,7 +2035,7 @@ class Step final : public StepBase {
     for (int p = 0; p < s.nphi; ++p)
       for (int q = 0; 8 * q < slots[p].y; ++q) tiles.push_back(make_int2(p, q));
     int teams = spo::pot4d::threads_of(s.nphi) / spo::pot4d::kTeam;
-    auto need = [&](int n) { return spo::pot4d::smem_bytes(s.nphi, n_fwd + n_back, static_cast<int>(tiles.size()), n); };
+    auto need = [&](int n) { return spo::pot4d::smem_bytes(s.n_rot, s.nphi, n_fwd + n_back, static_cast<int>(tiles.size()), n); };
     while (teams > 0 && need(teams) > static_cast<std::size_t>(smem_optin)) --teams;
     if (teams == 0) return;
     a.p = pot_;

@@ -13,9 +13,10 @@
 // psi comes scaled by the absorbers and rot(dt/2) (the xy pass). The projection is projection_finalize_kernel's.
 //
 // What bounds it: on configuration 2 the FP64 pipe (shared by the tensor products and the transforms) needs ~150
-// multiply-adds per value of psi with the padding of the fragments (2.1 ms), HBM 16.9 GB (2.6 ms). The register-tiled
-// form on FMAs (potential4_kernel) took 10.8 ms with 8 warps per SM: each term of its contractions loads its operands
-// from shared memory.
+// multiply-adds per value of psi with the padding of the fragments (2.1 ms), HBM 16.9 GB (2.6 ms). A register-tiled
+// form on FMAs took 10.8 ms with 8 warps per SM: each term of its contractions loads its operands from shared memory.
+// On Z 128, r 48, 12 x 12 (9.5 GB) the FMA form took 6.05 ms, this one with every load where its value is needed 3.77
+// (long-scoreboard stalls 2.7 of 7.7 cycles per issue), with psi and exp(i A) a phase ahead 3.00 (3.2 TB/s).
 #pragma once
 
 #include "spo_pot5.cuh"
@@ -26,6 +27,9 @@ namespace pot4d {
 // Threads per block: a line takes 4 nphi registers.
 constexpr int threads_of(int nphi) { return nphi > 20 ? 256 : nphi > 16 ? 384 : 512; }
 constexpr int kTeam = 128;
+// 256 threads leave a thread 255 registers: while the lines are not in registers they hold psi of the team's next item (the
+// 8 tasks of a warp; with one theta tile and two column groups they would be 16).
+constexpr bool ahead_of(int nphi, int h) { return threads_of(nphi) == 256 && h == 2; }
 }  // namespace pot4d
 
 struct Pot4dArgs {
@@ -57,8 +61,10 @@ __global__ void __launch_bounds__(pot4d::threads_of(NPHI), 1) potential4_dmma_ke
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int team = threadIdx.x / pot4d::kTeam, teams = blockDim.x / pot4d::kTeam;
   const int tid = threadIdx.x % pot4d::kTeam, warp = tid / 32, lane = tid % 32;
-  double2* const X = reinterpret_cast<double2*>(smem_raw) + team * NPHI * SLOT;
-  double* const mats = reinterpret_cast<double*>(reinterpret_cast<double2*>(smem_raw) + teams * NPHI * SLOT);
+  constexpr bool AHEAD = pot4d::ahead_of(NPHI, H);
+  double2* const X = reinterpret_cast<double2*>(smem_raw) + team * (NPHI * SLOT + n_rot);
+  double2* const rot_row = X + NPHI * SLOT;  // rot(dt/2) at the item's r point
+  double* const mats = reinterpret_cast<double*>(reinterpret_cast<double2*>(smem_raw) + teams * (NPHI * SLOT + n_rot));
   int4* const slots = reinterpret_cast<int4*>(mats + 32 * (g.n_fwd + g.n_back));
   int2* const tiles = reinterpret_cast<int2*>(slots + NPHI);
   int* const order = reinterpret_cast<int*>(tiles + g.n_back_tasks);
@@ -78,7 +84,26 @@ __global__ void __launch_bounds__(pot4d::threads_of(NPHI), 1) potential4_dmma_ke
   const int line_at = line_c * NT + (line_t ^ (4 * (line_c & 1)));
   const int step = gridDim.x * teams;
 
-  for (int item = blockIdx.x * teams + team; item < g.n_items; item += step) {
+  constexpr int TASKS = NPHI * GROUPS, MINE = (TASKS + 3) / 4;
+  auto load = [&](int task, int col0, double2 (&u)[4], int4& s) {
+    s = slots[order[task / GROUPS]];
+    const int col = col0 + (task % GROUPS) * 8 + c;
+    const double2* const p = a.psi + static_cast<long long>(min(col, g.n_cols - 1)) * n_rot;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      u[k] = 4 * k < s.y ? p[min(s.x + 4 * k + t, n_rot - 1)] : make_double2(0.0, 0.0);
+  };
+  double2 mine[AHEAD ? MINE : 1][4] = {};
+  auto load_mine = [&](int item) {
+    static_for<0, AHEAD ? MINE : 0>([&](auto k) {
+      int4 s;
+      load(min(warp + 4 * SPO_CV(k), TASKS - 1), item * COLS, mine[SPO_CV(k)], s);
+    });
+  };
+
+  int item = blockIdx.x * teams + team;
+  if (AHEAD && item < g.n_items) load_mine(item);
+  for (; item < g.n_items; item += step) {
     const int col0 = item * COLS;
     // the next item's columns and exp(i A) rows into L2
     {
@@ -90,23 +115,14 @@ __global__ void __launch_bounds__(pot4d::threads_of(NPHI), 1) potential4_dmma_ke
         pot5::prefetch_l2(a.psi + static_cast<long long>(col) * n_rot, static_cast<uint32_t>(n_rot * sizeof(double2)));
       }
     }
+    // the item's row of rot(dt/2), if it lies at one point
+    const int izr0 = col0 / n_xy;
+    const bool row = min(col0 + COLS - 1, g.n_cols - 1) / n_xy == izr0;
+    if (row)
+      for (int k = tid; k < n_rot; k += pot4d::kTeam) rot_row[k] = g.rot[(izr0 % nr) * n_rot + k];
 
-    // ---- forward: tasks (slot, group), the fragments of the next one requested before the products of this one
-    constexpr int TASKS = NPHI * GROUPS;
-    auto load = [&](int task, double2 (&u)[4], int4& s) {
-      s = slots[order[task / GROUPS]];
-      const int col = col0 + (task % GROUPS) * 8 + c;
-      const double2* const p = a.psi + static_cast<long long>(min(col, g.n_cols - 1)) * n_rot;
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        if (4 * k < s.y) u[k] = p[min(s.x + 4 * k + t, n_rot - 1)];
-    };
-    double2 u[4] = {}, un[4] = {};
-    int4 s, sn = make_int4(0, 0, 0, 0);
-    load(warp, u, s);
-#pragma unroll 1
-    for (int task = warp; task < TASKS; task += 4) {
-      if (task + 4 < TASKS) load(task + 4, un, sn);
+    // ---- forward: tasks (slot, group)
+    auto multiply = [&](int task, double2 (&u)[4], const int4& s) {
       const int slot = order[task / GROUPS], grp = task % GROUPS;
       const int col = col0 + grp * 8 + c;
       const int nj = s.y;
@@ -154,9 +170,24 @@ __global__ void __launch_bounds__(pot4d::threads_of(NPHI), 1) potential4_dmma_ke
         x[8 * h + (t ^ sw)] = make_double2(r[h][0], q[h][0]);
         x[8 * h + ((t + 4) ^ sw)] = make_double2(r[h][1], q[h][1]);
       }
-      s = sn;
+    };
+    if constexpr (AHEAD) {
+      static_for<0, MINE>([&](auto k) {
+        const int task = warp + 4 * SPO_CV(k);
+        if (task < TASKS) multiply(task, mine[SPO_CV(k)], slots[order[task / GROUPS]]);
+      });
+    } else {  // the fragments of the next task requested before the products of this one
+      double2 u[4] = {}, un[4] = {};
+      int4 s, sn = make_int4(0, 0, 0, 0);
+      load(warp, col0, u, s);
+#pragma unroll 1
+      for (int task = warp; task < TASKS; task += 4) {
+        if (task + 4 < TASKS) load(task + 4, col0, un, sn);
+        multiply(task, u, s);
+        s = sn;
 #pragma unroll
-      for (int k = 0; k < 4; ++k) u[k] = un[k];
+        for (int k = 0; k < 4; ++k) u[k] = un[k];
+      }
     }
     team_sync();
 
@@ -168,10 +199,18 @@ __global__ void __launch_bounds__(pot4d::threads_of(NPHI), 1) potential4_dmma_ke
         const double2* const e =
             g.table + (static_cast<long long>(izr) * a.n_rep + (g.phi_map ? __ldg(a.rep_of + ixy) : ixy)) * NPHI * a.n_theta + line_t;
         double2 x[NPHI];
+        constexpr int EARLY = AHEAD ? NPHI / 2 : 0;  // entries requested before the transform
+        double2 ex[EARLY > 0 ? EARLY : 1];
+        if (g.phi_map == nullptr) static_for<0, EARLY>([&](auto p) { ex[p] = __ldg(e + SPO_CV(p) * a.n_theta); });
         static_for<0, NPHI>([&](auto p) { x[p] = X[SPO_CV(p) * SLOT + line_at]; });
         rdft<NPHI, +1>(x);
         if (g.phi_map == nullptr) {
-          static_for<0, NPHI>([&](auto p) { x[p] = cmul(__ldg(e + SPO_CV(p) * a.n_theta), x[p]); });
+          static_for<0, EARLY>([&](auto p) {
+            x[p] = cmul(ex[p], x[p]);
+            ex[p] = __ldg(e + (SPO_CV(p) + EARLY) * a.n_theta);
+          });
+          static_for<EARLY, 2 * EARLY>([&](auto p) { x[p] = cmul(ex[SPO_CV(p) - EARLY], x[p]); });
+          static_for<2 * EARLY, NPHI>([&](auto p) { x[p] = cmul(__ldg(e + SPO_CV(p) * a.n_theta), x[p]); });
         } else {
           const uint8_t* const map = g.phi_map + ixy * NPHI;
           static_for<0, NPHI>([&](auto p) { x[p] = cmul(__ldg(e + __ldg(map + SPO_CV(p)) * a.n_theta), x[p]); });
@@ -182,7 +221,8 @@ __global__ void __launch_bounds__(pot4d::threads_of(NPHI), 1) potential4_dmma_ke
     }
     team_sync();
 
-    // ---- back: tasks (slot, 8 values of J, group)
+    // ---- back: tasks (slot, 8 values of J, group); psi of the next item on its way
+    if (AHEAD) load_mine(min(item + step, g.n_items - 1));  // (the last one's again: every value of `mine` is defined anew)
 #pragma unroll 1
     for (int task = warp; task < g.n_back_tasks * GROUPS; task += 4) {
       const int2 tile = tiles[task / GROUPS];
@@ -191,8 +231,8 @@ __global__ void __launch_bounds__(pot4d::threads_of(NPHI), 1) potential4_dmma_ke
       const int col = col0 + grp * 8 + c;
       const int ir = (min(col, g.n_cols - 1) / n_xy) % nr;
       const int j = 8 * tile.y + t;
-      const double2* const w = g.rot + ir * n_rot + s4.x;
-      const double2 wa = __ldg(w + min(j, s4.y - 1)), wb = __ldg(w + min(j + 4, s4.y - 1));
+      const double2* const w = (row ? rot_row : g.rot + ir * n_rot) + s4.x;
+      const double2 wa = w[min(j, s4.y - 1)], wb = w[min(j + 4, s4.y - 1)];
       const double2* const x = X + tile.x * SLOT + (grp * 8 + c) * NT;
       const double* const m = mb + 32 * (s4.w + tile.y * 2 * H);
       double r0 = 0, r1 = 0, q0 = 0, q1 = 0;
@@ -229,8 +269,8 @@ inline Kernel kernel_for(int nphi, int h) {
     if (!k) k = part(nphi, h);
   return k;
 }
-inline std::size_t smem_bytes(int nphi, int frags, int n_back_tasks, int teams) {
-  return 2048u * static_cast<std::size_t>(nphi) * teams + 256u * static_cast<std::size_t>(frags) +
+inline std::size_t smem_bytes(int n_rot, int nphi, int frags, int n_back_tasks, int teams) {
+  return (2048u * static_cast<std::size_t>(nphi) + 16u * static_cast<std::size_t>(n_rot)) * teams + 256u * static_cast<std::size_t>(frags) +
          (sizeof(int4) + sizeof(int)) * static_cast<std::size_t>(nphi) + sizeof(int2) * static_cast<std::size_t>(n_back_tasks);
 }
 }  // namespace pot4d
