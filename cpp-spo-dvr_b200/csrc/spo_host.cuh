@@ -245,7 +245,8 @@ KinLaunch<T> kin_configure(int map, int n1, int n2, bool unit, int lanes_per_til
 // them: where pairs measured faster (ms per launch of 0.2 to 0.8 GB, pairs against one lane per thread):
 //   Z, r: 48 0.242/0.259, 96 0.485/0.560, 128 1.56/1.64 (configuration 3), 160 0.256/0.296, 176 0.170/0.226, 192
 //     0.288/0.300, 224 0.182/0.223, 256 0.162/0.188;
-//   x = y: 2 0.034/0.036, 4 0.074/0.098, 8 0.173/0.227, 16 2.07/2.13 (configuration 3).
+//   x = y: 2 0.034/0.036, 4 0.074/0.098, 8 0.133/0.155, 16 1.75/1.84 (configuration 3); without a momentum shift only:
+//     with its two extra factors 16 took 2.07.
 // Not 24, 32 and 64 (short lines: the other kernels keep more warps in flight and run at 4.1 to 4.9 TB/s; 0.056/0.050,
 // 0.189/0.190, 0.232/0.224), 40, 56, 80 and 112 (radices 5 and 7 sum in FP64, line by line; 0.173/0.130, 0.090/0.066,
 // 0.120/0.114, 0.134/0.125), 6 and 12 (0.199/0.188, 0.463/0.445).
@@ -1534,8 +1535,11 @@ class Step final : public StepBase {
       };
       axis(kin_z_, s.nz, d.z_kinetic_full, d.z_kinetic_half);
       axis(kin_r_, s.nr, d.r_kinetic_full, d.r_kinetic_half);
-      if (kin_xy_size(s.nx) && kin_xy_size(s.ny) && (s.nx != s.ny || !xy2_supported(s.nx) || (mixed && kin_paired_xy(s.nx)))) {
-        kin_xy_.map = spo::kXy;
+      const std::vector<cplx> shift = complex_array(d.shift_forward, nxy, "shift_forward");  // as shift_f_ below
+      const bool shifted = std::any_of(shift.begin(), shift.end(), [](const cplx& c) { return c != cplx(1.0, 0.0); });
+      if (kin_xy_size(s.nx) && kin_xy_size(s.ny) &&
+          (s.nx != s.ny || !xy2_supported(s.nx) || (mixed && !shifted && kin_paired_xy(s.nx)))) {
+        kin_xy_.map = shifted ? spo::kXyShift : spo::kXy;
         kin_xy_.n1 = s.ny;
         kin_xy_.n2 = s.nx;
         kin_table(kin_xy_, 0, scaled(complex_array(d.xy_kinetic_full, nxy, "xy_kinetic_full"), xy_scale));

@@ -11,7 +11,7 @@
 // the instructions; the next tile's points are copied to shared memory (cp.async, each thread its own) while a tile is
 // transformed. Issue bound it before (65 to 75 % of the slots at 4 TB/s: every constant is exact to ~2^-48, which
 // costs two to three times the instructions of plain FP32 products); one lane per thread took 1.64, 1.59 and 1.84 ms
-// on configuration 3 (Z 128, r 48, 16 x 16). A grid of resident blocks loops over the tiles, so that the tables are
+// on configuration 3 (Z 128, r 48, 16 x 16), pairs 1.54, 1.51 and 1.75. A grid of resident blocks loops over the tiles, so that the tables are
 // staged in shared memory once per block, not once per tile. kinetic factors s e^{i phi} are applied as p (x + x g)
 // with p the power of two in s, folded into g and exact, and a product with the rest s / p only where it is not 1.
 //
@@ -24,7 +24,8 @@
 
 namespace spo {
 
-enum KinMap : int { kTwiddle = 0, kPrime = 1, kXy = 2 };
+enum KinMap : int { kTwiddle = 0, kPrime = 1, kXy = 2, kXyShift = 3 };  // kXy: without the momentum shift
+constexpr bool kin_is_xy(int map) { return map == kXy || map == kXyShift; }
 
 template <typename T>
 struct KinArgs {
@@ -80,12 +81,15 @@ __device__ __forceinline__ double2 kin_factor(double2 x, const double2* f, const
 template <bool ODD, int S>
 __device__ __forceinline__ C2 kin_twiddle(C2 x, const C2* tw, int j) {
   C2 w = tw[2 * j], l = tw[2 * j + 1];
-  if constexpr (S > 0) {
-    w.y = -w.y;
-    l.y = -l.y;
+  if constexpr (ODD) {
+    if constexpr (S > 0) {
+      w.y = -w.y;
+      l.y = -l.y;
+    }
+    return cmul_comp(x, w, l);
+  } else {
+    return S > 0 ? cmul2_conj(x, w, l) : cmul2(x, w, l);
   }
-  if constexpr (ODD) return cmul_comp(x, w, l);
-  else return cmul2(x, w, l);
 }
 template <bool ODD, int S>
 __device__ __forceinline__ double2 kin_twiddle(double2 x, const double2* tw, int j) {
@@ -183,7 +187,7 @@ struct KinTile {
 template <int MAP>
 __device__ __forceinline__ int kin_point(int n1, int n2, int N1, int N2) {
   if constexpr (MAP == kTwiddle) return n2 + N2 * n1;
-  else if constexpr (MAP == kXy) return n1 + N1 * n2;
+  else if constexpr (kin_is_xy(MAP)) return n1 + N1 * n2;
   else {
     const int n = N2 * n1 + N1 * n2;
     return n >= N1 * N2 ? n - N1 * N2 : n;
@@ -214,8 +218,7 @@ __device__ __forceinline__ void kin_forward(const KinTile<T>& t, const KinArgs<T
     L x[N1];
     static_for<0, N1>([&](auto n1) {
       x[n1] = kin_unpack(reinterpret_cast<const typename KinTile<T>::W*>(t.Y) + ((n2 * N1 + SPO_CV(n1)) << t.log_lines) + t.b);
-      if constexpr (MAP == kXy)
-        if (a.xy.shift_f) x[n1] = kin_shift(x[n1], a.xy.shift_f, N1 * N2, kin_point<MAP>(SPO_CV(n1), n2, N1, N2));
+      if constexpr (MAP == kXyShift) x[n1] = kin_shift(x[n1], a.xy.shift_f, N1 * N2, kin_point<MAP>(SPO_CV(n1), n2, N1, N2));
     });
     rdft<N1, -1>(x);
     static_for<0, N1>([&](auto k1) {
@@ -257,10 +260,9 @@ __device__ __forceinline__ void kin_back(const KinTile<T>& t, const KinArgs<T>& 
     rdft<N1, +1>(x);
     static_for<0, N1>([&](auto n1) {
       const int n = kin_point<MAP>(SPO_CV(n1), n2, N1, N2);
-      if constexpr (MAP == kXy) {
-        if (a.xy.shift_b) x[n1] = kin_shift(x[n1], a.xy.shift_b, N1 * N2, n);
+      if constexpr (MAP == kXyShift) x[n1] = kin_shift(x[n1], a.xy.shift_b, N1 * N2, n);
+      if constexpr (kin_is_xy(MAP))
         if (post) x[n1] = kin_apply(x[n1], w);
-      }
       kin_store(t.base + n * t.stride, x[n1], t.ok, t.aligned);
     });
   }
@@ -354,7 +356,7 @@ __global__ void __launch_bounds__(kin_max_threads(N1C > N2C ? N1C : N2C), kin_mi
     if constexpr (ANY) kin_switch(N2, [&](auto n) { kin_middle<T, MAP, SPO_CV(n), ODD>(t, a, N1, f, tw); });
     else kin_middle<T, MAP, N2C, ODD>(t, a, N1C, f, tw);
     __syncthreads();
-    if constexpr (MAP == kXy) {
+    if constexpr (kin_is_xy(MAP)) {
       const long long izr = a.xy.izr_offset + outer;
       const Vec<T>* const table = xy_post(a.xy, izr);
       decltype(kin_post(table, 0ll, 0ll, 0, T(0))) w{};

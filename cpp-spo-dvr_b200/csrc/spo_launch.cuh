@@ -278,7 +278,7 @@ KinKernel<T> kin_kernel_for(int map, int n1, int n2) {
       if (n1 == 3 && n2 == 32) return spo::kin_kernel<T, spo::kPrime, 3, 32>;
       if (n1 == 5 && n2 == 32) return spo::kin_kernel<T, spo::kPrime, 5, 32>;
       if (n1 == 7 && n2 == 32) return spo::kin_kernel<T, spo::kPrime, 7, 32>;
-    } else if (n1 == n2) {
+    } else if (map == spo::kXy && n1 == n2) {
       if (n1 == 2) return spo::kin_kernel<T, spo::kXy, 2, 2>;
       if (n1 == 4) return spo::kin_kernel<T, spo::kXy, 4, 4>;
       if (n1 == 8) return spo::kin_kernel<T, spo::kXy, 8, 8>;
@@ -287,7 +287,8 @@ KinKernel<T> kin_kernel_for(int map, int n1, int n2) {
   }
   return map == spo::kTwiddle ? spo::kin_kernel<T, spo::kTwiddle, 0, 0>
          : map == spo::kPrime ? spo::kin_kernel<T, spo::kPrime, 0, 0>
-                              : spo::kin_kernel<T, spo::kXy, 0, 0>;
+         : map == spo::kXy    ? spo::kin_kernel<T, spo::kXy, 0, 0>
+                              : spo::kin_kernel<T, spo::kXyShift, 0, 0>;
 }
 
 // Threads per line: the number that wastes the fewest thread slots over the two levels (N2 lines of N1 points, then N1 of

@@ -68,6 +68,13 @@ __device__ __forceinline__ C2 cmul2(C2 a, C2 w, C2 wl) {
   const F2 ci = fma2(a.x, wl.y, a.y * wl.x);
   return c2(fma2(a.x, w.x, fma2(n, w.y, cr)), fma2(a.x, w.y, fma2(a.y, w.x, ci)));
 }
+// a times the conjugate of w + wl: the same operations on (w.x, -w.y), one value negated instead of three.
+__device__ __forceinline__ C2 cmul2_conj(C2 a, C2 w, C2 wl) {
+  const F2 n = -a.x;
+  const F2 cr = fma2(a.x, wl.x, a.y * wl.y);
+  const F2 ci = fma2(n, wl.y, a.y * wl.x);
+  return c2(fma2(a.x, w.x, fma2(a.y, w.y, cr)), fma2(n, w.y, fma2(a.y, w.x, ci)));
+}
 // The same for one constant of both lines (the negated ones come with it, so that no value is negated).
 __device__ __forceinline__ C2 cmul2k(C2 a, float wx, float wy, float lx, float ly) {
   const F2 cr = fma2(a.x, f2(lx), a.y * f2(-ly));
@@ -111,8 +118,8 @@ __device__ __forceinline__ C2 twiddle_mul2(C2 a) {
   }
 }
 
-// rdft of spo_regfft.cuh on two lines: the same operations in the same order on each. The odd primes run line by
-// line (radices 5, 7 and 11 sum in FP64).
+// rdft of spo_regfft.cuh on two lines: the same operations in the same order on each. Radices 5, 7 and 11, which sum in
+// FP64, run line by line.
 template <int N, int S>
 __device__ __forceinline__ void rdft(C2 (&x)[N]) {
   if constexpr (N == 1) {
@@ -127,7 +134,17 @@ __device__ __forceinline__ void rdft(C2 (&x)[N]) {
     x[1] = cadd_i<S>(d02, d13);
     x[2] = csub(s02, s13);
     x[3] = cadd_i<-S>(d02, d13);
-  } else if constexpr (N == 3 || N == 5 || N == 7 || N == 11) {
+  } else if constexpr (N == 3) {  // the root's sine and cosine as two values each
+    constexpr float c = static_cast<float>(Root<1, 3, S>::re), sn = static_cast<float>(Root<1, 3, S>::im);
+    constexpr float cl = static_cast<float>(Root<1, 3, S>::re - static_cast<double>(c));
+    constexpr float sl = static_cast<float>(Root<1, 3, S>::im - static_cast<double>(sn));
+    const C2 s = cadd(x[1], x[2]), d = csub(x[1], x[2]);
+    const C2 re = c2(fma2(f2(c), s.x, fma2(f2(cl), s.x, x[0].x)), fma2(f2(c), s.y, fma2(f2(cl), s.y, x[0].y)));
+    const C2 im = c2(fma2(f2(sn), d.x, f2(sl) * d.x), fma2(f2(sn), d.y, f2(sl) * d.y));
+    x[0] = cadd(x[0], s);
+    x[1] = cadd_i<+1>(re, im);
+    x[2] = cadd_i<-1>(re, im);
+  } else if constexpr (N == 5 || N == 7 || N == 11) {
     float2 a[N], b[N];
     static_for<0, N>([&](auto t) { c2_split(x[t], a[t], b[t]); });
     rdft<N, S>(a);
