@@ -241,21 +241,25 @@ struct KinLaunch {
 template <typename T>
 KinLaunch<T> kin_configure(int map, int n1, int n2, bool unit, int lanes_per_tile, long long window);
 
-// The lengths and square grids whose mixed form runs kin_kernel on pairs of lanes although another register kernel has
-// them: where pairs measured faster (ms per launch of 0.2 to 0.8 GB, pairs against one lane per thread):
-//   Z, r: 48 0.242/0.259, 96 0.485/0.560, 128 1.56/1.64 (configuration 3), 160 0.256/0.296, 176 0.170/0.226, 192
-//     0.288/0.300, 224 0.182/0.223, 256 0.162/0.188;
-//   x = y: 2 0.034/0.036, 4 0.074/0.098, 8 0.133/0.155, 16 1.75/1.84 (configuration 3); without a momentum shift only:
-//     with its two extra factors 16 took 2.07.
-// Not 24, 32 and 64 (short lines: the other kernels keep more warps in flight and run at 4.1 to 4.9 TB/s; 0.056/0.050,
-// 0.189/0.190, 0.232/0.224), 40, 56, 80 and 112 (radices 5 and 7 sum in FP64, line by line; 0.173/0.130, 0.090/0.066,
-// 0.120/0.114, 0.134/0.125), 6 and 12 (0.199/0.188, 0.463/0.445).
-inline bool kin_paired(int n, int& map, int& n1, int& n2) {
+// The lengths and square grids that run kin_kernel although another register kernel has them: where it measured faster (ms
+// per launch of 0.1 to 1.6 GB, against the other kernel at its best tile width).
+//   mixed form, pairs of lanes: 48 0.242/0.259, 96 0.495/0.560, 128 0.228/0.250, 160 0.259/0.296, 176 0.168/0.226, 192
+//     0.273/0.300, 224 0.184/0.223, 256 0.156/0.188; x = y: 2 0.030/0.036, 4 0.064/0.097, 6 0.180/0.188, 8 0.151/0.227,
+//     12 0.372/0.445, 16 0.363/0.487;
+//   FP64: 48 0.374/0.418, 64 0.364/0.411, 128 0.348/0.390, 176 0.189/0.238, 192 0.279/0.312, 224 0.203/0.224, 256
+//     0.228/0.287; x = y: 2 0.0307/0.0312, 4 0.151/0.159, 6 0.176/0.214, 8 0.213/0.251, 12 0.384/0.518, 16 0.570/0.618.
+// The (x, y) pass without a momentum shift only: with its two extra factors the mixed 16 x 16 pass took 2.07 ms on
+// configuration 3, without 1.75 (the other kernel 1.84).
+// Not 24, 32 and, mixed, 64 (short lines: the other kernels keep more warps in flight; 0.056/0.050, 0.189/0.190,
+// 0.222/0.222; FP64 24 0.080/0.076, 32 0.171/0.166), 40, 56, 80 and 112 (mixed: radices 5 and 7 sum in FP64, line by line;
+// 0.173/0.130, 0.090/0.066, 0.120/0.114, 0.134/0.125), FP64 96 and 160 (0.618/0.593, 0.293/0.294).
+inline bool kin_preferred(int n, bool mixed, int& map, int& n1, int& n2) {
   switch (n) {
     case 48: map = spo::kPrime, n1 = 3, n2 = 16; return true;
-    case 96: map = spo::kPrime, n1 = 3, n2 = 32; return true;
+    case 64: map = spo::kTwiddle, n1 = 8, n2 = 8; return !mixed;
+    case 96: map = spo::kPrime, n1 = 3, n2 = 32; return mixed;
     case 128: map = spo::kTwiddle, n1 = 8, n2 = 16; return true;
-    case 160: map = spo::kPrime, n1 = 5, n2 = 32; return true;
+    case 160: map = spo::kPrime, n1 = 5, n2 = 32; return mixed;
     case 176: map = spo::kPrime, n1 = 11, n2 = 16; return true;
     case 192: map = spo::kTwiddle, n1 = 12, n2 = 16; return true;
     case 224: map = spo::kPrime, n1 = 7, n2 = 32; return true;
@@ -263,12 +267,12 @@ inline bool kin_paired(int n, int& map, int& n1, int& n2) {
     default: return false;
   }
 }
-inline bool kin_paired_xy(int n) { return n == 2 || n == 4 || n == 8 || n == 16; }
+inline bool kin_preferred_xy(int n) { return n == 2 || n == 4 || n == 6 || n == 8 || n == 12 || n == 16; }
 
-// The levels of kin_kernel for an axis of n points, false if another kernel takes it: the mixed form's pairs above, or for
+// The levels of kin_kernel for an axis of n points, false if another kernel takes it: those above, or for
 // lengths no register kernel has two coprime sizes up to 16 (no twiddles), else any two, the most balanced split first.
-inline bool kin_split(int n, bool mixed, bool prime, int& map, int& n1, int& n2) {
-  if (mixed && kin_paired(n, map, n1, n2) && (prime || map != spo::kPrime)) return true;
+inline bool kin_split(int n, bool mixed, bool preferred, bool prime, int& map, int& n1, int& n2) {
+  if (preferred && kin_preferred(n, mixed, map, n1, n2) && (prime || map != spo::kPrime)) return true;
   map = -1;
   if (axis2_supported(n)) return false;
   auto size_ok = [](int k) { return k >= 2 && k <= 16 && k != 13; };
@@ -604,7 +608,7 @@ class Step final : public StepBase {
     out += " r=" + axis_name(s_.nr, tile_r_, persist_r_, kin_r_);
     const bool xy2 = use_v2_ && s_.nx == s_.ny && xy2_supported(s_.nx);
     out += std::string(" xy=") + (xy2 ? std::string(persist_xy_ ? "xy2p<" : "xy2<") + std::to_string(s_.nx) + "," + lanes(tile_xy_, s_.nx > 8) + ">"
-                                      : std::string("xy_pass(general)"));
+                                : kin_xy_.map >= 0 ? "kin<" + std::to_string(s_.nx) + "x" + std::to_string(s_.ny) + ">" : std::string("xy_pass(general)"));
     if (pot_kind_ == 6) {
       out += " potential=potential6<nphi=" + std::to_string(s_.nphi) + ",nt=" + std::to_string(s_.nt) +
              ",tcgen05.tf32x3,tile=64,blocks=" + std::to_string(pot6_blocks_) + ">";
@@ -627,6 +631,9 @@ class Step final : public StepBase {
       out += " potential=potential2<nphi=" + std::to_string(s_.nphi) + ",cb=" + std::to_string(pot2_cb_) + ">";
     else
       out += " potential=potential(general)";
+    // axes named above by another register kernel of their size that run kin_kernel
+    out += std::string(" kin=") + (kin_z_.map >= 0 && axis2_supported(s_.nz) ? "z" : "") +
+           (kin_r_.map >= 0 && axis2_supported(s_.nr) ? "r" : "") + (kin_xy_.map >= 0 && xy2 ? "xy" : "");
     out += std::string(" balanced=") + (balanced_ ? "1" : "0") + " persistent=" + (persist_z_ ? "z" : "") + (persist_r_ ? "r" : "") + (persist_xy_ ? "xy" : "") +
            " zr_window=" + std::to_string(zr_window_) + " rxy_planes=" + std::to_string(rxy_planes_) + " tiles=" + tiles_source_ + " potential_choice=" + pot_source_;
     return out;
@@ -1296,7 +1303,9 @@ class Step final : public StepBase {
       }
       zr_window_ = best;
     }
-    // T_r and T_xy through L2, slabs of 1, 2 or 4 Z planes, against the full passes.
+    // T_r and T_xy through L2, slabs of 4, 2 or 1 Z planes, against the full passes. Smaller slabs take more launches:
+    // where the slabs of 4 are far behind (launch bound on small packets) the others are not timed, which were 4 of the
+    // 20 ms that creating a 20 MB handle took.
     rxy_planes_ = 0;
     if (zr_window_ == 0 && axis2_supported(s_.nr) && s_.nx == s_.ny && xy2_supported(s_.nx)) {
       auto run = [&] {
@@ -1309,7 +1318,7 @@ class Step final : public StepBase {
       };
       float best_ms = time_launches(run, reps);
       int best = 0;
-      for (const int g : {1, 2, 4}) {
+      for (const int g : {4, 2, 1}) {
         if (g >= s_.nz) continue;
         rxy_planes_ = g;
         const float ms = time_launches(run, reps);
@@ -1317,6 +1326,7 @@ class Step final : public StepBase {
           best = g;
           best_ms = ms;
         }
+        if (ms > 1.5f * best_ms) break;
       }
       rxy_planes_ = best;
     }
@@ -1523,13 +1533,14 @@ class Step final : public StepBase {
     const double xy_scale = (sx * sy) * ((1.0 / (s.nx * sx)) * (1.0 / (s.ny * sy)));
     xyk_full_ = upload_factor(scaled(complex_array(d.xy_kinetic_full, nxy, "xy_kinetic_full"), xy_scale));
     xyk_half_ = upload_factor(scaled(complex_array(d.xy_kinetic_half, nxy, "xy_kinetic_half"), xy_scale));
-    // kin_kernel: where the mixed form's pairs are faster, and both forms' sizes that no other register kernel has.
+    // kin_kernel: where it is the faster one, and the sizes that no other register kernel has.
     use_v2_ = !(std::getenv("SPO_B200_KERNELS") && std::string(std::getenv("SPO_B200_KERNELS")) == "v1");
     use_pfa_ = !(std::getenv("SPO_B200_PFA") && std::string(std::getenv("SPO_B200_PFA")) == "0");
     if (use_v2_) {
-      constexpr bool mixed = sizeof(T) == 4;
+      // An explicit SPO_B200_BALANCED or SPO_B200_PERSISTENT names a form of the other register kernels.
+      const bool preferred = !std::getenv("SPO_B200_BALANCED") && !std::getenv("SPO_B200_PERSISTENT");
       auto axis = [&](KinAxis& ax, int n, const double* full, const double* half) {
-        if (!kin_split(n, mixed, use_pfa_, ax.map, ax.n1, ax.n2)) return;
+        if (!kin_split(n, sizeof(T) == 4, preferred, use_pfa_, ax.map, ax.n1, ax.n2)) return;
         kin_table(ax, 0, scaled(complex_array(full, n, "kinetic factors"), 1.0 / n));
         kin_table(ax, 1, scaled(complex_array(half, n, "kinetic factors"), 1.0 / n));
       };
@@ -1538,7 +1549,7 @@ class Step final : public StepBase {
       const std::vector<cplx> shift = complex_array(d.shift_forward, nxy, "shift_forward");  // as shift_f_ below
       const bool shifted = std::any_of(shift.begin(), shift.end(), [](const cplx& c) { return c != cplx(1.0, 0.0); });
       if (kin_xy_size(s.nx) && kin_xy_size(s.ny) &&
-          (s.nx != s.ny || !xy2_supported(s.nx) || (mixed && !shifted && kin_paired_xy(s.nx)))) {
+          (s.nx != s.ny || !xy2_supported(s.nx) || (preferred && !shifted && kin_preferred_xy(s.nx)))) {
         kin_xy_.map = shifted ? spo::kXyShift : spo::kXy;
         kin_xy_.n1 = s.ny;
         kin_xy_.n2 = s.nx;
@@ -1829,7 +1840,7 @@ class Step final : public StepBase {
           sched[(2 * w) * len + k] = warp[w][k].a;
           sched[(2 * w + 1) * len + k] = warp[w][k].b;
         }
-      std::vector<double> rows(static_cast<std::size_t>(s.n_rot) * (nt_k + 4), 0.0), rows12(rows), rows_lo(rows);
+      std::vector<double> rows12(static_cast<std::size_t>(s.n_rot) * (nt_k + 4), 0.0), rows_lo(rows12);
       std::vector<int> irot_slot(s.n_rot);
       for (int b = 0; b < s.n_blocks; ++b)
         for (int j = 0; j < size[b]; ++j) {
@@ -1838,16 +1849,14 @@ class Step final : public StepBase {
             const int quads = nt_k / 4;  // theta t at the position where the forward tiles read it
             const int pos = (t % quads) * 4 + t / quads;
             const std::size_t k = static_cast<std::size_t>(first[b] + j) * (nt_k + 4) + pos;
-            rows[k] = legendre[offset[b] + t * size[b] + j];
             const double v = legendre64[offset[b] + t * size[b] + j];
             rows12[k] = round_bits(v, 12);
             rows_lo[k] = v - rows12[k];
           }
         }
       pot4_args_.p = pot2_.p;
-      pot4_args_.leg_rows = upload_real(rows);
-      pot4_args_.leg_rows12 = sizeof(T) == 4 ? upload_real(rows12) : nullptr;
-      pot4_args_.leg_rows_lo = sizeof(T) == 4 ? upload_real(rows_lo) : nullptr;
+      pot4_args_.leg_rows12 = upload_real(rows12);
+      pot4_args_.leg_rows_lo = upload_real(rows_lo);
       pot4_args_.slot_first = upload_int(slot_first);
       pot4_args_.slot_nj = upload_int(slot_nj);
       pot4_args_.irot_slot = upload_int(irot_slot);

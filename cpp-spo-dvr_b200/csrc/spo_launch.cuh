@@ -253,13 +253,15 @@ void launch_pot3(int nphi, const spo::Pot2Args<T>& a, dim3 grid, unsigned thread
 }
 
 template <typename T>
-Pot4Kernel<T> pot4_kernel_for(int nphi, int nt) {
-  if (nt == 16 && nphi == 32) return spo::potential4_kernel<T, 32, 16, 8>;
-  if (nt == 16 && nphi == 16) return spo::potential4_kernel<T, 16, 16, 8>;
-  if (nt == 8 && nphi == 16) return spo::potential4_kernel<T, 16, 8, 16>;
-  if (nt == 8 && nphi == 32) return spo::potential4_kernel<T, 32, 8, 16>;
-  if (nt == 4 && nphi == 8) return spo::potential4_kernel<T, 8, 4, 32>;
-  if (nt == 4 && nphi == 12) return spo::potential4_kernel<T, 12, 4, 32>;  // C6v grids
+Pot4Kernel<T> pot4_kernel_for(int nphi, int nt) {  // the mixed form's; FP64 has potential4_dmma_kernel
+  if constexpr (sizeof(T) == 4) {
+    if (nt == 16 && nphi == 32) return spo::potential4_kernel<T, 32, 16, 8>;
+    if (nt == 16 && nphi == 16) return spo::potential4_kernel<T, 16, 16, 8>;
+    if (nt == 8 && nphi == 16) return spo::potential4_kernel<T, 16, 8, 16>;
+    if (nt == 8 && nphi == 32) return spo::potential4_kernel<T, 32, 8, 16>;
+    if (nt == 4 && nphi == 8) return spo::potential4_kernel<T, 8, 4, 32>;
+    if (nt == 4 && nphi == 12) return spo::potential4_kernel<T, 12, 4, 32>;  // C6v grids
+  }
   return nullptr;
 }
 
@@ -267,23 +269,28 @@ template <typename T>
 using KinKernel = void (*)(spo::KinArgs<T>);
 template <typename T>
 KinKernel<T> kin_kernel_for(int map, int n1, int n2) {
-  if constexpr (sizeof(T) == 4) {  // kin_paired, kin_paired_xy
-    if (map == spo::kTwiddle) {
-      if (n1 == 8 && n2 == 16) return spo::kin_kernel<T, spo::kTwiddle, 8, 16>;
-      if (n1 == 12 && n2 == 16) return spo::kin_kernel<T, spo::kTwiddle, 12, 16>;
-      if (n1 == 16 && n2 == 16) return spo::kin_kernel<T, spo::kTwiddle, 16, 16>;
-    } else if (map == spo::kPrime) {
-      if (n1 == 3 && n2 == 16) return spo::kin_kernel<T, spo::kPrime, 3, 16>;
-      if (n1 == 11 && n2 == 16) return spo::kin_kernel<T, spo::kPrime, 11, 16>;
+  // kin_preferred, kin_preferred_xy
+  if (map == spo::kTwiddle) {
+    if constexpr (sizeof(T) == 8)
+      if (n1 == 8 && n2 == 8) return spo::kin_kernel<T, spo::kTwiddle, 8, 8>;
+    if (n1 == 8 && n2 == 16) return spo::kin_kernel<T, spo::kTwiddle, 8, 16>;
+    if (n1 == 12 && n2 == 16) return spo::kin_kernel<T, spo::kTwiddle, 12, 16>;
+    if (n1 == 16 && n2 == 16) return spo::kin_kernel<T, spo::kTwiddle, 16, 16>;
+  } else if (map == spo::kPrime) {
+    if (n1 == 3 && n2 == 16) return spo::kin_kernel<T, spo::kPrime, 3, 16>;
+    if (n1 == 11 && n2 == 16) return spo::kin_kernel<T, spo::kPrime, 11, 16>;
+    if constexpr (sizeof(T) == 4) {
       if (n1 == 3 && n2 == 32) return spo::kin_kernel<T, spo::kPrime, 3, 32>;
       if (n1 == 5 && n2 == 32) return spo::kin_kernel<T, spo::kPrime, 5, 32>;
-      if (n1 == 7 && n2 == 32) return spo::kin_kernel<T, spo::kPrime, 7, 32>;
-    } else if (map == spo::kXy && n1 == n2) {
-      if (n1 == 2) return spo::kin_kernel<T, spo::kXy, 2, 2>;
-      if (n1 == 4) return spo::kin_kernel<T, spo::kXy, 4, 4>;
-      if (n1 == 8) return spo::kin_kernel<T, spo::kXy, 8, 8>;
-      if (n1 == 16) return spo::kin_kernel<T, spo::kXy, 16, 16>;
     }
+    if (n1 == 7 && n2 == 32) return spo::kin_kernel<T, spo::kPrime, 7, 32>;
+  } else if (map == spo::kXy && n1 == n2) {
+    if (n1 == 2) return spo::kin_kernel<T, spo::kXy, 2, 2>;
+    if (n1 == 4) return spo::kin_kernel<T, spo::kXy, 4, 4>;
+    if (n1 == 6) return spo::kin_kernel<T, spo::kXy, 6, 6>;
+    if (n1 == 8) return spo::kin_kernel<T, spo::kXy, 8, 8>;
+    if (n1 == 12) return spo::kin_kernel<T, spo::kXy, 12, 12>;
+    if (n1 == 16) return spo::kin_kernel<T, spo::kXy, 16, 16>;
   }
   return map == spo::kTwiddle ? spo::kin_kernel<T, spo::kTwiddle, 0, 0>
          : map == spo::kPrime ? spo::kin_kernel<T, spo::kPrime, 0, 0>
@@ -299,9 +306,11 @@ KinLaunch<T> kin_configure(int map, int n1, int n2, bool unit, int lanes_per_til
   l.kernel = kin_kernel_for<T>(map, n1, n2);
   while ((spo::KinLine<T>::lanes << (l.log_lines + 1)) <= lanes_per_tile) ++l.log_lines;
   while (l.log_lines > 0 && (static_cast<long long>(spo::KinLine<T>::lanes) << (l.log_lines - 1)) >= window) --l.log_lines;
-  const int lines = 1 << l.log_lines, limit = spo::kin_max_threads(std::max(n1, n2));
   const std::size_t n = static_cast<std::size_t>(n1) * n2;
-  l.smem = 16 * (spo::kin_words<T>(map, n1 * n2, unit) + 2 * n * lines);
+  auto smem_of = [&](int log_lines) { return 16 * (spo::kin_words<T>(map, n1 * n2, unit) + (2 * n << log_lines)); };
+  while (l.log_lines > 0 && smem_of(l.log_lines) > static_cast<std::size_t>(smem_optin_bytes())) --l.log_lines;
+  const int lines = 1 << l.log_lines, limit = spo::kin_max_threads(std::max(n1, n2));
+  l.smem = smem_of(l.log_lines);
   const double fit = std::floor((228 << 10) / static_cast<double>(l.smem + 1024));
   double best = 0.0;
   for (int nt = 1; nt <= std::max(n1, n2) && nt * lines <= limit; ++nt) {

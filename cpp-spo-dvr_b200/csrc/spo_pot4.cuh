@@ -5,8 +5,8 @@
 // NT * CB = 128 threads. The angular matrix M_m[theta, J] = sqrt(w_theta / nphi) P_J^m(theta) has one
 // row per rotational state irot (its block m, its J), padded to NT + 4 values, so that the 16-byte
 // loads of consecutive rows fall on distinct bank groups; within a row theta is stored in the order in
-// which the forward tiles take it. The mixed form stages it in shared memory once per block, FP64 reads
-// it through L1 (pot4_matrix_shared). Per item:
+// which the forward tiles take it. It is staged in shared memory once per block. The mixed form only (FP64:
+// spo_pot4d.cuh). Per item:
 //   load:    F[irot][c] = opt_Z before(ir, irot) psi(c, irot), plus rot(dt/2) e0(c) chi(ir, iz) in the
 //            initial channel (potential_operator.cpp:116-123);
 //   forward: X[p][theta][c] = sum_J M_m[theta, J] F[first_m + J][c] for the slot p of every mJ block m,
@@ -30,12 +30,11 @@ namespace spo {
 template <typename T>
 struct Pot4Args {
   PotArgs<T> p;              // pointers and sizes shared with the other potential kernels
-  const T* leg_rows;         // n_rot rows of NT + 4: M_m[theta, J] of irot = first_m + J, theta at position
-                             // (theta % (NT / 4)) * 4 + theta / (NT / 4)
-  // mixed form: the same rows as a 12-bit high part and the FP32 rounding of the rest, so that hi + lo is the FP64
-  // matrix to ~2^-36 and each term's lo product stays well above the rounding unit of the running sum: with the
-  // matrix rounded to FP32 the contractions of a physical wave packet change its norm by up to ~1e-8 per step, the
-  // same sign every step
+  // n_rot rows of NT + 4: M_m[theta, J] of irot = first_m + J, theta at position (theta % (NT / 4)) * 4 +
+  // theta / (NT / 4), as a 12-bit high part and the FP32 rounding of the rest, so that hi + lo is the FP64 matrix to
+  // ~2^-36 and each term's lo product stays well above the rounding unit of the running sum: with the matrix rounded
+  // to FP32 the contractions of a physical wave packet change its norm by up to ~1e-8 per step, the same sign every
+  // step
   const T* leg_rows12;
   const T* leg_rows_lo;
   const int* slot_first;     // per phi slot: first irot of its mJ block
@@ -53,26 +52,12 @@ SPO_HD void ld4(const float* p, float (&o)[4]) {
   const float4 q = *reinterpret_cast<const float4*>(p);
   o[0] = q.x; o[1] = q.y; o[2] = q.z; o[3] = q.w;
 }
-SPO_HD void ld4(const double* p, double (&o)[4]) {
-  const double2 a = *reinterpret_cast<const double2*>(p);
-  const double2 b = *reinterpret_cast<const double2*>(p + 2);
-  o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y;
-}
 SPO_HD void ld2c(const float2* p, float2& a, float2& b) {
   const float4 q = *reinterpret_cast<const float4*>(p);
   a = make_float2(q.x, q.y);
   b = make_float2(q.z, q.w);
 }
-SPO_HD void ld2c(const double2* p, double2& a, double2& b) {
-  a = p[0];
-  b = p[1];
-}
 SPO_HD void st2c(float2* p, float2 a, float2 b) { *reinterpret_cast<float4*>(p) = make_float4(a.x, a.y, b.x, b.y); }
-SPO_HD void st2c(double2* p, double2 a, double2 b) {
-  p[0] = a;
-  p[1] = b;
-}
-
 // X holds one block of NT * CB values per phi slot, each followed by 16 bytes of padding: the back sums
 // of a warp read the blocks of two or three slots at once, which then start on different banks.
 template <typename T>
@@ -80,26 +65,19 @@ constexpr int pot4_slot_stride(int nt, int cb) {
   return nt * cb + static_cast<int>(16 / sizeof(Vec<T>));
 }
 
-// Where the matrix rows live: shared memory in the mixed form (20 KB on config 2); in FP64 (40 KB) they
-// are read through L1 instead, so that two FP64 blocks fit per SM (10.3 against 12.7 ms per launch on
-// config 2, where the mixed form is fastest with them staged).
-template <typename T>
-constexpr bool pot4_matrix_shared() {
-  return sizeof(T) == 4;
-}
-
 // Shared memory of potential4_kernel: F (n_rot CB), X (NPHI padded slot blocks), the matrix rows
-// (n_rot (NT + 4), when staged), irot -> slot (n_rot ints), the schedule (8 sched_len ints).
+// (n_rot (NT + 4)), irot -> slot (n_rot ints), the schedule (8 sched_len ints).
 template <typename T>
 constexpr std::size_t pot4_smem(int n_rot, int nphi, int nt, int cb, int sched_len) {
   return sizeof(Vec<T>) * (static_cast<std::size_t>(n_rot) * cb + static_cast<std::size_t>(nphi) * pot4_slot_stride<T>(nt, cb)) +
-         (pot4_matrix_shared<T>() ? sizeof(T) * static_cast<std::size_t>(n_rot) * (nt + 4) : 0) +
+         sizeof(T) * static_cast<std::size_t>(n_rot) * (nt + 4) +
          sizeof(int) * (static_cast<std::size_t>(n_rot) + 8 * sched_len);
 }
 
 template <typename T, int NPHI, int NT, int CB>
-__global__ void __launch_bounds__(NT * CB, sizeof(T) == 4 ? 3 : 1) potential4_kernel(Pot4Args<T> g) {
+__global__ void __launch_bounds__(NT * CB, 3) potential4_kernel(Pot4Args<T> g) {
   using V = Vec<T>;
+  static_assert(sizeof(T) == 4, "the mixed form");
   static_assert(NT * CB == 128 && NT % 4 == 0 && CB % 2 == 0, "tile shape");
   constexpr int NTH = NT * CB;
   constexpr int LDL = NT + 4;
@@ -112,16 +90,11 @@ __global__ void __launch_bounds__(NT * CB, sizeof(T) == 4 ? 3 : 1) potential4_ke
   extern __shared__ __align__(16) unsigned char smem_raw[];
   V* F = reinterpret_cast<V*>(smem_raw);                   // [irot][c]
   V* X = F + n_rot * CB;                                   // [p][theta][c], slot blocks of SS values
-  constexpr bool L_SHARED = pot4_matrix_shared<T>();
-  T* Ls = reinterpret_cast<T*>(X + NPHI * SS);             // [irot][position of theta], rows of LDL
-  // the mixed form's matrix as 12-bit high parts plus the rest, as potential5 uses it
-  const T* rows = sizeof(T) == 4 ? g.leg_rows12 : g.leg_rows;
-  const T* L = L_SHARED ? Ls : rows;
-  int* irot_slot = reinterpret_cast<int*>(Ls + (L_SHARED ? n_rot * LDL : 0));
+  T* L = reinterpret_cast<T*>(X + NPHI * SS);             // [irot][position of theta], rows of LDL
+  int* irot_slot = reinterpret_cast<int*>(L + n_rot * LDL);
   int* sched = irot_slot + n_rot;                          // [group][k]
   const int tid = threadIdx.x;
-  if constexpr (L_SHARED)
-    for (int k = tid; k < n_rot * LDL; k += NTH) Ls[k] = rows[k];
+  for (int k = tid; k < n_rot * LDL; k += NTH) L[k] = g.leg_rows12[k];
   for (int k = tid; k < n_rot; k += NTH) irot_slot[k] = g.irot_slot[k];
   for (int k = tid; k < 8 * g.sched_len; k += NTH) sched[k] = g.fwd_sched[k];
   __syncthreads();
@@ -177,21 +150,10 @@ __global__ void __launch_bounds__(NT * CB, sizeof(T) == 4 ? 3 : 1) potential4_ke
       }
       st2c(F + irot * CB + c, v0, v1);
     };
-    // FP64: batches of 4 tasks, all their loads issued before the first is used (in the mixed form the
-    // registers are taken by the exp(i A) line of the phase after next: batching there spills).
-    constexpr int LB = sizeof(T) == 4 ? 1 : 4;
-    for (int k0 = tid; k0 < n_tasks; k0 += NTH * LB) {
-      V v0[LB], v1[LB];
-#pragma unroll
-      for (int i = 0; i < LB; ++i) {
-        const int k = k0 + NTH * i;
-        if (k < n_tasks) load_task(col_base, ncol, k, v0[i], v1[i]);
-      }
-#pragma unroll
-      for (int i = 0; i < LB; ++i) {
-        const int k = k0 + NTH * i;
-        if (k < n_tasks) store_task(k, v0[i], v1[i]);
-      }
+    for (int k = tid; k < n_tasks; k += NTH) {
+      V v0, v1;
+      load_task(col_base, ncol, k, v0, v1);
+      store_task(k, v0, v1);
     }
     __syncthreads();
 
@@ -215,24 +177,14 @@ __global__ void __launch_bounds__(NT * CB, sizeof(T) == 4 ? 3 : 1) potential4_ke
         ld4(lp + j * LDL, l);
         V f0, f1;
         ld2c(fp + j * CB, f0, f1);
-        if constexpr (sizeof(T) == 4) {
-          T m[4];
-          ld4(g.leg_rows_lo + (first + j) * LDL + 4 * fq, m);
+        T m[4];
+        ld4(g.leg_rows_lo + (first + j) * LDL + 4 * fq, m);
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            acc[q][0] = fmaf(l[q], f0.x, fmaf(m[q], f0.x, acc[q][0]));
-            acc[q][1] = fmaf(l[q], f0.y, fmaf(m[q], f0.y, acc[q][1]));
-            acc[q][2] = fmaf(l[q], f1.x, fmaf(m[q], f1.x, acc[q][2]));
-            acc[q][3] = fmaf(l[q], f1.y, fmaf(m[q], f1.y, acc[q][3]));
-          }
-        } else {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            acc[q][0] += l[q] * f0.x;
-            acc[q][1] += l[q] * f0.y;
-            acc[q][2] += l[q] * f1.x;
-            acc[q][3] += l[q] * f1.y;
-          }
+        for (int q = 0; q < 4; ++q) {
+          acc[q][0] = fmaf(l[q], f0.x, fmaf(m[q], f0.x, acc[q][0]));
+          acc[q][1] = fmaf(l[q], f0.y, fmaf(m[q], f0.y, acc[q][1]));
+          acc[q][2] = fmaf(l[q], f1.x, fmaf(m[q], f1.x, acc[q][2]));
+          acc[q][3] = fmaf(l[q], f1.y, fmaf(m[q], f1.y, acc[q][3]));
         }
       }
 #pragma unroll
@@ -240,11 +192,10 @@ __global__ void __launch_bounds__(NT * CB, sizeof(T) == 4 ? 3 : 1) potential4_ke
         st2c(X + slot * SS + (fq + QUADS * q) * CB + 2 * fc, cmake<V>(acc[q][0], acc[q][1]),
              cmake<V>(acc[q][2], acc[q][3]));
     }
-    // Mixed form: exp(i A) of this thread's phi line (no symmetry maps), requested before the barrier,
-    // so that the loads overlap the other threads' last forward tiles (FP64 has no registers to spare).
-    constexpr bool EARLY_EXP = sizeof(T) == 4;
-    V e[EARLY_EXP ? NPHI : 1];
-    const bool direct = EARLY_EXP && g.identity_maps && has_line;
+    // exp(i A) of this thread's phi line (no symmetry maps), requested before the barrier, so that the loads overlap
+    // the other threads' last forward tiles.
+    V e[NPHI];
+    const bool direct = g.identity_maps && has_line;
     if (direct) {
       const V* ep = a.expia + ((static_cast<long long>(izr) * a.n_rep + c0 + line_c) * NT + line_t) * NPHI;
       static_for<0, NPHI / 2>([&](auto h) { ld2c(ep + 2 * SPO_CV(h), e[2 * SPO_CV(h)], e[2 * SPO_CV(h) + 1]); });
@@ -260,18 +211,7 @@ __global__ void __launch_bounds__(NT * CB, sizeof(T) == 4 ? 3 : 1) potential4_ke
       rdft<NPHI, +1>(x);
       if (direct) {
         const long long e0 = ((static_cast<long long>(izr) * a.n_rep + c0 + line_c) * NT + line_t) * NPHI;
-        if constexpr (EARLY_EXP)
-          static_for<0, NPHI>([&](auto p) { x[SPO_CV(p)] = exp_mul(x[SPO_CV(p)], e[SPO_CV(p)], a.exp_mod, e0 + SPO_CV(p)); });
-      } else if (g.identity_maps) {
-        const long long e0 = ((static_cast<long long>(izr) * a.n_rep + ixy) * NT + line_t) * NPHI;
-        const V* ep = a.expia + e0;
-        static_for<0, NPHI / 2>([&](auto h) {
-          constexpr int P = 2 * SPO_CV(h);
-          V ea, eb;
-          ld2c(ep + P, ea, eb);
-          x[P] = exp_mul(x[P], ea, a.exp_mod, e0 + P);
-          x[P + 1] = exp_mul(x[P + 1], eb, a.exp_mod, e0 + P + 1);
-        });
+        static_for<0, NPHI>([&](auto p) { x[SPO_CV(p)] = exp_mul(x[SPO_CV(p)], e[SPO_CV(p)], a.exp_mod, e0 + SPO_CV(p)); });
       } else {
         const long long e0 = ((static_cast<long long>(izr) * a.n_rep + __ldg(a.rep_of + ixy)) * NT + line_t) * NPHI;
         const int* map = a.phi_map + ixy * NPHI;
@@ -295,9 +235,9 @@ __global__ void __launch_bounds__(NT * CB, sizeof(T) == 4 ? 3 : 1) potential4_ke
       const V* ys = X + slot * SS;
 #pragma unroll 1
       for (int kq = 0; kq < QUADS; ++kq) {
-        T l[4], m[4] = {0, 0, 0, 0};
+        T l[4], m[4];
         ld4(lrow + 4 * kq, l);  // theta kq + QUADS q, q < 4
-        if constexpr (sizeof(T) == 4) ld4(g.leg_rows_lo + irot * LDL + 4 * kq, m);
+        ld4(g.leg_rows_lo + irot * LDL + 4 * kq, m);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const V* y = ys + (kq + QUADS * q) * CB;
@@ -305,17 +245,10 @@ __global__ void __launch_bounds__(NT * CB, sizeof(T) == 4 ? 3 : 1) potential4_ke
           for (int c = 0; c < CB; c += 2) {
             V y0, y1;
             ld2c(y + c, y0, y1);
-            if constexpr (sizeof(T) == 4) {
-              acc[c][0] = fmaf(l[q], y0.x, fmaf(m[q], y0.x, acc[c][0]));
-              acc[c][1] = fmaf(l[q], y0.y, fmaf(m[q], y0.y, acc[c][1]));
-              acc[c + 1][0] = fmaf(l[q], y1.x, fmaf(m[q], y1.x, acc[c + 1][0]));
-              acc[c + 1][1] = fmaf(l[q], y1.y, fmaf(m[q], y1.y, acc[c + 1][1]));
-            } else {
-              acc[c][0] += l[q] * y0.x;
-              acc[c][1] += l[q] * y0.y;
-              acc[c + 1][0] += l[q] * y1.x;
-              acc[c + 1][1] += l[q] * y1.y;
-            }
+            acc[c][0] = fmaf(l[q], y0.x, fmaf(m[q], y0.x, acc[c][0]));
+            acc[c][1] = fmaf(l[q], y0.y, fmaf(m[q], y0.y, acc[c][1]));
+            acc[c + 1][0] = fmaf(l[q], y1.x, fmaf(m[q], y1.x, acc[c + 1][0]));
+            acc[c + 1][1] = fmaf(l[q], y1.y, fmaf(m[q], y1.y, acc[c + 1][1]));
           }
         }
       }

@@ -1,0 +1,163 @@
+"""The kernels that take any sizes, at the sizes where they can go wrong, against the general kernels
+(SPO_B200_KERNELS=v1, which the oracle checks) or a numpy restatement (needs a B200).
+
+  - kin_kernel: axis lengths and (x, y) grids without an instantiation, rectangular cells, odd basis sizes (lanes that
+    do not pair up on 16-byte boundaries), one lane, the momentum shift;
+  - potential5 (mixed) and potential4 (FP64) on the FP64 tensor cores: theta 1 to 16, phi 6 to 32, columns that do not
+    fill an item or belong to several points, symmetry maps, the homonuclear basis;
+  - the step as one graph against its kernels launched one by one;
+  - host copies by several threads; prediction of the network for ragged numbers of points.
+
+The bars are those of test_gpu_kernels.py: 1e-12 (FP64) and 2e-6 (mixed) of the largest value per operator, 1e-11 and 2e-5
+relative L2 for an analysis step.
+"""
+
+import numpy as np
+import pytest
+
+from conftest import rel_err, rel_l2
+from test_gpu_kernels import make
+
+pytestmark = pytest.mark.gpu
+
+TOL = {"fp64": (1e-12, 1e-11), "mixed": (2e-6, 2e-5)}
+
+
+def random_state(case, seed):
+    rng = np.random.default_rng(seed)
+    psi = rng.standard_normal(case.psi_shape) + 1j * rng.standard_normal(case.psi_shape)
+    return psi, rng.standard_normal(case.chi_shape) + 1j * rng.standard_normal(case.chi_shape)
+
+
+def compare(case, precision, stages):
+    """The default kernels against the general ones: the given operators one after another, then an analysis step."""
+    psi, chi = random_state(case, 3)
+    stage_bar, step_bar = TOL[precision]
+    with make(case, "v1", precision) as ref, make(case, None, precision) as new:
+        text = new.describe()
+        for be in (ref, new):
+            be.read_wave_packet(psi, chi)
+        for stage in stages:
+            for be in (ref, new):
+                be.apply_stage(stage)
+            a, b = ref.wave_packet_on_host(), new.wave_packet_on_host()
+            assert rel_err(b[0], a[0]) < stage_bar and rel_err(b[1], a[1]) < stage_bar, (stage, text)
+        for be in (ref, new):
+            be.read_wave_packet(psi, chi)
+            be.propagate_analysis_step()
+        a, b = ref.wave_packet_on_host(), new.wave_packet_on_host()
+        assert rel_l2(b[0], a[0]) < step_bar and rel_l2(b[1], a[1]) < step_bar, text
+    return text
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("nz,nr,nx,ny,j_max", [(90, 36, 10, 10, 2), (72, 45, 5, 9, 1), (110, 30, 9, 4, 2), (84, 44, 7, 7, 3),
+                                               (60, 20, 16, 2, 1), (128, 48, 16, 16, 1), (176, 56, 4, 4, 2),
+                                               (96, 40, 12, 12, 1), (36, 22, 3, 11, 0), (28, 18, 1, 1, 2)])
+def test_kinetic_passes_of_any_lengths(nz, nr, nx, ny, j_max, precision):
+    from spo_b200 import capi, workload
+    case = workload.config_case({"nz": nz, "nr": nr, "nx": nx, "ny": ny, "j_max": j_max, "mj_max": j_max,
+                                 "nz_specular": 2 * nz, "nz_potential": nz // 3})
+    phase = np.exp(1j * np.random.default_rng(1).uniform(0, 6, nx * ny))
+    case.a["shift_forward"], case.a["shift_backward"] = phase, np.conj(phase)
+    compare(case, precision, (capi.STAGE_ZR, capi.STAGE_XY))
+
+
+def fold(case, n):
+    """C3v maps on an n x n cell: every point takes the potential of the smallest point of its orbit."""
+    nphi, nt = case.n_phi, case.n_theta
+    ix, iy = np.meshgrid(np.arange(n), np.arange(n), indexing="ij")
+    best, op, maps = np.full(n * n, n * n), np.zeros(n * n, dtype=np.int32), []
+    for r in range(3):
+        for s in (1, -1):
+            x, y = (ix, iy) if s > 0 else (iy, ix)
+            for _ in range(r):
+                x, y = (-y) % n, (x - y) % n
+            k = (x * n + y).ravel()
+            op[k < best] = len(maps)
+            best = np.minimum(best, k)
+            maps.append((s * np.arange(nphi) + r * nphi // 3) % nphi)
+    reps = np.unique(best)
+    full = case.a["potential"].reshape(-1, n * n, nt * nphi)
+    case.a["potential"] = np.ascontiguousarray(full[:, reps]).reshape(-1)
+    case.a["representative_of"] = np.searchsorted(reps, best).astype(np.int32)
+    case.a["operation_of"], case.a["phi_index"] = op, np.concatenate(maps).astype(np.int32)
+    case.m["n_rep"], case.m["n_ops"] = len(reps), 6
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("j_max,homonuclear,nx,ny,symmetry",
+                         [(j, False, 5, 3, False) for j in (2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 13, 14, 15)] +
+                         [(4, True, 5, 3, False), (10, True, 4, 4, False), (14, True, 2, 2, False), (14, True, 8, 8, False),
+                          (15, False, 2, 2, False), (15, False, 8, 8, False), (7, False, 1, 1, False),
+                          (11, False, 6, 6, True), (8, False, 4, 4, True), (5, False, 3, 3, True)])
+def test_potential_step_of_any_angular_grid(j_max, homonuclear, nx, ny, symmetry, precision):
+    from spo_b200 import capi, workload
+    case = workload.config_case({"nz": 16, "nr": 6, "nx": nx, "ny": ny, "j_max": j_max, "mj_max": j_max,
+                                 "homonuclear": homonuclear, "nz_specular": 32, "nz_potential": 11})
+    if symmetry:
+        fold(case, nx)
+    text = compare(case, precision, (capi.STAGE_POTENTIAL,))
+    kernel = "potential4" if precision == "fp64" else "potential5"
+    assert ",dmma" in text and f"potential={kernel}<nphi={case.n_phi}," in text, text
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_a_step_as_one_graph_is_bitwise_its_kernels_one_by_one(precision):
+    """With profiling on the kernels are launched one after another on the handle's stream; the graph runs the specular
+    grid's beside the kinetic passes. The same kernels on the same data, also on a caller's stream."""
+    import torch
+    from spo_b200 import workload
+    case = workload.config_case({"nz": 48, "nr": 24, "nx": 6, "ny": 6, "j_max": 5, "mj_max": 5, "nz_specular": 96,
+                                 "nz_potential": 30})
+    psi, chi = random_state(case, 8)
+    out = []
+    for mode in ("graph", "launches", "stream"):
+        with make(case, None, precision) as be:
+            be.read_wave_packet(psi, chi)
+            if mode == "launches":
+                be.profile(True)
+            if mode == "stream":
+                stream = torch.cuda.Stream()
+                be.set_stream(stream.cuda_stream)
+            for _ in range(3):
+                be.propagate_analysis_step()
+            out.append(be.wave_packet_on_host() + (be.last_launch_count(),))
+    for other in out[1:]:
+        assert np.array_equal(out[0][0], other[0]) and np.array_equal(out[0][1], other[1]) and out[0][2] == other[2]
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_large_packets_cross_to_the_device_and_back_unchanged(precision):
+    """Copies of 4 MiB and more by several threads: a packet that does not fill the last chunk, into ordinary and into
+    pinned memory (which takes the other path)."""
+    import torch
+    from spo_b200 import workload
+    case = workload.config_case({"nz": 64, "nr": 30, "nx": 7, "ny": 5, "j_max": 4, "mj_max": 4, "nz_specular": 128,
+                                 "nz_potential": 4})
+    psi, chi = random_state(case, 5)
+    want = psi if precision == "fp64" else psi.astype(np.complex64).astype(np.complex128)
+    with make(case, None, precision) as be:
+        be.read_wave_packet(psi, chi)
+        got, _ = be.wave_packet_on_host()
+        assert np.array_equal(got, want)
+        pinned = torch.empty(case.psi_shape, dtype=torch.complex128).pin_memory().numpy()
+        pinned[...] = psi[::-1]
+        be.read_wave_packet(pinned, None)
+        got, _ = be.wave_packet_on_host()
+        assert np.array_equal(got, want[::-1])
+
+
+@pytest.mark.parametrize("n,n_in,width,depth", [(1, 1, 64, 1), (127, 12, 128, 2), (128, 64, 256, 4), (129, 7, 64, 8),
+                                                (40001, 12, 256, 3), (200000, 12, 128, 4)])
+def test_predictions_of_ragged_numbers_of_points(n, n_in, width, depth):
+    """Against the numpy oracle, to 1e-2 of the output scale (BF16 activations, as test_gpu_mlp.py)."""
+    import mlp_oracle
+    from spo_b200.mlp import Mlp
+    x = np.random.default_rng(n).uniform(-1.0, 1.0, (n, n_in)).astype(np.float32)
+    with Mlp(n_in, width, depth, seed=n) as net:
+        some = np.unique(np.concatenate([np.arange(min(n, 300)), np.arange(max(0, n - 300), n)]))
+        want, _, _ = mlp_oracle.forward(net.get_parameters(), x[some], net.input_width, width, depth)
+        got = net.predict(x)
+    assert got.shape == (n,) and np.all(np.isfinite(got))
+    assert np.max(np.abs(got[some] - want)) <= 1e-2 * max(np.max(np.abs(want)), 1e-3)
