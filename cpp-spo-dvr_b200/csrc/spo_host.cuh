@@ -234,18 +234,18 @@ Pot4Kernel<T> pot4_kernel_for(int nphi, int nt);
 template <typename T>
 struct KinLaunch {
   void (*kernel)(spo::KinArgs<T>) = nullptr;
-  int threads = 0, log_lines = 0;
+  int threads = 0, log_lines = 0, lanes = 1;  // lanes per line
   long long blocks = 0;  // resident blocks of the device
   std::size_t smem = 0;
 };
 template <typename T>
-KinLaunch<T> kin_configure(int map, int n1, int n2, bool unit, int lanes_per_tile, long long window);
+KinLaunch<typename spo::KinStored<T>::type> kin_configure(int map, int n1, int n2, bool unit, int lanes_per_tile, long long window);
 
 // The lengths and square grids that run kin_kernel although another register kernel has them: where it measured faster (ms
 // per launch of 0.1 to 1.6 GB, against the other kernel at its best tile width).
 //   mixed form, pairs of lanes: 48 0.242/0.259, 96 0.495/0.560, 128 0.228/0.250, 160 0.259/0.296, 176 0.168/0.226, 192
-//     0.273/0.300, 224 0.184/0.223, 256 0.156/0.188; x = y: 2 0.030/0.036, 4 0.064/0.097, 6 0.180/0.188, 8 0.151/0.227,
-//     12 0.372/0.445, 16 0.363/0.487;
+//     0.273/0.300, 224 0.184/0.223, 256 0.156/0.188; x = y: 2 0.030/0.036, 4 0.064/0.097, 6 0.174/0.188, 8 0.151/0.227,
+//     12 0.372/0.445, 16 0.363/0.487 (6: Wide);
 //   FP64: 48 0.374/0.418, 64 0.364/0.411, 128 0.348/0.390, 176 0.189/0.238, 192 0.279/0.312, 224 0.203/0.224, 256
 //     0.228/0.287; x = y: 2 0.0307/0.0312, 4 0.151/0.159, 6 0.176/0.214, 8 0.213/0.251, 12 0.384/0.518, 16 0.570/0.618.
 // The (x, y) pass without a momentum shift only: with its two extra factors the mixed 16 x 16 pass took 2.07 ms on
@@ -268,6 +268,15 @@ inline bool kin_preferred(int n, bool mixed, int& map, int& n1, int& n2) {
   }
 }
 inline bool kin_preferred_xy(int n) { return n == 2 || n == 4 || n == 6 || n == 8 || n == 12 || n == 16; }
+
+// The mixed form's Wide kernel (FP64 between load and store) takes the sizes that have no kernel of their own, and 6 x 6:
+// pairs sum radices 5, 7, 9 and 11 line by line and compensate every twiddle of an odd length, Wide is bound by the FP64
+// pipe at 2.0 to 2.9 TB/s (ms, Wide/pairs): 100 1.14/1.88, 90 0.323/0.424, 140 1.51/2.57, 36 0.257/0.293, 50 1.08/1.59,
+// 63 0.072/0.086; x = y: 10 0.319/0.460, 14 0.269/0.379, 15 1.51/1.67, 9 0.309/0.395, 6 0.174/0.180 (a few are the other way
+// round: 42 0.183/0.175, 20 0.177/0.171, 7 0.221/0.209). Not where pairs have a kernel of powers of two, 3 and 12 (128
+// 0.345/0.228, 96 0.676/0.494, 48 0.321/0.242; x = y: 16 0.565/0.365, 8 0.210/0.151, 12 0.376/0.372), nor 5 and 7 with 32
+// (160 0.307/0.259, 224 0.203/0.183), nor the lengths of axis2pfa_kernel (40 0.178/0.130, 112 0.158/0.124).
+inline bool kin_wide_xy(int nx, int ny, bool shifted) { return shifted || nx != ny || nx == 6 || !kin_preferred_xy(nx); }
 
 // The levels of kin_kernel for an axis of n points, false if another kernel takes it: those above, or for
 // lengths no register kernel has two coprime sizes up to 16 (no twiddles), else any two, the most balanced split first.
@@ -487,6 +496,7 @@ class Step final : public StepBase {
   // shapes by (lanes per tile, lanes).
   struct KinAxis {
     int map = -1, n1 = 0, n2 = 0;
+    bool wide = false;  // mixed form: FP64 between load and store
     double2* table[2] = {nullptr, nullptr};
     T scale[2] = {T(1), T(1)};
     int unit[2] = {1, 1};
@@ -1038,10 +1048,15 @@ class Step final : public StepBase {
   void kin_launch(KinAxis& ax, bool half, int tile, spo::KinArgs<T>& a, long long outer) {
     const int lanes = tile > 0 ? tile : ax.n1 * ax.n2 >= 80 ? 16 : 32;
     auto it = ax.launches.find({lanes, a.window});
-    if (it == ax.launches.end())
-      it = ax.launches.emplace(std::make_pair(lanes, a.window), kin_configure<T>(ax.map, ax.n1, ax.n2, ax.unit[0] && ax.unit[1], lanes, a.window)).first;
+    if (it == ax.launches.end()) {
+      const bool unit = ax.unit[0] && ax.unit[1];
+      KinLaunch<T> made;
+      if constexpr (sizeof(T) == 4) made = ax.wide ? kin_configure<spo::Wide>(ax.map, ax.n1, ax.n2, unit, lanes, a.window) : kin_configure<T>(ax.map, ax.n1, ax.n2, unit, lanes, a.window);
+      else made = kin_configure<T>(ax.map, ax.n1, ax.n2, unit, lanes, a.window);
+      it = ax.launches.emplace(std::make_pair(lanes, a.window), made).first;
+    }
     const KinLaunch<T>& l = it->second;
-    const long long per_tile = static_cast<long long>(spo::KinLine<T>::lanes) << l.log_lines;
+    const long long per_tile = static_cast<long long>(l.lanes) << l.log_lines;
     const long long blocks_per_group = (a.window + per_tile - 1) / per_tile, n_tiles = blocks_per_group * a.groups * outer;
     require(n_tiles < (1ll << 32), "kinetic pass: too many tiles");
     a.n1 = ax.n1;
@@ -1424,7 +1439,7 @@ class Step final : public StepBase {
     const std::vector<cplx> tw = ax.map == spo::kTwiddle ? twiddles(n) : std::vector<cplx>();
     ax.scale[half] = T(1);
     ax.unit[half] = 1;
-    if constexpr (sizeof(T) == 8) {
+    if (sizeof(T) == 8 || ax.wide) {
       std::vector<cplx> t = f;
       t.insert(t.end(), tw.begin(), tw.end());
       ax.table[half] = upload_c128(t);
@@ -1541,6 +1556,7 @@ class Step final : public StepBase {
       const bool preferred = !std::getenv("SPO_B200_BALANCED") && !std::getenv("SPO_B200_PERSISTENT");
       auto axis = [&](KinAxis& ax, int n, const double* full, const double* half) {
         if (!kin_split(n, sizeof(T) == 4, preferred, use_pfa_, ax.map, ax.n1, ax.n2)) return;
+        ax.wide = sizeof(T) == 4 && !axis2_supported(n);
         kin_table(ax, 0, scaled(complex_array(full, n, "kinetic factors"), 1.0 / n));
         kin_table(ax, 1, scaled(complex_array(half, n, "kinetic factors"), 1.0 / n));
       };
@@ -1551,6 +1567,7 @@ class Step final : public StepBase {
       if (kin_xy_size(s.nx) && kin_xy_size(s.ny) &&
           (s.nx != s.ny || !xy2_supported(s.nx) || (preferred && !shifted && kin_preferred_xy(s.nx)))) {
         kin_xy_.map = shifted ? spo::kXyShift : spo::kXy;
+        kin_xy_.wide = sizeof(T) == 4 && kin_wide_xy(s.nx, s.ny, shifted);
         kin_xy_.n1 = s.ny;
         kin_xy_.n2 = s.nx;
         kin_table(kin_xy_, 0, scaled(complex_array(d.xy_kinetic_full, nxy, "xy_kinetic_full"), xy_scale));

@@ -23,7 +23,7 @@ namespace spo_host {
 // The streams and pinned buffers of a device's large copies: at most 8 MiB of pinned memory, made for the first handle
 // that needs them, shared by all handles of the device (one copy at a time) and freed with the last of them. With a set
 // per handle the first copy of each further handle paid for its own pinned memory (14 of 19 ms of a network's first
-// prediction of 1.6 M points; 8.7 ms with the shared set).
+// prediction of 1 M points; 8.7 ms with the shared set).
 class CopyPool {
  public:
   static constexpr std::size_t kChunk = 512 << 10;  // bytes on the device per chunk

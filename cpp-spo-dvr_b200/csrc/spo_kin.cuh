@@ -16,8 +16,11 @@
 // with p the power of two in s, folded into g and exact, and a product with the rest s / p only where it is not 1.
 //
 // N1, N2 > 0: compile-time sizes. N1 = N2 = 0: any two sizes up to 16 that rdft has (a switch per level), for the
-// lengths without an instantiation and for rectangular (x, y) grids, in both forms; the shared-memory Stockham kernels
+// lengths without an instantiation and for rectangular (x, y) grids, as FP64 and Wide; the shared-memory Stockham kernels
 // they ran on before are 3 to 10 times slower (T_Z of 90 points, r 36, x = y = 10: 1.12 ms).
+//
+// FP64 and Wide take one lane per thread. FP64 passes run at 4.3 to 5.6 TB/s (other register kernels: 3.9 to 5.0), Wide
+// at 2.0 to 2.9, where the FP64 pipe is the limit.
 #pragma once
 
 #include "spo_pot5.cuh"
@@ -26,6 +29,13 @@ namespace spo {
 
 enum KinMap : int { kTwiddle = 0, kPrime = 1, kXy = 2, kXyShift = 3 };  // kXy: without the momentum shift
 constexpr bool kin_is_xy(int map) { return map == kXy || map == kXyShift; }
+
+// The forms of the kernel: float (complex64, pairs of lanes as packed FP32), double (complex128), and Wide: complex64 in
+// memory, FP64 in between, one lane per thread, the constants as they are and one rounding per pass.
+struct Wide {};
+template <typename T> struct KinStored { using type = T; };
+template <> struct KinStored<Wide> { using type = float; };
+template <typename T> using KinVec = Vec<typename KinStored<T>::type>;
 
 template <typename T>
 struct KinArgs {
@@ -44,7 +54,7 @@ struct KinArgs {
 };
 
 // Table entries: mixed form: N pairs (p g.x, p g.x, p g.y, p g.y) and (their low parts), for kTwiddle N twiddles
-// (w.x, w.x, w.y, w.y) and (their low parts), and where some s is not p N scales (s/p, s/p, low, low); FP64 form: N
+// (w.x, w.x, w.y, w.y) and (their low parts), and where some s is not p N scales (s/p, s/p, low, low); FP64 and Wide: N
 // factors, then N twiddles.
 template <typename T> struct KinLine;
 template <> struct KinLine<float> {
@@ -57,6 +67,7 @@ template <> struct KinLine<double> {
   static constexpr int lanes = 1;
   static constexpr int factor_words = 1, twiddle_words = 1, scale_words = 0;
 };
+template <> struct KinLine<Wide> : KinLine<double> {};
 // 16-byte words of a table in shared memory.
 template <typename T>
 constexpr int kin_words(int map, int n, bool unit) {
@@ -95,8 +106,11 @@ template <bool ODD, int S>
 __device__ __forceinline__ double2 kin_twiddle(double2 x, const double2* tw, int j) {
   return S > 0 ? cmul(x, cconj(tw[j])) : cmul(x, tw[j]);
 }
-__device__ __forceinline__ F2 kin_scale(float p) { return f2(p); }
-__device__ __forceinline__ double kin_scale(double p) { return p; }
+template <typename T, typename P>
+__device__ __forceinline__ auto kin_scale(P p) {
+  if constexpr (std::is_same_v<T, float>) return f2(p);
+  else return static_cast<double>(p);
+}
 
 // The lane(s) of a line: `ok` counts those that exist.
 __device__ __forceinline__ C2 kin_load(const float2* p, int ok, bool aligned) {
@@ -132,6 +146,13 @@ __device__ __forceinline__ float4 kin_pack(C2 v) {
   c2_split(v, a, b);
   return make_float4(a.x, a.y, b.x, b.y);
 }
+struct alignas(16) KinWideWord {
+  float2 v;
+};
+__device__ __forceinline__ double2 kin_unpack(const KinWideWord* w) { return make_double2(w->v.x, w->v.y); }
+__device__ __forceinline__ void kin_store(float2* p, double2 v, int ok, bool) {
+  if (ok) *p = make_float2(static_cast<float>(v.x), static_cast<float>(v.y));
+}
 __device__ __forceinline__ double2 kin_unpack(const double2* w) { return *w; }
 __device__ __forceinline__ double2 kin_pack(double2 v) { return v; }
 __device__ __forceinline__ void kin_store(double2* p, double2 v, int ok, bool) {
@@ -164,19 +185,29 @@ __device__ __forceinline__ C2 kin_apply(C2 x, const KinPostPair& w) {
 __device__ __forceinline__ KinPostF64 kin_post(const double2* t, long long, long long k, int ok, double oz) {
   return KinPostF64{ok ? t[k] : make_double2(0.0, 0.0), oz};
 }
+// entry k of a mixed form's factor table (g, its low part, the scale's two parts)
+__device__ __forceinline__ double2 kin_entry(const float2* t, long long n, long long k) {
+  const float2 g = t[k], l = t[n + k], s = t[2 * n + k];
+  const double sc = static_cast<double>(s.x) + s.y;
+  return make_double2(sc * (1.0 + (static_cast<double>(g.x) + l.x)), sc * (static_cast<double>(g.y) + l.y));
+}
+// the form's kin_post
+template <typename T, typename V, typename R>
+__device__ __forceinline__ auto kin_post_of(const V* t, long long n, long long k, int ok, R oz) {
+  if constexpr (std::is_same_v<T, Wide>) return KinPostF64{ok ? kin_entry(t, n, k) : make_double2(0.0, 0.0), oz};
+  else return kin_post(t, n, k, ok, oz);
+}
 __device__ __forceinline__ double2 kin_apply(double2 x, const KinPostF64& w) { return cscale(cmul(w.g, x), w.oz); }
 // x times entry k of a factor table in global memory (the momentum shift), the same for every lane
-__device__ __forceinline__ C2 kin_shift(C2 x, const float2* t, int n, int k) {
-  return fmul_parts(x, __ldg(t + k), __ldg(t + n + k), __ldg(t + 2 * n + k));
-}
 __device__ __forceinline__ double2 kin_shift(double2 x, const double2* t, int, int k) { return cmul(t[k], x); }
+__device__ __forceinline__ double2 kin_shift(double2 x, const float2* t, int n, int k) { return cmul(kin_entry(t, n, k), x); }
 
 // A thread's share of a tile.
 template <typename T>
 struct KinTile {
   using L = typename KinLine<T>::type;
-  using W = std::conditional_t<sizeof(T) == 4, float4, double2>;
-  Vec<T>* base;   // the line's first point
+  using W = std::conditional_t<std::is_same_v<T, float>, float4, std::conditional_t<std::is_same_v<T, Wide>, KinWideWord, double2>>;
+  KinVec<T>* base;   // the line's first point
   long long stride;
   int ok;         // existing lanes of the line
   bool aligned;
@@ -196,10 +227,17 @@ __device__ __forceinline__ int kin_point(int n1, int n2, int N1, int N2) {
 
 // The thread's points of a tile into its own words of `buffer` (asynchronous copies; the ragged edge by plain loads).
 template <typename T, int MAP>
-__device__ __forceinline__ void kin_request(const KinTile<T>& t, typename KinTile<T>::L* buffer, const Vec<T>* base, int ok, int N1, int N2) {
+__device__ __forceinline__ void kin_request(const KinTile<T>& t, typename KinTile<T>::L* buffer, const KinVec<T>* base, int ok, int N1, int N2) {
   for (int n2 = t.s; n2 < N2; n2 += t.nt) {
     auto* const to = reinterpret_cast<typename KinTile<T>::W*>(buffer) + ((n2 * N1) << t.log_lines) + t.b;
-    if (ok == KinLine<T>::lanes && t.aligned) {
+    if constexpr (std::is_same_v<T, Wide>) {
+      if (ok) {
+#pragma unroll 4
+        for (int n1 = 0; n1 < N1; ++n1) pot5::copy8(to + (n1 << t.log_lines), base + kin_point<MAP>(n1, n2, N1, N2) * t.stride);
+      } else {
+        for (int n1 = 0; n1 < N1; ++n1) to[n1 << t.log_lines].v = make_float2(0.0f, 0.0f);
+      }
+    } else if (ok == KinLine<T>::lanes && t.aligned) {
 #pragma unroll 4
       for (int n1 = 0; n1 < N1; ++n1) pot5::copy16(to + (n1 << t.log_lines), base + kin_point<MAP>(n1, n2, N1, N2) * t.stride);
     } else {
@@ -211,7 +249,7 @@ __device__ __forceinline__ void kin_request(const KinTile<T>& t, typename KinTil
 }
 // Level 1: DFT over n1 for the thread's n2.
 template <typename T, int MAP, int N1, bool ODD>
-__device__ __forceinline__ void kin_forward(const KinTile<T>& t, const KinArgs<T>& a, int N2, const typename KinLine<T>::type* tw) {
+__device__ __forceinline__ void kin_forward(const KinTile<T>& t, const KinArgs<typename KinStored<T>::type>& a, int N2, const typename KinLine<T>::type* tw) {
   using L = typename KinLine<T>::type;
 #pragma unroll 1
   for (int n2 = t.s; n2 < N2; n2 += t.nt) {
@@ -229,10 +267,10 @@ __device__ __forceinline__ void kin_forward(const KinTile<T>& t, const KinArgs<T
 }
 // Level 2: DFT over n2 for the thread's k1, the factor, and back.
 template <typename T, int MAP, int N2, bool ODD>
-__device__ __forceinline__ void kin_middle(const KinTile<T>& t, const KinArgs<T>& a, int N1, const typename KinLine<T>::type* f,
+__device__ __forceinline__ void kin_middle(const KinTile<T>& t, const KinArgs<typename KinStored<T>::type>& a, int N1, const typename KinLine<T>::type* f,
                                            const typename KinLine<T>::type* tw) {
   using L = typename KinLine<T>::type;
-  const auto p = kin_scale(a.scale);
+  const auto p = kin_scale<T>(a.scale);
   const bool unit = a.unit != 0;
   const L* const scale = f + (KinLine<T>::factor_words + (MAP == kTwiddle ? KinLine<T>::twiddle_words : 0)) * N1 * N2;
 #pragma unroll 1
@@ -250,7 +288,7 @@ __device__ __forceinline__ void kin_middle(const KinTile<T>& t, const KinArgs<T>
   }
 }
 template <typename T, int MAP, int N1, typename P>
-__device__ __forceinline__ void kin_back(const KinTile<T>& t, const KinArgs<T>& a, int N2, bool post, const P& w) {
+__device__ __forceinline__ void kin_back(const KinTile<T>& t, const KinArgs<typename KinStored<T>::type>& a, int N2, bool post, const P& w) {
   using L = typename KinLine<T>::type;
   if (t.ok == 0) return;
 #pragma unroll 1
@@ -296,7 +334,7 @@ constexpr int kin_min_blocks(int n) { return n > 16 ? 3 : n > 8 || n == 0 ? 2 : 
 
 template <typename T, int MAP, int N1C, int N2C>
 __global__ void __launch_bounds__(kin_max_threads(N1C > N2C ? N1C : N2C), kin_min_blocks(N1C > N2C ? N1C : N2C))
-    kin_kernel(const __grid_constant__ KinArgs<T> a) {
+    kin_kernel(const __grid_constant__ KinArgs<typename KinStored<T>::type> a) {
   using L = typename KinLine<T>::type;
   constexpr bool ANY = N1C == 0;
   const int N1 = ANY ? a.n1 : N1C, N2 = ANY ? a.n2 : N2C, N = N1 * N2;
@@ -318,7 +356,7 @@ __global__ void __launch_bounds__(kin_max_threads(N1C > N2C ? N1C : N2C), kin_mi
   t.aligned = a.aligned != 0;
   // twiddle products of lengths with an odd factor are nearly correctly rounded (cmul_comp)
   constexpr bool ODD = ANY || ((N1C * N2C) & (N1C * N2C - 1)) != 0;
-  auto locate = [&](unsigned tile, Vec<T>*& base, int& ok, unsigned& outer, long long& lane) {
+  auto locate = [&](unsigned tile, KinVec<T>*& base, int& ok, unsigned& outer, long long& lane) {
     const unsigned rest = tile / a.blocks_per_group, blk = tile - rest * a.blocks_per_group;
     outer = rest / a.groups;
     const unsigned grp = rest - outer * a.groups;
@@ -338,7 +376,7 @@ __global__ void __launch_bounds__(kin_max_threads(N1C > N2C ? N1C : N2C), kin_mi
   int side = 0;
   for (; tile < a.n_tiles; tile += gridDim.x, side ^= 1) {
     // the next tile's points, on their way during this one
-    Vec<T>* next_base = nullptr;
+    KinVec<T>* next_base = nullptr;
     int next_ok = 0;
     unsigned next_outer = 0;
     long long next_lane = 0;
@@ -358,10 +396,10 @@ __global__ void __launch_bounds__(kin_max_threads(N1C > N2C ? N1C : N2C), kin_mi
     __syncthreads();
     if constexpr (kin_is_xy(MAP)) {
       const long long izr = a.xy.izr_offset + outer;
-      const Vec<T>* const table = xy_post(a.xy, izr);
-      decltype(kin_post(table, 0ll, 0ll, 0, T(0))) w{};
+      const KinVec<T>* const table = xy_post(a.xy, izr);
+      decltype(kin_post_of<T>(table, 0ll, 0ll, 0, a.scale)) w{};
       if (table && t.ok)
-        w = kin_post(table, static_cast<long long>(a.xy.nr) * a.xy.n_rot, (izr % a.xy.nr) * a.xy.n_rot + lane, t.ok, a.xy.opt_z[izr / a.xy.nr]);
+        w = kin_post_of<T>(table, static_cast<long long>(a.xy.nr) * a.xy.n_rot, (izr % a.xy.nr) * a.xy.n_rot + lane, t.ok, a.xy.opt_z[izr / a.xy.nr]);
       if constexpr (ANY) kin_switch(N1, [&](auto n) { kin_back<T, MAP, SPO_CV(n)>(t, a, N2, table != nullptr, w); });
       else kin_back<T, MAP, N1C>(t, a, N2C, table != nullptr, w);
     } else {

@@ -15,6 +15,8 @@ template void launch_pot2<T>(int, const spo::Pot2Args<T>&, unsigned, std::size_t
 template void launch_pot3<T>(int, const spo::Pot2Args<T>&, dim3, unsigned, std::size_t, cudaStream_t);
 #elif SPO_LAUNCH_PART == 5
 template KinLaunch<T> kin_configure<T>(int, int, int, bool, int, long long);
+#elif SPO_LAUNCH_PART == 6
+template KinLaunch<float> kin_configure<spo::Wide>(int, int, int, bool, int, long long);
 #else
 template Pot4Kernel<T> pot4_kernel_for<T>(int, int);
 #endif

@@ -266,12 +266,14 @@ Pot4Kernel<T> pot4_kernel_for(int nphi, int nt) {  // the mixed form's; FP64 has
 }
 
 template <typename T>
-using KinKernel = void (*)(spo::KinArgs<T>);
+using KinKernel = void (*)(spo::KinArgs<typename spo::KinStored<T>::type>);
 template <typename T>
-KinKernel<T> kin_kernel_for(int map, int n1, int n2) {
-  // kin_preferred, kin_preferred_xy
-  if (map == spo::kTwiddle) {
-    if constexpr (sizeof(T) == 8)
+KinKernel<T> kin_kernel_for(int map, int n1, int n2) {  // kin_preferred, kin_preferred_xy, kin_wide_xy
+  constexpr bool mixed = std::is_same_v<T, float>, fp64 = std::is_same_v<T, double>, wide = std::is_same_v<T, spo::Wide>;
+  if constexpr (wide) {
+    if (map == spo::kXy && n1 == 6 && n2 == 6) return spo::kin_kernel<T, spo::kXy, 6, 6>;
+  } else if (map == spo::kTwiddle) {
+    if constexpr (fp64)
       if (n1 == 8 && n2 == 8) return spo::kin_kernel<T, spo::kTwiddle, 8, 8>;
     if (n1 == 8 && n2 == 16) return spo::kin_kernel<T, spo::kTwiddle, 8, 16>;
     if (n1 == 12 && n2 == 16) return spo::kin_kernel<T, spo::kTwiddle, 12, 16>;
@@ -279,7 +281,7 @@ KinKernel<T> kin_kernel_for(int map, int n1, int n2) {
   } else if (map == spo::kPrime) {
     if (n1 == 3 && n2 == 16) return spo::kin_kernel<T, spo::kPrime, 3, 16>;
     if (n1 == 11 && n2 == 16) return spo::kin_kernel<T, spo::kPrime, 11, 16>;
-    if constexpr (sizeof(T) == 4) {
+    if constexpr (mixed) {
       if (n1 == 3 && n2 == 32) return spo::kin_kernel<T, spo::kPrime, 3, 32>;
       if (n1 == 5 && n2 == 32) return spo::kin_kernel<T, spo::kPrime, 5, 32>;
     }
@@ -287,22 +289,26 @@ KinKernel<T> kin_kernel_for(int map, int n1, int n2) {
   } else if (map == spo::kXy && n1 == n2) {
     if (n1 == 2) return spo::kin_kernel<T, spo::kXy, 2, 2>;
     if (n1 == 4) return spo::kin_kernel<T, spo::kXy, 4, 4>;
-    if (n1 == 6) return spo::kin_kernel<T, spo::kXy, 6, 6>;
+    if constexpr (fp64)
+      if (n1 == 6) return spo::kin_kernel<T, spo::kXy, 6, 6>;
     if (n1 == 8) return spo::kin_kernel<T, spo::kXy, 8, 8>;
     if (n1 == 12) return spo::kin_kernel<T, spo::kXy, 12, 12>;
     if (n1 == 16) return spo::kin_kernel<T, spo::kXy, 16, 16>;
   }
-  return map == spo::kTwiddle ? spo::kin_kernel<T, spo::kTwiddle, 0, 0>
-         : map == spo::kPrime ? spo::kin_kernel<T, spo::kPrime, 0, 0>
-         : map == spo::kXy    ? spo::kin_kernel<T, spo::kXy, 0, 0>
-                              : spo::kin_kernel<T, spo::kXyShift, 0, 0>;
+  if constexpr (mixed) throw SpoError(SPO_ERR_STATE, "kin_kernel: no pair kernel of these sizes");
+  else
+    return map == spo::kTwiddle ? spo::kin_kernel<T, spo::kTwiddle, 0, 0>
+           : map == spo::kPrime ? spo::kin_kernel<T, spo::kPrime, 0, 0>
+           : map == spo::kXy    ? spo::kin_kernel<T, spo::kXy, 0, 0>
+                                : spo::kin_kernel<T, spo::kXyShift, 0, 0>;
 }
 
 // Threads per line: the number that wastes the fewest thread slots over the two levels (N2 lines of N1 points, then N1 of
 // N2) in whole warps, among those that keep about 14 warps per SM beside the tiles' shared memory.
 template <typename T>
-KinLaunch<T> kin_configure(int map, int n1, int n2, bool unit, int lanes_per_tile, long long window) {
-  KinLaunch<T> l;
+KinLaunch<typename spo::KinStored<T>::type> kin_configure(int map, int n1, int n2, bool unit, int lanes_per_tile, long long window) {
+  KinLaunch<typename spo::KinStored<T>::type> l;
+  l.lanes = spo::KinLine<T>::lanes;
   l.kernel = kin_kernel_for<T>(map, n1, n2);
   while ((spo::KinLine<T>::lanes << (l.log_lines + 1)) <= lanes_per_tile) ++l.log_lines;
   while (l.log_lines > 0 && (static_cast<long long>(spo::KinLine<T>::lanes) << (l.log_lines - 1)) >= window) --l.log_lines;
