@@ -53,13 +53,17 @@ def compare(case, precision, stages):
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 @pytest.mark.parametrize("nz,nr,nx,ny,j_max", [(90, 36, 10, 10, 2), (72, 45, 5, 9, 1), (110, 30, 9, 4, 2), (84, 44, 7, 7, 3),
                                                (60, 20, 16, 2, 1), (128, 48, 16, 16, 1), (176, 56, 4, 4, 2),
-                                               (96, 40, 12, 12, 1), (36, 22, 3, 11, 0), (28, 18, 1, 1, 2)])
-def test_kinetic_passes_of_any_lengths(nz, nr, nx, ny, j_max, precision):
+                                               (96, 40, 12, 12, 1), (36, 22, 3, 11, 0), (28, 18, 1, 1, 2),
+                                               (192, 64, 6, 6, 1), (256, 48, 8, 8, 0), (224, 160, 2, 2, 1),
+                                               (240, 14, 15, 14, 0)])
+@pytest.mark.parametrize("shifted", [True, False])
+def test_kinetic_passes_of_any_lengths(nz, nr, nx, ny, j_max, shifted, precision):
     from spo_b200 import capi, workload
     case = workload.config_case({"nz": nz, "nr": nr, "nx": nx, "ny": ny, "j_max": j_max, "mj_max": j_max,
                                  "nz_specular": 2 * nz, "nz_potential": nz // 3})
-    phase = np.exp(1j * np.random.default_rng(1).uniform(0, 6, nx * ny))
-    case.a["shift_forward"], case.a["shift_backward"] = phase, np.conj(phase)
+    if shifted:
+        phase = np.exp(1j * np.random.default_rng(1).uniform(0, 6, nx * ny))
+        case.a["shift_forward"], case.a["shift_backward"] = phase, np.conj(phase)
     compare(case, precision, (capi.STAGE_ZR, capi.STAGE_XY))
 
 
