@@ -271,6 +271,10 @@ __global__ void __launch_bounds__(pot5::threads_of(NPHI), 1) potential5_kernel(P
     }
   };
   // The columns, exp(i A) rows and corrections of an item into L2 (column c by one lane).
+  // The next item's data into L2. Not in the ring form, whose copies run 12 phi ahead by themselves: 888 teams have 29 MB of
+  // rows ahead besides those in use, and about as much as the table was read again from DRAM (1.49 times the algorithmic
+  // bytes; configuration 3: 4.12 ms with the rows and psi requested, 4.11 with the request after the phi phase, 3.90 with
+  // psi alone, 3.83 without).
   auto prefetch = [&](int item) {
     const int col = item * kCols + lane;
     if (h == 0 && lane < kCols && col < g.n_cols) {
@@ -287,7 +291,7 @@ __global__ void __launch_bounds__(pot5::threads_of(NPHI), 1) potential5_kernel(P
   uint32_t parity = 0;
   if (item < g.n_items) {
     issue(item);
-    prefetch(item);
+    if constexpr (!RING) prefetch(item);
   }
   for (; item < g.n_items; item += step) {
     const bool ok = !g.bulk || mbar_wait(bar, parity, g.poll_limit);
@@ -348,7 +352,7 @@ __global__ void __launch_bounds__(pot5::threads_of(NPHI), 1) potential5_kernel(P
     const int next = item + step;
     if (next < g.n_items) {
       if (H == 1 && g.bulk) issue(next);  // every lane of the team has read F
-      prefetch(next);
+      if constexpr (!RING) prefetch(next);
     }
 
     // ---- phi transform, exp(i A), inverse phi transform of the lane's two lines
