@@ -513,7 +513,6 @@ class Step final : public StepBase {
     if (side_) cudaStreamDestroy(side_);
     for (cudaEvent_t e : fork_)
       if (e) cudaEventDestroy(e);
-    if (host_flag_) cudaFreeHost(host_flag_);
   }
 
   void propagate_analysis_step() override {
@@ -522,8 +521,8 @@ class Step final : public StepBase {
       check_cuda(cudaGraphLaunch(graph_, stream_), "propagate_analysis_step launch");
     } else {
       enqueue_analysis_step();
-      read_device_error();
     }
+    read_device_error();
     check_cuda(cudaStreamSynchronize(stream_), "propagate_analysis_step");
     prof_.resolve();
     check_device_error();
@@ -538,23 +537,25 @@ class Step final : public StepBase {
     capture_graph();  // the graph holds the kernels' arguments
   }
 
-  // A kernel whose bounded wait gave up has set the device flag, which each step copies to host_flag_ at its end: report
-  // it (and clear it).
+  // A kernel whose bounded wait gave up has set the device flag, which is copied to host_flag_ behind each step: report it
+  // (and clear it). An ordinary int: the copy behind a graph of 40 short kernels costs 7 us, 1 us more than a copy into
+  // pinned memory (and 5 less than one after the wait for the step), but pinned memory costs 1 to 4 ms to get and 0.4 to 9
+  // ms to give back, for every handle.
   void read_device_error() {
     if (error_flag_)
-      check_cuda(cudaMemcpyAsync(host_flag_, error_flag_, sizeof(int), cudaMemcpyDeviceToHost, stream_), "error flag");
+      check_cuda(cudaMemcpyAsync(&host_flag_, error_flag_, sizeof(int), cudaMemcpyDeviceToHost, stream_), "error flag");
   }
   void check_device_error() {
-    if (!error_flag_ || *host_flag_ == 0) return;
-    *host_flag_ = 0;
+    if (!error_flag_ || host_flag_ == 0) return;
+    host_flag_ = 0;
     check_cuda(cudaMemset(error_flag_, 0, sizeof(int)), "error flag");
     throw SpoError(SPO_ERR_TIMEOUT, std::string(pot_kind_ == 6 ? "potential6" : "potential5") +
                                         ": a bounded wait for an asynchronous copy or tensor-core work gave up");
   }
 
   // One analysis step as a CUDA graph (about 8 (n + 1) small kernels: on the smallest grids the gaps between separate
-  // launches and the wait for the copy of the error flag cost as much as the kernels). Captured on a stream of its own
-  // when the handle is built, so it can be launched into any stream.
+  // launches cost as much as the kernels). Captured on a stream of its own when the handle is built, so it can be launched
+  // into any stream.
   void capture_graph() {
     if (graph_) {
       check_cuda(cudaStreamSynchronize(stream_), "graph");
@@ -573,7 +574,6 @@ class Step final : public StepBase {
       try {
         require(!was_on, "profiling");
         enqueue_analysis_step();
-        read_device_error();
       } catch (const std::exception& x) {
         failed = x.what();
       }
@@ -2097,8 +2097,6 @@ class Step final : public StepBase {
   void make_error_flag() {
     error_flag_ = dev<int>(1);
     check_cuda(cudaMemset(error_flag_, 0, sizeof(int)), "error flag");
-    check_cuda(cudaMallocHost(&host_flag_, sizeof(int)), "error flag");
-    *host_flag_ = 0;
   }
 
   // The phi maps as bytes, or null without symmetry.
@@ -2275,7 +2273,7 @@ class Step final : public StepBase {
   int graph_launches_ = 0;
   cudaStream_t side_ = nullptr;      // the specular grid's passes
   cudaEvent_t fork_[2] = {nullptr, nullptr};
-  int* host_flag_ = nullptr;         // pinned copy of the error flag
+  int host_flag_ = 0;                // copy of the error flag
   DeviceArena arena_;
   HostCopier<T> copier_;
   Profiler prof_;

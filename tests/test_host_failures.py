@@ -1,0 +1,65 @@
+"""The library's host code where calls of the CUDA runtime fail, and what it leaves behind (CPU only).
+
+tests/support/fake_cudart.cpp stands in for the runtime: device memory is host memory, kernels are not run, every object
+is counted, and a chosen call can be made to fail. Each check runs in a process of its own with that library preloaded.
+"""
+
+import os
+import subprocess
+import sys
+
+import pytest
+
+from conftest import ROOT
+
+PKG = os.path.join(ROOT, "cpp-spo-dvr_b200")
+PRELUDE = """
+import ctypes, os, sys
+import numpy as np
+sys.path.insert(0, %r)
+from spo_b200 import B200Backend, Ensemble, capi, workload
+from spo_b200.mlp import Mlp
+fake = ctypes.CDLL(None)
+fake.fake_launches.restype = ctypes.c_long
+KINDS = (b"malloc", b"host", b"stream", b"event", b"graph", b"exec")
+live = lambda: {k.decode(): fake.fake_live(k) for k in KINDS if fake.fake_live(k)}
+def status(call):
+    try:
+        call()
+        return capi.SPO_OK
+    except capi.B200Error as e:
+        return e.status
+def case(nz=24, nr=12, nx=4, ny=4, j=3, nzp=10, **kw):
+    return workload.config_case({"nz": nz, "nr": nr, "nx": nx, "ny": ny, "j_max": j, "mj_max": j, "nz_specular": 2 * nz,
+                                 "nz_potential": nzp, **kw})
+""" % PKG
+
+
+@pytest.fixture(scope="session")
+def run(tmp_path_factory):
+    """run(code): the code after PRELUDE, with the stand-in preloaded; fails with its output unless it ends well."""
+    lib = os.path.join(PKG, "lib", "libspo_b200.so")
+    if not os.path.exists(lib):
+        subprocess.run(["make", "-C", PKG, "-j4"], check=True, stdout=subprocess.DEVNULL)
+    fake = str(tmp_path_factory.mktemp("fake") / "libfake_cudart.so")
+    include = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", f"-I{include}", "-o", fake,
+                    os.path.join(ROOT, "tests", "support", "fake_cudart.cpp")], check=True)
+
+    def go(code, env=None):
+        r = subprocess.run([sys.executable, "-c", PRELUDE + code], env={**os.environ, "LD_PRELOAD": fake, **(env or {})},
+                           capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stdout + r.stderr
+
+    return go
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_a_handle_asks_for_no_pinned_memory(run, precision):
+    """Page-locked memory takes milliseconds to get and to give back; a handle that copies nothing large needs none."""
+    run(f"""
+with B200Backend(case(), precision="{precision}") as be:
+    be.propagate_analysis_step()
+    be.block_densities()
+assert fake.fake_calls(b"host") == 0
+""")
