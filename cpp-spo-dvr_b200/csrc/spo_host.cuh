@@ -135,6 +135,20 @@ class DeviceArena {
   unsigned long long bytes_ = 0;
 };
 
+// A stream and an event that go with their owner, also when its constructor throws.
+struct OwnedStream {
+  cudaStream_t s = nullptr;
+  ~OwnedStream() {
+    if (s) cudaStreamDestroy(s);
+  }
+};
+struct OwnedEvent {
+  cudaEvent_t e = nullptr;
+  ~OwnedEvent() {
+    if (e) cudaEventDestroy(e);
+  }
+};
+
 struct Sizes {
   int n_rot, nx, ny, nr, nz, nzp, nzs, nt, nphi, i0, ra, rb, spa, n_rep, n_ops, n_blocks, mj_max;
   double dt;
@@ -510,9 +524,6 @@ class Step final : public StepBase {
 
   ~Step() override {
     if (graph_) cudaGraphExecDestroy(graph_);
-    if (side_) cudaStreamDestroy(side_);
-    for (cudaEvent_t e : fork_)
-      if (e) cudaEventDestroy(e);
   }
 
   void propagate_analysis_step() override {
@@ -918,15 +929,15 @@ class Step final : public StepBase {
   // The specular grid's step needs nothing of the scattering wave's kinetic step, so its three short passes (20 to 50 us
   // each, a few blocks) run beside it on a second stream; profiling runs them one after another.
   void sub_step(bool half, bool kinetic_only) {
-    const bool fork = side_ && !prof_.on();
+    const bool fork = side_.s && !prof_.on();
     if (fork) {
       const cudaStream_t main = stream_;
-      check_cuda(cudaEventRecord(fork_[0], main), "cudaEventRecord");
-      check_cuda(cudaStreamWaitEvent(side_, fork_[0], 0), "cudaStreamWaitEvent");
-      stream_ = side_;
+      check_cuda(cudaEventRecord(fork_[0].e, main), "cudaEventRecord");
+      check_cuda(cudaStreamWaitEvent(side_.s, fork_[0].e, 0), "cudaStreamWaitEvent");
+      stream_ = side_.s;
       specular(half, kinetic_only);
       stream_ = main;
-      check_cuda(cudaEventRecord(fork_[1], side_), "cudaEventRecord");
+      check_cuda(cudaEventRecord(fork_[1].e, side_.s), "cudaEventRecord");
     } else {
       specular(half, kinetic_only);
     }
@@ -936,7 +947,7 @@ class Step final : public StepBase {
       kinetic_zr(half);
       kinetic_xy(half, !kinetic_only);  // the gas-phase potential step rides along
     }
-    if (fork) check_cuda(cudaStreamWaitEvent(stream_, fork_[1], 0), "cudaStreamWaitEvent");
+    if (fork) check_cuda(cudaStreamWaitEvent(stream_, fork_[1].e, 0), "cudaStreamWaitEvent");
     if (!kinetic_only) interaction();
   }
 
@@ -1199,18 +1210,16 @@ class Step final : public StepBase {
   // Mean device milliseconds of `launch` over `reps` launches on the handle's stream, after one warm-up.
   template <typename F>
   float time_launches(F&& launch, int reps) {
-    cudaEvent_t e0 = nullptr, e1 = nullptr;
-    check_cuda(cudaEventCreate(&e0), "cudaEventCreate");
-    check_cuda(cudaEventCreate(&e1), "cudaEventCreate");
+    OwnedEvent e0, e1;
+    check_cuda(cudaEventCreate(&e0.e), "cudaEventCreate");
+    check_cuda(cudaEventCreate(&e1.e), "cudaEventCreate");
     launch();
-    check_cuda(cudaEventRecord(e0, stream_), "cudaEventRecord");
+    check_cuda(cudaEventRecord(e0.e, stream_), "cudaEventRecord");
     for (int i = 0; i < reps; ++i) launch();
-    check_cuda(cudaEventRecord(e1, stream_), "cudaEventRecord");
-    check_cuda(cudaEventSynchronize(e1), "cudaEventSynchronize");
+    check_cuda(cudaEventRecord(e1.e, stream_), "cudaEventRecord");
+    check_cuda(cudaEventSynchronize(e1.e), "cudaEventSynchronize");
     float ms = 0.0f;
-    check_cuda(cudaEventElapsedTime(&ms, e0, e1), "cudaEventElapsedTime");
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
+    check_cuda(cudaEventElapsedTime(&ms, e0.e, e1.e), "cudaEventElapsedTime");
     check_cuda(cudaGetLastError(), "autotune launch");
     return ms / reps;
   }
@@ -1994,8 +2003,8 @@ class Step final : public StepBase {
     build_exp_table(d);
     check_cuda(cudaStreamSynchronize(stream_), "set-up");
     autotune();
-    check_cuda(cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking), "cudaStreamCreate");
-    for (cudaEvent_t& e : fork_) check_cuda(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
+    check_cuda(cudaStreamCreateWithFlags(&side_.s, cudaStreamNonBlocking), "cudaStreamCreate");
+    for (OwnedEvent& e : fork_) check_cuda(cudaEventCreateWithFlags(&e.e, cudaEventDisableTiming), "cudaEventCreate");
     capture_graph();
   }
 
@@ -2271,8 +2280,8 @@ class Step final : public StepBase {
   cudaStream_t own_stream_;
   cudaGraphExec_t graph_ = nullptr;  // one analysis step
   int graph_launches_ = 0;
-  cudaStream_t side_ = nullptr;      // the specular grid's passes
-  cudaEvent_t fork_[2] = {nullptr, nullptr};
+  OwnedStream side_;                 // the specular grid's passes
+  OwnedEvent fork_[2];
   int host_flag_ = 0;                // copy of the error flag
   DeviceArena arena_;
   HostCopier<T> copier_;

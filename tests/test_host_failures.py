@@ -63,3 +63,20 @@ with B200Backend(case(), precision="{precision}") as be:
     be.block_densities()
 assert fake.fake_calls(b"host") == 0
 """)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("kind", ["malloc", "stream", "event"])
+def test_a_handle_that_cannot_be_made_leaves_nothing_behind(run, kind, precision):
+    """Every call of a kind that making a handle needs, failing once: the status says so and nothing stays alive."""
+    run(f"""
+c = case()
+B200Backend(c, precision="{precision}").close()
+n = fake.fake_calls(b"{kind}")
+assert n > 0 and not live(), (n, live())
+for k in range(1, n + 1):
+    fake.fake_fail(b"{kind}", k)
+    st = status(lambda: B200Backend(c, precision="{precision}").close())
+    assert st == capi.SPO_ERR_OOM, (k, st)
+    assert not live(), (k, live())
+""")
