@@ -527,6 +527,7 @@ class Step final : public StepBase {
   }
 
   void propagate_analysis_step() override {
+    if (graph_stale_ && !prof_.on()) capture_graph();
     if (graph_ && !prof_.on()) {
       launches_ = graph_launches_;
       check_cuda(cudaGraphLaunch(graph_, stream_), "propagate_analysis_step launch");
@@ -545,7 +546,7 @@ class Step final : public StepBase {
     const int limit = poll_limit > 0 ? poll_limit : spo::pot5::kWaitLimit;
     pot5_args_.poll_limit = pot6_args_.poll_limit = limit;
     pot5_args_.extra_tx = pot6_args_.extra_tx = extra_bytes;
-    capture_graph();  // the graph holds the kernels' arguments
+    graph_stale_ = true;  // the graph holds the kernels' arguments
   }
 
   // A kernel whose bounded wait gave up has set the device flag, which is copied to host_flag_ behind each step: report it
@@ -568,36 +569,35 @@ class Step final : public StepBase {
   // launches cost as much as the kernels). Captured on a stream of its own when the handle is built, so it can be launched
   // into any stream.
   void capture_graph() {
+    graph_stale_ = false;
     if (graph_) {
       check_cuda(cudaStreamSynchronize(stream_), "graph");
       cudaGraphExecDestroy(graph_);
       graph_ = nullptr;
     }
     const cudaStream_t current = stream_;
-    cudaStream_t capture = nullptr;
-    check_cuda(cudaStreamCreateWithFlags(&capture, cudaStreamNonBlocking), "cudaStreamCreate");
+    OwnedStream capture;
+    check_cuda(cudaStreamCreateWithFlags(&capture.s, cudaStreamNonBlocking), "cudaStreamCreate");
     cudaGraph_t graph = nullptr;
-    cudaError_t e = cudaStreamBeginCapture(capture, cudaStreamCaptureModeThreadLocal);
+    graph_missing_.clear();
+    cudaError_t e = cudaStreamBeginCapture(capture.s, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-      stream_ = capture;
-      const bool was_on = prof_.on();
-      std::string failed;
+      stream_ = capture.s;
       try {
-        require(!was_on, "profiling");
         enqueue_analysis_step();
       } catch (const std::exception& x) {
-        failed = x.what();
+        graph_missing_ = x.what();
       }
       stream_ = current;
-      e = cudaStreamEndCapture(capture, &graph);
-      if (e == cudaSuccess && failed.empty()) e = cudaGraphInstantiate(&graph_, graph, 0);
+      e = cudaStreamEndCapture(capture.s, &graph);
+      if (e == cudaSuccess && graph_missing_.empty()) e = cudaGraphInstantiate(&graph_, graph, 0);
       if (graph) cudaGraphDestroy(graph);
       graph_launches_ = launches_;
     }
-    cudaStreamDestroy(capture);
     if (e != cudaSuccess) {  // the step then launches its kernels one by one
       (void)cudaGetLastError();
       graph_ = nullptr;
+      if (graph_missing_.empty()) graph_missing_ = cudaGetErrorString(e);
     }
   }
 
@@ -657,6 +657,7 @@ class Step final : public StepBase {
            (kin_r_.map >= 0 && axis2_supported(s_.nr) ? "r" : "") + (kin_xy_.map >= 0 && xy2 ? "xy" : "");
     out += std::string(" balanced=") + (balanced_ ? "1" : "0") + " persistent=" + (persist_z_ ? "z" : "") + (persist_r_ ? "r" : "") + (persist_xy_ ? "xy" : "") +
            " zr_window=" + std::to_string(zr_window_) + " rxy_planes=" + std::to_string(rxy_planes_) + " tiles=" + tiles_source_ + " potential_choice=" + pot_source_;
+    out += graph_ || graph_stale_ ? " graph=1" : " graph=0 (" + graph_missing_ + ")";
     return out;
   }
 
@@ -2279,6 +2280,8 @@ class Step final : public StepBase {
   cudaStream_t stream_;
   cudaStream_t own_stream_;
   cudaGraphExec_t graph_ = nullptr;  // one analysis step
+  bool graph_stale_ = false;         // to be captured again before the next step that is not profiled
+  std::string graph_missing_;        // why there is none
   int graph_launches_ = 0;
   OwnedStream side_;                 // the specular grid's passes
   OwnedEvent fork_[2];

@@ -118,6 +118,7 @@ def test_a_step_as_one_graph_is_bitwise_its_kernels_one_by_one(precision):
     out = []
     for mode in ("graph", "launches", "stream"):
         with make(case, None, precision) as be:
+            assert be.describe().endswith(" graph=1"), be.describe()
             be.read_wave_packet(psi, chi)
             if mode == "launches":
                 be.profile(True)

@@ -80,3 +80,29 @@ for k in range(1, n + 1):
     assert st == capi.SPO_ERR_OOM, (k, st)
     assert not live(), (k, live())
 """)
+
+
+def test_a_step_is_one_graph_and_says_so_when_it_is_not(run):
+    """describe() names the graph; new arguments of the kernels are captured again, also after a profiled stretch; a
+    capture that fails leaves launches one by one and its reason."""
+    run("""
+with B200Backend(case(), precision="mixed") as be:
+    assert be.describe().endswith(" graph=1"), be.describe()
+    n = fake.fake_launches(b"graph")
+    be.propagate_analysis_step()
+    assert fake.fake_launches(b"graph") == n + 1
+    be.profile(True)
+    be.test_wait_timeout(100, 16)
+    be.test_wait_timeout(0, 0)
+    be.propagate_analysis_step()
+    be.profile(False)
+    be.propagate_analysis_step()
+    assert fake.fake_launches(b"graph") == n + 2, be.describe()
+fake.fake_fail(b"capture", 1)
+with B200Backend(case(), precision="mixed") as be:
+    n, k = fake.fake_launches(b"graph"), fake.fake_launches(b"potential5")
+    assert " graph=0 (" in be.describe(), be.describe()
+    be.propagate_analysis_step()
+    assert fake.fake_launches(b"graph") == n and fake.fake_launches(b"potential5") > k
+assert not live()
+""")
