@@ -479,6 +479,10 @@ class StepBase {
   virtual void propagate_analysis_step() = 0;
   // Queues one analysis step on the current stream without synchronising (graph capture).
   virtual void enqueue_analysis_step() = 0;
+  // The device flag that a bounded wait of this handle's kernels sets when it gives up (null: none waits), and the report
+  // of one that was set: clears it and throws SPO_ERR_TIMEOUT.
+  virtual const int* device_flag() const = 0;
+  virtual void report_device_error() = 0;
   virtual std::string describe() const = 0;
   virtual void averages(const double* z, const double* zs, const double* r, double vol_scat, double vol_spec,
                         int iz_analysis, int surface_index, double* out) = 0;
@@ -558,9 +562,13 @@ class Step final : public StepBase {
       check_cuda(cudaMemcpyAsync(&host_flag_, error_flag_, sizeof(int), cudaMemcpyDeviceToHost, stream_), "error flag");
   }
   void check_device_error() {
-    if (!error_flag_ || host_flag_ == 0) return;
+    if (error_flag_ && host_flag_ != 0) report_device_error();
+  }
+  const int* device_flag() const override { return error_flag_; }
+  void report_device_error() override {
     host_flag_ = 0;
-    check_cuda(cudaMemset(error_flag_, 0, sizeof(int)), "error flag");
+    check_cuda(cudaMemsetAsync(error_flag_, 0, sizeof(int), stream_), "error flag");
+    check_cuda(cudaStreamSynchronize(stream_), "error flag");
     throw SpoError(SPO_ERR_TIMEOUT, std::string(pot_kind_ == 6 ? "potential6" : "potential5") +
                                         ": a bounded wait for an asynchronous copy or tensor-core work gave up");
   }
@@ -828,8 +836,10 @@ class Step final : public StepBase {
       default: require(false, "unknown stage");
     }
     check_cuda(cudaGetLastError(), "apply_stage launch");
+    read_device_error();
     check_cuda(cudaStreamSynchronize(stream_), "apply_stage");
     prof_.resolve();
+    check_device_error();
   }
 
   void analysis_setup(const spo_analysis_desc& d) override {

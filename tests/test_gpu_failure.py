@@ -52,3 +52,52 @@ def test_unmatched_bytes_must_be_a_multiple_of_16():
         with pytest.raises(capi.B200Error) as err:
             be.test_wait_timeout(100, 8)
         assert err.value.status == capi.SPO_ERR_INVALID
+
+
+@pytest.mark.parametrize("failing", [(0,), (1,), (0, 2)])
+def test_an_ensemble_reports_a_wait_that_gave_up_and_its_members_recover(failing):
+    """The graph holds the arguments its members had when it was made."""
+    from spo_b200 import Ensemble, capi, workload
+    case = workload.config_case({"nz": 24, "nr": 16, "nx": 4, "ny": 4, "j_max": 7, "mj_max": 7,
+                                 "nz_specular": 64, "nz_potential": 14})
+    rng = np.random.default_rng(5)
+    psi0 = rng.standard_normal(case.psi_shape) + 1j * rng.standard_normal(case.psi_shape)
+    chi0 = rng.standard_normal(case.chi_shape) + 1j * rng.standard_normal(case.chi_shape)
+    members = [make(case, None, p) for p in ("mixed", "mixed", "mixed", "fp64")]
+    try:
+        members[0].read_wave_packet(psi0, chi0)
+        members[0].propagate_analysis_step()
+        expected = members[0].wave_packet_on_host()
+        for k in failing:
+            members[k].test_wait_timeout(1 << 16, 16)
+        with Ensemble(members) as ensemble:
+            for _ in range(2):  # the flags are cleared by the report, and set again by the next step
+                with pytest.raises(capi.B200Error) as err:
+                    ensemble.propagate_analysis_step()
+                assert err.value.status == capi.SPO_ERR_TIMEOUT and f"member {failing[0]}:" in str(err.value), str(err.value)
+        for k in failing:
+            members[k].test_wait_timeout(0, 0)
+        with Ensemble(members) as ensemble:
+            for m in members:
+                m.read_wave_packet(psi0, chi0)
+            ensemble.propagate_analysis_step()
+            for m in members[:3]:
+                psi, chi = m.wave_packet_on_host()
+                assert np.array_equal(psi, expected[0]) and np.array_equal(chi, expected[1])
+    finally:
+        for m in members:
+            m.close()
+
+
+def test_a_single_operator_reports_a_wait_that_gave_up():
+    from spo_b200 import capi, workload
+    case = workload.config_case({"nz": 24, "nr": 16, "nx": 4, "ny": 4, "j_max": 7, "mj_max": 7,
+                                 "nz_specular": 64, "nz_potential": 14})
+    with make(case, None, "mixed") as be:
+        be.test_wait_timeout(1 << 16, 16)
+        with pytest.raises(capi.B200Error) as err:
+            be.apply_stage(capi.STAGE_POTENTIAL)
+        assert err.value.status == capi.SPO_ERR_TIMEOUT
+        be.test_wait_timeout(0, 0)
+        be.apply_stage(capi.STAGE_POTENTIAL)
+        be.propagate_analysis_step()

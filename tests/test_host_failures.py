@@ -106,3 +106,16 @@ with B200Backend(case(), precision="mixed") as be:
     assert fake.fake_launches(b"graph") == n and fake.fake_launches(b"potential5") > k
 assert not live()
 """)
+
+
+def test_a_wait_that_gave_up_is_reported_by_every_call_that_runs_the_kernels(run):
+    run("""
+with B200Backend(case(), precision="mixed") as a, B200Backend(case(), precision="mixed") as b:
+    fake.fake_raise(b"potential5", 1)
+    assert status(lambda: a.apply_stage(capi.STAGE_POTENTIAL)) == capi.SPO_ERR_TIMEOUT
+    with Ensemble([a, b]) as both:  # the stand-in runs a graph's kernels when it is captured
+        fake.fake_raise(b"", 0)
+        assert status(both.propagate_analysis_step) == capi.SPO_ERR_TIMEOUT
+    assert status(a.propagate_analysis_step) == status(b.propagate_analysis_step) == capi.SPO_OK
+assert not live(), live()
+""")
