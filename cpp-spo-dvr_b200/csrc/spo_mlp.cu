@@ -735,6 +735,7 @@ struct spo_mlp {
   DevBuf<float> px, py, pbias;
   DevBuf<bf16> packed;
   int sms = 0;
+  bool predict_ready = false;  // all of these are there
   spo_host::RawCopier copier;
 
   ~spo_mlp() {
@@ -749,30 +750,32 @@ struct spo_mlp {
 
   void ensure_capacity(long long rows) {
     if (rows <= cap) return;
-    cap = ((rows + 127) / 128) * 128;
-    x16.alloc(cap * in_pad);
-    x16t.alloc(cap * in_pad);
+    cap = 0;  // until the last allocation has succeeded: a call after one that failed starts over
+    const long long grown = ((rows + 127) / 128) * 128;
+    x16.alloc(grown * in_pad);
+    x16t.alloc(grown * in_pad);
     z.clear();
     act.clear();
     act_t.clear();
     for (int l = 0; l < depth; ++l) {
       z.push_back(std::make_unique<DevBuf<float>>());
-      z.back()->alloc(cap * width);
+      z.back()->alloc(grown * width);
       for (auto* v : {&act, &act_t}) {
         v->push_back(std::make_unique<DevBuf<bf16>>());
-        v->back()->alloc(cap * width);
+        v->back()->alloc(grown * width);
       }
     }
-    yb.alloc(cap);
-    d.alloc(cap);
-    db.alloc(cap / 64 * width);
-    dwo.alloc(cap / 64 * width);
-    dbo.alloc(cap / 64);
-    g16.alloc(cap * width);
-    dz16.alloc(cap * width);
-    dzt.alloc(cap * width);
-    loss_parts.alloc(cap / 64);
+    yb.alloc(grown);
+    d.alloc(grown);
+    db.alloc(grown / 64 * width);
+    dwo.alloc(grown / 64 * width);
+    dbo.alloc(grown / 64);
+    g16.alloc(grown * width);
+    dz16.alloc(grown * width);
+    dzt.alloc(grown * width);
+    loss_parts.alloc(grown / 64);
     if (!loss.p) loss.alloc(1);
+    cap = grown;
   }
 
   void refresh_bf16() {
@@ -1040,7 +1043,7 @@ int spo_mlp_predict(spo_mlp* m, const float* x, long long n, float* y) {
     const long long most = std::min(n, spo_mlp::kPredictRows);
     if (m->px.n < static_cast<std::size_t>(most * m->n_in)) m->px.alloc(static_cast<std::size_t>(most * m->n_in));
     if (m->py.n < static_cast<std::size_t>(most)) m->py.alloc(static_cast<std::size_t>(most));
-    if (!m->packed.p) {
+    if (!m->predict_ready) {
       std::size_t total = 0;
       for (const auto& l : m->layers) total += static_cast<std::size_t>(l->in) * l->out;
       m->packed.alloc(total);
@@ -1048,6 +1051,7 @@ int spo_mlp_predict(spo_mlp* m, const float* x, long long n, float* y) {
       ck(cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, m->device), "SM count");
       ck(cudaFuncSetAttribute(mlp_predict_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               static_cast<int>(predict_smem(256))), "predict smem");
+      m->predict_ready = true;
     }
     std::size_t off = 0;
     for (int l = 0; l < m->depth; ++l) {

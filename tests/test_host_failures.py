@@ -119,3 +119,31 @@ with B200Backend(case(), precision="mixed") as a, B200Backend(case(), precision=
     assert status(a.propagate_analysis_step) == status(b.propagate_analysis_step) == capi.SPO_OK
 assert not live(), live()
 """)
+
+
+@pytest.mark.parametrize("call", ["train", "gradients", "predict"])
+def test_a_network_works_on_after_a_call_that_ran_out_of_memory(run, call):
+    """Every allocation of a call's work space failing once: the status says so, and a smaller call then makes all of its
+    own, as it does on a network that never failed (no buffer is taken for one that was not made)."""
+    run(f"""
+rng = np.random.default_rng(1)
+x, y = rng.uniform(-1, 1, (1024, 12)).astype(np.float32), np.zeros(1024, np.float32)
+calls = dict(train=lambda net, n: net.train(x[:n], y[:n], epochs=1, batch=n),
+             gradients=lambda net, n: net.gradients(x[:n], y[:n]), predict=lambda net, n: net.predict(x[:n]))
+go = calls["{call}"]
+with Mlp(12, 128, 3) as net:
+    go(net, 128)
+    want = live()
+with Mlp(12, 128, 3) as net:
+    n = fake.fake_calls(b"malloc")
+    go(net, 1024)
+    n = fake.fake_calls(b"malloc") - n
+assert n > 1 and not live()
+for k in range(1, n + 1):
+    with Mlp(12, 128, 3) as net:
+        fake.fake_fail(b"malloc", k)
+        assert status(lambda: go(net, 1024)) == capi.SPO_ERR_OOM, k
+        go(net, 128)
+        assert live() == want, (k, live(), want)
+    assert not live(), k
+""")
