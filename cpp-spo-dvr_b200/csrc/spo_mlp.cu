@@ -714,11 +714,14 @@ struct spo_mlp {
   DevBuf<double> loss_parts, loss;                         // per 64 rows; per step of an epoch
   DevBuf<bf16> g16, dz16, dzt;
   long long step = 0;
-  // prediction: features and outputs of a chunk of points (grown to the largest call's, at most kPredictRows points),
-  // packed weights and the biases of all layers
-  static constexpr long long kPredictRows = 1 << 20;
-  // and the points of a training set, kept for the next call up to kKeepBytes
+  // Device memory for a call's points, kept for the next call: at most this much for a training set (which is given back
+  // above it) and as much for the predictions' points, which go in chunks that fit: 2^20 points of up to 15 features, 258048
+  // of 64. (Chunks of 2^20 whatever the features kept 268 MB.)
   static constexpr std::size_t kKeepBytes = 64ull << 20;
+  long long predict_rows() const {
+    const long long fit = static_cast<long long>(kKeepBytes / (sizeof(float) * (n_in + 1))) / kBM * kBM;
+    return std::min(fit, 1ll << 20);
+  }
   DevBuf<float> tx, ty;
   DevBuf<long long> tperm;
   void training_set(long long n, bool order) {
@@ -726,6 +729,10 @@ struct spo_mlp {
     if (ty.n < static_cast<std::size_t>(n)) ty.alloc(static_cast<std::size_t>(n));
     if (order && tperm.n < static_cast<std::size_t>(n)) tperm.alloc(static_cast<std::size_t>(n));
   }
+  struct TrainingSetKeeper {  // at the end of a call, also of one that failed
+    spo_mlp* m;
+    ~TrainingSetKeeper() { m->release_training_set(); }
+  };
   void release_training_set() {
     if (sizeof(float) * (tx.n + ty.n) + sizeof(long long) * tperm.n <= kKeepBytes) return;
     tx.free();
@@ -1040,7 +1047,7 @@ int spo_mlp_set_parameters(spo_mlp* m, const float* in) {
 int spo_mlp_predict(spo_mlp* m, const float* x, long long n, float* y) {
   return guarded_mlp(m, [&] {
     need(x && y && n > 0, "spo_mlp_predict: bad arguments");
-    const long long most = std::min(n, spo_mlp::kPredictRows);
+    const long long most = std::min(n, m->predict_rows());
     if (m->px.n < static_cast<std::size_t>(most * m->n_in)) m->px.alloc(static_cast<std::size_t>(most * m->n_in));
     if (m->py.n < static_cast<std::size_t>(most)) m->py.alloc(static_cast<std::size_t>(most));
     if (!m->predict_ready) {
@@ -1115,6 +1122,7 @@ int spo_mlp_train(spo_mlp* m, const float* x, const float* y, long long n, int e
     need(x && y && n >= batch && epochs > 0 && batch >= 128 && batch % 128 == 0 && batch <= 65536 && lr > 0.0f,
          "spo_mlp_train: bad arguments");
     m->ensure_capacity(batch);
+    const spo_mlp::TrainingSetKeeper keeper{m};
     m->training_set(n, true);
     ck(cudaMemcpyAsync(m->tx.p, x, sizeof(float) * n * m->n_in, cudaMemcpyHostToDevice, m->stream), "upload");
     ck(cudaMemcpyAsync(m->ty.p, y, sizeof(float) * n, cudaMemcpyHostToDevice, m->stream), "upload");
@@ -1147,7 +1155,6 @@ int spo_mlp_train(spo_mlp* m, const float* x, const float* y, long long n, int e
     }
     ck(cudaStreamSynchronize(m->stream), "train");
     m->check_flag();
-    m->release_training_set();
     if (last_epoch_loss) *last_epoch_loss = epoch_loss;
   });
 }

@@ -2,6 +2,7 @@
 // without a GPU: device memory is host memory, copies are memcpy, kernels are not run (their launches are counted). It
 // keeps count of what is alive and can let a call fail, which no real device does on request.
 //   fake_live(kind), fake_calls(kind) ... objects of a kind that are alive, calls that made one so far
+//   fake_bytes(kind) .................... bytes of those alive
 //   fake_fail(kind, n) .................. the n-th call from now (1: the next) that makes one fails, once
 //   fake_launches(part) ................. launches so far of kernels whose (mangled) name contains `part`
 //   fake_raise(part, value) ............. kernels whose name contains `part` store `value` at their second argument, an int*
@@ -12,13 +13,12 @@
 #include <cstring>
 #include <map>
 #include <mutex>
-#include <set>
 #include <string>
 #include <vector>
 
 namespace {
 struct Kind {
-  std::set<void*> live;
+  std::map<void*, std::size_t> live;
   int calls = 0, fail_in = 0;
 };
 std::recursive_mutex mutex;
@@ -43,7 +43,7 @@ cudaError_t make(const char* kind, std::size_t bytes, void** out) {
   ++k.calls;
   if (k.fail_in > 0 && --k.fail_in == 0) return cudaErrorMemoryAllocation;
   *out = std::calloc(1, bytes < 16 ? 16 : bytes);
-  k.live.insert(*out);
+  k.live[*out] = bytes;
   return cudaSuccess;
 }
 cudaError_t drop(const char* kind, void* p) {
@@ -65,6 +65,11 @@ cudaError_t make_handle(const char* kind, H* out) {
 extern "C" {
 
 int fake_live(const char* kind) { return static_cast<int>(kinds()[kind].live.size()); }
+long long fake_bytes(const char* kind) {
+  long long n = 0;
+  for (const auto& l : kinds()[kind].live) n += static_cast<long long>(l.second);
+  return n;
+}
 int fake_calls(const char* kind) { return kinds()[kind].calls; }
 void fake_fail(const char* kind, int n) { kinds()[kind].fail_in = n; }
 long fake_launches(const char* part) {

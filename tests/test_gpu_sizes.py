@@ -154,7 +154,7 @@ def test_large_packets_cross_to_the_device_and_back_unchanged(precision):
 
 
 @pytest.mark.parametrize("n,n_in,width,depth", [(1, 1, 64, 1), (127, 12, 128, 2), (128, 64, 256, 4), (129, 7, 64, 8),
-                                                (40001, 12, 256, 3), (200000, 12, 128, 4)])
+                                                (40001, 12, 256, 3), (200000, 12, 128, 4), (300001, 64, 64, 1)])
 def test_predictions_of_ragged_numbers_of_points(n, n_in, width, depth):
     """Against the numpy oracle, to 1e-2 of the output scale (BF16 activations, as test_gpu_mlp.py)."""
     import mlp_oracle

@@ -21,6 +21,7 @@ from spo_b200 import B200Backend, Ensemble, capi, workload
 from spo_b200.mlp import Mlp
 fake = ctypes.CDLL(None)
 fake.fake_launches.restype = ctypes.c_long
+fake.fake_bytes.restype = ctypes.c_longlong
 KINDS = (b"malloc", b"host", b"stream", b"event", b"graph", b"exec")
 live = lambda: {k.decode(): fake.fake_live(k) for k in KINDS if fake.fake_live(k)}
 def status(call):
@@ -146,4 +147,27 @@ for k in range(1, n + 1):
         go(net, 128)
         assert live() == want, (k, live(), want)
     assert not live(), k
+""")
+
+
+def test_what_a_network_keeps_for_the_next_call_is_bounded(run):
+    """64 MiB for the points of predictions and 64 MiB for a training set, also after a call that failed."""
+    run("""
+n = 300001
+x, y = np.ones((n, 64), np.float32), np.zeros(n, np.float32)
+with Mlp(64, 64, 1) as net:
+    net.predict(x[:128])
+    before = fake.fake_bytes(b"malloc")
+    k = fake.fake_launches(b"mlp_predict_kernel")
+    net.predict(x)
+    assert fake.fake_launches(b"mlp_predict_kernel") - k == 2
+    assert 0 < fake.fake_bytes(b"malloc") - before <= 64 << 20, fake.fake_bytes(b"malloc") - before
+with Mlp(64, 64, 1) as net:
+    net.train(x[:128], y[:128], epochs=1, batch=128)
+    before = fake.fake_bytes(b"malloc")
+    net.train(x, y, epochs=1, batch=128)
+    assert fake.fake_bytes(b"malloc") - before <= 64 << 20
+    fake.fake_fail(b"malloc", 3)  # the third buffer of the training set
+    assert status(lambda: net.train(x, y, epochs=1, batch=128)) == capi.SPO_ERR_OOM
+    assert fake.fake_bytes(b"malloc") - before <= 64 << 20
 """)
