@@ -66,9 +66,9 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 constexpr int kWaitLimit = 1 << 22;
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int limit = kWaitLimit) {
   const uint32_t addr = smem_addr(bar);
-  for (int i = 0; i < kWaitLimit; ++i) {
+  for (int i = 0; i < limit; ++i) {
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -156,6 +156,7 @@ struct GemmArgs {
   bf16* out16t;  // kEpiBiasSilu: the activation transposed (column c at c * ldt), or null
   long long ldt;
   int* error_flag;
+  int poll_limit;  // polls before a wait gives up; those of a block that leaves take kWaitLimit
 };
 
 constexpr int kBM = 128, kBK = 64, kBN = 64;
@@ -244,7 +245,7 @@ __global__ void __launch_bounds__(128) gemm_tn_kernel(GemmArgs g) {
       // the other stage's previous chunk (kc - 1) must be multiplied before it is overwritten
       bool ok = true;
       if (kc > kc_first) {
-        ok = tc::mbar_wait(bar + (st ^ 1), parity >> (st ^ 1) & 1u);
+        ok = tc::mbar_wait(bar + (st ^ 1), parity >> (st ^ 1) & 1u, g.poll_limit);
         if (ok) {
           parity ^= 1u << (st ^ 1);
           pending &= ~(1u << (st ^ 1));
@@ -263,7 +264,7 @@ __global__ void __launch_bounds__(128) gemm_tn_kernel(GemmArgs g) {
   // completed, so the accumulator is final (the second-to-last commit needs no wait of its own).
   if (!failed && kc_last > kc_first) {
     const int last = (kc_last - kc_first - 1) & 1;
-    const bool ok = tc::mbar_wait(bar + last, parity >> last & 1u);
+    const bool ok = tc::mbar_wait(bar + last, parity >> last & 1u, g.poll_limit);
     if (ok) pending = 0;  // the last commit arrives after every earlier MMA of the issuing thread
     failed = __syncthreads_or(!ok) != 0;
   }
@@ -339,6 +340,7 @@ struct PredictArgs {
   const float* bo;
   float* y;
   int* error_flag;
+  int poll_limit;
 };
 constexpr int kPredictSlots = 3, kPredictChunk = 32;
 constexpr std::size_t predict_smem(int width) {
@@ -378,7 +380,7 @@ __global__ void __launch_bounds__(128) mlp_predict_kernel(PredictArgs g) {
     while (requested < chunks && requested < used + kPredictSlots) {
       const int slot = static_cast<int>(requested % kPredictSlots);
       if (requested >= kPredictSlots &&
-          !tc::mbar_wait(empty + slot, static_cast<uint32_t>(requested / kPredictSlots - 1) & 1u))
+          !tc::mbar_wait(empty + slot, static_cast<uint32_t>(requested / kPredictSlots - 1) & 1u, g.poll_limit))
         return false;
       tc::mbar_arrive_tx(full + slot, chunk_bytes);
       tc::bulk_copy(W + slot * chunk_bytes, reinterpret_cast<const unsigned char*>(g.weights) + (requested % per_tile) * chunk_bytes,
@@ -411,7 +413,7 @@ __global__ void __launch_bounds__(128) mlp_predict_kernel(PredictArgs g) {
         bool ok = true;
         for (int c = 0; c < nc && ok; ++c) {
           const int slot = static_cast<int>(used % kPredictSlots);
-          ok = tc::mbar_wait(full + slot, static_cast<uint32_t>(used / kPredictSlots) & 1u);
+          ok = tc::mbar_wait(full + slot, static_cast<uint32_t>(used / kPredictSlots) & 1u, g.poll_limit);
           if (!ok) break;
           const uint32_t b0 = tc::smem_addr(W + slot * chunk_bytes);
 #pragma unroll
@@ -433,7 +435,7 @@ __global__ void __launch_bounds__(128) mlp_predict_kernel(PredictArgs g) {
         }
         if (!ok) atomicExch(g.error_flag, 1);
       }
-      const bool ok = tc::mbar_wait(done, done_parity);
+      const bool ok = tc::mbar_wait(done, done_parity, g.poll_limit);
       if (__syncthreads_or(!ok)) {
         failed = true;
         break;
@@ -630,7 +632,11 @@ constexpr int kAdamTensors = 18;  // 8 layers of W and b, the output layer's
 struct AdamArgs {
   AdamTensor t[kAdamTensors];
 };
-__global__ void adam_kernel(const __grid_constant__ AdamArgs args, float lr, float b1, float b2, float c1, float c2, float eps) {
+// A step whose gradients are not complete (a bounded wait gave up) changes nothing, nor do the steps queued behind it.
+__global__ void adam_kernel(const __grid_constant__ AdamArgs args, float lr, float b1, float b2, float c1, float c2, float eps,
+                            const int* __restrict__ error_flag, long long* __restrict__ steps_done) {
+  if (*error_flag != 0) return;
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) ++*steps_done;
   const AdamTensor& a = args.t[blockIdx.y];
   for (long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; t < a.n;
        t += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -713,7 +719,9 @@ struct spo_mlp {
   DevBuf<float> yb, d, db, dwo, dbo, partials;             // db, dwo, dbo: column sums per 64 rows
   DevBuf<double> loss_parts, loss;                         // per 64 rows; per step of an epoch
   DevBuf<bf16> g16, dz16, dzt;
-  long long step = 0;
+  long long step = 0;             // of Adam; on the device those that were applied
+  DevBuf<long long> steps_done;
+  int poll_limit = tc::kWaitLimit;
   // Device memory for a call's points, kept for the next call: at most this much for a training set (which is given back
   // above it) and as much for the predictions' points, which go in chunks that fit: 2^20 points of up to 15 features, 258048
   // of 64. (Chunks of 2^20 whatever the features kept 268 MB.)
@@ -796,7 +804,7 @@ struct spo_mlp {
             long long ldc, const float* bias, bf16* out16, long long ld16, int splits = 1, long long split_stride = 0,
             bf16* out16t = nullptr, long long ldt = 0) {
     need(k % kBK == 0 && n % kBN == 0 && n > 0 && lda % 8 == 0 && ldb % 8 == 0, "gemm shape");
-    GemmArgs g{a, lda, b, ldb, m, n, k, epi, c, ldc, split_stride, bias, out16, ld16, out16t, ldt, error_flag.p};
+    GemmArgs g{a, lda, b, ldb, m, n, k, epi, c, ldc, split_stride, bias, out16, ld16, out16t, ldt, error_flag.p, poll_limit};
     const dim3 grid(static_cast<unsigned>((m + kBM - 1) / kBM), static_cast<unsigned>(splits), static_cast<unsigned>(n / kBN));
     gemm_tn_kernel<<<grid, 128, kGemmLaunchSmem, stream>>>(g);
     ck(cudaGetLastError(), "gemm launch");
@@ -846,6 +854,7 @@ struct spo_mlp {
     int f = 0;
     ck(cudaMemcpy(&f, error_flag.p, sizeof(int), cudaMemcpyDeviceToHost), "error flag");
     if (f) {
+      ck(cudaMemcpy(&step, steps_done.p, sizeof step, cudaMemcpyDeviceToHost), "steps done");
       ck(cudaMemset(error_flag.p, 0, sizeof(int)), "error flag");
       throw MlpError(SPO_ERR_TIMEOUT, "mlp: a bounded wait for the tensor cores gave up");
     }
@@ -868,7 +877,7 @@ struct spo_mlp {
     }
     args.t[n++] = {wo.p, mwo.p, vwo.p, gwo.p, width, 0, nullptr, nullptr};
     args.t[n++] = {bo.p, mbo.p, vbo.p, gbo.p, 1, 0, nullptr, nullptr};
-    adam_kernel<<<dim3(64, static_cast<unsigned>(n)), 256, 0, stream>>>(args, lr, b1, b2, c1, c2, eps);
+    adam_kernel<<<dim3(64, static_cast<unsigned>(n)), 256, 0, stream>>>(args, lr, b1, b2, c1, c2, eps, error_flag.p, steps_done.p);
     ck(cudaGetLastError(), "adam");
   }
 
@@ -987,6 +996,8 @@ int spo_mlp_create(int n_in, int width, int depth, unsigned long long seed, int 
     zeros(m->vbo, 1);
     m->error_flag.alloc(1);
     ck(cudaMemset(m->error_flag.p, 0, sizeof(int)), "error flag");
+    m->steps_done.alloc(1);
+    ck(cudaMemset(m->steps_done.p, 0, sizeof(long long)), "steps done");
     m->partials.alloc(static_cast<std::size_t>(kSplits) * width * std::max(width, m->in_pad));
     m->refresh_bf16();
     ck(cudaStreamSynchronize(m->stream), "create");
@@ -1076,7 +1087,7 @@ int spo_mlp_predict(spo_mlp* m, const float* x, long long n, float* y) {
         ck(m->copier.to_device(x + i0 * m->n_in, m->px.p, in_bytes, m->device), "upload");
       else
         ck(cudaMemcpyAsync(m->px.p, x + i0 * m->n_in, in_bytes, cudaMemcpyHostToDevice, m->stream), "upload");
-      PredictArgs g{m->px.p, rows, m->n_in, m->width, m->depth, m->packed.p, m->pbias.p, m->wo.p, m->bo.p, m->py.p, m->error_flag.p};
+      PredictArgs g{m->px.p, rows, m->n_in, m->width, m->depth, m->packed.p, m->pbias.p, m->wo.p, m->bo.p, m->py.p, m->error_flag.p, m->poll_limit};
       const long long tiles = (rows + kBM - 1) / kBM;
       mlp_predict_kernel<<<static_cast<unsigned>(std::min<long long>(tiles, 2ll * m->sms)), 128, predict_smem(m->width), m->stream>>>(g);
       ck(cudaGetLastError(), "predict launch");
@@ -1090,6 +1101,12 @@ int spo_mlp_predict(spo_mlp* m, const float* x, long long n, float* y) {
     }
     m->check_flag();
   });
+}
+
+int spo_mlp_test_wait_timeout(spo_mlp* m, int poll_limit) {
+  if (!m) return SPO_ERR_INVALID;
+  m->poll_limit = poll_limit < 0 ? tc::kWaitLimit : poll_limit;
+  return SPO_OK;
 }
 
 int spo_mlp_gradients(spo_mlp* m, const float* x, const float* y, long long n, double* loss, float* grad) {

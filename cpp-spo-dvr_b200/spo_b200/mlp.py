@@ -16,7 +16,7 @@ from . import capi
 
 _EXPORTS = ["spo_mlp_create", "spo_mlp_destroy", "spo_mlp_last_error", "spo_mlp_parameter_count",
             "spo_mlp_get_parameters", "spo_mlp_set_parameters", "spo_mlp_input_width", "spo_mlp_predict",
-            "spo_mlp_gradients", "spo_mlp_train"]
+            "spo_mlp_gradients", "spo_mlp_train", "spo_mlp_test_wait_timeout"]
 
 
 def _bind(lib):
@@ -38,6 +38,7 @@ def _bind(lib):
     lib.spo_mlp_gradients.argtypes = [h, fp, fp, ctypes.c_longlong, dp, fp]
     lib.spo_mlp_train.argtypes = [h, fp, fp, ctypes.c_longlong, ctypes.c_int, ctypes.c_int, ctypes.c_float,
                                   ctypes.c_ulonglong, dp]
+    lib.spo_mlp_test_wait_timeout.argtypes = [h, ctypes.c_int]
     for name in _EXPORTS:
         if name != "spo_mlp_last_error":
             getattr(lib, name).restype = ctypes.c_int
@@ -127,6 +128,10 @@ class Mlp:
         loss = ctypes.c_double()
         self._check(self._lib.spo_mlp_train(self._h, xp, yp, x.shape[0], epochs, batch, lr, seed, ctypes.byref(loss)))
         return loss.value
+
+    def test_wait_timeout(self, poll_limit: int) -> None:
+        """Failure-detection test: the products' waits give up after poll_limit polls (negative: the default)."""
+        self._check(self._lib.spo_mlp_test_wait_timeout(self._h, poll_limit))
 
 
 def potential_features(z: np.ndarray, r: np.ndarray, nx: int, ny: int, theta: np.ndarray, phi: np.ndarray,

@@ -50,6 +50,12 @@ int spo_mlp_gradients(spo_mlp* m, const float* x, const float* y, long long n, d
 int spo_mlp_train(spo_mlp* m, const float* x, const float* y, long long n, int epochs, int batch, float lr,
                   unsigned long long seed, double* last_epoch_loss);
 
+/* Failure-detection test of the products' bounded device-side waits: each gives up after poll_limit polls (0: at once;
+ * negative: the default limit). The block records the failure, waits (bounded) for its work in flight and leaves, and the
+ * call returns SPO_ERR_TIMEOUT. A training call then leaves the parameters and Adam's state as they were before the step
+ * that failed. */
+int spo_mlp_test_wait_timeout(spo_mlp* m, int poll_limit);
+
 #ifdef __cplusplus
 }
 #endif

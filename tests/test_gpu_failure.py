@@ -101,3 +101,32 @@ def test_a_single_operator_reports_a_wait_that_gave_up():
         be.test_wait_timeout(0, 0)
         be.apply_stage(capi.STAGE_POTENTIAL)
         be.propagate_analysis_step()
+
+
+def test_a_training_step_that_failed_changes_nothing_and_the_network_recovers():
+    """With a poll limit of 0 every wait for the tensor cores gives up at once (the products in flight are then waited for
+    before a block leaves). The parameters and Adam's state stay as they were, so the training that follows is bitwise
+    that of a network that never failed."""
+    from spo_b200 import capi
+    from spo_b200.mlp import Mlp
+    rng = np.random.default_rng(3)
+    x = rng.uniform(-1.0, 1.0, (2048, 12)).astype(np.float32)
+    y = np.sin(x.sum(axis=1)).astype(np.float32)
+    results = []
+    for failing in (False, True):
+        with Mlp(12, 128, 3, seed=4) as net:
+            net.train(x, y, epochs=1, batch=512, seed=1)
+            if failing:
+                before = net.get_parameters()
+                net.test_wait_timeout(0)
+                for call in (lambda: net.train(x, y, epochs=1, batch=512, seed=2), lambda: net.gradients(x, y),
+                             lambda: net.predict(x)):
+                    with pytest.raises(capi.B200Error) as err:
+                        call()
+                    assert err.value.status == capi.SPO_ERR_TIMEOUT, str(err.value)
+                net.test_wait_timeout(-1)
+                assert np.array_equal(net.get_parameters(), before)
+            loss = net.train(x, y, epochs=1, batch=512, seed=5)
+            results.append((loss, net.get_parameters(), net.predict(x)))
+    assert results[0][0] == results[1][0]
+    assert all(np.array_equal(a, b) for a, b in zip(results[0][1:], results[1][1:]))
