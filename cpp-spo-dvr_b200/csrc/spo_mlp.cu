@@ -375,6 +375,7 @@ __global__ void __launch_bounds__(128) mlp_predict_kernel(PredictArgs g) {
   // Thread 0: chunks requested and multiplied so far; chunk k is the k % per_tile-th of the weights, in slot k % 3.
   long long requested = 0, used = 0;
   uint32_t done_parity = 0;
+  bool done_pending = false;  // thread 0: a commit on `done` not yet waited for
   bool failed = false;
   auto request = [&] {  // every slot whose products are done, in order; false when a wait gave up
     while (requested < chunks && requested < used + kPredictSlots) {
@@ -424,7 +425,10 @@ __global__ void __launch_bounds__(128) mlp_predict_kernel(PredictArgs g) {
           }
           tc::commit(empty + slot);
           ++used;
-          if (c == nc - 1) tc::commit(done);
+          if (c == nc - 1) {
+            tc::commit(done);
+            done_pending = true;
+          }
           // the chunk after the next two, into the slot of the chunk before this one
           if (c + 1 < nc || l + 1 < g.depth || tile + gridDim.x < tiles) {
             const long long keep = used;
@@ -441,6 +445,7 @@ __global__ void __launch_bounds__(128) mlp_predict_kernel(PredictArgs g) {
         break;
       }
       done_parity ^= 1u;
+      done_pending = false;
       tc::fence_after_sync();
       // bias, SiLU, BF16: the next layer's A operand, or the output layer's sum
       const float* const bias = g.bias + l * width;
@@ -466,11 +471,13 @@ __global__ void __launch_bounds__(128) mlp_predict_kernel(PredictArgs g) {
   if (failed) {
     if (tid == 0) {
       atomicExch(g.error_flag, 1);
-      // bounded waits for this block's copies and products in flight, so that none lands after the block has left
+      // bounded waits for this block's copies and products in flight and all they arrive on, so that nothing reaches its
+      // shared memory after the block has left
       for (long long k = used; k < requested; ++k)
         tc::mbar_wait(full + k % kPredictSlots, static_cast<uint32_t>(k / kPredictSlots) & 1u);
       for (long long k = used > kPredictSlots ? used - kPredictSlots : 0; k < used; ++k)
         tc::mbar_wait(empty + k % kPredictSlots, static_cast<uint32_t>(k / kPredictSlots) & 1u);
+      if (done_pending) tc::mbar_wait(done, done_parity);
     }
   }
   tc::fence_before_sync();

@@ -130,3 +130,26 @@ def test_a_training_step_that_failed_changes_nothing_and_the_network_recovers():
             results.append((loss, net.get_parameters(), net.predict(x)))
     assert results[0][0] == results[1][0]
     assert all(np.array_equal(a, b) for a, b in zip(results[0][1:], results[1][1:]))
+
+
+def test_a_prediction_that_gives_up_anywhere_leaves_the_next_one_intact():
+    """Poll limits from 0 upwards end a block's work at different waits: before its weights, between two products, before a
+    layer's end. Each call either succeeds or says that it timed out, and a block that leaves has nothing in flight that
+    could reach the shared memory of the next."""
+    from spo_b200 import capi
+    from spo_b200.mlp import Mlp
+    x = np.random.default_rng(6).uniform(-1.0, 1.0, (100000, 12)).astype(np.float32)
+    with Mlp(12, 256, 4, seed=4) as net:
+        want = net.predict(x)
+        outcomes = set()
+        for polls in [0, 1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 64, 128, 256] * 3:
+            net.test_wait_timeout(polls)
+            try:
+                assert np.array_equal(net.predict(x), want)
+                outcomes.add("done")
+            except capi.B200Error as e:
+                assert e.status == capi.SPO_ERR_TIMEOUT, str(e)
+                outcomes.add("timeout")
+            net.test_wait_timeout(-1)
+            assert np.array_equal(net.predict(x), want), polls
+        assert "timeout" in outcomes, outcomes
