@@ -346,8 +346,12 @@ struct AxisArgs {
   int tb;
 };
 
+// Two blocks per SM, i.e. at most 128 registers, here and in xy_pass_kernel: without the second bound the compiler takes 136
+// to 156 and one block is left, whose stages wait for one another at every barrier. Milliseconds per launch, one block / two:
+// Z 512 x r 30 x 4 x 4, mixed 0.761/0.478, FP64 0.905/0.550; the specular grid's r passes 0.029/0.020; the (x, y) pass of 20 x 20
+// cells, mixed 2.22/1.39, FP64 2.51/1.47.
 template <typename T>
-__global__ void __launch_bounds__(256) axis_pass_kernel(AxisArgs<T> a) {
+__global__ void __launch_bounds__(256, 2) axis_pass_kernel(AxisArgs<T> a) {
   using V = Vec<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   V* buf0 = reinterpret_cast<V*>(smem_raw);
@@ -433,7 +437,7 @@ __device__ __forceinline__ const Vec<T>* xy_post(const XyArgs<T>& a, long long i
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) xy_pass_kernel(XyArgs<T> a) {
+__global__ void __launch_bounds__(256, 2) xy_pass_kernel(XyArgs<T> a) {
   using V = Vec<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int nxy = a.nx * a.ny;

@@ -1,0 +1,36 @@
+"""Register counts of the built kernels, from the compiler's own report beside the library (CPU only): those whose launch
+shapes were chosen for a number of resident blocks keep to it."""
+
+import os
+import re
+import subprocess
+
+import pytest
+
+from conftest import ROOT
+
+PKG = os.path.join(ROOT, "cpp-spo-dvr_b200")
+
+
+@pytest.fixture(scope="module")
+def kernels():
+    """Mangled name -> (registers, bytes of spill stores)."""
+    log = os.path.join(PKG, "lib", "ptxas.log")
+    if not os.path.exists(log):
+        subprocess.run(["make", "-C", PKG, "-j4"], check=True, stdout=subprocess.DEVNULL)
+    out, name, spill = {}, None, 0
+    for line in open(log):
+        if m := re.search(r"Compiling entry function '(\S+)'", line):
+            name = m.group(1)
+        elif m := re.search(r"(\d+) bytes spill stores", line):
+            spill = int(m.group(1))
+        elif (m := re.search(r"Used (\d+) registers", line)) and name:
+            out[name] = (int(m.group(1)), spill)
+    return out
+
+
+@pytest.mark.parametrize("kernel", ["axis_pass_kernel", "xy_pass_kernel"])
+def test_general_kernels_leave_room_for_two_blocks_of_256_threads(kernels, kernel):
+    forms = {n: r for n, r in kernels.items() if f"{len(kernel)}{kernel}I" in n}
+    assert len(forms) == 2, forms  # float and double
+    assert all(r <= 65536 // (2 * 256) for r, _ in forms.values()), forms
