@@ -622,22 +622,35 @@ class Step final : public StepBase {
 
   std::string describe() const override {
     auto lanes = [](int tile, bool has_tiles) { return "tb" + std::to_string(!has_tiles ? 32 : tile ? tile : 16); };
-    auto axis_name = [&](int n, int tile, bool persistent, const KinAxis& kin) {
-      if (kin.map >= 0 && !axis2_supported(n))
-        return "kin<" + std::to_string(n) + "=" + std::to_string(kin.n1) + "x" + std::to_string(kin.n2) + ">";
+    auto kin_name = [](const KinAxis& kin, const std::string& size, int lanes_per_tile) {
+      return "kin<" + size + ",tb" + std::to_string(lanes_per_tile) + (kin.wide ? ",wide>" : ">");
+    };
+    bool any_balanced = false;
+    std::string any_persistent;
+    auto axis_name = [&](const char* which, int n, int tile, bool persistent, const KinAxis& kin) {
+      if (kin.map >= 0)
+        return kin_name(kin, std::to_string(n) + "=" + std::to_string(kin.n1) + "x" + std::to_string(kin.n2), kin_axis_lanes(kin, tile));
       if (!(use_v2_ && axis2_supported(n))) return std::string("axis_pass(general)");
       int n1 = 0, n2 = 0;
-      if (use_pfa_ && !persistent && pfa_split(n, n1, n2))
+      const bool p = zr_window_ == 0 && persistent;  // windows and slabs have the plain forms
+      if (use_pfa_ && !p && pfa_split(n, n1, n2))
         return "axis2pfa<" + std::to_string(n) + "=" + std::to_string(n1) + "x" + std::to_string(n2) + ",tb32>";
-      const char* form = zr_window_ > 0 ? "axis2" : persistent ? "axis2p" : balanced_ && axis2_balanced(n) ? "axis2b" : "axis2";
-      return form + std::string("<") + std::to_string(n) + "," + lanes(tile, axis2_has_tiles(n)) + ">";
+      const bool b = zr_window_ == 0 && rxy_planes_ == 0 && !p && balanced_ && axis2_balanced(n);
+      if (p) any_persistent += which;
+      any_balanced = any_balanced || b;
+      return std::string(p ? "axis2p" : b ? "axis2b" : "axis2") + "<" + std::to_string(n) + "," + lanes(tile, axis2_has_tiles(n)) + ">";
     };
     std::string out = std::string(sizeof(T) == 8 ? "fp64" : "mixed");
-    out += " z=" + axis_name(s_.nz, tile_z_, persist_z_, kin_z_);
-    out += " r=" + axis_name(s_.nr, tile_r_, persist_r_, kin_r_);
-    const bool xy2 = use_v2_ && s_.nx == s_.ny && xy2_supported(s_.nx);
-    out += std::string(" xy=") + (xy2 ? std::string(persist_xy_ ? "xy2p<" : "xy2<") + std::to_string(s_.nx) + "," + lanes(tile_xy_, s_.nx > 8) + ">"
-                                : kin_xy_.map >= 0 ? "kin<" + std::to_string(s_.nx) + "x" + std::to_string(s_.ny) + ">" : std::string("xy_pass(general)"));
+    out += " z=" + axis_name("z", s_.nz, tile_z_, persist_z_, kin_z_);
+    out += " r=" + axis_name("r", s_.nr, tile_r_, persist_r_, kin_r_);
+    if (kin_xy_.map >= 0) {
+      out += " xy=" + kin_name(kin_xy_, std::to_string(s_.nx) + "x" + std::to_string(s_.ny), kin_xy_lanes());
+    } else if (use_v2_ && s_.nx == s_.ny && xy2_supported(s_.nx)) {
+      if (persist_xy_) any_persistent += "xy";
+      out += std::string(persist_xy_ ? " xy=xy2p<" : " xy=xy2<") + std::to_string(s_.nx) + "," + lanes(tile_xy_, s_.nx > 8) + ">";
+    } else {
+      out += " xy=xy_pass(general)";
+    }
     if (pot_kind_ == 6) {
       out += " potential=potential6<nphi=" + std::to_string(s_.nphi) + ",nt=" + std::to_string(s_.nt) +
              ",tcgen05.tf32x3,tile=64,blocks=" + std::to_string(pot6_blocks_) + ">";
@@ -660,10 +673,7 @@ class Step final : public StepBase {
       out += " potential=potential2<nphi=" + std::to_string(s_.nphi) + ",cb=" + std::to_string(pot2_cb_) + ">";
     else
       out += " potential=potential(general)";
-    // axes named above by another register kernel of their size that run kin_kernel
-    out += std::string(" kin=") + (kin_z_.map >= 0 && axis2_supported(s_.nz) ? "z" : "") +
-           (kin_r_.map >= 0 && axis2_supported(s_.nr) ? "r" : "") + (kin_xy_.map >= 0 && xy2 ? "xy" : "");
-    out += std::string(" balanced=") + (balanced_ ? "1" : "0") + " persistent=" + (persist_z_ ? "z" : "") + (persist_r_ ? "r" : "") + (persist_xy_ ? "xy" : "") +
+    out += std::string(" balanced=") + (any_balanced ? "1" : "0") + " persistent=" + any_persistent +
            " zr_window=" + std::to_string(zr_window_) + " rxy_planes=" + std::to_string(rxy_planes_) + " tiles=" + tiles_source_ + " potential_choice=" + pot_source_;
     out += graph_ || graph_stale_ ? " graph=1" : " graph=0 (" + graph_missing_ + ")";
     return out;
@@ -1067,8 +1077,11 @@ class Step final : public StepBase {
     a.groups = static_cast<unsigned>(groups);
     kin_launch(ax, half, tile, a, outer);
   }
+  // Lanes per tile of kin_kernel for a tuned width (0: none).
+  static int kin_axis_lanes(const KinAxis& ax, int tile) { return tile > 0 ? tile : ax.n1 * ax.n2 >= 80 ? 16 : 32; }
+  int kin_xy_lanes() const { return tile_xy_ > 0 ? tile_xy_ : s_.nx > 8 || s_.ny > 8 ? 16 : 32; }
   void kin_launch(KinAxis& ax, bool half, int tile, spo::KinArgs<T>& a, long long outer) {
-    const int lanes = tile > 0 ? tile : ax.n1 * ax.n2 >= 80 ? 16 : 32;
+    const int lanes = kin_axis_lanes(ax, tile);
     auto it = ax.launches.find({lanes, a.window});
     if (it == ax.launches.end()) {
       const bool unit = ax.unit[0] && ax.unit[1];
@@ -1151,7 +1164,7 @@ class Step final : public StepBase {
       x.izr_offset = izr_first;
       a.xy = x;
       prof_.begin(stream_);
-      kin_launch(kin_xy_, half, tile_xy_ > 0 ? tile_xy_ : s_.nx > 8 || s_.ny > 8 ? 16 : 32, a, n);
+      kin_launch(kin_xy_, half, kin_xy_lanes(), a, n);
       prof_.end(stream_, "kinetic_xy", 2.0 * sizeof(V) * n * s_.n_xy() * s_.n_rot);
       ++launches_;
       return;

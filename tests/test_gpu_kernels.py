@@ -92,7 +92,8 @@ def test_register_kernels_match_general_kernels(shape, precision, kernels):
 
 
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
-def test_tile_widths_are_bitwise_equal(precision):
+@pytest.mark.parametrize("z,xy", [("kin<128=8x16", "kin<16x16"), ("axis2b<128", "xy2p<16")])
+def test_tile_widths_are_bitwise_equal(z, xy, precision, monkeypatch):
     from spo_b200 import workload
     # Z 128 = 8 x 16 and (x, y) 16 x 16: the lengths whose kernels have 8, 16 and 32 lane tiles
     case = workload.config_case({"nz": 128, "nr": 24, "nx": 16, "ny": 16, "j_max": 3, "mj_max": 3,
@@ -101,9 +102,11 @@ def test_tile_widths_are_bitwise_equal(precision):
     psi0 = rng.standard_normal(case.psi_shape) + 1j * rng.standard_normal(case.psi_shape)
     chi0 = rng.standard_normal(case.chi_shape) + 1j * rng.standard_normal(case.chi_shape)
     out = []
+    if z.startswith("axis2b"):
+        monkeypatch.setenv("SPO_B200_BALANCED", "1")  # the register kernels other than kin_kernel
     for tiles in ("8", "16", "32"):
         be = make(case, "v3", precision, tiles)
-        assert f"z=axis2b<128,tb{tiles}>" in be.describe() and f"xy=xy2p<16,tb{tiles}>" in be.describe(), be.describe()
+        assert f"z={z},tb{tiles}>" in be.describe() and f"xy={xy},tb{tiles}>" in be.describe(), be.describe()
         be.read_wave_packet(psi0, chi0)
         be.propagate_analysis_step()
         out.append(be.wave_packet_on_host())
@@ -285,6 +288,7 @@ def test_prime_factor_axis_kernel_agrees(nz, nr, precision, monkeypatch):
     two-level kernel with twiddles (SPO_B200_PFA=0) over an analysis step: the same wave packet to rounding
     (1e-12 FP64, 1e-5 mixed)."""
     from spo_b200 import workload
+    monkeypatch.setenv("SPO_B200_BALANCED", "1")  # 48 by this kernel, too, not by kin_kernel
     case = workload.config_case({"nz": nz, "nr": nr, "nx": 4, "ny": 4, "j_max": 3, "mj_max": 3,
                                  "nz_specular": 2 * nz, "nz_potential": nz // 2})
     rng = np.random.default_rng(43)

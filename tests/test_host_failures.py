@@ -171,3 +171,26 @@ with Mlp(64, 64, 1) as net:
     assert status(lambda: net.train(x, y, epochs=1, batch=128)) == capi.SPO_ERR_OOM
     assert fake.fake_bytes(b"malloc") - before <= 64 << 20
 """)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("env", [{}, {"SPO_B200_BALANCED": "1"}, {"SPO_B200_PERSISTENT": "1"}, {"SPO_B200_KERNELS": "v1"},
+                                 {"SPO_B200_PFA": "0"}])
+@pytest.mark.parametrize("nz,nr,nx,ny", [(128, 48, 16, 16), (90, 36, 10, 10), (32, 27, 6, 4), (512, 24, 8, 8)])
+def test_describe_names_the_kernels_that_run(run, nz, nr, nx, ny, env, precision):
+    """The names of an analysis step's kinetic passes against the kernels that a step launches."""
+    run(f"""
+c = workload.config_case(dict(nz={nz}, nr={nr}, nx={nx}, ny={ny}, j_max=1, mj_max=1, nz_specular={nz}, nz_potential=2))
+families = ("kin_kernel", "axis2_kernel", "axis2b_kernel", "axis2p_kernel", "axis2pfa_kernel", "xy2_kernel", "xy2p_kernel",
+            "xy_pass_kernel")
+with B200Backend(c, precision="{precision}") as be:
+    be.profile(True)  # launch by launch
+    before = [fake.fake_launches(f.encode()) for f in families]
+    be.propagate_analysis_step()
+    ran = {{f for f, b in zip(families, before) if fake.fake_launches(f.encode()) > b}}
+    text = be.describe()
+fields = dict(w.split("=", 1) for w in text.split() if "=" in w)
+named = {{fields[k].split("<")[0].split("(")[0] + "_kernel" for k in ("z", "r", "xy")}}
+assert named - {{"axis_pass_kernel"}} == ran, (named, ran, text)
+assert (fields["balanced"] == "1") == ("axis2b_kernel" in ran) and (fields["persistent"] != "") == bool(ran & {{"axis2p_kernel", "xy2p_kernel"}}), text
+""", env)
