@@ -839,8 +839,8 @@ class Step final : public StepBase {
       case SPO_STAGE_ZR: kinetic_zr(half); break;
       case SPO_STAGE_XY: kinetic_xy(half, false); break;
       case SPO_STAGE_POTENTIAL:
-        scale_points("gas_phase", static_cast<long long>(s_.nzp) * s_.nr, s_.n_zr(), gas_step_);
-        if (prescaled_) scale_points("scaling", 0, static_cast<long long>(s_.nzp) * s_.nr, before_);
+        scale_points("gas_phase", static_cast<long long>(s_.nzp) * s_.nr, s_.n_zr(), 0);
+        if (prescaled_) scale_points("scaling", 0, static_cast<long long>(s_.nzp) * s_.nr, static_cast<long long>(s_.nr) * s_.n_rot);
         interaction();
         break;
       default: require(false, "unknown stage");
@@ -1145,12 +1145,11 @@ class Step final : public StepBase {
     x.shift_f = shift_f_;
     x.shift_b = shift_b_;
     x.tb = xy_tb_;
-    x.apply_gas = with_gas ? 1 : 0;
+    x.apply_gas = !with_gas ? 0 : prescaled_ ? 2 : 1;
     x.izr_gas_first = static_cast<long long>(s_.nzp) * s_.nr;
     x.nr = s_.nr;
     x.opt_z = opt_z_;
-    x.gas_step = gas_step_;
-    x.before = prescaled_ ? before_ : nullptr;
+    x.post_step = post_step_;
     x.tile = tile_xy_;
     x.persistent = persist_xy_ ? 1 : 0;
     if (kin_xy_.map >= 0) {
@@ -1184,11 +1183,11 @@ class Step final : public StepBase {
     ++launches_;
   }
 
-  void scale_points(const char* name, long long first, long long last, const V* table) {
+  void scale_points(const char* name, long long first, long long last, long long entry) {
     if (first >= last) return;
     prof_.begin(stream_);
     spo::scale_points_kernel<T><<<1184, 256, 0, stream_>>>(psi_, first, last, s_.n_rot, static_cast<int>(s_.n_xy()), s_.nr,
-                                                           opt_z_, table);
+                                                           opt_z_, post_step_, entry);
     prof_.end(stream_, name, 2.0 * sizeof(V) * (last - first) * s_.n_xy() * s_.n_rot);
     ++launches_;
   }
@@ -1587,9 +1586,10 @@ class Step final : public StepBase {
     if (use_v2_) {
       // An explicit SPO_B200_BALANCED or SPO_B200_PERSISTENT names a form of the other register kernels.
       const bool preferred = !std::getenv("SPO_B200_BALANCED") && !std::getenv("SPO_B200_PERSISTENT");
+      constexpr bool mixed = sizeof(T) == 4;
       auto axis = [&](KinAxis& ax, int n, const double* full, const double* half) {
-        if (!kin_split(n, sizeof(T) == 4, preferred, use_pfa_, ax.map, ax.n1, ax.n2)) return;
-        ax.wide = sizeof(T) == 4 && !axis2_supported(n);
+        if (!kin_split(n, mixed, preferred, use_pfa_, ax.map, ax.n1, ax.n2)) return;
+        ax.wide = mixed && !axis2_supported(n);
         kin_table(ax, 0, scaled(complex_array(full, n, "kinetic factors"), 1.0 / n));
         kin_table(ax, 1, scaled(complex_array(half, n, "kinetic factors"), 1.0 / n));
       };
@@ -1600,7 +1600,7 @@ class Step final : public StepBase {
       if (kin_xy_size(s.nx) && kin_xy_size(s.ny) &&
           (s.nx != s.ny || !xy2_supported(s.nx) || (preferred && !shifted && kin_preferred_xy(s.nx)))) {
         kin_xy_.map = shifted ? spo::kXyShift : spo::kXy;
-        kin_xy_.wide = sizeof(T) == 4 && kin_wide_xy(s.nx, s.ny, shifted);
+        kin_xy_.wide = mixed && kin_wide_xy(s.nx, s.ny, shifted);
         kin_xy_.n1 = s.ny;
         kin_xy_.n2 = s.nx;
         kin_table(kin_xy_, 0, scaled(complex_array(d.xy_kinetic_full, nxy, "xy_kinetic_full"), xy_scale));
@@ -1648,7 +1648,8 @@ class Step final : public StepBase {
       return v;
     }());
     before_ = upload_factor(before);
-    gas_step_ = upload_factor(gas_step);
+    gas_step.insert(gas_step.end(), before.begin(), before.end());
+    post_step_ = upload_factor(gas_step);
     spec_w_ = upload_factor(spec_w);
     opt_z_ = upload_real(opt_z);
 
@@ -2317,7 +2318,7 @@ class Step final : public StepBase {
   V *tw_z_ = nullptr, *tw_r_ = nullptr, *tw_x_ = nullptr, *tw_y_ = nullptr, *tw_zs_ = nullptr, *tw_phi_ = nullptr;
   V *zk_full_ = nullptr, *zk_half_ = nullptr, *rk_full_ = nullptr, *rk_half_ = nullptr;
   V *xyk_full_ = nullptr, *xyk_half_ = nullptr, *spec_full_ = nullptr, *spec_half_ = nullptr;
-  V *rot_half_ = nullptr, *before_ = nullptr, *gas_step_ = nullptr, *spec_w_ = nullptr;
+  V *rot_half_ = nullptr, *before_ = nullptr, *post_step_ = nullptr, *spec_w_ = nullptr;
   V *shift_f_ = nullptr, *shift_b_ = nullptr;
   T* opt_z_ = nullptr;
   V *psi_ = nullptr, *chi_ = nullptr, *expia_ = nullptr;

@@ -403,7 +403,7 @@ __global__ void __launch_bounds__(256, 2) axis_pass_kernel(AxisArgs<T> a) {
 // shift, 2D (x, y) FFT, kinetic factor, inverse, shift back (src/propagation/kinetic_operators.cpp:
 // 134-172). In the gas-phase region (izr >= izr_gas_first) the potential step of that region,
 // optical_z * rot exp(-i vasy dt) rot (src/propagation/potential_operator.cpp:104-112), is applied
-// in the same pass when `apply_gas` is set.
+// in the same pass (`apply_gas`), or the scaling before the interaction region's step.
 // ---------------------------------------------------------------------------------------------
 template <typename T>
 struct XyArgs {
@@ -416,24 +416,27 @@ struct XyArgs {
   const Vec<T>* shift_f;  // nx*ny or null (no momentum shift)
   const Vec<T>* shift_b;
   int tb;
-  int apply_gas;
+  int apply_gas;           // 0: nothing follows T_xy; 1: the gas-phase step at the points from izr_gas_first on; 2: and before them
+                           // the scaling of the interaction region's step (a potential kernel that takes psi scaled follows)
   long long izr_gas_first;
   int nr;
   const T* opt_z;          // nz
-  const Vec<T>* gas_step;  // (ir, irot): opt_r rot gas rot
-  const Vec<T>* before;    // (ir, irot): opt_r rot(dt/2), applied with opt_z to the points below izr_gas_first when
-                           // `apply_gas` is set (a potential kernel that takes psi scaled follows); or null
+  const Vec<T>* post_step;  // 2 nr n_rot factors, applied with opt_z: (ir, irot) opt_r rot gas rot, then opt_r rot(dt/2)
   int tile;                // launch choice of the register-DFT xy kernel: rotational states per block
                            // (8, 16 or 32; 0: the default) for grids of more than 8 points per axis
   long long izr_offset;    // register-DFT xy kernel: block y serves point izr = izr_offset + y
   int persistent;          // launch choice: the persistent form of the register-DFT xy kernel (xy2p_kernel)
 };
 
-// The factor table (ir, irot) that follows T_xy at a point: the gas-phase step, or the scaling of the interaction
-// region's potential step, or none (null).
+// Whether a factor of post_step follows T_xy at a point, and its entry at irot = 0. (One table and an index: a pointer that
+// depends on the point took 4 to 8 registers more in xy2_kernel and xy2p_kernel, a block per SM less at some sizes.)
 template <typename T>
-__device__ __forceinline__ const Vec<T>* xy_post(const XyArgs<T>& a, long long izr) {
-  return !a.apply_gas ? nullptr : izr >= a.izr_gas_first ? a.gas_step : a.before;
+__device__ __forceinline__ bool xy_post(const XyArgs<T>& a, long long izr) {
+  return a.apply_gas > (izr >= a.izr_gas_first ? 0 : 1);
+}
+template <typename T>
+__device__ __forceinline__ unsigned xy_post_entry(const XyArgs<T>& a, long long izr) {
+  return (static_cast<unsigned>(izr % a.nr) + (izr >= a.izr_gas_first ? 0u : a.nr)) * a.n_rot;
 }
 
 template <typename T>
@@ -472,8 +475,8 @@ __global__ void __launch_bounds__(256, 2) xy_pass_kernel(XyArgs<T> a) {
   cur = smem_fft(cur, oth, twx, a.px, +1, a.ny * tb, a.ny * tb, 0, a.ny * tb);
   oth = cur == buf0 ? buf1 : buf0;
   cur = smem_fft(cur, oth, twy, a.py, +1, a.nx * tb, tb, a.ny * tb, tb);
-  const Vec<T>* const post = xy_post(a, izr);
-  const int ir = static_cast<int>(izr % a.nr);
+  const bool post = xy_post(a, izr);
+  const unsigned entry = xy_post_entry(a, izr);
   const T oz = post ? a.opt_z[izr / a.nr] : T(1);
   for (int e = threadIdx.x; e < nxy * tb; e += blockDim.x) {
     const int ixy = e / tb, b = e % tb;
@@ -481,7 +484,7 @@ __global__ void __launch_bounds__(256, 2) xy_pass_kernel(XyArgs<T> a) {
       V v = cur[e];
       if (a.shift_b) v = fmul_t(v, a.shift_b, nxy, ixy);
       if (post) {
-        v = fmul_t(v, post, static_cast<long long>(a.nr) * a.n_rot, ir * a.n_rot + r0 + b);
+        v = fmul_t(v, a.post_step, 2ll * a.nr * a.n_rot, entry + r0 + b);
         v = cscale(v, oz);
       }
       a.psi[(col0 + ixy) * a.n_rot + r0 + b] = v;
@@ -637,13 +640,13 @@ __global__ void __launch_bounds__(256) potential_kernel(PotArgs<T> a) {
 // Utilities
 // ---------------------------------------------------------------------------------------------
 
-// The factors opt_z * table(ir, irot) of the potential step at the points izr_first <= izr < izr_last: the whole
+// The factors opt_z * table(ir, irot) (XyArgs::post_step from `entry` on) of the potential step at the points izr_first <= izr < izr_last: the whole
 // step in the gas-phase region (src/propagation/potential_operator.cpp:104-112), or the scaling before a potential
 // kernel that takes psi scaled. The propagation fuses this into the xy pass; this kernel serves the stage-by-stage
 // entry point.
 template <typename T>
 __global__ void scale_points_kernel(Vec<T>* __restrict__ psi, long long izr_first, long long izr_last, int n_rot, int n_xy,
-                                    int nr, const T* __restrict__ opt_z, const Vec<T>* __restrict__ table) {
+                                    int nr, const T* __restrict__ opt_z, const Vec<T>* __restrict__ post_step, long long entry) {
   const long long per_izr = static_cast<long long>(n_xy) * n_rot;
   const long long n = (izr_last - izr_first) * per_izr;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
@@ -652,7 +655,7 @@ __global__ void scale_points_kernel(Vec<T>* __restrict__ psi, long long izr_firs
     const int irot = static_cast<int>(i % n_rot);
     const int ir = static_cast<int>(izr % nr);
     const long long g = izr_first * per_izr + i;
-    psi[g] = cscale(fmul_t(psi[g], table, static_cast<long long>(nr) * n_rot, ir * n_rot + irot), opt_z[izr / nr]);
+    psi[g] = cscale(fmul_t(psi[g], post_step, 2ll * nr * n_rot, entry + ir * n_rot + irot), opt_z[izr / nr]);
   }
 }
 

@@ -396,10 +396,11 @@ __global__ void __launch_bounds__(kin_max_threads(N1C > N2C ? N1C : N2C), kin_mi
     __syncthreads();
     if constexpr (kin_is_xy(MAP)) {
       const long long izr = a.xy.izr_offset + outer;
-      const KinVec<T>* const table = xy_post(a.xy, izr);
+      const long long half = static_cast<long long>(a.xy.nr) * a.xy.n_rot;
+      const KinVec<T>* const table = xy_post(a.xy, izr) ? a.xy.post_step + (izr >= a.xy.izr_gas_first ? 0 : half) : nullptr;
       decltype(kin_post_of<T>(table, 0ll, 0ll, 0, a.scale)) w{};
       if (table && t.ok)
-        w = kin_post_of<T>(table, static_cast<long long>(a.xy.nr) * a.xy.n_rot, (izr % a.xy.nr) * a.xy.n_rot + lane, t.ok, a.xy.opt_z[izr / a.xy.nr]);
+        w = kin_post_of<T>(table, 2 * half, (izr % a.xy.nr) * a.xy.n_rot + lane, t.ok, a.xy.opt_z[izr / a.xy.nr]);
       if constexpr (ANY) kin_switch(N1, [&](auto n) { kin_back<T, MAP, SPO_CV(n)>(t, a, N2, table != nullptr, w); });
       else kin_back<T, MAP, N1C>(t, a, N2C, table != nullptr, w);
     } else {

@@ -167,14 +167,13 @@ __global__ void __launch_bounds__(TB*(NX > NY ? NX : NY)) xy2p_kernel(XyArgs<T> 
       V z[NY];
       static_for<0, NY>([&](auto ky) { z[ky] = S[(ix * NY + ky) * TB + b]; });
       rdft<NY, +1>(z);
-      const V* const post = xy_post(a, izr);
-      const int ir = static_cast<int>(izr % a.nr);
-      const long long n_gas = static_cast<long long>(a.nr) * a.n_rot, k_gas = ir * a.n_rot + irot;
+      const bool post = xy_post(a, izr);
+      const long long n_post = 2ll * a.nr * a.n_rot, k_post = xy_post_entry(a, izr) + irot;
       const T oz = post ? a.opt_z[izr / a.nr] : T(1);
       static_for<0, NY>([&](auto iy) {
         V v = z[iy];
         if (a.shift_b) v = fmul_t(v, a.shift_b, NXY, ix * NY + iy);
-        if (post) v = cscale(fmul_t(v, post, n_gas, k_gas), oz);
+        if (post) v = cscale(fmul_t(v, a.post_step, n_post, k_post), oz);
         a.psi[(col0 + ix * NY + iy) * a.n_rot + irot] = v;
       });
     }
