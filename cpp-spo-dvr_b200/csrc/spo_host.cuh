@@ -282,6 +282,16 @@ inline bool kin_preferred(int n, bool mixed, int& map, int& n1, int& n2) {
   }
 }
 inline bool kin_preferred_xy(int n) { return n == 2 || n == 4 || n == 6 || n == 8 || n == 12 || n == 16; }
+// Not where the lanes along a pass are odd in number (n_rot for the (x, y) pass, n_xy n_rot for r, nr n_xy n_rot for Z). Mixed
+// form: every second row of lanes then starts between two 16-byte words, and kin_request fetches the tile by plain loads and
+// waits for them (ms, kin_kernel/other, n_rot 81: r 48 0.050/0.033, 96 0.18/0.12, 128 0.17/0.15, 160 0.34/0.23, 192 0.31/0.24, 224
+// 0.45/0.34, 256 0.51/0.25; Z likewise; x = y: 4 0.119/0.114, 8 0.133/0.120, 12 0.193/0.140, 16 0.210/0.122; 2 the same on both). Not 6,
+// whose Wide form copies lane by lane (0.204/0.212). FP64 loses only on the smallest cells with long rows (n_rot 121, 169, 225,
+// x = y = 2: 0.194/0.179, 0.284/0.254, 0.382/0.333; 4: 0.194/0.189, 0.291/0.273, 0.400/0.357; 81 and below: as fast or faster).
+inline bool kin_lanes(bool mixed, long long lanes) { return !mixed || lanes % 2 == 0; }
+inline bool kin_lanes_xy(int n, bool mixed, int n_rot) {
+  return n_rot % 2 == 0 || (mixed ? n == 6 : n > 4 || n_rot <= 100);
+}
 
 // The mixed form's Wide kernel (FP64 between load and store) takes the sizes that have no kernel of their own, and 6 x 6:
 // pairs sum radices 5, 7, 9 and 11 line by line and compensate every twiddle of an odd length, Wide is bound by the FP64
@@ -1587,18 +1597,18 @@ class Step final : public StepBase {
       // An explicit SPO_B200_BALANCED or SPO_B200_PERSISTENT names a form of the other register kernels.
       const bool preferred = !std::getenv("SPO_B200_BALANCED") && !std::getenv("SPO_B200_PERSISTENT");
       constexpr bool mixed = sizeof(T) == 4;
-      auto axis = [&](KinAxis& ax, int n, const double* full, const double* half) {
-        if (!kin_split(n, mixed, preferred, use_pfa_, ax.map, ax.n1, ax.n2)) return;
+      auto axis = [&](KinAxis& ax, int n, long long lanes, const double* full, const double* half) {
+        if (!kin_split(n, mixed, preferred && kin_lanes(mixed, lanes), use_pfa_, ax.map, ax.n1, ax.n2)) return;
         ax.wide = mixed && !axis2_supported(n);
         kin_table(ax, 0, scaled(complex_array(full, n, "kinetic factors"), 1.0 / n));
         kin_table(ax, 1, scaled(complex_array(half, n, "kinetic factors"), 1.0 / n));
       };
-      axis(kin_z_, s.nz, d.z_kinetic_full, d.z_kinetic_half);
-      axis(kin_r_, s.nr, d.r_kinetic_full, d.r_kinetic_half);
+      axis(kin_z_, s.nz, s.nr * nxy * s.n_rot, d.z_kinetic_full, d.z_kinetic_half);
+      axis(kin_r_, s.nr, nxy * s.n_rot, d.r_kinetic_full, d.r_kinetic_half);
       const std::vector<cplx> shift = complex_array(d.shift_forward, nxy, "shift_forward");  // as shift_f_ below
       const bool shifted = std::any_of(shift.begin(), shift.end(), [](const cplx& c) { return c != cplx(1.0, 0.0); });
       if (kin_xy_size(s.nx) && kin_xy_size(s.ny) &&
-          (s.nx != s.ny || !xy2_supported(s.nx) || (preferred && !shifted && kin_preferred_xy(s.nx)))) {
+          (s.nx != s.ny || !xy2_supported(s.nx) || (preferred && !shifted && kin_preferred_xy(s.nx) && kin_lanes_xy(s.nx, mixed, s.n_rot)))) {
         kin_xy_.map = shifted ? spo::kXyShift : spo::kXy;
         kin_xy_.wide = mixed && kin_wide_xy(s.nx, s.ny, shifted);
         kin_xy_.n1 = s.ny;

@@ -194,3 +194,23 @@ named = {{fields[k].split("<")[0].split("(")[0] + "_kernel" for k in ("z", "r", 
 assert named - {{"axis_pass_kernel"}} == ran, (named, ran, text)
 assert (fields["balanced"] == "1") == ("axis2b_kernel" in ran) and (fields["persistent"] != "") == bool(ran & {{"axis2p_kernel", "xy2p_kernel"}}), text
 """, env)
+
+
+def test_odd_numbers_of_lanes_take_the_kernels_that_load_them_one_by_one(run):
+    """n_rot 81 (J 8) and 169 (J 12) against 100 (J 9): the pairs of kin_kernel need even rows, the FP64 form short ones on
+    the smallest cells."""
+    run("""
+def names(precision, n, j, nz=24, nr=24, homo=False):
+    c = workload.config_case(dict(nz=nz, nr=nr, nx=n, ny=n, j_max=j, mj_max=j, nz_specular=nz, nz_potential=2))
+    with B200Backend(c, precision=precision) as be:
+        return {k: v.split("<")[0] for k, v in (w.split("=", 1) for w in be.describe().split() if "=" in w) if k in "z r xy"}
+for n in (4, 8, 12, 16):
+    assert names("mixed", n, 9)["xy"] == "kin" and names("mixed", n, 8)["xy"] in ("xy2", "xy2p"), n
+assert names("mixed", 6, 8)["xy"] == "kin" and names("mixed", 10, 8)["xy"] == "kin"
+for n in (2, 4):
+    assert names("fp64", n, 8)["xy"] == "kin" and names("fp64", n, 12)["xy"] == "xy2", n
+assert names("fp64", 8, 12)["xy"] == "kin"
+assert names("mixed", 5, 8, 128, 48) == {"z": "kin", "r": "axis2pfa", "xy": "kin"}  # 48 r points: even rows for Z
+assert names("mixed", 5, 8, 128, 27)["z"] == "axis2b" and names("mixed", 5, 9, 128, 27)["z"] == "kin"
+assert names("fp64", 5, 8, 128, 48) == {"z": "kin", "r": "kin", "xy": "kin"}
+""")
