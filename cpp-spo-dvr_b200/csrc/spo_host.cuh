@@ -257,13 +257,16 @@ KinLaunch<typename spo::KinStored<T>::type> kin_configure(int map, int n1, int n
 
 // The lengths and square grids that run kin_kernel although another register kernel has them: where it measured faster (ms
 // per launch of 0.1 to 1.6 GB, against the other kernel at its best tile width).
-//   mixed form, pairs of lanes: 48 0.242/0.259, 96 0.495/0.560, 128 0.228/0.250, 160 0.259/0.296, 176 0.168/0.226, 192
+//   mixed form, pairs of lanes: 48 0.242/0.259, 96 0.879/0.989, 128 0.228/0.250, 160 0.259/0.296, 176 0.168/0.226, 192
 //     0.273/0.300, 224 0.184/0.223, 256 0.156/0.188; x = y: 2 0.030/0.036, 4 0.064/0.097, 6 0.174/0.188, 8 0.151/0.227,
 //     12 0.372/0.445, 16 0.363/0.487 (6: Wide);
 //   FP64: 48 0.374/0.418, 64 0.364/0.411, 128 0.348/0.390, 176 0.189/0.238, 192 0.279/0.312, 224 0.203/0.224, 256
 //     0.228/0.287; x = y: 2 0.0307/0.0312, 4 0.151/0.159, 6 0.176/0.214, 8 0.213/0.251, 12 0.384/0.518, 16 0.570/0.618.
 // The (x, y) pass without a momentum shift only: with its two extra factors the mixed 16 x 16 pass took 2.07 ms on
 // configuration 3, without 1.75 (the other kernel 1.84).
+// 96 is 8 x 12 with twiddles, as the other kernel has it: 3 x 32 is no faster (0.875) and another order of roundings, with which the
+// planes and densities of a step on smooth packets were 1 to 4 % further from 64 bits. 160 and 224 as 5 x 32 and 7 x 32 are closer
+// to 64 bits than the other kernel's splits, by 2 %.
 // Not 24, 32 and, mixed, 64 (short lines: the other kernels keep more warps in flight; 0.056/0.050, 0.189/0.190,
 // 0.222/0.222; FP64 24 0.080/0.076, 32 0.171/0.166), 40, 56, 80 and 112 (mixed: radices 5 and 7 sum in FP64, line by line;
 // 0.173/0.130, 0.090/0.066, 0.120/0.114, 0.134/0.125), FP64 96 and 160 (0.618/0.593, 0.293/0.294).
@@ -271,7 +274,7 @@ inline bool kin_preferred(int n, bool mixed, int& map, int& n1, int& n2) {
   switch (n) {
     case 48: map = spo::kPrime, n1 = 3, n2 = 16; return true;
     case 64: map = spo::kTwiddle, n1 = 8, n2 = 8; return !mixed;
-    case 96: map = spo::kPrime, n1 = 3, n2 = 32; return mixed;
+    case 96: map = spo::kTwiddle, n1 = 8, n2 = 12; return mixed;
     case 128: map = spo::kTwiddle, n1 = 8, n2 = 16; return true;
     case 160: map = spo::kPrime, n1 = 5, n2 = 32; return mixed;
     case 176: map = spo::kPrime, n1 = 11, n2 = 16; return true;

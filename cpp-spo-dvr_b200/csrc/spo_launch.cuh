@@ -275,16 +275,16 @@ KinKernel<T> kin_kernel_for(int map, int n1, int n2) {  // kin_preferred, kin_pr
   } else if (map == spo::kTwiddle) {
     if constexpr (fp64)
       if (n1 == 8 && n2 == 8) return spo::kin_kernel<T, spo::kTwiddle, 8, 8>;
+    if constexpr (mixed)
+      if (n1 == 8 && n2 == 12) return spo::kin_kernel<T, spo::kTwiddle, 8, 12>;
     if (n1 == 8 && n2 == 16) return spo::kin_kernel<T, spo::kTwiddle, 8, 16>;
     if (n1 == 12 && n2 == 16) return spo::kin_kernel<T, spo::kTwiddle, 12, 16>;
     if (n1 == 16 && n2 == 16) return spo::kin_kernel<T, spo::kTwiddle, 16, 16>;
   } else if (map == spo::kPrime) {
     if (n1 == 3 && n2 == 16) return spo::kin_kernel<T, spo::kPrime, 3, 16>;
     if (n1 == 11 && n2 == 16) return spo::kin_kernel<T, spo::kPrime, 11, 16>;
-    if constexpr (mixed) {
-      if (n1 == 3 && n2 == 32) return spo::kin_kernel<T, spo::kPrime, 3, 32>;
+    if constexpr (mixed)
       if (n1 == 5 && n2 == 32) return spo::kin_kernel<T, spo::kPrime, 5, 32>;
-    }
     if (n1 == 7 && n2 == 32) return spo::kin_kernel<T, spo::kPrime, 7, 32>;
   } else if (map == spo::kXy && n1 == n2) {
     if (n1 == 2) return spo::kin_kernel<T, spo::kXy, 2, 2>;
