@@ -2271,9 +2271,9 @@ class Step final : public StepBase {
 
   // Host FP64 complex -> device T, by several threads or through the staging buffer.
   void copy_in(const double* src, V* dst, long long n) {
-    if (HostCopier<T>::wanted(src, n)) {
-      int device = 0;
-      check_cuda(cudaGetDevice(&device), "cudaGetDevice");
+    int device = 0;
+    check_cuda(cudaGetDevice(&device), "cudaGetDevice");
+    if (copier_.wanted(src, n, device)) {
       check_cuda(cudaStreamSynchronize(stream_), "upload");
       check_cuda(copier_.to_device(src, dst, n, device), "upload");
       return;
@@ -2291,9 +2291,9 @@ class Step final : public StepBase {
     }
   }
   void copy_out(const V* src, double* dst, long long n) {
-    if (HostCopier<T>::wanted(dst, n)) {
-      int device = 0;
-      check_cuda(cudaGetDevice(&device), "cudaGetDevice");
+    int device = 0;
+    check_cuda(cudaGetDevice(&device), "cudaGetDevice");
+    if (copier_.wanted(dst, n, device)) {
       check_cuda(cudaStreamSynchronize(stream_), "download");
       check_cuda(copier_.to_host(src, dst, n, device), "download");
       return;

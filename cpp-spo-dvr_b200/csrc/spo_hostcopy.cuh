@@ -21,9 +21,7 @@
 namespace spo_host {
 
 // The streams and pinned buffers of a device's large copies: at most 8 MiB of pinned memory, made for the first handle
-// that needs them, shared by all handles of the device (one copy at a time) and freed with the last of them. With a set
-// per handle the first copy of each further handle paid for its own pinned memory (14 of 19 ms of a network's first
-// prediction of 1 M points; 8.7 ms with the shared set).
+// that needs them, shared by all handles of the device (one copy at a time) and freed with the last of them.
 class CopyPool {
  public:
   static constexpr std::size_t kChunk = 512 << 10;  // bytes on the device per chunk
@@ -35,16 +33,18 @@ class CopyPool {
   std::mutex busy;
   std::vector<Worker> workers;
 
-  // The pool of a device (the current one); null with the reason in `e`.
-  static std::shared_ptr<CopyPool> of_device(int device, cudaError_t& e) {
+  // The pool of a device (the current one), made if `make` and there is none; null if there is none or it cannot be had.
+  static std::shared_ptr<CopyPool> of_device(int device, bool make) {
     static std::mutex mutex;
     static std::map<int, std::weak_ptr<CopyPool>> pools;
     std::lock_guard<std::mutex> lock(mutex);
-    e = cudaSuccess;
-    if (std::shared_ptr<CopyPool> p = pools[device].lock()) return p;
-    auto p = std::make_shared<CopyPool>();
-    e = p->prepare();
-    if (e != cudaSuccess) return nullptr;
+    std::shared_ptr<CopyPool> p = pools[device].lock();
+    if (p || !make) return p;
+    p = std::make_shared<CopyPool>();
+    if (p->prepare() != cudaSuccess) {
+      (void)cudaGetLastError();
+      return nullptr;
+    }
     pools[device] = p;
     return p;
   }
@@ -79,21 +79,33 @@ class CopyPool {
 class RawCopier {
  public:
   static constexpr std::size_t kChunk = CopyPool::kChunk;
-  static constexpr std::size_t kMin = 4 << 20;  // smaller copies go through one cudaMemcpyAsync
+  // Host bytes from which a copy is faster this way (18 MiB of a mixed packet up 1.2 -> 0.8 ms, down 1.1 -> 0.9; 9 MiB up 0.6
+  // -> 0.5, down 0.6 -> 0.8).
+  static constexpr std::size_t kMin = 16 << 20;
+  // The pool costs 6 to 13 ms to make and 1 to 8 to give back; the copies gain about 0.2 ms per MiB. So a handle that finds
+  // none uses plain copies for the first 64 MiB of those that would have taken this path: a program that reads one small
+  // packet at its end does not pay for it (10 ms against 1), one that goes on has it after a few copies.
+  static constexpr std::size_t kWorth = 64 << 20;
   using Worker = CopyPool::Worker;
 
-  // Whether a copy of n bytes from or to p takes this path: large, and p not pinned (whose copies run at bus speed).
-  static bool wanted(const void* p, std::size_t n) {
+  // Whether a copy of n host bytes from or to p takes this path: large, p not pinned (whose copies run at bus speed), and the
+  // pool is there, or worth making and to be had. If not, the caller copies by cudaMemcpyAsync.
+  bool wanted(const void* p, std::size_t n, int device) {
     if (n < kMin) return false;
     cudaPointerAttributes a{};
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
       (void)cudaGetLastError();
       return false;
     }
-    return a.type == cudaMemoryTypeUnregistered;
+    if (a.type != cudaMemoryTypeUnregistered) return false;
+    if (pool_) return true;
+    copied_ += n;
+    pool_ = CopyPool::of_device(device, copied_ >= kWorth);
+    if (!pool_ && copied_ >= kWorth) copied_ = 0;  // cannot be had: asked for again after as much
+    return pool_ != nullptr;
   }
 
-  // n bytes of host memory to the device, chunk by chunk through fill(pinned, offset, bytes); returns when done. The
+  // (after wanted() said so) n bytes of host memory to the device, chunk by chunk through fill(pinned, offset, bytes); returns when done. The
   // caller has synchronised the last use of dst.
   template <typename Fill>
   cudaError_t fill_device(void* dst, std::size_t n, int device, Fill&& fill) {
@@ -143,11 +155,6 @@ class RawCopier {
  private:
   template <typename F>
   cudaError_t run(std::size_t n, int device, F&& body) {
-    if (!pool_) {
-      cudaError_t e = cudaSuccess;
-      pool_ = CopyPool::of_device(device, e);
-      if (!pool_) return e;
-    }
     std::lock_guard<std::mutex> lock(pool_->busy);
     std::vector<Worker>& workers_ = pool_->workers;
     const std::size_t chunks = (n + kChunk - 1) / kChunk;
@@ -175,6 +182,7 @@ class RawCopier {
   }
 
   std::shared_ptr<CopyPool> pool_;
+  std::size_t copied_ = 0;  // host bytes copied without it that would have taken this path
 };
 
 // Wave packets: n complex128 on the host, complex128 or complex64 on the device.
@@ -182,7 +190,7 @@ template <typename T>
 class HostCopier {
  public:
   using V = std::conditional_t<sizeof(T) == 4, float2, double2>;
-  static bool wanted(const void* p, long long n) { return RawCopier::wanted(p, sizeof(V) * static_cast<std::size_t>(n)); }
+  bool wanted(const void* p, long long n, int device) { return raw_.wanted(p, sizeof(double2) * static_cast<std::size_t>(n), device); }
   cudaError_t to_device(const double* src, V* dst, long long n, int device) {
     if constexpr (sizeof(T) == 8) return raw_.to_device(src, dst, sizeof(V) * n, device);
     else

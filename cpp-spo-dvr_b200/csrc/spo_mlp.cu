@@ -1090,7 +1090,7 @@ int spo_mlp_predict(spo_mlp* m, const float* x, long long n, float* y) {
     for (long long i0 = 0; i0 < n; i0 += most) {
       const long long rows = std::min(most, n - i0);
       const std::size_t in_bytes = sizeof(float) * static_cast<std::size_t>(rows * m->n_in), out_bytes = sizeof(float) * rows;
-      if (spo_host::RawCopier::wanted(x, in_bytes))
+      if (m->copier.wanted(x, in_bytes, m->device))
         ck(m->copier.to_device(x + i0 * m->n_in, m->px.p, in_bytes, m->device), "upload");
       else
         ck(cudaMemcpyAsync(m->px.p, x + i0 * m->n_in, in_bytes, cudaMemcpyHostToDevice, m->stream), "upload");
@@ -1098,7 +1098,7 @@ int spo_mlp_predict(spo_mlp* m, const float* x, long long n, float* y) {
       const long long tiles = (rows + kBM - 1) / kBM;
       mlp_predict_kernel<<<static_cast<unsigned>(std::min<long long>(tiles, 2ll * m->sms)), 128, predict_smem(m->width), m->stream>>>(g);
       ck(cudaGetLastError(), "predict launch");
-      if (spo_host::RawCopier::wanted(y, out_bytes)) {
+      if (m->copier.wanted(y, out_bytes, m->device)) {
         ck(cudaStreamSynchronize(m->stream), "predict");
         ck(m->copier.to_host(m->py.p, y + i0, out_bytes, m->device), "download");
       } else {

@@ -214,3 +214,48 @@ assert names("mixed", 5, 8, 128, 48) == {"z": "kin", "r": "axis2pfa", "xy": "kin
 assert names("mixed", 5, 8, 128, 27)["z"] == "axis2b" and names("mixed", 5, 9, 128, 27)["z"] == "kin"
 assert names("fp64", 5, 8, 128, 48) == {"z": "kin", "r": "kin", "xy": "kin"}
 """)
+
+
+COPIES = """
+def packet(be, c, seed):
+    psi = np.random.default_rng(seed).standard_normal(c.psi_shape).astype(np.float32) + 0j
+    be.read_wave_packet(psi, None)
+    return np.array_equal(be.wave_packet_on_host()[0], psi)
+big, mid, small = (case(nz=nz, nr=32, nx=8, ny=8, j=5, nzp=1) for nz in (64, 16, 4))
+mib = [c.nz * c.nr * c.nx * c.ny * c.n_rot * 16 / 2**20 for c in (big, mid, small)]
+assert mib == [72.0, 18.0, 4.5], mib
+"""
+
+
+def test_copies_go_on_without_pinned_memory(run):
+    """A packet of 72 MiB where the pinned buffers or their streams cannot be had: by plain copies, nothing left behind."""
+    run(COPIES + """
+for kind, nth in ((b"host", 1), (b"stream", 2), (b"event", 3)):
+    with B200Backend(big, precision="fp64") as be:
+        fake.fake_fail(kind, nth)
+        assert packet(be, big, 1), kind
+        assert fake.fake_live(b"host") == 1, kind  # asked for again by the second copy
+    assert not live(), live()
+x, calls = np.ones((1500000, 12), np.float32), fake.fake_calls(b"host")
+with Mlp(12, 64, 1) as net:
+    fake.fake_fail(b"host", 1)
+    net.predict(x)
+    assert fake.fake_calls(b"host") == calls + 1 and fake.fake_live(b"host") == 0
+""")
+
+
+def test_pinned_buffers_are_made_when_the_copies_pay_for_them(run):
+    """Not for one packet of 18 MiB up and down, but at the fourth such copy; at once for a large one; not for small ones
+    however often; and shared by the handles of the device."""
+    run(COPIES + """
+with B200Backend(mid, precision="fp64") as be:
+    assert packet(be, mid, 1) and fake.fake_calls(b"host") == 0
+    assert packet(be, mid, 2) and fake.fake_calls(b"host") == 1
+    with B200Backend(mid, precision="fp64") as other, B200Backend(big, precision="fp64") as third:
+        assert packet(other, mid, 3) and packet(third, big, 4) and fake.fake_calls(b"host") == 1
+with B200Backend(big, precision="fp64") as be:
+    assert packet(be, big, 5) and fake.fake_calls(b"host") == 2
+with B200Backend(small, precision="fp64") as be:
+    assert all(packet(be, small, k) for k in range(40)) and fake.fake_calls(b"host") == 2
+assert not live()
+""")
