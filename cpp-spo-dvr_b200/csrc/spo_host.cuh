@@ -2163,6 +2163,10 @@ class Step final : public StepBase {
     const Sizes& s = s_;
     const long long n_cols = static_cast<long long>(s.nzp) * s.nr * s.n_xy();
     if (s.nt > 16 || s.nphi > 255 || s.n_rot > 8192 || n_cols > (1ll << 30) || static_cast<long long>(s.nr) * s.n_rot > (1ll << 30)) return;
+    // Both blocks of a pair (m, -m) take the steps of the longer one; the shorter one's last steps multiply what lies behind
+    // it by zero, which has to be the column or the 4 zeros behind the column (blocks of equal length end 3 behind at most).
+    for (int b = 0; b < s.n_blocks; ++b)
+      if (first[b] + (std::max(size[b], size[s.n_blocks - 1 - b]) + 3) / 4 * 4 > s.n_rot + 4) return;
     const int h_n = s.nt > 8 ? 2 : 1;
     auto kernel = spo::pot5::kernel_for(s.nphi, h_n);
     if (!kernel) return;

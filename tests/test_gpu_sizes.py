@@ -106,6 +106,35 @@ def test_potential_step_of_any_angular_grid(j_max, homonuclear, nx, ny, symmetry
     assert ",dmma" in text and f"potential={kernel}<nphi={case.n_phi}," in text, text
 
 
+def uneven_blocks(sizes):
+    """A case whose mJ blocks have the given lengths, m = -M .. M, and any matrices."""
+    from spo_b200 import workload
+    m_max = len(sizes) // 2
+    case = workload.config_case({"nz": 16, "nr": 6, "nx": 5, "ny": 3, "j_max": m_max, "mj_max": m_max, "nz_specular": 32,
+                                 "nz_potential": 11})
+    rng = np.random.default_rng(sum(sizes))
+    first = np.concatenate([[0], np.cumsum(sizes)[:-1]])
+    case.m["n_rot"] = n_rot = sum(sizes)
+    case.m["mj_blocks"] = [[int(f), n, b[2]] for f, n, b in zip(first, sizes, case.m["mj_blocks"])]
+    case.m["initial_channel"] = int(first[m_max])
+    case.a["legendre"] = rng.standard_normal(case.n_theta * n_rot) * 0.2
+    case.a["rotation_half"] = np.exp(1j * rng.uniform(0, 6, n_rot * case.nr))
+    return case
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("sizes,mma", [([1, 2, 3, 4, 3, 2, 1], True), ([2, 2, 3, 4, 3, 2, 1], True), ([1, 2, 3, 4, 3, 2, 5], True),
+                                       ([13, 2, 3, 4, 3, 2, 1], False), ([4, 3, 2, 9, 9, 9, 30], True),
+                                       ([30, 9, 9, 9, 2, 3, 4], False)])
+def test_blocks_of_m_and_minus_m_may_differ_in_length(sizes, mma, precision):
+    """The descriptor allows it. potential5 runs both with the steps of the longer one; where those would read more than the
+    zeros behind a column, another kernel takes the grid."""
+    from spo_b200 import capi
+    text = compare(uneven_blocks(sizes), precision, (capi.STAGE_POTENTIAL,))
+    if precision == "mixed":
+        assert ("potential=potential5<" in text) == mma, text
+
+
 @pytest.mark.parametrize("nz,nr", [(96, 24), (24, 96), (48, 24), (128, 24), (192, 24), (256, 24)])
 def test_pairs_of_lanes_round_as_one_lane(nz, nr, monkeypatch):
     """Mixed form: where both kernels split a length the same way, a pair of lanes takes the same operations in the same order
