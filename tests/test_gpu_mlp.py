@@ -140,3 +140,30 @@ def test_learned_potential_of_a_reference_grid(ref_case):
           f"(host round trip included), reference exact evaluation {t_exact * 1e3:.1f} ms")
     assert rms_mev < 50.0 and rms_low_mev < 50.0
     assert dpsi < 0.05  # measured 6e-3 (the LCG packet has amplitude everywhere, the steep wall included)
+
+
+def test_sums_over_many_rows_and_units_keep_their_bits():
+    """Equal terms show what a long FP32 chain loses (each addition rounds the same way).
+    Gradients: 1024 times the same 64 rows have the same bias and output gradients as 64 of them (each term a 1024th, exactly).
+    The sums of 64 rows are the same on both sides; 1024 of them go through 16 chains of 64 equal terms, whose k-th addition
+    rounds by at most 2^-24 of k terms (32.5 x 2^-24 of the sum together), and an exact tree; 1.5 x 2^-24 for the rest.
+    Predictions: zero weights, so that every unit is 8 in BF16 (SiLU(8) = 7.997), and 256 equal products: each rounded
+    once, the sum of 16 of them exact, then FP64 and one rounding: 2 x 2^-24."""
+    from spo_b200.mlp import Mlp
+    rng = np.random.default_rng(8)
+    with Mlp(12, 128, 2, seed=6) as net:
+        x = np.repeat(rng.uniform(-1, 1, (1, 12)).astype(np.float32), 65536, axis=0)
+        y = np.full(65536, 0.3, np.float32)
+        few, many = net.gradients(x[:64], y[:64])[1], net.gradients(x, y)[1]
+        n = 128 * 64
+        for k, size in ((n, 128), (n + 128 + 128 * 128, 128 + 128 + 1)):  # b of layer 0; b of layer 1, output weights and bias
+            a, b = few[k:k + size].astype(np.float64), many[k:k + size]
+            assert np.all(np.abs(b - a) <= 34 * 2.0 ** -24 * np.abs(a)), np.max(np.abs(b / a - 1))
+    with Mlp(1, 256, 1, seed=1) as net:
+        for w in rng.uniform(0.1, 1.0, 20).astype(np.float32):
+            p = np.zeros(net.parameter_count(), np.float32)
+            p[256 * 64:256 * 65] = 8.0
+            p[256 * 65:256 * 66] = w
+            net.set_parameters(p)
+            got, want = net.predict(np.zeros((1, 1), np.float32))[0], 256 * 8.0 * float(w)
+            assert abs(got - want) <= 2 * 2.0 ** -24 * want, (got, want)
