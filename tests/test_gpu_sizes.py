@@ -106,6 +106,25 @@ def test_potential_step_of_any_angular_grid(j_max, homonuclear, nx, ny, symmetry
     assert ",dmma" in text and f"potential={kernel}<nphi={case.n_phi}," in text, text
 
 
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("j_max,mj_max,homonuclear,nx,ny,symmetry",
+                         [(13, 13, False, 4, 4, True), (15, 15, False, 4, 4, True), (12, 12, False, 6, 6, True),
+                          (14, 13, False, 4, 4, True), (14, 13, False, 5, 3, False), (12, 12, False, 8, 8, False),
+                          (15, 13, False, 5, 3, False), (13, 12, False, 2, 2, False), (9, 7, False, 5, 3, False),
+                          (12, 7, False, 4, 4, True), (14, 11, True, 5, 3, False), (15, 2, False, 3, 3, False)])
+def test_potential_step_where_lines_fill_the_registers_and_with_shorter_mj(j_max, mj_max, homonuclear, nx, ny, symmetry, precision):
+    """potential5's ring (theta above 8, phi 28 and 32) with symmetry maps and with odd basis sizes (no bulk copies), and
+    bases whose blocks are longer than phi asks for (mJ below J)."""
+    from spo_b200 import capi, workload
+    case = workload.config_case({"nz": 16, "nr": 6, "nx": nx, "ny": ny, "j_max": j_max, "mj_max": mj_max,
+                                 "homonuclear": homonuclear, "nz_specular": 32, "nz_potential": 11})
+    if symmetry:
+        fold(case, nx)
+    text = compare(case, precision, (capi.STAGE_POTENTIAL,))
+    kernel = "potential4" if precision == "fp64" else "potential5"
+    assert ",dmma" in text and f"potential={kernel}<nphi={case.n_phi}," in text, text
+
+
 def uneven_blocks(sizes):
     """A case whose mJ blocks have the given lengths, m = -M .. M, and any matrices."""
     from spo_b200 import workload
