@@ -787,46 +787,43 @@ static __global__ void norm_budget_finish_kernel(const double* __restrict__ part
   else if (a < n_absorbers) out[(k / kBudgetMaxAbsorbers) * n_absorbers + a] = v;
 }
 
-// sum |psi|^2 over one (Z, r) block (n_block values) in FP64, fixed order: strided per thread into four sums (16-byte
-// loads where the blocks are aligned), then a fixed tree (src/propagation/averages.cpp:20-29). Bound by the one read of psi.
+// sum |psi|^2 over one (Z, r) block (n_block values) in FP64, fixed order: strided per thread (16-byte loads where the blocks
+// are aligned), then a fixed tree (src/propagation/averages.cpp:20-29). Bound by the one read of psi for blocks of 4000
+// values and more (6.4 to 7.2 TB/s); below that by what a block costs: eight of them per SM (32 registers) and shuffles, with one
+// barrier instead of nine. Four sums per thread and a tree through shared memory (40 registers, six blocks) took, on 0.4 to 1.7
+// GB, blocks of 100 values 856 us mixed and 816 FP64 (now 477 and 478), of 676 355 and 426 (224, 304), of 1600 172 and 284 (131, 238).
 template <typename T>
-__global__ void __launch_bounds__(256) block_density_kernel(const Vec<T>* __restrict__ psi, long long n_block,
-                                                            double* __restrict__ out) {
-  __shared__ double part[256];
+__global__ void __launch_bounds__(256, 8) block_density_kernel(const Vec<T>* __restrict__ psi, long long n_block,
+                                                               double* __restrict__ out) {
+  __shared__ double part[8];
   const Vec<T>* const p = psi + static_cast<long long>(blockIdx.x) * n_block;
-  double s[4] = {0.0, 0.0, 0.0, 0.0};
-  auto add = [](double& t, T re, T im) {
+  double s = 0.0;
+  auto add = [&](T re, T im) {
     const double x = re, y = im;
-    t = fma(x, x, fma(y, y, t));
+    s = fma(x, x, fma(y, y, s));
   };
-  long long done = 0;  // values taken by the 16-byte loads
-  if (sizeof(T) == 8 || (n_block % 2 == 0 && reinterpret_cast<uintptr_t>(psi) % 16 == 0)) {
-    using W = std::conditional_t<sizeof(T) == 4, float4, double2>;
-    constexpr int per = sizeof(W) / sizeof(Vec<T>);
-    const W* const w = reinterpret_cast<const W*>(p);
-    const long long n = n_block / per, whole = n / 1024 * 1024;
-    auto take = [&](double& t, const W& v) {
-      add(t, v.x, v.y);
-      if constexpr (per == 2) add(t, v.z, v.w);
-    };
-    for (long long i = threadIdx.x; i < whole; i += 1024) {
-      const W v0 = w[i], v1 = w[i + 256], v2 = w[i + 512], v3 = w[i + 768];
-      take(s[0], v0);
-      take(s[1], v1);
-      take(s[2], v2);
-      take(s[3], v3);
+  bool paired = false;  // two values per load
+  if constexpr (sizeof(T) == 4) {
+    paired = n_block % 2 == 0 && reinterpret_cast<uintptr_t>(psi) % 16 == 0;
+    if (paired) {
+      const float4* const w = reinterpret_cast<const float4*>(p);
+      for (long long i = threadIdx.x; i < n_block / 2; i += 256) {
+        const float4 v = w[i];
+        add(v.z, v.w);
+        add(v.x, v.y);
+      }
     }
-    for (long long i = whole + threadIdx.x; i < n; i += 256) take(s[0], w[i]);
-    done = n * per;
   }
-  for (long long i = done + threadIdx.x; i < n_block; i += 256) add(s[0], p[i].x, p[i].y);
-  part[threadIdx.x] = (s[0] + s[1]) + (s[2] + s[3]);
+  if (!paired)
+    for (long long i = threadIdx.x; i < n_block; i += 256) add(p[i].x, p[i].y);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (threadIdx.x % 32 == 0) part[threadIdx.x / 32] = s;
   __syncthreads();
-  for (int w = 128; w > 0; w >>= 1) {
-    if (threadIdx.x < w) part[threadIdx.x] += part[threadIdx.x + w];
-    __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 1; k < 8; ++k) s += part[k];
+    out[blockIdx.x] = s;
   }
-  if (threadIdx.x == 0) out[blockIdx.x] = part[0];
 }
 
 // (izr, irot) column of one (x, y) point: out[izr + n_zr * irot] = psi[irot + n_rot*(ixy + n_xy*izr)].

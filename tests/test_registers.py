@@ -42,3 +42,8 @@ def test_xy_kernels_keep_their_resident_blocks(kernels, kernel, most):
     """256, 192, 192 and 96 threads: 6, 10, 4 and 5 blocks per SM."""
     (registers, _), = [r for n, r in kernels.items() if kernel in n]
     assert registers <= most, registers
+
+
+def test_block_density_kernel_leaves_room_for_eight_blocks(kernels):
+    forms = {n: r for n, r in kernels.items() if "20block_density_kernelI" in n}
+    assert forms and all(r <= 32 and spill == 0 for r, spill in forms.values()), forms
