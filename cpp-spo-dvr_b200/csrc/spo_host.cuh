@@ -797,9 +797,9 @@ class Step final : public StepBase {
     spo::block_density_kernel<T><<<static_cast<unsigned>(s_.n_zr()), 256, 0, stream_>>>(
         psi_, s_.n_xy() * s_.n_rot, densities_);
     double* const partial = budget_out_ + spo::kBudgetSums;
-    spo::norm_budget_kernel<T><<<spo::kSumBlocks, 256, 0, stream_>>>(densities_, budget_vol_scat_, chi_, budget_vol_spec_,
-                                                                    budget_scat_, budget_spec_, budget_has_previous_ ? 1 : 0, partial);
-    spo::norm_budget_finish_kernel<<<1, 32, 0, stream_>>>(partial, spo::kSumBlocks, budget_abs_, budget_out_);
+    spo::norm_budget_kernel<T><<<spo::sum_blocks(std::max(budget_scat_.cells, budget_spec_.cells)), 256, 0, stream_>>>(
+        densities_, budget_vol_scat_, chi_, budget_vol_spec_, budget_scat_, budget_spec_, budget_has_previous_ ? 1 : 0, budget_abs_,
+        partial, arrived_, budget_out_);
     check_cuda(cudaGetLastError(), "norm budget launch");
     const bool window = budget_has_previous_;
     if (window)
@@ -824,9 +824,8 @@ class Step final : public StepBase {
                "averages grids");
     spo::block_density_kernel<T><<<static_cast<unsigned>(s_.n_zr()), 256, 0, stream_>>>(
         psi_, s_.n_xy() * s_.n_rot, densities_);
-    spo::averages_kernel<T><<<spo::kSumBlocks, 256, 0, stream_>>>(densities_, chi_, g, s_.nz, s_.nr, s_.nzs, iz_analysis,
-                                                                 surface_index, g + ng + 4);
-    spo::averages_finish_kernel<<<1, 32, 0, stream_>>>(g + ng + 4, spo::kSumBlocks, vol_scat, vol_spec, g + ng);
+    spo::averages_kernel<T><<<spo::sum_blocks(std::max(s_.n_zr(), s_.n_chi())), 256, 0, stream_>>>(
+        densities_, chi_, g, s_.nz, s_.nr, s_.nzs, iz_analysis, surface_index, vol_scat, vol_spec, g + ng + 4, arrived_, g + ng);
     check_cuda(cudaGetLastError(), "averages launch");
     check_cuda(cudaMemcpyAsync(out, g + ng, sizeof(double) * 4, cudaMemcpyDeviceToHost, stream_), "averages copy");
     check_cuda(cudaStreamSynchronize(stream_), "averages");
@@ -1738,6 +1737,8 @@ class Step final : public StepBase {
     check_cuda(cudaMemsetAsync(psi_, 0, sizeof(V) * s.n_psi(), stream_), "zero psi");
     chi_ = dev<V>(s.n_chi());
     densities_ = dev<double>(s.n_zr());
+    arrived_ = dev<unsigned>(1);
+    check_cuda(cudaMemsetAsync(arrived_, 0, sizeof(unsigned), stream_), "zero counter");
     staging_elems_ = std::max<long long>(s.n_zr() * s.n_rot, 4ll << 20);
     staging_ = dev<double2>(staging_elems_);
     require(d.chi_initial != nullptr, "chi_initial is null");
@@ -2339,6 +2340,7 @@ class Step final : public StepBase {
   V *shift_f_ = nullptr, *shift_b_ = nullptr;
   T* opt_z_ = nullptr;
   V *psi_ = nullptr, *chi_ = nullptr, *expia_ = nullptr;
+  unsigned* arrived_ = nullptr;  // blocks that have left their partial sums (grid_sums), 0 between launches
   double* densities_ = nullptr;
   double2* staging_ = nullptr;
   long long staging_elems_ = 0;

@@ -703,13 +703,18 @@ struct BudgetGrid {
   double* previous;        // the cells of the previous call
   long long cells;
 };
-// kSumBlocks blocks leave their partial sums, one block adds them in order: a single block took 0.1 ms of latency for
-// 3e4 cells.
+// Up to kSumBlocks blocks leave their partial sums, and the last of them to finish adds those: a single block took 0.1 ms of
+// latency for 3e4 cells, a second launch for the addition 5 us, a tenth of the whole call on the smallest grids.
 constexpr int kSumBlocks = 64;
-// The block's sums of NV values per thread (fixed tree) into out[k * gridDim.x + blockIdx.x].
+inline unsigned sum_blocks(long long cells) {
+  return static_cast<unsigned>(cells < 256ll * kSumBlocks ? (cells + 255) / 256 : kSumBlocks);
+}
+// The sums over all blocks of 256 threads of NV values per thread, in fixed trees: true in the last block to arrive, with the
+// sums in `total`, false in the others. `partial` holds NV values per block, `arrived` is 0 before and after.
 template <int NV>
-__device__ __forceinline__ void block_sums(const double (&acc)[NV], double* __restrict__ out) {
+__device__ __forceinline__ bool grid_sums(const double (&acc)[NV], double* partial, unsigned* arrived, double (&total)[NV]) {
   __shared__ double part[NV][8];
+  __shared__ bool last;
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
     double v = acc[k];
@@ -721,16 +726,33 @@ __device__ __forceinline__ void block_sums(const double (&acc)[NV], double* __re
   if (threadIdx.x < NV) {
     double v = 0.0;
     for (int w = 0; w < 8; ++w) v += part[threadIdx.x][w];
-    out[threadIdx.x * gridDim.x + blockIdx.x] = v;
+    __stcg(partial + threadIdx.x * gridDim.x + blockIdx.x, v);
+    __threadfence();
   }
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicInc(arrived, gridDim.x - 1) == gridDim.x - 1;  // back to 0 with the last
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  for (int k = threadIdx.x / 32; k < NV; k += 8) {
+    double v = 0.0;
+    for (int b = threadIdx.x % 32; b < static_cast<int>(gridDim.x); b += 32) v += __ldcg(partial + k * gridDim.x + b);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (threadIdx.x % 32 == 0) total[k] = v;
+  }
+  __syncthreads();
+  return true;
 }
 constexpr int kBudgetSums = 2 * kBudgetMaxAbsorbers + 2;  // loss, error per absorber; norm at start, at end
 template <typename T>
 __global__ void __launch_bounds__(256) norm_budget_kernel(const double* __restrict__ densities, double vol_scat,
                                                           const Vec<T>* __restrict__ chi, double vol_spec,
                                                           BudgetGrid scat, BudgetGrid spec, int has_previous,
-                                                          double* __restrict__ partial) {
+                                                          int n_absorbers, double* partial, unsigned* arrived,
+                                                          double* __restrict__ out) {
   constexpr int NV = kBudgetSums;
+  __shared__ double total[NV];
   double acc[NV];
 #pragma unroll
   for (int k = 0; k < NV; ++k) acc[k] = 0.0;
@@ -773,18 +795,13 @@ __global__ void __launch_bounds__(256) norm_budget_kernel(const double* __restri
       g.previous[k] = rho_end;
     }
   }
-  block_sums(acc, partial);
-}
-// out = losses, errors (n_absorbers each), norm at start, at end, from the blocks' partial sums.
-static __global__ void norm_budget_finish_kernel(const double* __restrict__ partial, int blocks, int n_absorbers,
-                                                 double* __restrict__ out) {
+  if (!grid_sums(acc, partial, arrived, total)) return;
+  // losses, errors (n_absorbers each), norm at start, at end
   const int k = threadIdx.x;
-  if (k >= kBudgetSums) return;
-  double v = 0.0;
-  for (int b = 0; b < blocks; ++b) v += partial[k * blocks + b];
+  if (k >= NV) return;
   const int a = k % kBudgetMaxAbsorbers;
-  if (k >= 2 * kBudgetMaxAbsorbers) out[2 * n_absorbers + k - 2 * kBudgetMaxAbsorbers] = v;
-  else if (a < n_absorbers) out[(k / kBudgetMaxAbsorbers) * n_absorbers + a] = v;
+  if (k >= 2 * kBudgetMaxAbsorbers) out[2 * n_absorbers + k - 2 * kBudgetMaxAbsorbers] = total[k];
+  else if (a < n_absorbers) out[(k / kBudgetMaxAbsorbers) * n_absorbers + a] = total[k];
 }
 
 // sum |psi|^2 over one (Z, r) block (n_block values) in FP64, fixed order: strided per thread (16-byte loads where the blocks
@@ -944,12 +961,14 @@ __global__ void convert_kernel(const Vec<TI>* __restrict__ in, Vec<TO>* __restri
 // Norm and position averages of the scattering plus specular wave, FP64 (src/propagation/averages.cpp:37-80). grids =
 // [z (nz) | z_specular (nzs) | r (nr)]; densities are the block densities (izr = ir + nr iz). Seven sums (the scattering
 // norm, Z and r moments, the same three on the specular grid, and the specular norm between the analysis line
-// (exclusive) and the analysis surface (inclusive)) as block sums, which one block adds in order:
+// (exclusive) and the analysis surface (inclusive)):
 // out = {norm, <Z>, <r>, rest norm}.
 template <typename T>
 __global__ void __launch_bounds__(256) averages_kernel(const double* __restrict__ densities, const Vec<T>* __restrict__ chi,
                                                        const double* __restrict__ grids, int nz, int nr, int nzs,
-                                                       int iz_analysis, int surface_index, double* __restrict__ partial) {
+                                                       int iz_analysis, int surface_index, double vol_scat, double vol_spec,
+                                                       double* partial, unsigned* arrived, double* __restrict__ out) {
+  __shared__ double total[7];
   const double* zg = grids;
   const double* zsg = grids + nz;
   const double* rg = grids + nz + nzs;
@@ -973,23 +992,12 @@ __global__ void __launch_bounds__(256) averages_kernel(const double* __restrict_
     acc[5] += rg[ir] * d;
     if (iz > iz_analysis && iz <= surface_index) acc[6] += d;
   }
-  block_sums(acc, partial);
-}
-static __global__ void averages_finish_kernel(const double* __restrict__ partial, int blocks, double vol_scat, double vol_spec,
-                                              double* __restrict__ out) {
-  __shared__ double part[7];
-  if (threadIdx.x < 7) {
-    double v = 0.0;
-    for (int b = 0; b < blocks; ++b) v += partial[threadIdx.x * blocks + b];
-    part[threadIdx.x] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const double norm = part[0] * vol_scat + part[3] * vol_spec;
+  if (grid_sums(acc, partial, arrived, total) && threadIdx.x == 0) {
+    const double norm = total[0] * vol_scat + total[3] * vol_spec;
     out[0] = norm;
-    out[1] = (part[1] * vol_scat + part[4] * vol_spec) / norm;
-    out[2] = (part[2] * vol_scat + part[5] * vol_spec) / norm;
-    out[3] = part[6] * vol_spec;
+    out[1] = (total[1] * vol_scat + total[4] * vol_spec) / norm;
+    out[2] = (total[2] * vol_scat + total[5] * vol_spec) / norm;
+    out[3] = total[6] * vol_spec;
   }
 }
 

@@ -125,6 +125,39 @@ def test_potential_step_where_lines_fill_the_registers_and_with_shorter_mj(j_max
     assert ",dmma" in text and f"potential={kernel}<nphi={case.n_phi}," in text, text
 
 
+@pytest.mark.parametrize("nz,nr,nzs", [(6, 5, 6), (16, 16, 16), (16, 16, 33), (128, 64, 256), (128, 64, 512), (200, 90, 200)])
+def test_sums_over_any_number_of_cells(nz, nr, nzs):
+    """Averages and norm budget on grids of one block of cells, two, all 64 and more, twice each, one after the other (they share
+    the count of blocks that have finished): the restatements' values to 1e-12, the second time to the last bit."""
+    import norm_budget_oracle
+    import spo_oracle
+    from spo_b200 import workload
+    case = workload.config_case({"nz": nz, "nr": nr, "nx": 1, "ny": 1, "j_max": 1, "mj_max": 1, "nz_specular": nzs,
+                                 "nz_potential": 2})
+    psi, chi = random_state(case, 4)
+    for name, n in (("z_optical", nz), ("r_optical", nr), ("z_specular_optical", nzs)):
+        case.a[name] = np.exp(-np.clip(np.linspace(-0.5, 0.2, n), 0.0, None))
+    z, zs, r = 1.5 + 0.1 * np.arange(nz), 1.5 + 0.1 * np.arange(nzs), 0.4 + 0.1 * np.arange(nr)
+    vols, line, surface = (0.02, 0.05), nz // 2, nzs - 2
+    budget = norm_budget_oracle.NormBudgetOracle(case.a["z_optical"], case.a["r_optical"], case.a["z_specular_optical"],
+                                                 case.steps_per_analysis, *vols, None, None)
+    with make(case, None, "fp64") as be:
+        be.norm_budget_setup(*vols)
+        be.read_wave_packet(psi, chi)
+        got = []
+        for _ in range(3):
+            got.append((be.averages(z, zs, r, *vols, line, surface), be.norm_budget_add()))
+        dens = be.block_densities()
+    want = spo_oracle.averages(dens, chi, z, zs, r, *vols, line, surface)
+    assert np.max(np.abs(got[0][0] - want) / np.abs(want)) <= 1e-12
+    budget.add(dens, chi)
+    loss, err, start, end = budget.add(dens, chi)
+    assert got[0][1] is None
+    assert np.max(np.abs(got[1][1][0] - loss)) <= 1e-12 * end and np.max(np.abs(got[1][1][1] - err)) <= 1e-12 * end
+    assert abs(got[1][1][2] - start) <= 1e-12 * end and abs(got[1][1][3] - end) <= 1e-12 * end
+    assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[1][1][0], got[2][1][0]) and got[1][1][2:] == got[2][1][2:]
+
+
 def uneven_blocks(sizes):
     """A case whose mJ blocks have the given lengths, m = -M .. M, and any matrices."""
     from spo_b200 import workload
