@@ -1695,21 +1695,6 @@ class Step final : public StepBase {
     require(total_j == s.n_rot, "mj blocks do not cover the rotational basis");
     std::vector<double> legendre = real_array(d.legendre, static_cast<std::size_t>(off), "legendre");
     const std::vector<double> legendre64 = legendre;  // the FP64 matrix (the low parts of the mixed form's tables)
-    if constexpr (sizeof(T) == 4) {
-      // The mixed form's matrix, rounded once for every potential kernel so that each rotational state's
-      // sum of squares over theta keeps its FP64 value: the forward and the transposed contraction of a step
-      // multiply the state by that sum (times nphi), every step (norm_preserving_rows).
-      std::vector<double> by_state(static_cast<std::size_t>(s.n_rot) * s.nt);
-      for (int b = 0; b < s.n_blocks; ++b)
-        for (int t = 0; t < s.nt; ++t)
-          for (int j = 0; j < size[b]; ++j)
-            by_state[static_cast<std::size_t>(first[b] + j) * s.nt + t] = legendre[offset[b] + t * size[b] + j];
-      const std::vector<float> rounded = norm_preserving_rows(by_state, s.n_rot, s.nt);
-      for (int b = 0; b < s.n_blocks; ++b)
-        for (int t = 0; t < s.nt; ++t)
-          for (int j = 0; j < size[b]; ++j)
-            legendre[offset[b] + t * size[b] + j] = rounded[static_cast<std::size_t>(first[b] + j) * s.nt + t];
-    }
 
     // Symmetry maps, expanded to one phi map per (x, y) point.
     const std::vector<int> rep = int_array(d.representative_of, nxy, "representative_of");
@@ -1785,7 +1770,6 @@ class Step final : public StepBase {
     pot_.cb = cb;
     pot_.pphi = plan_phi_;
     pot_.twphi = tw_phi_;
-    pot_.legendre = upload_real_lo(legendre, legendre64);
     pot_.block_first = upload_int(first);
     pot_.block_size = upload_int(size);
     pot_.block_slot = upload_int(slot);
@@ -1799,10 +1783,37 @@ class Step final : public StepBase {
     pot_.rep_of = upload_int(rep);
     pot_.phi_map = upload_int(phi_map);
 
+    // potential5 (mixed form): the contractions on the FP64 tensor cores, any ntheta up to 16.
+    pot5_kernel_ = nullptr;
+    if constexpr (std::is_same_v<T, float>) build_pot5(pot5_args_, first, size, slot, offset, legendre64, phi_map, smem_optin, dev_id);
+    // potential4 of the FP64 form: the same for FP64 columns.
+    if constexpr (std::is_same_v<T, double>) build_pot4d(pot4d_args_, first, size, slot, offset, legendre64, phi_map, smem_optin, dev_id);
+    // The other potential kernels' tables (the mixed form's matrix with its rounding searched row by row takes milliseconds):
+    // where neither of these takes the grid, or SPO_B200_KERNELS names one.
+    const bool others = !(pot5_kernel_ || pot4d_kernel_) || std::getenv("SPO_B200_KERNELS");
+    if (others) {
+      if constexpr (sizeof(T) == 4) {
+        // The mixed form's matrix, rounded once for every potential kernel so that each rotational state's
+        // sum of squares over theta keeps its FP64 value: the forward and the transposed contraction of a step
+        // multiply the state by that sum (times nphi), every step (norm_preserving_rows).
+        std::vector<double> by_state(static_cast<std::size_t>(s.n_rot) * s.nt);
+        for (int b = 0; b < s.n_blocks; ++b)
+          for (int t = 0; t < s.nt; ++t)
+            for (int j = 0; j < size[b]; ++j)
+              by_state[static_cast<std::size_t>(first[b] + j) * s.nt + t] = legendre[offset[b] + t * size[b] + j];
+        const std::vector<float> rounded = norm_preserving_rows(by_state, s.n_rot, s.nt);
+        for (int b = 0; b < s.n_blocks; ++b)
+          for (int t = 0; t < s.nt; ++t)
+            for (int j = 0; j < size[b]; ++j)
+              legendre[offset[b] + t * size[b] + j] = rounded[static_cast<std::size_t>(first[b] + j) * s.nt + t];
+      }
+      pot_.legendre = upload_real_lo(legendre, legendre64);
+    }
+
     // The register-phi potential kernel: CB columns per chunk with CB * ntheta lines <= 128 threads and
     // at most ~110 KiB of shared memory (two blocks per SM), when nphi has an instantiation.
     pot2_cb_ = 0;
-    if (pot2_phi_supported(s.nphi) && s.nt <= 32) {
+    if (others && pot2_phi_supported(s.nphi) && s.nt <= 32) {
       for (const int cb : {32, 8, 4}) {
         if (cb * s.nt > 128 || cb > nxy * 2) continue;
         const std::size_t need = pot2_smem<T>(cb, s.n_rot, s.nt, s.nphi, nxy);
@@ -1945,11 +1956,6 @@ class Step final : public StepBase {
         pot4_kernel_ = nullptr;
       }
     }
-    // potential5 (mixed form): the contractions on the FP64 tensor cores, any ntheta up to 16.
-    pot5_kernel_ = nullptr;
-    if constexpr (std::is_same_v<T, float>) build_pot5(pot5_args_, first, size, slot, offset, legendre64, phi_map, smem_optin, dev_id);
-    // potential4 of the FP64 form: the same for FP64 columns.
-    if constexpr (std::is_same_v<T, double>) build_pot4d(pot4d_args_, first, size, slot, offset, legendre64, phi_map, smem_optin, dev_id);
     // potential6 (mixed form): both theta contractions as split-precision TF32 tcgen05 GEMMs over 64-column
     // tiles, for the square heteronuclear basis JMax = MJMax = 15 with ntheta 16 and nphi 32 (configuration
     // 2's angular grid); one block of 256 threads per SM holding all 512 tensor-memory columns.

@@ -259,3 +259,19 @@ with B200Backend(small, precision="fp64") as be:
     assert all(packet(be, small, k) for k in range(40)) and fake.fake_calls(b"host") == 2
 assert not live()
 """)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_a_handle_holds_no_tables_of_kernels_it_does_not_launch(run, precision):
+    """The same potential kernel by default and named: only the named one can fall back to others, whose tables it holds."""
+    run(f"""
+c = case(j=15, nx=8, ny=8)
+out = []
+for kernels in (None, "v5"):
+    if kernels:
+        os.environ["SPO_B200_KERNELS"] = kernels
+    with B200Backend(c, precision="{precision}") as be:
+        out.append((be.device_bytes(), [w for w in be.describe().split() if w.startswith("potential=")], fake.fake_live(b"malloc")))
+(few, a, n), (all_tables, b, m) = out
+assert a == b and few < all_tables and n < m, out
+""")
