@@ -257,7 +257,8 @@ def precision_record():
             "bar": 1e-6, "time_steps": r["time_steps"], "energies": r["energies"],
             "open_channels": r["open_channels"],
             "source": "tests/golden/precision_config3.json: configuration 2 (FP64) and 3 (mixed) through the "
-                      "reference program with the B200 backend (oracle/_ref/spodvr_b200), 20000 time steps"}
+                      "reference program with the B200 backend (oracle/_ref/spodvr_b200), 20000 time steps; a stored record, taken "
+                      "with the potential5 before its FP64 tensor-core products"}
 
 
 def run_reference(args, rank):
@@ -291,10 +292,10 @@ ENSEMBLE_SHAPES = [
 
 # DRAM bytes per algorithmic byte of the mixed-form potential kernel (potential5), from one ncu capture of
 # the small case (nX = nY = 8; profiles/dmma_potential_and_kin_small_nx8.md): dram__bytes_read.sum +
-# dram__bytes_write.sum = 2.940 + 0.600 GB against 2.378 GB algorithmic (interaction-region psi read and written once, the
+# dram__bytes_write.sum = 1.854 + 0.522 GB against 2.378 GB algorithmic (interaction-region psi read and written once, the
 # exp(i A) table read once with its 2-byte modulus corrections). The traffic grows with the columns processed, so the
 # ratio carries over to configuration 3.
-POTENTIAL_DRAM_PER_ALGORITHMIC = (2.940481e9 + 0.600490e9) / 2.378170368e9
+POTENTIAL_DRAM_PER_ALGORITHMIC = (1.853975e9 + 0.521808e9) / 2.378170368e9
 
 
 def run_ensemble(args):
@@ -433,7 +434,7 @@ def main():
                          "traffic": top["bytes_per_launch"] * POTENTIAL_DRAM_PER_ALGORITHMIC
                          if top["name"] == "potential" else None,
                          "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one potential5 launch "
-                                           "on the small case (nX = nY = 8: 3.541 GB for 2.378 GB algorithmic), "
+                                           "on the small case (nX = nY = 8: 2.376 GB for 2.378 GB algorithmic), "
                                            "scaled to this launch by the columns processed",
                          "bytes_per_launch": top["bytes_per_launch"], "avg_launch_ms": avg_ms,
                          "share_of_kernel_time": top["ms"] / total_kernel_ms},

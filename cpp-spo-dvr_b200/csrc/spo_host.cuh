@@ -422,9 +422,9 @@ inline double round_bits(double v, int bits) {
 // search over the entries' alternatives (rows of up to 24 non-zero entries; longer rows keep the nearest
 // rounding). A matrix applied with its transpose at every time step (the theta contractions) then keeps the
 // norm of a random state (whose rotational components have independent phases); on a physical wave packet
-// the other entries of the Gram matrix still act, which is why potential5 and the small-grid kernels use
-// the matrix to ~2^-36 (12-bit high parts with their remainders, or FP64 sums) and only potential4's mixed
-// form uses these FP32 rows alone.
+// the other entries of the Gram matrix still act, which is why potential5 multiplies by the FP64 matrix itself,
+// potential4's mixed form by 12-bit high parts with their remainders, and the general and small-grid kernels add the low
+// parts of these rows.
 inline std::vector<float> norm_preserving_rows(const std::vector<double>& m, int rows, int stride) {
   std::vector<float> out(m.size());
   for (std::size_t i = 0; i < m.size(); ++i) out[i] = static_cast<float>(m[i]);
@@ -1270,14 +1270,15 @@ class Step final : public StepBase {
     rxy_planes_ = 0;
     // The persistent forms are a fixed choice, not a timed one: they agree with the plain kernels to
     // rounding only (the compiler may contract a complex product into FMAs differently in each), and a
-    // timed choice could make two runs of one case differ in the last bits. On configuration 3 the
-    // persistent xy pass (16 x 16) takes 1.50 ms against 1.66; the persistent Z and r passes are slower
-    // (2.17 against 1.43 ms for Z: 127 registers leave one block of 512 threads per SM).
+    // timed choice could make two runs of one case differ in the last bits. Where kin_kernel does not run
+    // (shifted cells, odd n_rot): on a 16 x 16 cell of configuration 3's sizes the persistent xy pass took 1.50 ms
+    // against 1.66; the persistent Z and r passes are slower (2.17 against 1.43 ms for Z = 128: 127 registers leave
+    // one block of 512 threads per SM).
     persist_z_ = persist_r_ = false;
     persist_xy_ = use_v2_ && s_.nx == s_.ny && xy2_supported(s_.nx) && s_.nx >= 12;
     // The balanced axis kernel (lengths N1 x 2 N1: 32 and 128) is a fixed choice for the same reason:
-    // Z = 128 on configuration 3 takes 1.38 ms against 1.43 (mixed), 2.69 against 2.71 (FP64). An explicit
-    // persistent request takes precedence over it.
+    // Z = 128 took 1.38 ms against 1.43 (mixed), 2.69 against 2.71 (FP64) by it; kin_kernel takes that length now
+    // unless its lanes are odd in number. An explicit persistent request takes precedence over it.
     balanced_ = use_v2_;
     tiles_source_ = "default";
     if (!use_v2_) return;
@@ -1448,8 +1449,6 @@ class Step final : public StepBase {
     check_cuda(cudaMemcpy(d, h.data(), sizeof(V) * h.size(), cudaMemcpyHostToDevice), "upload table");
     return d;
   }
-  // A real matrix with, in the mixed form, its low parts: the entries v (as T) followed by the roundings of
-  // exact - v; the FP64 form uploads exact.
   // A table of factors s e^{i phi} (s >= 0 real: kinetic and rotation phases with FFT scales or absorbers). The
   // mixed form stores g = e^{i phi} - 1 (n values), the roundings of g's remainders (n values) and, per factor,
   // (s, the rounding of s's remainder) (n pairs): spo::fmul_t applies the factor as s (x + x g), which FP32 rounds
@@ -1515,6 +1514,8 @@ class Step final : public StepBase {
       ax.table[half] = d;
     }
   }
+  // A real matrix with, in the mixed form, its low parts: the entries v (as T) followed by the roundings of
+  // exact - v; the FP64 form uploads exact.
   T* upload_real_lo(const std::vector<double>& v, const std::vector<double>& exact) {
     if constexpr (sizeof(T) == 4) {
       std::vector<double> both(2 * v.size());

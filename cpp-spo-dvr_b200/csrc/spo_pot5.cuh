@@ -26,7 +26,8 @@
 // mbarrier; odd n_rot, whose columns are not 16-byte multiples, by plain loads). The exp(i A) entries are stored
 // in the order in which the lanes read them: per (Z, r) point and representative [phi][pair of theta] as
 // (re, re', im, im') with the modulus corrections of G phi together, so the four lanes of a column read 64
-// contiguous bytes; the next item's are requested into L2 one item ahead.
+// contiguous bytes; the next item's are requested into L2 one item ahead, except by the ring form (ring_of), whose own
+// copies run ahead.
 //
 // psi comes scaled by the absorbers and rot(dt/2): the xy pass before this kernel multiplies every value anyway.
 //
@@ -179,8 +180,8 @@ constexpr int f_stride(int n_rot) {
 constexpr int threads_of(int nphi) { return nphi > 16 ? 384 : nphi > 8 ? 512 : 640; }
 // With two warps per team and 28 or 32 phi, the lines (112 or 128 registers) leave no registers for exp(i A) entries in
 // flight: each lane copies its entries into the team's buffer instead, kBatches batches of 4 phi (and their corrections)
-// ahead, and the row of rot(dt/2) comes with the columns. Configuration 3: 4.31 ms against 4.92 with loads two batches of
-// two phi ahead in registers and rot(dt/2) through L1; phi 24 with symmetry maps 1.35 against 1.25 ms, phi 18 0.547
+// ahead, and the row of rot(dt/2) comes with the columns. Configuration 3: 4.08 ms against 4.92 with loads two batches of
+// two phi ahead in registers and rot(dt/2) through L1 (3.83 since the ring requests nothing into L2); phi 24 with symmetry maps 1.35 against 1.25 ms, phi 18 0.547
 // against 0.525, one warp per team 0.78 against 0.55: there the loads in registers stay.
 constexpr bool ring_of(int nphi, int h) { return h == 2 && nphi >= 28 && nphi % 4 == 0; }
 constexpr int kBatches = 3, kBatchBytes = 5 * 512;
@@ -270,11 +271,12 @@ __global__ void __launch_bounds__(pot5::threads_of(NPHI), 1) potential5_kernel(P
       }
     }
   };
-  // The columns, exp(i A) rows and corrections of an item into L2 (column c by one lane).
-  // The next item's data into L2. Not in the ring form, whose copies run 12 phi ahead by themselves: 888 teams have 29 MB of
-  // rows ahead besides those in use, and about as much as the table was read again from DRAM (1.49 times the algorithmic
-  // bytes; configuration 3: 4.12 ms with the rows and psi requested, 4.11 with the request after the phi phase, 3.90 with
-  // psi alone, 3.83 without).
+  // The columns, exp(i A) rows and corrections of an item into L2 (column c by one lane). Not in the ring form, whose copies run
+  // 12 phi ahead by themselves: 888 teams had 29 MB of rows ahead besides those in use, and about as much as the table was
+  // read again from DRAM (1.49 times the algorithmic bytes; configuration 3: 4.12 ms with the rows and psi requested, 4.11 with
+  // the request after the phi phase, 3.90 with psi alone, 3.83 without). Nor does it pay for phi 28, symmetry maps or odd n_rot
+  // (64 x 48 x 12 x 12, without/with: J 13 1.30/1.34, with maps 1.33/1.35; J 12, n_rot 169, 1.26/1.29, with maps 1.33/1.33; J 15 with
+  // maps 1.14/1.22).
   auto prefetch = [&](int item) {
     const int col = item * kCols + lane;
     if (h == 0 && lane < kCols && col < g.n_cols) {

@@ -219,9 +219,10 @@ int spo_profile_entry(const spo_handle* h, int i, char* name, int name_len, doub
  * potential kernels that move their data by bulk asynchronous copies (potential5, potential6) announces that
  * many bytes more on its first barrier than its copies deliver, so the barrier's phase cannot complete;
  * every copy stays valid and lands. Each wait gives up after poll_limit polls (<= 0: the default limit), the
- * block records the failure, waits (bounded) for its work in flight and leaves, and the next
- * spo_propagate_analysis_step returns SPO_ERR_TIMEOUT; the wave packet is then undefined until the next
- * spo_upload_state. spo_test_wait_timeout(h, 0, 0) restores normal operation. */
+ * block records the failure, waits (bounded) for its work in flight and leaves, and the
+ * spo_propagate_analysis_step, spo_apply_stage or spo_ensemble_step that launched it returns SPO_ERR_TIMEOUT; the
+ * wave packet is then undefined until the next spo_upload_state. spo_test_wait_timeout(h, 0, 0) restores normal
+ * operation. An ensemble's graph keeps the setting that its members had when it was created. */
 int spo_test_wait_timeout(spo_handle* h, int poll_limit, int unmatched_bytes);
 
 /* Bytes of device memory the handle holds. */
@@ -231,8 +232,8 @@ int spo_device_bytes(const spo_handle* h, unsigned long long* bytes);
 int spo_last_launch_count(const spo_handle* h, int* launches);
 
 /* The kernels and tile shapes the handle chose (kernel per pass, tile width per kinetic pass, and
- * whether the autotuner or an environment setting chose them), as one NUL-terminated line truncated
- * to out_len bytes. No counterpart in the reference (its CUDA backend has one fixed plan). */
+ * whether the autotuner or an environment setting chose them; whether the step is one graph, or why not), as one
+ * NUL-terminated line truncated to out_len bytes. No counterpart in the reference (its CUDA backend has one fixed plan). */
 int spo_describe(const spo_handle* h, char* out, int out_len);
 
 /* Norm and position averages of the resident wave packet, computed on the device in FP64:
@@ -284,7 +285,8 @@ typedef struct spo_ensemble spo_ensemble;
 
 int spo_ensemble_create(spo_handle* const* members, int n_members, spo_ensemble** out);
 
-/* One analysis step of every member (one graph launch); returns when all are done. */
+/* One analysis step of every member (one graph launch); returns when all are done. SPO_ERR_TIMEOUT with the
+ * member's index in the message if a bounded wait of one of them gave up. */
 int spo_ensemble_step(spo_ensemble* e);
 
 /* Kernel launches in one ensemble step (the sum over the members). */
