@@ -250,16 +250,12 @@ struct spo_ensemble {
   cudaGraphExec_t exec = nullptr;
   int launches = 0;
   std::vector<spo_handle*> members;
-  // The members' error flags after a step: copied side by side at the end of the branches, then read by one copy.
-  int* flags = nullptr;
-  std::vector<int> host_flags;
   ~spo_ensemble() {
     for (spo_handle* m : members) --m->ensembles;
     cudaSetDevice(device);
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
     if (stream) cudaStreamDestroy(stream);
-    if (flags) cudaFree(flags);
   }
 };
 
@@ -292,9 +288,6 @@ int spo_ensemble_create(spo_handle* const* members, int n_members, spo_ensemble*
     for (spo_handle* m : e->members) ++m->ensembles;
     check_cuda(cudaSetDevice(e->device), "cudaSetDevice");
     check_cuda(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking), "cudaStreamCreate");
-    check_cuda(cudaMalloc(reinterpret_cast<void**>(&e->flags), sizeof(int) * n_members), "ensemble flags");
-    check_cuda(cudaMemsetAsync(e->flags, 0, sizeof(int) * n_members, e->stream), "ensemble flags");
-    e->host_flags.assign(n_members, 0);
     events.resize(n_members + 1, nullptr);
     for (cudaEvent_t& ev : events) check_cuda(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "cudaEventCreate");
     branch.resize(n_members, nullptr);
@@ -315,8 +308,6 @@ int spo_ensemble_create(spo_handle* const* members, int n_members, spo_ensemble*
       m.set_stream(branch[i]);
       m.enqueue_analysis_step();
       m.set_stream(nullptr);
-      if (const int* flag = m.device_flag())
-        check_cuda(cudaMemcpyAsync(e->flags + i, flag, sizeof(int), cudaMemcpyDeviceToDevice, branch[i]), "ensemble flags");
       e->launches += m.launches();
       check_cuda(cudaEventRecord(events[i + 1], branch[i]), "cudaEventRecord");
       check_cuda(cudaStreamWaitEvent(e->stream, events[i + 1], 0), "cudaStreamWaitEvent");
@@ -346,14 +337,11 @@ int spo_ensemble_step(spo_ensemble* e) {
   try {
     check_cuda(cudaSetDevice(e->device), "cudaSetDevice");
     check_cuda(cudaGraphLaunch(e->exec, e->stream), "cudaGraphLaunch");
-    check_cuda(cudaMemcpyAsync(e->host_flags.data(), e->flags, sizeof(int) * e->host_flags.size(), cudaMemcpyDeviceToHost,
-                               e->stream), "ensemble flags");
     check_cuda(cudaStreamSynchronize(e->stream), "spo_ensemble_step");
     int code = SPO_OK;
     for (std::size_t i = 0; i < e->members.size(); ++i) {
-      if (e->host_flags[i] == 0) continue;
       try {
-        e->members[i]->impl->report_device_error();
+        e->members[i]->impl->check_device_error();
       } catch (const SpoError& ex) {
         if (code == SPO_OK) e->err = "member " + std::to_string(i) + ": " + ex.what();
         code = ex.code;

@@ -121,6 +121,16 @@ class DeviceArena {
     bytes_ += bytes;
     return p;
   }
+  // One value of managed memory that stays on the host and is mapped to the device.
+  template <typename U>
+  U* alloc_on_host(int device) {
+    U* p = nullptr;
+    check_cuda(cudaMallocManaged(&p, sizeof(U)), "cudaMallocManaged");
+    ptrs_.push_back(p);
+    check_cuda(cudaMemAdvise(p, sizeof(U), cudaMemAdviseSetPreferredLocation, cudaCpuDeviceId), "cudaMemAdvise");
+    check_cuda(cudaMemAdvise(p, sizeof(U), cudaMemAdviseSetAccessedBy, device), "cudaMemAdvise");
+    return p;
+  }
   void release(void* p, std::size_t bytes) {
     auto it = std::find(ptrs_.begin(), ptrs_.end(), p);
     if (it == ptrs_.end()) return;
@@ -492,10 +502,9 @@ class StepBase {
   virtual void propagate_analysis_step() = 0;
   // Queues one analysis step on the current stream without synchronising (graph capture).
   virtual void enqueue_analysis_step() = 0;
-  // The device flag that a bounded wait of this handle's kernels sets when it gives up (null: none waits), and the report
-  // of one that was set: clears it and throws SPO_ERR_TIMEOUT.
-  virtual const int* device_flag() const = 0;
-  virtual void report_device_error() = 0;
+  // With the work that may set it synchronised: whether a bounded wait of this handle's kernels gave up, reported as
+  // SPO_ERR_TIMEOUT (and the flag cleared).
+  virtual void check_device_error() = 0;
   virtual std::string describe() const = 0;
   virtual void averages(const double* z, const double* zs, const double* r, double vol_scat, double vol_spec,
                         int iz_analysis, int surface_index, double* out) = 0;
@@ -551,7 +560,6 @@ class Step final : public StepBase {
     } else {
       enqueue_analysis_step();
     }
-    read_device_error();
     check_cuda(cudaStreamSynchronize(stream_), "propagate_analysis_step");
     prof_.resolve();
     check_device_error();
@@ -566,24 +574,27 @@ class Step final : public StepBase {
     graph_stale_ = true;  // the graph holds the kernels' arguments
   }
 
-  // A kernel whose bounded wait gave up has set the device flag, which is copied to host_flag_ behind each step: report it
-  // (and clear it). An ordinary int: the copy behind a graph of 40 short kernels costs 7 us, 1 us more than a copy into
-  // pinned memory (and 5 less than one after the wait for the step), but pinned memory costs 1 to 4 ms to get and 0.4 to 9
-  // ms to give back, for every handle.
-  void read_device_error() {
-    if (error_flag_)
-      check_cuda(cudaMemcpyAsync(&host_flag_, error_flag_, sizeof(int), cudaMemcpyDeviceToHost, stream_), "error flag");
-  }
-  void check_device_error() {
-    if (error_flag_ && host_flag_ != 0) report_device_error();
-  }
-  const int* device_flag() const override { return error_flag_; }
-  void report_device_error() override {
-    host_flag_ = 0;
-    check_cuda(cudaMemsetAsync(error_flag_, 0, sizeof(int), stream_), "error flag");
-    check_cuda(cudaStreamSynchronize(stream_), "error flag");
+  // A kernel whose bounded wait gave up has set the error flag: report it (and clear it). The flag lies in managed memory that
+  // stays on the host, so looking at it costs nothing: a copy of it behind a graph of 40 short kernels takes 7 to 13 us (from
+  // inside the graph, into pinned memory, 4 to 6; pinned memory costs 1 to 4 ms to get and 0.4 to 9 ms to give back for
+  // every handle, managed 0.5 and 0.7). Where the host may not touch managed memory while kernels run, it is copied.
+  void check_device_error() override {
+    if (!error_flag_) return;
+    int raised = 0;
+    if (flag_on_host_) raised = *static_cast<volatile int*>(error_flag_);
+    else check_cuda(cudaMemcpy(&raised, error_flag_, sizeof(int), cudaMemcpyDeviceToHost), "error flag");
+    if (raised == 0) return;
+    clear_error_flag();
     throw SpoError(SPO_ERR_TIMEOUT, std::string(pot_kind_ == 6 ? "potential6" : "potential5") +
                                         ": a bounded wait for an asynchronous copy or tensor-core work gave up");
+  }
+  void clear_error_flag() {
+    if (flag_on_host_) {
+      *static_cast<volatile int*>(error_flag_) = 0;
+    } else {
+      check_cuda(cudaMemsetAsync(error_flag_, 0, sizeof(int), stream_), "error flag");
+      check_cuda(cudaStreamSynchronize(stream_), "error flag");
+    }
   }
 
   // One analysis step as a CUDA graph (about 8 (n + 1) small kernels: on the smallest grids the gaps between separate
@@ -858,7 +869,6 @@ class Step final : public StepBase {
       default: require(false, "unknown stage");
     }
     check_cuda(cudaGetLastError(), "apply_stage launch");
-    read_device_error();
     check_cuda(cudaStreamSynchronize(stream_), "apply_stage");
     prof_.resolve();
     check_device_error();
@@ -2150,8 +2160,12 @@ class Step final : public StepBase {
   }
 
   void make_error_flag() {
-    error_flag_ = dev<int>(1);
-    check_cuda(cudaMemset(error_flag_, 0, sizeof(int)), "error flag");
+    int device = 0, concurrent = 0;
+    check_cuda(cudaGetDevice(&device), "cudaGetDevice");
+    check_cuda(cudaDeviceGetAttribute(&concurrent, cudaDevAttrConcurrentManagedAccess, device), "managed memory");
+    flag_on_host_ = concurrent != 0;
+    error_flag_ = flag_on_host_ ? arena_.alloc_on_host<int>(device) : dev<int>(1);
+    clear_error_flag();
   }
 
   // The phi maps as bytes, or null without symmetry.
@@ -2334,7 +2348,6 @@ class Step final : public StepBase {
   int graph_launches_ = 0;
   OwnedStream side_;                 // the specular grid's passes
   OwnedEvent fork_[2];
-  int host_flag_ = 0;                // copy of the error flag
   DeviceArena arena_;
   HostCopier<T> copier_;
   Profiler prof_;
@@ -2379,6 +2392,7 @@ class Step final : public StepBase {
   std::vector<cplx> host_rot_;   // rot(dt/2), (ir, irot)
   bool identity_maps_ = true;    // no symmetry: representative = (x, y) point and phi maps = identity
   int* error_flag_ = nullptr;  // set by a kernel whose bounded wait gave up
+  bool flag_on_host_ = false;  // it is managed memory on the host
   // the norm budget (norm_budget_setup / norm_budget_add) and the FP64 absorber factors it is built from
   std::vector<double> host_opt_z_, host_opt_r_, host_opt_zs_;
   spo::BudgetGrid budget_scat_{}, budget_spec_{};

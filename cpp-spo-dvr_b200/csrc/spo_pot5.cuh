@@ -218,7 +218,7 @@ struct Pot5Args {
 };
 
 template <int NPHI, int H>
-__global__ void __launch_bounds__(pot5::threads_of(NPHI), 1) potential5_kernel(Pot5Args g, int* __restrict__ error_flag) {
+__global__ void __launch_bounds__(pot5::threads_of(NPHI), 1) potential5_kernel(Pot5Args g, int* error_flag) {
   using namespace pot5;
   constexpr int G = group_of(NPHI);
   constexpr bool RING = ring_of(NPHI, H);
@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(pot5::threads_of(NPHI), 1) potential5_kernel(P
     const bool ok = !g.bulk || mbar_wait(bar, parity, g.poll_limit);
     if (team_any<H>(bar_id, !ok)) {
       if (lane == 0 && h == 0) {
-        atomicExch(error_flag, 1);
+        *static_cast<volatile int*>(error_flag) = 1;  // host memory: a plain store, no atomic
         mbar_wait(bar, parity, g.poll_limit);  // bounded: no copy lands after the team has left
       }
       return;

@@ -6,6 +6,7 @@
 //   fake_fail(kind, n) .................. the n-th call from now (1: the next) that makes one fails, once
 //   fake_launches(part) ................. launches so far of kernels whose (mangled) name contains `part`
 //   fake_raise(part, value) ............. kernels whose name contains `part` store `value` at their second argument, an int*
+// With FAKE_NO_MANAGED_ACCESS in the environment the host may not touch managed memory while kernels run.
 // Kinds: "malloc" (device), "host" (pinned), "stream", "event", "graph", "exec", "capture".
 #include <cuda_runtime_api.h>
 
@@ -84,6 +85,8 @@ void fake_raise(const char* part, int value) {
 }
 
 cudaError_t cudaMalloc(void** p, size_t n) { return make("malloc", n, p); }
+cudaError_t cudaMallocManaged(void** p, size_t n, unsigned int) { return make("malloc", n, p); }
+cudaError_t cudaMemAdvise(const void*, size_t, cudaMemoryAdvise, int) { return cudaSuccess; }
 cudaError_t cudaFree(void* p) { return drop("malloc", p); }
 cudaError_t cudaMallocHost(void** p, size_t n) { return make("host", n, p); }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned int) { return make("host", n, p); }
@@ -150,7 +153,8 @@ cudaError_t cudaGetDevice(int* d) {
 }
 cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
   *v = a == cudaDevAttrMultiProcessorCount ? 148 : a == cudaDevAttrMaxSharedMemoryPerBlockOptin ? 232448
-       : a == cudaDevAttrComputeCapabilityMajor ? 10 : 0;
+       : a == cudaDevAttrComputeCapabilityMajor ? 10
+       : a == cudaDevAttrConcurrentManagedAccess ? std::getenv("FAKE_NO_MANAGED_ACCESS") == nullptr : 0;
   return cudaSuccess;
 }
 cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) { return cudaSuccess; }

@@ -109,7 +109,8 @@ assert not live()
 """)
 
 
-def test_a_wait_that_gave_up_is_reported_by_every_call_that_runs_the_kernels(run):
+@pytest.mark.parametrize("env", [{}, {"FAKE_NO_MANAGED_ACCESS": "1"}])
+def test_a_wait_that_gave_up_is_reported_by_every_call_that_runs_the_kernels(run, env):
     run("""
 with B200Backend(case(), precision="mixed") as a, B200Backend(case(), precision="mixed") as b:
     fake.fake_raise(b"potential5", 1)
@@ -119,7 +120,7 @@ with B200Backend(case(), precision="mixed") as a, B200Backend(case(), precision=
         assert status(both.propagate_analysis_step) == capi.SPO_ERR_TIMEOUT
     assert status(a.propagate_analysis_step) == status(b.propagate_analysis_step) == capi.SPO_OK
 assert not live(), live()
-""")
+""", env)
 
 
 @pytest.mark.parametrize("call", ["train", "gradients", "predict"])
