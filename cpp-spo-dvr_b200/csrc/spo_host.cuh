@@ -298,12 +298,16 @@ inline bool kin_preferred_xy(int n) { return n == 2 || n == 4 || n == 6 || n == 
 // Not where the lanes along a pass are odd in number (n_rot for the (x, y) pass, n_xy n_rot for r, nr n_xy n_rot for Z). Mixed
 // form: every second row of lanes then starts between two 16-byte words, and kin_request fetches the tile by plain loads and
 // waits for them (ms, kin_kernel/other, n_rot 81: r 48 0.050/0.033, 96 0.18/0.12, 128 0.17/0.15, 160 0.34/0.23, 192 0.31/0.24, 224
-// 0.45/0.34, 256 0.51/0.25; Z likewise; x = y: 4 0.119/0.114, 8 0.133/0.120, 12 0.193/0.140, 16 0.210/0.122; 2 the same on both). Not 6,
-// whose Wide form copies lane by lane (0.204/0.212). FP64 loses only on the smallest cells with long rows (n_rot 121, 169, 225,
-// x = y = 2: 0.194/0.179, 0.284/0.254, 0.382/0.333; 4: 0.194/0.189, 0.291/0.273, 0.400/0.357; 81 and below: as fast or faster).
+// 0.45/0.34, 256 0.51/0.25; Z likewise; x = y: 8 0.133/0.120, 12 0.193/0.140, 16 0.210/0.122). Not 6, whose Wide form copies lane
+// by lane (0.204/0.212). The smallest cells lose only with long rows and beyond the 126 MB of L2, in both forms (n_rot 121, 169,
+// 225: mixed 4 x 4 0.160/0.152, 0.233/0.219, 0.308/0.288; FP64 2 x 2 0.194/0.179, 0.284/0.254, 0.382/0.333, 4 x 4 0.194/0.189,
+// 0.291/0.273, 0.400/0.357), within L2 the other way round (92 MB, 225: FP64 4 x 4 0.038/0.043; mixed 81 0.029/0.034). The other
+// (x, y) kernels have one block row per (Z, r) point, 65535 at most.
 inline bool kin_lanes(bool mixed, long long lanes) { return !mixed || lanes % 2 == 0; }
-inline bool kin_lanes_xy(int n, bool mixed, int n_rot) {
-  return n_rot % 2 == 0 || (mixed ? n == 6 : n > 4 || n_rot <= 100);
+inline bool kin_lanes_xy(int n, bool mixed, int n_rot, long long packet_bytes, long long n_zr) {
+  if (n_rot % 2 == 0 || n_zr > 65535) return true;
+  if (n <= 4) return n_rot <= 100 || packet_bytes <= 128ll << 20;
+  return !mixed || n == 6;
 }
 
 // The mixed form's Wide kernel (FP64 between load and store) takes the sizes that have no kernel of their own, and 6 x 6:
@@ -1621,7 +1625,8 @@ class Step final : public StepBase {
       const std::vector<cplx> shift = complex_array(d.shift_forward, nxy, "shift_forward");  // as shift_f_ below
       const bool shifted = std::any_of(shift.begin(), shift.end(), [](const cplx& c) { return c != cplx(1.0, 0.0); });
       if (kin_xy_size(s.nx) && kin_xy_size(s.ny) &&
-          (s.nx != s.ny || !xy2_supported(s.nx) || (preferred && !shifted && kin_preferred_xy(s.nx) && kin_lanes_xy(s.nx, mixed, s.n_rot)))) {
+          (s.nx != s.ny || !xy2_supported(s.nx) || (preferred && !shifted && kin_preferred_xy(s.nx) &&
+            kin_lanes_xy(s.nx, mixed, s.n_rot, static_cast<long long>(sizeof(V)) * s.n_psi(), s.n_zr())))) {
         kin_xy_.map = shifted ? spo::kXyShift : spo::kXy;
         kin_xy_.wide = mixed && kin_wide_xy(s.nx, s.ny, shifted);
         kin_xy_.n1 = s.ny;

@@ -198,19 +198,21 @@ assert (fields["balanced"] == "1") == ("axis2b_kernel" in ran) and (fields["pers
 
 
 def test_odd_numbers_of_lanes_take_the_kernels_that_load_them_one_by_one(run):
-    """n_rot 81 (J 8) and 169 (J 12) against 100 (J 9): the pairs of kin_kernel need even rows, the FP64 form short ones on
-    the smallest cells."""
+    """n_rot 81 (J 8) and 169 (J 12) against 100 (J 9): the pairs of kin_kernel need even rows; the smallest cells only where
+    long rows do not fit L2; and more points than the other kernels have block rows stay where they run."""
     run("""
-def names(precision, n, j, nz=24, nr=24, homo=False):
-    c = workload.config_case(dict(nz=nz, nr=nr, nx=n, ny=n, j_max=j, mj_max=j, nz_specular=nz, nz_potential=2))
+def names(precision, n, j, nz=24, nr=24):
+    c = workload.config_case(dict(nz=nz, nr=nr, nx=n, ny=n, j_max=j, mj_max=j, nz_specular=nz, nz_potential=1))
     with B200Backend(c, precision=precision) as be:
         return {k: v.split("<")[0] for k, v in (w.split("=", 1) for w in be.describe().split() if "=" in w) if k in "z r xy"}
-for n in (4, 8, 12, 16):
+for n in (8, 12, 16):
     assert names("mixed", n, 9)["xy"] == "kin" and names("mixed", n, 8)["xy"] in ("xy2", "xy2p"), n
 assert names("mixed", 6, 8)["xy"] == "kin" and names("mixed", 10, 8)["xy"] == "kin"
-for n in (2, 4):
-    assert names("fp64", n, 8)["xy"] == "kin" and names("fp64", n, 12)["xy"] == "xy2", n
+for precision, nz in (("fp64", 160), ("mixed", 320)):  # 150 MB of 4 x 4 cells
+    assert names(precision, 4, 8, nz, 24)["xy"] == "kin" and names(precision, 4, 12, 24, 24)["xy"] == "kin", precision
+    assert names(precision, 4, 12, nz, 24)["xy"] == "xy2", precision
 assert names("fp64", 8, 12)["xy"] == "kin"
+assert names("mixed", 8, 2, 2048, 33)["xy"] == "kin"  # 67584 points
 assert names("mixed", 5, 8, 128, 48) == {"z": "kin", "r": "axis2pfa", "xy": "kin"}  # 48 r points: even rows for Z
 assert names("mixed", 5, 8, 128, 27)["z"] == "axis2b" and names("mixed", 5, 9, 128, 27)["z"] == "kin"
 assert names("fp64", 5, 8, 128, 48) == {"z": "kin", "r": "kin", "xy": "kin"}
