@@ -374,10 +374,24 @@ __global__ void __launch_bounds__(TB*(NX > NY ? NX : NY)) xy2_kernel(XyArgs<T> a
     const bool post = xy_post(a, izr);
     const long long n_post = 2ll * a.nr * a.n_rot, k_post = xy_post_entry(a, izr) + irot;
     const T oz = post ? a.opt_z[izr / a.nr] : T(1);
+    // The factor held (4 registers, mixed 6) rather than loaded behind every store, which may alias it for the compiler; mixed
+    // from 8 points on it would cost a block per SM.
+    constexpr bool HOLD = sizeof(T) == 8 || NY < 8;
+    V held[sizeof(T) == 8 ? 1 : 3] = {};
+    if constexpr (HOLD)
+      if (post)
+#pragma unroll
+        for (int k = 0; k < (sizeof(T) == 8 ? 1 : 3); ++k) held[k] = a.post_step[k * n_post + k_post];
     static_for<0, NY>([&](auto iy) {
       V v = x[iy];
       if (a.shift_b) v = fmul_t(v, a.shift_b, NXY, ix * NY + iy);
-      if (post) v = cscale(fmul_t(v, a.post_step, n_post, k_post), oz);
+      if constexpr (sizeof(T) == 8) {
+        if (post) v = cscale(cmul(held[0], v), oz);
+      } else if constexpr (HOLD) {
+        if (post) v = cscale(fmul_parts(v, held[0], held[1], held[2]), oz);
+      } else {
+        if (post) v = cscale(fmul_t(v, a.post_step, n_post, k_post), oz);
+      }
       a.psi[(col0 + ix * NY + iy) * a.n_rot + irot] = v;
     });
   }
