@@ -301,13 +301,15 @@ inline bool kin_preferred_xy(int n) { return n == 2 || n == 4 || n == 6 || n == 
 // 0.45/0.34, 256 0.51/0.25; Z likewise; x = y: 8 0.133/0.120, 12 0.193/0.140, 16 0.210/0.122). Not 6, whose Wide form copies lane
 // by lane (0.204/0.212). The smallest cells lose only with long rows and beyond the 126 MB of L2, in both forms (n_rot 121, 169,
 // 225: mixed 4 x 4 0.160/0.152, 0.233/0.219, 0.308/0.288; FP64 2 x 2 0.194/0.179, 0.284/0.254, 0.382/0.333, 4 x 4 0.194/0.189,
-// 0.291/0.273, 0.400/0.357), within L2 the other way round (92 MB, 225: FP64 4 x 4 0.038/0.043; mixed 81 0.029/0.034). The other
-// (x, y) kernels have one block row per (Z, r) point, 65535 at most.
+// 0.291/0.273, 0.400/0.357), within L2 the other way round (92 MB, 225: FP64 4 x 4 0.038/0.043; mixed 81 0.029/0.034). On (x, y)
+// cells few lanes stay, to which kin_kernel fits its tile: 8 x 8 with n_rot 1, 9, 15 0.031/0.104, 0.062/0.115, 0.071/0.116, 25
+// 0.140/0.126; 12 x 12 and 16 x 16 with n_rot 1 0.058/0.089, 0.098/0.118, 9 0.225/0.180, 0.381/0.268 (for r few lanes are no
+// different: 48 0.013/0.009). The other (x, y) kernels have one block row per (Z, r) point, 65535 at most.
 inline bool kin_lanes(bool mixed, long long lanes) { return !mixed || lanes % 2 == 0; }
 inline bool kin_lanes_xy(int n, bool mixed, int n_rot, long long packet_bytes, long long n_zr) {
   if (n_rot % 2 == 0 || n_zr > 65535) return true;
   if (n <= 4) return n_rot <= 100 || packet_bytes <= 128ll << 20;
-  return !mixed || n == 6;
+  return !mixed || n == 6 || n_rot <= (n == 8 ? 16 : 1);
 }
 
 // The mixed form's Wide kernel (FP64 between load and store) takes the sizes that have no kernel of their own, and 6 x 6:

@@ -212,7 +212,8 @@ for precision, nz in (("fp64", 160), ("mixed", 320)):  # 150 MB of 4 x 4 cells
     assert names(precision, 4, 8, nz, 24)["xy"] == "kin" and names(precision, 4, 12, 24, 24)["xy"] == "kin", precision
     assert names(precision, 4, 12, nz, 24)["xy"] == "xy2", precision
 assert names("fp64", 8, 12)["xy"] == "kin"
-assert names("mixed", 8, 2, 2048, 33)["xy"] == "kin"  # 67584 points
+assert names("mixed", 8, 2)["xy"] == "kin" and names("mixed", 16, 0)["xy"] == "kin" and names("mixed", 16, 2)["xy"] == "xy2p"
+assert names("mixed", 12, 2, 2048, 33)["xy"] == "kin"  # 67584 points
 assert names("mixed", 5, 8, 128, 48) == {"z": "kin", "r": "axis2pfa", "xy": "kin"}  # 48 r points: even rows for Z
 assert names("mixed", 5, 8, 128, 27)["z"] == "axis2b" and names("mixed", 5, 9, 128, 27)["z"] == "kin"
 assert names("fp64", 5, 8, 128, 48) == {"z": "kin", "r": "kin", "xy": "kin"}
